@@ -4,15 +4,16 @@
 //   mean       the time average of every point, summed over the snapshots in order (the order
 //              numpy's mean along axis 0 adds them), so it equals the reference bit for bit;
 //   X'         X - mean, kept on the device;
-//   C          X' X'^T / M, an M x M Gram matrix: 32 x 32 output tiles, the point range split
-//              over blocks (each block accumulates its slice in FP64 from shared-memory tiles),
-//              the slices then summed in a fixed order;
+//   C          X' X'^T / M, an M x M Gram matrix: 16 x 16 output tiles of the upper triangle, the
+//              point range split over blocks (each block accumulates its slice in FP64 from
+//              shared-memory tiles), the slices then summed in a fixed order;
 // the host takes the eigen-decomposition of C (M is small), and the device forms
-//   phi_i      = X'^T v_i / sigma_i, one thread per point for all requested modes;
-//   a_i        = X' phi_i, dot products over the points (per-block partials, fixed-order sums).
+//   phi_i      = X'^T v_i / sigma_i, one thread per point for a group of modes;
+//   a_i        = X' phi_i, dot products over the points (per-slice partials, fixed-order sums).
 // All arithmetic is FP64.  Input snapshots may be host or device memory.
 #include <cuda_runtime.h>
 
+#include <algorithm>
 #include <cmath>
 #include <cstring>
 #include <string>
@@ -41,9 +42,6 @@ struct gm_pod {
 
 namespace {
 
-constexpr int T = 32;             // Gram tile edge
-constexpr int KCHUNK = 32;        // points per shared-memory stage
-constexpr int SLICE = 16384;      // points per Gram block (its slice of the point range)
 constexpr int MAXM = 4096;
 
 __global__ void k_pod_mean(const double* __restrict__ X, int M, int64_t N, double* __restrict__ mean,
@@ -57,91 +55,196 @@ __global__ void k_pod_mean(const double* __restrict__ X, int M, int64_t N, doubl
   for (int i = 0; i < M; ++i) Xp[(int64_t)i * N + p] = X[(int64_t)i * N + p] - m;
 }
 
-// part[slice][i][j] = sum over the slice's points of X'[i][p] X'[j][p], for the tile (bi, bj)
-__global__ void __launch_bounds__(T * 8) k_pod_gram(const double* __restrict__ Xp, int M, int64_t N,
-                                                    double* __restrict__ part) {
+// The Gram matrix is bound by the FP64 pipe (M (M + 1) / 2 fused multiply-adds a point).  One
+// block forms a 16 x 16 tile of the upper triangle over one slice of the points: 16-wide tiles
+// waste little on the diagonal (5,376 products a point for M = 96, of 4,656 needed; 32-wide tiles
+// 6,144), and the slice count fills the GPU whatever M and N are (GRAM_BLOCKS blocks, slices of at
+// least GRAM_MIN points), where a fixed slice of 16,384 points left 110 of 152 SMs idle on
+// 96 x 80,000 values (5.32 ms, now 0.72 ms: 0.60 T products/s, the FP64 pipe's rate).  Four groups of 64 threads take a quarter of every staged chunk
+// each, four outputs a thread, and add their sums in group order.
+constexpr int T = 16, KCHUNK = 64, GROUPS = 4;
+constexpr int GRAM_BLOCKS = 152 * 8, GRAM_MIN = 512;
+__device__ __forceinline__ void tri_tile(int e, int nt, int& bi, int& bj) {  // row-major upper triangle
+  bi = 0;
+  while (e >= nt - bi) { e -= nt - bi; ++bi; }
+  bj = bi + e;
+}
+__global__ void __launch_bounds__(64 * GROUPS) k_pod_gram(const double* __restrict__ Xp, int M, int64_t N,
+                                                          int64_t slice, double* __restrict__ part) {
   __shared__ double a[T][KCHUNK + 1];
   __shared__ double b[T][KCHUNK + 1];
-  const int bi = blockIdx.x, bj = blockIdx.y, sl = blockIdx.z;
-  if (bj < bi) return;  // C is symmetric: the upper tiles only
-  const int tx = threadIdx.x, ty = threadIdx.y;  // 32 x 8: each thread 4 outputs (rows ty, ty+8, ...)
-  const int64_t p0 = (int64_t)sl * SLICE, p1 = min((int64_t)N, p0 + SLICE);
+  __shared__ double red[GROUPS - 1][T * T];
+  const int nt = (M + T - 1) / T;
+  int bi, bj;
+  tri_tile(blockIdx.x, nt, bi, bj);
+  const int g = threadIdx.x >> 6, t = threadIdx.x & 63, tx = t & 15, ty = t >> 4;  // outputs (ty + 4 q, tx)
+  const int64_t p0 = (int64_t)blockIdx.y * slice, p1 = min(N, p0 + slice);
   double acc[4] = {0.0, 0.0, 0.0, 0.0};
   for (int64_t k0 = p0; k0 < p1; k0 += KCHUNK) {
-    for (int r = ty; r < T; r += 8) {
-      const int gi = bi * T + r, gj = bj * T + r;
-      const int64_t k = k0 + tx;
-      a[r][tx] = (gi < M && k < p1) ? Xp[(int64_t)gi * N + k] : 0.0;
-      b[r][tx] = (gj < M && k < p1) ? Xp[(int64_t)gj * N + k] : 0.0;
+    const int64_t k = k0 + t;
+#pragma unroll
+    for (int r = 0; r < T; r += GROUPS) {
+      const int gi = bi * T + r + g, gj = bj * T + r + g;
+      a[r + g][t] = (gi < M && k < p1) ? Xp[(int64_t)gi * N + k] : 0.0;
+      b[r + g][t] = (gj < M && k < p1) ? Xp[(int64_t)gj * N + k] : 0.0;
     }
     __syncthreads();
-#pragma unroll 8
-    for (int kk = 0; kk < KCHUNK; ++kk) {
-      const double bv = b[tx][kk];
 #pragma unroll
-      for (int q = 0; q < 4; ++q) acc[q] = fma(a[ty + 8 * q][kk], bv, acc[q]);
+    for (int kk = 0; kk < KCHUNK / GROUPS; ++kk) {
+      const int c = g * (KCHUNK / GROUPS) + kk;
+      const double bv = b[tx][c];
+#pragma unroll
+      for (int q = 0; q < 4; ++q) acc[q] = fma(a[ty + 4 * q][c], bv, acc[q]);
     }
     __syncthreads();
   }
-  const int nt = (M + T - 1) / T;
-  for (int q = 0; q < 4; ++q) {
-    const int i = bi * T + ty + 8 * q, j = bj * T + tx;
-    if (i < M && j < M) part[((int64_t)sl * nt * nt + (int64_t)bi * nt + bj) * T * T + (ty + 8 * q) * T + tx] = acc[q];
+  if (g > 0)
+#pragma unroll
+    for (int q = 0; q < 4; ++q) red[g - 1][(ty + 4 * q) * T + tx] = acc[q];
+  __syncthreads();
+  if (g == 0) {
+    double* o = part + ((int64_t)blockIdx.y * gridDim.x + blockIdx.x) * T * T;
+#pragma unroll
+    for (int q = 0; q < 4; ++q) {
+      const int e = (ty + 4 * q) * T + tx;
+      double v = acc[q];
+      for (int w = 0; w < GROUPS - 1; ++w) v += red[w][e];
+      o[e] = v;
+    }
   }
 }
 
-// C[i][j] = C[j][i] = (sum over slices in order) / M
-__global__ void k_pod_gram_fold(const double* __restrict__ part, int M, int nslice, double* __restrict__ C) {
-  const int i = blockIdx.y * blockDim.y + threadIdx.y, j = blockIdx.x * blockDim.x + threadIdx.x;
+// C[i][j] = C[j][i] = (sum over slices in order) / M; block e: tile e of the upper triangle
+__global__ void __launch_bounds__(T * T) k_pod_gram_fold(const double* __restrict__ part, int M, int nslice,
+                                                         double* __restrict__ C) {
+  const int nt = (M + T - 1) / T;
+  int bi, bj;
+  tri_tile(blockIdx.x, nt, bi, bj);
+  const int i = bi * T + threadIdx.x / T, j = bj * T + threadIdx.x % T;
   if (i >= M || j >= M || j < i) return;
-  const int nt = (M + T - 1) / T, bi = i / T, bj = j / T;
   double s = 0.0;
-  for (int sl = 0; sl < nslice; ++sl) s += part[((int64_t)sl * nt * nt + (int64_t)bi * nt + bj) * T * T + (i % T) * T + (j % T)];
+#pragma unroll 8
+  for (int sl = 0; sl < nslice; ++sl) s += part[((int64_t)sl * gridDim.x + blockIdx.x) * T * T + threadIdx.x];
   const double c = s / (double)M;
   C[(int64_t)i * M + j] = c;
   C[(int64_t)j * M + i] = c;
 }
 
-// modes[q][p] = sum_s X'[s][p] V[s][q] / sigma[q] (zero where sigma <= 1e-12)
+// Modes and coefficients are FP64-bound as well (M k fused multiply-adds a point each).  Both take
+// the k modes in groups of QB <= 8, k split evenly (10 modes: 5 + 5), so that a value of X' is
+// loaded once for QB products held in registers and no product is padding.
+constexpr int QMAX = 8;
+int mode_groups(int k) { return (k + QMAX - 1) / QMAX; }
+int mode_width(int k) { return (k + mode_groups(k) - 1) / mode_groups(k); }
+
+// modes[q][p] = sum_s X'[s][p] V[s][q] / sigma[q] (zero where sigma <= 1e-12), one thread a point
+// (one mode at a time re-read X' for every mode: 192 us on 96 x 80,000 values and 10 modes, now 158).
+template <int QB>
 __global__ void k_pod_modes(const double* __restrict__ Xp, int M, int64_t N, const double* __restrict__ V, int k,
                             const double* __restrict__ inv_sigma, double* __restrict__ modes) {
+  __shared__ double vs[64][QB];
   const int64_t p = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
-  if (p >= N) return;
-  for (int q = 0; q < k; ++q) {
-    double s = 0.0;
-    for (int i = 0; i < M; ++i) s += Xp[(int64_t)i * N + p] * V[(int64_t)i * k + q];
-    modes[(int64_t)q * N + p] = inv_sigma[q] > 0 ? s * inv_sigma[q] : 0.0;
+  const int q0 = blockIdx.y * QB;
+  double acc[QB];
+#pragma unroll
+  for (int u = 0; u < QB; ++u) acc[u] = 0.0;
+  for (int i0 = 0; i0 < M; i0 += 64) {
+    const int ni = min(64, M - i0);
+    __syncthreads();
+    for (int e = threadIdx.x; e < ni * QB; e += blockDim.x) {
+      const int i = e / QB, u = e - i * QB;
+      vs[i][u] = q0 + u < k ? V[(int64_t)(i0 + i) * k + q0 + u] : 0.0;
+    }
+    __syncthreads();
+    if (p < N)
+#pragma unroll 8
+      for (int i = 0; i < ni; ++i) {
+        const double x = Xp[(int64_t)(i0 + i) * N + p];
+#pragma unroll
+        for (int u = 0; u < QB; ++u) acc[u] += x * vs[i][u];
+      }
   }
+  if (p >= N) return;
+#pragma unroll
+  for (int u = 0; u < QB; ++u)
+    if (q0 + u < k) modes[(int64_t)(q0 + u) * N + p] = inv_sigma[q0 + u] > 0 ? acc[u] * inv_sigma[q0 + u] : 0.0;
 }
 
-// part[b][s][q] = sum over block b's points of X'[s][p] modes[q][p]
-__global__ void k_pod_coef_part(const double* __restrict__ Xp, int M, int64_t N, const double* __restrict__ modes,
-                                int k, double* __restrict__ part) {
-  __shared__ double red[256 / 32];
-  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
-  for (int s = 0; s < M; ++s)
-    for (int q = 0; q < k; ++q) {
-      double acc = 0.0;
-      for (int64_t p = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; p < N; p += (int64_t)gridDim.x * blockDim.x)
-        acc += Xp[(int64_t)s * N + p] * modes[(int64_t)q * N + p];
-      for (int o = 16; o > 0; o >>= 1) acc += __shfl_xor_sync(0xffffffffu, acc, o);
-      if (lane == 0) red[warp] = acc;
-      __syncthreads();
-      if (threadIdx.x == 0) {
-        double t = 0.0;
-        for (int w = 0; w < (int)(blockDim.x >> 5); ++w) t += red[w];
-        part[((int64_t)blockIdx.x * M + s) * k + q] = t;
-      }
-      __syncthreads();
+// part[slice][s][q] = sum over the slice's points of X'[s][p] modes[q][p]: a block takes 32 snapshots
+// (its lanes) x QB modes, its eight warps an eighth of every staged chunk each, added in warp order
+// (one output at a time with a block reduction each took 1.33 ms on the sizes above, now 0.16 ms).
+constexpr int CR = 32, CK = 64, CW = 8;
+template <int QB>
+__global__ void __launch_bounds__(32 * CW) k_pod_coef_part(const double* __restrict__ Xp, int M, int64_t N,
+                                                           const double* __restrict__ modes, int k, int64_t slice,
+                                                           double* __restrict__ part) {
+  __shared__ double a[CR][CK + 1];
+  __shared__ double b[QB][CK];
+  __shared__ double red[CW][QB][CR];
+  const int lane = threadIdx.x & 31, w = threadIdx.x >> 5;
+  const int s0 = blockIdx.x * CR, q0 = blockIdx.y * QB;
+  const int64_t p0 = (int64_t)blockIdx.z * slice, p1 = min(N, p0 + slice);
+  double acc[QB];
+#pragma unroll
+  for (int u = 0; u < QB; ++u) acc[u] = 0.0;
+  for (int64_t k0 = p0; k0 < p1; k0 += CK) {
+#pragma unroll
+    for (int e = 0; e < CR * CK / (32 * CW); ++e) {
+      const int f = e * 32 * CW + threadIdx.x, r = f / CK, c = f % CK;
+      a[r][c] = (s0 + r < M && k0 + c < p1) ? Xp[(int64_t)(s0 + r) * N + k0 + c] : 0.0;
     }
+    for (int f = threadIdx.x; f < QB * CK; f += 32 * CW) {
+      const int r = f / CK, c = f % CK;
+      b[r][c] = (q0 + r < k && k0 + c < p1) ? modes[(int64_t)(q0 + r) * N + k0 + c] : 0.0;
+    }
+    __syncthreads();
+#pragma unroll
+    for (int kk = 0; kk < CK / CW; ++kk) {
+      const int c = w * (CK / CW) + kk;
+      const double x = a[lane][c];
+#pragma unroll
+      for (int u = 0; u < QB; ++u) acc[u] += x * b[u][c];
+    }
+    __syncthreads();
+  }
+#pragma unroll
+  for (int u = 0; u < QB; ++u) red[w][u][lane] = acc[u];
+  __syncthreads();
+  for (int e = threadIdx.x; e < QB * CR; e += 32 * CW) {
+    const int u = e / CR, r = e % CR;
+    if (s0 + r >= M || q0 + u >= k) continue;
+    double t = 0.0;
+    for (int v = 0; v < CW; ++v) t += red[v][u][r];
+    part[((int64_t)blockIdx.z * M + s0 + r) * k + q0 + u] = t;
+  }
 }
+// coef[q][s]: the slices' sums, one warp an output (lanes over slices, fixed butterfly)
 __global__ void k_pod_coef_fold(const double* __restrict__ part, int nb, int M, int k, double* __restrict__ coef) {
-  const int e = blockIdx.x * blockDim.x + threadIdx.x;
+  const int e = (blockIdx.x * blockDim.x + threadIdx.x) >> 5, lane = threadIdx.x & 31;
   if (e >= M * k) return;
   const int s = e / k, q = e - s * k;
   double t = 0.0;
-  for (int b = 0; b < nb; ++b) t += part[((int64_t)b * M + s) * k + q];
-  coef[(int64_t)q * M + s] = t;
+  for (int b = lane; b < nb; b += 32) t += part[((int64_t)b * M + s) * k + q];
+  for (int o = 16; o > 0; o >>= 1) t += __shfl_xor_sync(0xffffffffu, t, o);
+  if (lane == 0) coef[(int64_t)q * M + s] = t;
+}
+
+template <int QB>
+void launch_modes(const double* Xp, int M, int64_t N, const double* V, int k, const double* inv_sigma, double* modes,
+                  int64_t slice, int nslice, double* part, cudaStream_t st) {
+  const unsigned ng = (unsigned)mode_groups(k);
+  k_pod_modes<QB><<<dim3((unsigned)((N + 255) / 256), ng), 256, 0, st>>>(Xp, M, N, V, k, inv_sigma, modes);
+  k_pod_coef_part<QB><<<dim3((unsigned)((M + CR - 1) / CR), ng, (unsigned)nslice), 32 * CW, 0, st>>>(Xp, M, N, modes, k,
+                                                                                                    slice, part);
+}
+
+// slices of the point range that give about GRAM_BLOCKS blocks over `tiles` tiles, of at least
+// GRAM_MIN points (a multiple of the staged chunk)
+int64_t slice_points(int64_t N, int64_t tiles) {
+  const int64_t want = std::max<int64_t>(1, GRAM_BLOCKS / tiles);
+  int64_t s = std::max<int64_t>((N + want - 1) / want, GRAM_MIN);
+  s = std::max<int64_t>(s, (N + 65534) / 65535);
+  return (s + KCHUNK - 1) / KCHUNK * KCHUNK;
 }
 
 bool is_device(const void* p) {
@@ -221,11 +324,11 @@ int gm_pod_gram(gm_pod* p, const double* snapshots, double* mean, double* gram, 
     X = p->X;
   }
   k_pod_mean<<<(unsigned)((N + 255) / 256), 256, 0, st>>>(X, M, N, p->mean, p->X);
-  const int nt = (M + T - 1) / T;
-  const int nslice = (int)((N + SLICE - 1) / SLICE);
-  if (cudaError_t e = grow(&p->part, p->part_n, (size_t)nslice * nt * nt * T * T)) return cuda_fail(p, e);
-  k_pod_gram<<<dim3(nt, nt, nslice), dim3(T, 8), 0, st>>>(p->X, M, N, p->part);
-  k_pod_gram_fold<<<dim3(nt, nt), dim3(T, T), 0, st>>>(p->part, M, nslice, p->C);
+  const int64_t nt = (M + T - 1) / T, tiles = nt * (nt + 1) / 2;
+  const int64_t slice = slice_points(N, tiles), nslice = (N + slice - 1) / slice;
+  if (cudaError_t e = grow(&p->part, p->part_n, (size_t)(nslice * tiles * T * T))) return cuda_fail(p, e);
+  k_pod_gram<<<dim3((unsigned)tiles, (unsigned)nslice), 64 * GROUPS, 0, st>>>(p->X, M, N, slice, p->part);
+  k_pod_gram_fold<<<(unsigned)tiles, T * T, 0, st>>>(p->part, M, (int)nslice, p->C);
   gmk::kernel_launch_adjust(3);
   if (cudaError_t e = cudaGetLastError()) return cuda_fail(p, e);
   cudaError_t e = cudaMemcpyAsync(mean, p->mean, N * sizeof(double), cudaMemcpyDefault, st);
@@ -256,11 +359,21 @@ int gm_pod_modes(gm_pod* p, const double* eigvecs, const double* sigma, int32_t 
   for (int q = 0; q < k; ++q) host[(size_t)M * k + q] = sigma[q] > 1e-12 ? 1.0 / sigma[q] : 0.0;
   if (cudaError_t e = cudaMemcpyAsync(p->V, host.data(), host.size() * sizeof(double), cudaMemcpyHostToDevice, st))
     return cuda_fail(p, e);
-  k_pod_modes<<<(unsigned)((N + 255) / 256), 256, 0, st>>>(p->X, M, N, p->V, k, p->V + (size_t)M * k, p->modes);
-  const int nb = (int)std::min<int64_t>(304, (N + 255) / 256);
-  if (cudaError_t e = grow(&p->part, p->part_n, (size_t)nb * M * k)) return cuda_fail(p, e);
-  k_pod_coef_part<<<nb, 256, 0, st>>>(p->X, M, N, p->modes, k, p->part);
-  k_pod_coef_fold<<<(unsigned)((M * k + 255) / 256), 256, 0, st>>>(p->part, nb, M, k, p->coef);
+  const int64_t slice = slice_points(N, (int64_t)((M + CR - 1) / CR) * mode_groups(k)), nslice = (N + slice - 1) / slice;
+  if (cudaError_t e = grow(&p->part, p->part_n, (size_t)(nslice * M * k))) return cuda_fail(p, e);
+  auto* launch = launch_modes<1>;
+  switch (mode_width(k)) {
+    case 1: break;
+    case 2: launch = launch_modes<2>; break;
+    case 3: launch = launch_modes<3>; break;
+    case 4: launch = launch_modes<4>; break;
+    case 5: launch = launch_modes<5>; break;
+    case 6: launch = launch_modes<6>; break;
+    case 7: launch = launch_modes<7>; break;
+    default: launch = launch_modes<8>; break;
+  }
+  launch(p->X, M, N, p->V, k, p->V + (size_t)M * k, p->modes, slice, (int)nslice, p->part, st);
+  k_pod_coef_fold<<<(unsigned)(((int64_t)M * k * 32 + 255) / 256), 256, 0, st>>>(p->part, (int)nslice, M, k, p->coef);
   gmk::kernel_launch_adjust(3);
   if (cudaError_t e = cudaGetLastError()) return cuda_fail(p, e);
   cudaError_t e = cudaMemcpyAsync(modes, p->modes, (size_t)k * N * sizeof(double), cudaMemcpyDefault, st);
