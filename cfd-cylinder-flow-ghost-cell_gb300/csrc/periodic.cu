@@ -10,6 +10,12 @@
 // right-hand side and the Fourier solves in FP32 and refines both solves against the FP64
 // operators (the CN system to the reference's residual gate, the pressure until the
 // projected divergence is below 1e-11).
+//
+// A Fourier solve is three kernels: rows forward, columns (forward, symbol, inverse, in place),
+// rows inverse.  In FP64 the real fields share complex transforms: the two velocity components as
+// u + i v (the CN operator is real and the same for both), two rows of the divergence for the
+// pressure, whose spectrum then has n / 2 + 1 columns.  An FP64 step decides nothing on the
+// host: its launches are queued for all steps and the failed-gate word is read once.
 #include <cuda_runtime.h>
 
 #include <algorithm>
@@ -113,6 +119,7 @@ __device__ __forceinline__ T lap_p(const S* f, int n, int j, int i, T h, T nu) {
 // ---- kernels ------------------------------------------------------------------------------
 // AB2/CN right-hand sides (solver/time_integration.py:20-67): mode 0 AB2, mode 1 start-up
 // midpoint, mode 2 start-up CN right-hand side from the half-step velocity
+// (the FP32 mode's; FP64: k_tg_rhs64)
 template <typename T>
 __global__ void k_tg_rhs(int n, double h, double nu, int mode, double dt, double alpha, const double* __restrict__ q,
                          const double* __restrict__ qh, const double* __restrict__ p, const double* __restrict__ prev,
@@ -150,40 +157,117 @@ __global__ void k_tg_rhs(int n, double h, double nu, int mode, double dt, double
   out[t] = qv + (double)(ddt * (expl + (T)0.5 * lq - gp));
 }
 
-// r = b - H x (H = I - dt/2 nu L, FP64) with max |r| and, on request, max |b|
-__global__ void k_tg_hres(int n, double h, double nu, double hdt, const double* __restrict__ b,
-                          const double* __restrict__ x, double* __restrict__ r, unsigned long long* rmax,
-                          unsigned long long* bmax) {
+// ---- FP64 stencils: 1/h and the products of the step formed on the host (GB300 issues FP64 at
+// 1/64 of the FP32 rate and a divide costs about seven instructions) --------------------------
+// A step's reductions and its failed-gate word (bits of non-negative doubles).
+enum : int { RED_CN = 0, RED_RHS = 1, RED_DIV = 2, RED_COUPLED = 3, RED_PRES = 4, RED_ERR = 5 };
+// Whether an earlier gate of this call failed: the state writers of the steps queued behind it return.
+__device__ __forceinline__ bool tg_failed(const unsigned long long* red) {
+  return *(const volatile unsigned long long*)(red + RED_ERR) != 0;
+}
+__device__ __forceinline__ double lap4(const double* __restrict__ f, int n, int j, int i, int k, double c) {
+  const double e = f[i + 1 < n ? k + 1 : k + 1 - n], w = f[i > 0 ? k - 1 : k - 1 + n];
+  const double u = f[j + 1 < n ? k + n : k + n - n * n], d = f[j > 0 ? k - n : k - n + n * n];
+  return fma(-4.0, c, (e + w) + (u + d));
+}
+
+// FP64 right-hand sides (modes as k_tg_rhs), one thread per cell for its u and v face: the corner
+// products u v are formed once for both, sums stay unhalved (ka = -1/(4h)), and the constants
+// multiply last: about 45 FP64 instructions a cell.  The form with its divides took 369 us at
+// 1024^2.
+struct TgRhsC {
+  double ka, kl, kg, c1, c2;  // -1/(4h); for the step e: nu e/(2 h^2) (mode 1: nu e/h^2), e/h, e (1 + alpha), e alpha
+};
+template <int MODE>
+__global__ void k_tg_rhs64(int n, TgRhsC c, const double* __restrict__ q, const double* __restrict__ qh,
+                           const double* __restrict__ p, const double* __restrict__ prev, double* __restrict__ now,
+                           double* __restrict__ out, unsigned long long* red) {
+  if (tg_failed(red)) return;
+  const int nn = n * n, k = blockIdx.x * blockDim.x + threadIdx.x;
+  if (k == 0) red[RED_CN] = red[RED_RHS] = 0;  // this step's; the previous step's were read by its gate
+  if (k >= nn) return;
+  const int j = k / n, i = k - j * n;
+  const int jp = j + 1 < n ? k + n : k + n - nn, jm = j > 0 ? k - n : k - n + nn;  // (j + 1, i), (j - 1, i)
+  const int dp = i + 1 < n ? 1 : 1 - n, dm = i > 0 ? -1 : n - 1;                     // to i + 1, i - 1
+  const double* u = q;
+  const double* v = q + nn;
+  const double uc = u[k], ue = u[k + dp], uw = u[k + dm], un = u[jp], us = u[jm];
+  const double vc = v[k], ve = v[k + dp], vw = v[k + dm], vn = v[jp], vs = v[jm];
+  double au, av;
+  {
+    const double* a = MODE == 2 ? qh : q;
+    const double* b = a + nn;
+    const double Uc = MODE == 2 ? a[k] : uc, Ue = MODE == 2 ? a[k + dp] : ue, Uw = MODE == 2 ? a[k + dm] : uw;
+    const double Un = MODE == 2 ? a[jp] : un, Us = MODE == 2 ? a[jm] : us, Use = a[jm + dp];
+    const double Vc = MODE == 2 ? b[k] : vc, Ve = MODE == 2 ? b[k + dp] : ve, Vw = MODE == 2 ? b[k + dm] : vw;
+    const double Vn = MODE == 2 ? b[jp] : vn, Vs = MODE == 2 ? b[jm] : vs, Vnw = b[jp + dm];
+    // corner products at (j, i), (j + 1, i), (j, i + 1), times 4
+    const double c00 = (Vw + Vc) * (Us + Uc), c10 = (Vnw + Vn) * (Uc + Un), c01 = (Vc + Ve) * (Use + Ue);
+    const double e = Uc + Ue, w = Uw + Uc, nn_ = Vc + Vn, ss = Vs + Vc;
+    au = fma(e, e, -(w * w)) + (c10 - c00);
+    av = fma(nn_, nn_, -(ss * ss)) + (c01 - c00);
+  }
+  const double lu = fma(-4.0, uc, (ue + uw) + (un + us)), lv = fma(-4.0, vc, (ve + vw) + (vn + vs));
+  const double pc = p[k], gu = pc - p[k + dm], gv = pc - p[jm];
+  au *= c.ka;
+  av *= c.ka;
+  if (MODE != 2) {
+    now[k] = au;
+    now[nn + k] = av;
+  }
+  double xu = c.c1 * au, xv = c.c1 * av;
+  if (MODE == 0) {
+    xu = fma(-c.c2, prev[k], xu);
+    xv = fma(-c.c2, prev[nn + k], xv);
+  }
+  out[k] = uc + fma(c.kl, lu, fma(-c.kg, gu, xu));
+  out[nn + k] = vc + fma(c.kl, lv, fma(-c.kg, gv, xv));
+}
+
+// The stencils that both precisions share, in two forms.  P64: as above, reciprocals on the host.
+// Otherwise with the divides: the FP32 mode's pressure holds the FP32 rounding of its state, which
+// another last bit of these stencils moves by 4e-8 in 20 steps, and its small grids gain little.
+struct TgC {
+  double h, nu, hdt;     // with divides: spacing, viscosity, dt / 2
+  double ih, kh;         // P64: 1 / h, dt nu / (2 h^2)
+};
+template <bool P64>
+__device__ __forceinline__ double helm_p(const TgC& c, const double* __restrict__ f, int n, int j, int i, int k, double x) {
+  if (P64) return fma(-c.kh, lap4(f, n, j, i, k, x), x);
+  return x - c.hdt * lap_p<double>(f, n, j, i, c.h, c.nu);
+}
+__device__ __forceinline__ double div_sum(const double* __restrict__ q, int n, int j, int i, int k) {
+  const int nn = n * n;
+  return q[i + 1 < n ? k + 1 : k + 1 - n] - q[k] + q[nn + (j + 1 < n ? k + n : k + n - nn)] - q[nn + k];
+}
+
+// r = b - H x (H = I - dt/2 nu L) with max |r| and max |b|
+template <bool P64>
+__global__ void k_tg_hres(int n, TgC c, const double* __restrict__ b, const double* __restrict__ x,
+                          double* __restrict__ r, unsigned long long* red) {
   const int nn = n * n;
   unsigned long long rm = 0, bm = 0;
   for (int t = blockIdx.x * blockDim.x + threadIdx.x; t < 2 * nn; t += gridDim.x * blockDim.x) {
     const int comp = t >= nn, k = t - comp * nn, j = k / n, i = k - j * n;
-    const double* f = x + comp * nn;
-    const double hx = x[t] - hdt * lap_p<double>(f, n, j, i, h, nu);
-    const double rv = b[t] - hx;
+    const double bv = b[t], rv = bv - helm_p<P64>(c, x + comp * nn, n, j, i, k, x[t]);
     if (r) r[t] = rv;
     rm = max(rm, absbits_(rv));
-    if (bmax) bm = max(bm, absbits_(b[t]));
+    bm = max(bm, absbits_(bv));
   }
-  commit_max(rm, rmax);
-  if (bmax) commit_max(bm, bmax);
+  commit_max(rm, red + RED_CN);
+  commit_max(bm, red + RED_RHS);
 }
 
-// d = div(q) / step on the cell grid, max |div q| on request
-__global__ void k_tg_div(int n, double h, double inv_step, const double* __restrict__ q, double* __restrict__ d,
-                         unsigned long long* dmax) {
+// FP32 mode: d = div(q) / step on the cell grid
+__global__ void k_tg_div(int n, double h, double inv_step, const double* __restrict__ q, double* __restrict__ d) {
   const int nn = n * n;
-  unsigned long long m = 0;
   for (int k = blockIdx.x * blockDim.x + threadIdx.x; k < nn; k += gridDim.x * blockDim.x) {
     const int j = k / n, i = k - j * n;
-    const double dv = (q[j * n + wrapi(i + 1, n)] - q[k] + q[nn + wrapi(j + 1, n) * n + i] - q[nn + k]) / h;
-    if (d) d[k] = dv * inv_step;
-    m = max(m, absbits_(dv));
+    d[k] = div_sum(q, n, j, i, k) / h * inv_step;
   }
-  if (dmax) commit_max(m, dmax);
 }
 
-// r = b - A phi with A = div grad (periodic 5-point / h^2), max |r|
+// FP32 mode: r = b - A phi with A = div grad (periodic 5-point / h^2), max |r|
 __global__ void k_tg_pres(int n, double h, const double* __restrict__ b, const double* __restrict__ x,
                           double* __restrict__ r, unsigned long long* rmax) {
   const int nn = n * n;
@@ -199,125 +283,250 @@ __global__ void k_tg_pres(int n, double h, const double* __restrict__ b, const d
   commit_max(rm, rmax);
 }
 
-// out = q - step grad(phi)
-__global__ void k_tg_update(int n, double h, double step, const double* __restrict__ q, const double* __restrict__ phi,
-                            double* __restrict__ out) {
-  const int nn = n * n;
-  const int t = blockIdx.x * blockDim.x + threadIdx.x;
-  if (t >= 2 * nn) return;
-  const int comp = t >= nn, k = t - comp * nn, j = k / n, i = k - j * n;
-  const double g = comp == 0 ? (phi[k] - phi[j * n + wrapi(i - 1, n)]) / h : (phi[k] - phi[wrapi(j - 1, n) * n + i]) / h;
-  out[t] = q[t] - step * g;
-}
-
-// action = H result, proj = result + (rhs - action)   (solver/time_integration.py:107-113)
-__global__ void k_tg_defect(int n, double h, double nu, double hdt, const double* __restrict__ res,
-                            const double* __restrict__ rhs, double* __restrict__ action, double* __restrict__ proj) {
-  const int nn = n * n;
-  const int t = blockIdx.x * blockDim.x + threadIdx.x;
-  if (t >= 2 * nn) return;
-  const int comp = t >= nn, k = t - comp * nn, j = k / n, i = k - j * n;
-  const double a = res[t] - hdt * lap_p<double>(res + comp * nn, n, j, i, h, nu);
-  action[t] = a;
-  proj[t] = res[t] + (rhs[t] - a);
-}
-
-// half = p + inc, out = half + factor inc, max |action - rhs + dt grad inc|
-__global__ void k_tg_pout(int n, double h, double dt, double factor, const double* __restrict__ p,
-                          const double* __restrict__ inc, const double* __restrict__ action,
-                          const double* __restrict__ rhs, double* __restrict__ half, double* __restrict__ pout,
-                          unsigned long long* cmax) {
-  const int nn = n * n;
-  unsigned long long m = 0;
-  for (int t = blockIdx.x * blockDim.x + threadIdx.x; t < 2 * nn; t += gridDim.x * blockDim.x) {
-    const int comp = t >= nn, k = t - comp * nn, j = k / n, i = k - j * n;
-    const double g = comp == 0 ? (inc[k] - inc[j * n + wrapi(i - 1, n)]) / h : (inc[k] - inc[wrapi(j - 1, n) * n + i]) / h;
-    m = max(m, absbits_(action[t] - rhs[t] + dt * g));
-    if (comp == 0) {
-      const double hv = p[k] + inc[k];
-      half[k] = hv;
-      pout[k] = hv + factor * inc[k];
+// out = q - step grad(phi), one thread per cell.  With gate_step > 0 (the projection of the CN
+// velocity) it first applies the CN gate max |H star - rhs| <= 1e-10 max(1, max |rhs|)
+// (solver/time_integration.py:100-104): every block reads the same two words, a failed gate records
+// the step and leaves the state alone.
+template <bool P64>
+__global__ void k_tg_update(int n, TgC c, double step, double kg, const double* __restrict__ q,
+                            const double* __restrict__ phi, double* __restrict__ out, unsigned long long* red,
+                            int gate_step) {
+  if (gate_step > 0) {
+    if (tg_failed(red)) return;
+    const double r = __longlong_as_double((long long)red[RED_CN]), b = __longlong_as_double((long long)red[RED_RHS]);
+    if (!(r <= 1e-10 * (b > 1.0 ? b : 1.0)) || !isfinite(r)) {
+      if (blockIdx.x == 0 && threadIdx.x == 0) red[RED_ERR] = (unsigned long long)gate_step;
+      return;
     }
   }
-  commit_max(m, cmax);
+  const int nn = n * n, k = blockIdx.x * blockDim.x + threadIdx.x;
+  if (k >= nn) return;
+  const int j = k / n, i = k - j * n;
+  const double f = phi[k];
+  const double gu = f - phi[i > 0 ? k - 1 : k - 1 + n], gv = f - phi[j > 0 ? k - n : k - n + nn];
+  out[k] = P64 ? fma(-kg, gu, q[k]) : q[k] - step * (gu / c.h);
+  out[nn + k] = P64 ? fma(-kg, gv, q[nn + k]) : q[nn + k] - step * (gv / c.h);
 }
 
-// ---- Fourier solves: rows (x) -> transpose -> rows (y) with the symbol -> transpose -> rows ----
+// action = H result, proj = result + (rhs - action)   (solver/time_integration.py:107-113), and
+// the largest |div result|
+template <bool P64>
+__global__ void k_tg_defect(int n, TgC c, const double* __restrict__ res, const double* __restrict__ rhs,
+                            double* __restrict__ action, double* __restrict__ proj, unsigned long long* red) {
+  if (tg_failed(red)) return;
+  const int nn = n * n;
+  unsigned long long m = 0;
+  for (int k = blockIdx.x * blockDim.x + threadIdx.x; k < nn; k += gridDim.x * blockDim.x) {
+    const int j = k / n, i = k - j * n;
+#pragma unroll
+    for (int comp = 0; comp < 2; ++comp) {
+      const int t = comp * nn + k;
+      const double x = res[t], a = helm_p<P64>(c, res + comp * nn, n, j, i, k, x);
+      action[t] = a;
+      proj[t] = x + (rhs[t] - a);
+    }
+    const double d = div_sum(res, n, j, i, k);
+    m = max(m, absbits_(P64 ? d * c.ih : d / c.h));
+  }
+  commit_max(m, red + RED_DIV);
+}
+
+// half = p + inc, out = half + factor inc, max |action - rhs + dt grad inc| (kg = dt / h)
+template <bool P64>
+__global__ void k_tg_pout(int n, TgC c, double dt, double kg, double factor, const double* __restrict__ p,
+                          const double* __restrict__ inc, const double* __restrict__ action,
+                          const double* __restrict__ rhs, double* __restrict__ half, double* __restrict__ pout,
+                          unsigned long long* red) {
+  if (tg_failed(red)) return;
+  const int nn = n * n;
+  unsigned long long m = 0;
+  for (int k = blockIdx.x * blockDim.x + threadIdx.x; k < nn; k += gridDim.x * blockDim.x) {
+    const int j = k / n, i = k - j * n;
+    const double f = inc[k];
+    const double gu = f - inc[i > 0 ? k - 1 : k - 1 + n], gv = f - inc[j > 0 ? k - n : k - n + nn];
+    const double au = action[k] - rhs[k], av = action[nn + k] - rhs[nn + k];
+    m = max(m, absbits_(P64 ? fma(kg, gu, au) : au + dt * (gu / c.h)));
+    m = max(m, absbits_(P64 ? fma(kg, gv, av) : av + dt * (gv / c.h)));
+    const double hv = p[k] + f;
+    half[k] = hv;
+    pout[k] = hv + factor * f;
+  }
+  commit_max(m, red + RED_COUPLED);
+}
+
+// ---- Fourier solves: rows (x) forward -> columns (y) forward, symbol, inverse -> rows inverse ----
 // The symbol of the periodic 5-point Laplacian is lam(k, l) = -4 (s_k + s_l) / h^2 with
 // s_k = sin^2(pi k / n).  kind 0: phi = F^-1[F b / lam] with the mean mode set to zero
 // (verification/taylor_green.py:41-45); kind 1: x = F^-1[F b / (1 - c lam)].
+//
+// How a real field goes through the complex transforms:
+//   LINE_REAL  one real row per transform (FP32: its rounding is kept as it is)
+//   LINE_PAIR  two rows of s div(q) as real and imaginary part (FP64 pressure): the spectra of both
+//              rows separate by their symmetry, n / 2 + 1 modes each, so the column pass runs
+//              half the columns.  2 A and 2 B are stored, the halves are in the final scale
+//   LINE_UV    u + i v (FP64 CN solve): the operator is real, so both parts solve at once
+// FP64 transforms are bound by the FP64 pipe (about 33 instructions a complex point and pass): with
+// these a pressure solve takes half and a CN solve half of the one-row form's work.  At 1024^2
+// (8 8 8 2) the column pass takes 150 us for u + i v and 77 for a pressure (0.80 and 0.77 of the pipe's
+// rate), row passes 82-87 and 47-54; a solve of seven kernels with transposes took 366 us a field,
+// now 186 a pressure and 319 both components
+enum : int { LINE_REAL = 0, LINE_PAIR = 1, LINE_UV = 2 };
+
+// A block holds gpb groups of gt threads, each with two length-n buffers (pad entries apart, so that
+// a quarter warp's column loads touch distinct banks), behind the plan's twiddles.
 template <typename T>
-__host__ __device__ inline size_t tg_row_smem(int n, int tw) {
-  return ((size_t)tw * sizeof(cplx<T>) + 15) / 16 * 16 + 2 * (size_t)n * sizeof(cplx<T>);
+__host__ __device__ inline int tg_pad(int gpb) { return gpb > 1 ? (sizeof(T) == 8 ? 2 : 4) : 0; }
+template <typename T>
+__host__ __device__ inline size_t tg_smem(int n, int tw, int gpb) {
+  return ((size_t)tw * sizeof(cplx<T>) + 15) / 16 * 16 + (size_t)gpb * (2 * (size_t)n + tg_pad<T>(gpb)) * sizeof(cplx<T>);
+}
+template <typename T>
+__device__ __forceinline__ const cplx<T>* tw_of(const unsigned char* smem) { return reinterpret_cast<const cplx<T>*>(smem); }
+template <typename T>
+__device__ __forceinline__ cplx<T>* tg_stage(const FftPlan& plan, const cplx<T>* __restrict__ tw_g, unsigned char* smem) {
+  cplx<T>* tw = reinterpret_cast<cplx<T>*>(smem);
+  for (int q = threadIdx.x; q < plan.tw_len; q += blockDim.x) tw[q] = tw_g[q];
+  __syncthreads();
+  return reinterpret_cast<cplx<T>*>(smem + ((size_t)plan.tw_len * sizeof(cplx<T>) + 15) / 16 * 16);
 }
 
-// mode 0: real row in -> forward FFT -> complex out; mode 1: complex row in -> forward FFT ->
-// divide by the symbol -> inverse FFT -> complex out; mode 2: complex row in -> inverse FFT ->
-// real part times scale out.  One block per row.
-template <typename T, int MODE>
-__global__ void k_tg_rows(int n, FftPlan plan, const cplx<T>* __restrict__ tw_g, const void* __restrict__ in,
-                          void* __restrict__ out, const T* __restrict__ s2, int kind, T hh2, T coef, T scale) {
+// Rows forward.  in: the real field (LINE_REAL; field blockIdx.y of n n values), q (LINE_PAIR), the
+// two components (LINE_UV).
+template <typename T, int LINE>
+__global__ void k_tg_rows_fwd(int n, FftPlan plan, const cplx<T>* __restrict__ tw_g, const double* __restrict__ in,
+                              cplx<T>* __restrict__ S, int pitch, double s, int gt, int gpb) {
   extern __shared__ __align__(16) unsigned char smem_raw[];
-  cplx<T>* tw = reinterpret_cast<cplx<T>*>(smem_raw);
-  for (int q = threadIdx.x; q < plan.tw_len; q += blockDim.x) tw[q] = tw_g[q];
-  cplx<T>* a = reinterpret_cast<cplx<T>*>(smem_raw + ((size_t)plan.tw_len * sizeof(cplx<T>) + 15) / 16 * 16);
+  cplx<T>* base = tg_stage<T>(plan, tw_g, smem_raw);
+  const int grp = threadIdx.x / gt, tid = threadIdx.x - grp * gt, nn = n * n;
+  const int line = blockIdx.x * gpb + grp, row = LINE == LINE_PAIR ? 2 * line : line;
+  if (row >= n) return;
+  cplx<T>* a = base + (size_t)grp * (2 * n + tg_pad<T>(gpb));
   cplx<T>* b = a + n;
-  const int row = blockIdx.x;
-  if (MODE == 0) {
-    const T* src = reinterpret_cast<const T*>(in) + (size_t)row * n;
-    for (int e = threadIdx.x; e < n; e += blockDim.x) a[e] = {src[e], (T)0};
+  const Grp G{tid, gt, grp + 1};
+  if (LINE == LINE_REAL) {
+    const double* src = in + (size_t)blockIdx.y * nn + (size_t)row * n;
+    for (int e = tid; e < n; e += gt) a[e] = {(T)src[e], (T)0};
+  } else if (LINE == LINE_UV) {
+    const double* src = in + (size_t)row * n;
+    for (int e = tid; e < n; e += gt) a[e] = {(T)src[e], (T)src[nn + e]};
   } else {
-    const cplx<T>* src = reinterpret_cast<const cplx<T>*>(in) + (size_t)row * n;
-    for (int e = threadIdx.x; e < n; e += blockDim.x) a[e] = src[e];
-  }
-  __syncthreads();
-  const Grp G{(int)threadIdx.x, (int)blockDim.x, 1};
-  cplx<T>* r = fft_run<T>(a, b, plan, 1, tw, MODE == 2 ? +1 : -1, G);
-  if (MODE == 1) {
-    cplx<T>* o = r == a ? b : a;
-    for (int e = threadIdx.x; e < n; e += blockDim.x) {
-      const T lam = (T)-4 * (s2[row] + s2[e]) / hh2;
-      T f;
-      if (kind == 0) f = (row == 0 && e == 0) ? (T)0 : (T)1 / lam;
-      else f = (T)1 / ((T)1 - coef * lam);
-      r[e] = {r[e].x * f, r[e].y * f};
+    const bool two = row + 1 < n;
+    for (int e = tid; e < n; e += gt) {
+      const double d0 = div_sum(in, n, row, e, row * n + e) * s;
+      const double d1 = two ? div_sum(in, n, row + 1, e, (row + 1) * n + e) * s : 0.0;
+      a[e] = {(T)d0, (T)d1};
     }
-    __syncthreads();
+  }
+  G.sync();
+  const cplx<T>* r = fft_run<T>(a, b, plan, 1, tw_of<T>(smem_raw), -1, G);
+  cplx<T>* dst = S + (size_t)blockIdx.y * nn + (size_t)row * pitch;
+  if (LINE == LINE_PAIR) {
+    const bool two = row + 1 < n;
+    for (int k = tid; k <= n / 2; k += gt) {
+      const cplx<T> z = r[k], c = r[k ? n - k : 0];
+      dst[k] = {z.x + c.x, z.y - c.y};
+      if (two) dst[pitch + k] = {z.y + c.y, c.x - z.x};
+    }
+  } else {
+    for (int e = tid; e < n; e += gt) dst[e] = r[e];
+  }
+}
+
+// Columns forward, symbol, columns inverse, in place: a block's groups take gpb neighbouring
+// columns, loaded and stored by the whole block along the rows (64-byte pieces for FP64).  f: the
+// FP64 symbol table (n x (n / 2 + 1), lam(k, n - l) = lam(k, l)); FP32 forms the symbol as it goes.
+template <typename T>
+__global__ void k_tg_cols(int n, FftPlan plan, const cplx<T>* __restrict__ tw_g, cplx<T>* __restrict__ S, int pitch,
+                          int ncols, const double* __restrict__ f, const T* __restrict__ s2, int kind, T hh2, T coef,
+                          int gt, int gpb) {
+  extern __shared__ __align__(16) unsigned char smem_raw[];
+  cplx<T>* base = tg_stage<T>(plan, tw_g, smem_raw);
+  const int stride = 2 * n + tg_pad<T>(gpb), c0 = blockIdx.x * gpb;
+  cplx<T>* field = S + (size_t)blockIdx.y * n * n;
+  const int lc = threadIdx.x % gpb, lr = threadIdx.x / gpb, ls = blockDim.x / gpb;
+  if (c0 + lc < ncols)
+    for (int e = lr; e < n; e += ls) base[lc * stride + e] = field[(size_t)e * pitch + c0 + lc];
+  __syncthreads();
+  const int grp = threadIdx.x / gt, tid = threadIdx.x - grp * gt, col = c0 + grp;
+  cplx<T>* r = base + grp * stride;  // where the column ends up (group-uniform)
+  if (col < ncols) {
+    cplx<T>* a = r;
+    cplx<T>* b = a + n;
+    const Grp G{tid, gt, grp + 1};
+    const cplx<T>* tw = tw_of<T>(smem_raw);
+    r = fft_run<T>(a, b, plan, 1, tw, -1, G);
+    cplx<T>* o = r == a ? b : a;
+    if (sizeof(T) == 8) {
+      const int nh = n / 2 + 1, kc = col < nh ? col : n - col;
+      for (int e = tid; e < n; e += gt) {
+        const T g = (T)f[(size_t)e * nh + kc];
+        r[e] = {r[e].x * g, r[e].y * g};
+      }
+    } else {
+      for (int e = tid; e < n; e += gt) {
+        const T lam = (T)-4 * (s2[col] + s2[e]) / hh2;
+        T g;
+        if (kind == 0) g = (col == 0 && e == 0) ? (T)0 : (T)1 / lam;
+        else g = (T)1 / ((T)1 - coef * lam);
+        r[e] = {r[e].x * g, r[e].y * g};
+      }
+    }
+    G.sync();
     r = fft_run<T>(r, o, plan, 1, tw, +1, G);
   }
-  if (MODE == 2) {
-    T* dst = reinterpret_cast<T*>(out) + (size_t)row * n;
-    for (int e = threadIdx.x; e < n; e += blockDim.x) dst[e] = r[e].x * scale;
-  } else {
-    cplx<T>* dst = reinterpret_cast<cplx<T>*>(out) + (size_t)row * n;
-    for (int e = threadIdx.x; e < n; e += blockDim.x) dst[e] = r[e];
-  }
-}
-
-template <typename T>
-__global__ void k_tg_transpose(int n, const cplx<T>* __restrict__ in, cplx<T>* __restrict__ out) {
-  __shared__ cplx<T> tile[32][33];
-  const int bx = blockIdx.x * 32, by = blockIdx.y * 32;
-  for (int yy = threadIdx.y; yy < 32; yy += blockDim.y) {
-    const int y = by + yy, x = bx + threadIdx.x;
-    if (y < n && x < n) tile[yy][threadIdx.x] = in[(size_t)y * n + x];
-  }
+  // two transforms of equal length end in the buffer they began in: column c is at base + c stride
   __syncthreads();
-  for (int xx = threadIdx.y; xx < 32; xx += blockDim.y) {
-    const int x = bx + xx, y = by + threadIdx.x;
-    if (y < n && x < n) out[(size_t)x * n + y] = tile[threadIdx.x][xx];
+  if (c0 + lc < ncols)
+    for (int e = lr; e < n; e += ls) field[(size_t)e * pitch + c0 + lc] = base[lc * stride + e];
+}
+
+// Rows inverse: the real parts (LINE_PAIR: two rows, LINE_UV: both components) times scale, FP64.
+template <typename T, int LINE>
+__global__ void k_tg_rows_inv(int n, FftPlan plan, const cplx<T>* __restrict__ tw_g, const cplx<T>* __restrict__ S,
+                              int pitch, double* __restrict__ out, T scale, int accumulate, int gt, int gpb) {
+  extern __shared__ __align__(16) unsigned char smem_raw[];
+  cplx<T>* base = tg_stage<T>(plan, tw_g, smem_raw);
+  const int grp = threadIdx.x / gt, tid = threadIdx.x - grp * gt, nn = n * n;
+  const int line = blockIdx.x * gpb + grp, row = LINE == LINE_PAIR ? 2 * line : line;
+  if (row >= n) return;
+  cplx<T>* a = base + (size_t)grp * (2 * n + tg_pad<T>(gpb));
+  cplx<T>* b = a + n;
+  const Grp G{tid, gt, grp + 1};
+  const cplx<T>* src = S + (size_t)blockIdx.y * nn + (size_t)row * pitch;
+  const bool two = LINE == LINE_PAIR && row + 1 < n;
+  if (LINE == LINE_PAIR) {
+    for (int k = tid; k <= n / 2; k += gt) {
+      const cplx<T> A = src[k], B = two ? src[pitch + k] : cplx<T>{(T)0, (T)0};
+      a[k] = {A.x - B.y, A.y + B.x};
+      if (k && n - k != k) a[n - k] = {A.x + B.y, B.x - A.y};
+    }
+  } else {
+    for (int e = tid; e < n; e += gt) a[e] = src[e];
+  }
+  G.sync();
+  const cplx<T>* r = fft_run<T>(a, b, plan, 1, tw_of<T>(smem_raw), +1, G);
+  double* dst = out + (size_t)blockIdx.y * nn + (size_t)row * n;
+  for (int e = tid; e < n; e += gt) {
+    const double re = (double)(r[e].x * scale);
+    if (LINE == LINE_REAL) {
+      dst[e] = accumulate ? dst[e] + re : re;
+    } else {
+      const double im = (double)(r[e].y * scale);
+      dst[e] = re;
+      if (LINE == LINE_UV) dst[nn + e] = im;
+      else if (two) dst[n + e] = im;
+    }
   }
 }
 
-template <typename T>
-__global__ void k_tg_to_t(int64_t n, const double* __restrict__ src, T* __restrict__ dst) {
-  for (int64_t t = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; t < n; t += (int64_t)gridDim.x * blockDim.x)
-    dst[t] = (T)src[t];
-}
-template <typename T>
-__global__ void k_tg_from_t(int64_t n, const T* __restrict__ src, double* __restrict__ dst, int accumulate) {
-  for (int64_t t = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; t < n; t += (int64_t)gridDim.x * blockDim.x)
-    dst[t] = accumulate ? dst[t] + (double)src[t] : (double)src[t];
+// FP64 symbol tables (n x (n / 2 + 1)): the factor of each mode
+__global__ void k_tg_symbol(int n, const double* __restrict__ s2, int kind, double hh2, double coef, double* __restrict__ f) {
+  const int nh = n / 2 + 1;
+  for (int t = blockIdx.x * blockDim.x + threadIdx.x; t < n * nh; t += gridDim.x * blockDim.x) {
+    const int l = t / nh, k = t - l * nh;
+    const double lam = -4 * (s2[l] + s2[k]) / hh2;
+    f[t] = kind == 0 ? (t == 0 ? 0.0 : 1 / lam) : 1 / (1 - coef * lam);
+  }
 }
 
 unsigned grid_for(int64_t n) { return (unsigned)std::min<int64_t>((n + PT - 1) / PT, 152 * 8); }
@@ -330,57 +539,53 @@ struct gm_tg {
   std::string err;
   cudaStream_t st = nullptr;
   FftPlan plan{};
-  size_t smem = 0, smem32 = 0;
-  int threads = 256;
-  Buf<double> q, qn, hist, now, rhs, star, mid, half_q, action, proj, phalf, phalf_n, pout, phi, inc, div, work, corr;
-  Buf<double> tw64, s2_64;
-  Buf<float> tw32, s2_32, real32;
-  Buf<double> real64;
-  Buf<unsigned char> cbuf_a, cbuf_b;  // complex n x n work arrays (T precision)
-  Buf<unsigned long long> red;        // reductions: 0 cn residual, 1 rhs max, 2 div, 3 coupled, 4 pressure residual
+  int gt = 32, gpb[2] = {1, 1};  // threads per transform, transforms per block (FP32, FP64)
+  size_t smem[2] = {0, 0};
+  Buf<double> q, qn, hist, now, rhs, star, mid, half_q, action, proj, phalf, phalf_n, pout, phi, inc, div, work;
+  Buf<double> tw64, s2_64, sym_p, sym_h;  // FP64 symbol tables of the pressure and the CN operator (for sym_dt)
+  Buf<float> tw32, s2_32;
+  double sym_dt = 0;
+  Buf<unsigned char> spec;            // the spectrum: n x n complex FP64, or two of FP32
+  Buf<unsigned long long> red;        // RED_*
+  unsigned long long* host_red = nullptr;  // its page-locked copy (a pageable one costs the FP32 refinement's read-backs a staging copy each)
+  ~gm_tg() { if (host_red) cudaFreeHost(host_red); }
   bool has_history = false;
   double prev_dt = 0;
-  double last_cn_residual = 0, last_coupled = 0;
 };
 
 namespace {
 
-// x = S^-1 b on the cell grid (n x n, FP64 in and out, T arithmetic); kind 0 Poisson, 1 Helmholtz
+// One solve: kind 0 Poisson, 1 Helmholtz (coef = dt nu / 2).
+//   FP32: x (+)= S^-1 b for `fields` cell grids of n n values.
+//   FP64: kind 0 takes the velocity b and solves for s div(b); kind 1 takes both components.
 template <typename T>
-void fourier_solve(gm_tg* t, int kind, double coef, const double* b, double* x, bool accumulate) {
-  const int n = t->n;
-  const int64_t nn = (int64_t)n * n;
+void fourier_solve(gm_tg* t, int kind, double coef, const double* b, double* x, bool accumulate, int fields, double s) {
+  constexpr bool D = sizeof(T) == 8;
+  const int n = t->n, gt = t->gt, gpb = t->gpb[D], thr = gt * gpb;
+  const size_t sm = t->smem[D];
   cudaStream_t st = t->st;
-  T* rb = sizeof(T) == 4 ? (T*)t->real32.p : (T*)t->real64.p;
-  const cplx<T>* tw = sizeof(T) == 4 ? (const cplx<T>*)t->tw32.p : (const cplx<T>*)t->tw64.p;
-  const T* s2 = sizeof(T) == 4 ? (const T*)t->s2_32.p : (const T*)t->s2_64.p;
-  const size_t smem = sizeof(T) == 4 ? t->smem32 : t->smem;
-  cplx<T>* A = reinterpret_cast<cplx<T>*>(t->cbuf_a.p);
-  cplx<T>* B = reinterpret_cast<cplx<T>*>(t->cbuf_b.p);
-  gmk::kernel_launch_adjust(1);
-  k_tg_to_t<T><<<grid_for(nn), PT, 0, st>>>(nn, b, rb);
-  gmk::kernel_launch_adjust(1);
-  k_tg_rows<T, 0><<<n, t->threads, smem, st>>>(n, t->plan, tw, rb, A, s2, kind, (T)(t->h * t->h), (T)coef, (T)1);
-  const dim3 tg((n + 31) / 32, (n + 31) / 32), tb(32, 8);
-  gmk::kernel_launch_adjust(1);
-  k_tg_transpose<T><<<tg, tb, 0, st>>>(n, A, B);
-  gmk::kernel_launch_adjust(1);
-  k_tg_rows<T, 1><<<n, t->threads, smem, st>>>(n, t->plan, tw, B, B, s2, kind, (T)(t->h * t->h), (T)coef, (T)1);
-  gmk::kernel_launch_adjust(1);
-  k_tg_transpose<T><<<tg, tb, 0, st>>>(n, B, A);
-  gmk::kernel_launch_adjust(1);
-  k_tg_rows<T, 2><<<n, t->threads, smem, st>>>(n, t->plan, tw, A, rb, s2, kind, (T)(t->h * t->h), (T)coef,
-                                                (T)(1.0 / ((double)n * n)));
-  gmk::kernel_launch_adjust(1);
-  k_tg_from_t<T><<<grid_for(nn), PT, 0, st>>>(nn, rb, x, accumulate ? 1 : 0);
+  const cplx<T>* tw = D ? (const cplx<T>*)t->tw64.p : (const cplx<T>*)t->tw32.p;
+  const T* s2 = D ? (const T*)t->s2_64.p : (const T*)t->s2_32.p;
+  cplx<T>* S = reinterpret_cast<cplx<T>*>(t->spec.p);
+  const T scale = (T)((D && kind == 0 ? 0.5 : 1.0) / ((double)n * n));
+  const int pair = D && kind == 0, ncols = pair ? n / 2 + 1 : n, lines = pair ? (n + 1) / 2 : n;
+  const dim3 gr((unsigned)((lines + gpb - 1) / gpb), (unsigned)fields), gc((unsigned)((ncols + gpb - 1) / gpb), (unsigned)fields);
+  const double* f = kind == 0 ? t->sym_p.p : t->sym_h.p;
+  gmk::kernel_launch_adjust(3);
+  if constexpr (!D) k_tg_rows_fwd<T, LINE_REAL><<<gr, thr, sm, st>>>(n, t->plan, tw, b, S, n, 0.0, gt, gpb);
+  else if (pair) k_tg_rows_fwd<T, LINE_PAIR><<<gr, thr, sm, st>>>(n, t->plan, tw, b, S, ncols, s, gt, gpb);
+  else k_tg_rows_fwd<T, LINE_UV><<<gr, thr, sm, st>>>(n, t->plan, tw, b, S, n, 0.0, gt, gpb);
+  k_tg_cols<T><<<gc, thr, sm, st>>>(n, t->plan, tw, S, ncols, ncols, f, s2, kind, (T)(t->h * t->h), (T)coef, gt, gpb);
+  if constexpr (!D) k_tg_rows_inv<T, LINE_REAL><<<gr, thr, sm, st>>>(n, t->plan, tw, S, n, x, scale, accumulate ? 1 : 0, gt, gpb);
+  else if (pair) k_tg_rows_inv<T, LINE_PAIR><<<gr, thr, sm, st>>>(n, t->plan, tw, S, ncols, x, scale, 0, gt, gpb);
+  else k_tg_rows_inv<T, LINE_UV><<<gr, thr, sm, st>>>(n, t->plan, tw, S, n, x, scale, 0, gt, gpb);
   TG_CK(cudaGetLastError());
 }
 
-unsigned long long read_max(gm_tg* t, int slot) {
-  unsigned long long v = 0;
-  TG_CK(cudaMemcpyAsync(&v, t->red.p + slot, sizeof v, cudaMemcpyDeviceToHost, t->st));
+const unsigned long long* read_red(gm_tg* t) {
+  TG_CK(cudaMemcpyAsync(t->host_red, t->red.p, 8 * sizeof(unsigned long long), cudaMemcpyDeviceToHost, t->st));
   TG_CK(cudaStreamSynchronize(t->st));
-  return v;
+  return t->host_red;
 }
 double bitsd(unsigned long long b) {
   double d;
@@ -388,110 +593,141 @@ double bitsd(unsigned long long b) {
   return d;
 }
 
+unsigned blocks_of(int64_t n) { return (unsigned)((n + PT - 1) / PT); }
+TgC stencil_consts(const gm_tg* t, double dt) {
+  return TgC{t->h, t->nu, 0.5 * dt, 1.0 / t->h, 0.5 * dt * t->nu / (t->h * t->h)};
+}
+
 // project(q, step): phi = A^-1 (div q / step), out = q - step grad phi (refined in FP32 mode
 // until the projected divergence max |step (b - A phi)| is below 1e-11)
-void tg_project(gm_tg* t, const double* q, double step, double* out, double* phi) {
+void tg_project(gm_tg* t, const double* q, double step, double* out, double* phi, int gate_step) {
   const int n = t->n;
   const int64_t nn = (int64_t)n * n;
   cudaStream_t st = t->st;
-  gmk::kernel_launch_adjust(1);
-  k_tg_div<<<grid_for(nn), PT, 0, st>>>(n, t->h, 1.0 / step, q, t->div.p, nullptr);
   if (t->precision == 0) {
-    fourier_solve<double>(t, 0, 0.0, t->div.p, phi, false);
+    fourier_solve<double>(t, 0, 0.0, q, phi, false, 1, 1.0 / (t->h * step));
   } else {
-    fourier_solve<float>(t, 0, 0.0, t->div.p, phi, false);
+    gmk::kernel_launch_adjust(1);
+    k_tg_div<<<grid_for(nn), PT, 0, st>>>(n, t->h, 1.0 / step, q, t->div.p);
+    fourier_solve<float>(t, 0, 0.0, t->div.p, phi, false, 1, 0.0);
     for (int sweep = 0; sweep < 8; ++sweep) {
-      TG_CK(cudaMemsetAsync(t->red.p + 4, 0, sizeof(unsigned long long), st));
+      TG_CK(cudaMemsetAsync(t->red.p + RED_PRES, 0, sizeof(unsigned long long), st));
       gmk::kernel_launch_adjust(1);
-      k_tg_pres<<<grid_for(nn), PT, 0, st>>>(n, t->h, t->div.p, phi, t->work.p, t->red.p + 4);
-      if (bitsd(read_max(t, 4)) * step <= 1e-11) break;
-      fourier_solve<float>(t, 0, 0.0, t->work.p, phi, true);
+      k_tg_pres<<<grid_for(nn), PT, 0, st>>>(n, t->h, t->div.p, phi, t->work.p, t->red.p + RED_PRES);
+      if (bitsd(read_red(t)[RED_PRES]) * step <= 1e-11) break;
+      fourier_solve<float>(t, 0, 0.0, t->work.p, phi, true, 1, 0.0);
     }
   }
+  if (!out) return;
   gmk::kernel_launch_adjust(1);
-  k_tg_update<<<(unsigned)((2 * nn + PT - 1) / PT), PT, 0, st>>>(n, t->h, step, q, phi, out);
+  (t->precision ? k_tg_update<false> : k_tg_update<true>)<<<blocks_of(nn), PT, 0, st>>>(n, stencil_consts(t, 0.0), step,
+                                                                                    step / t->h, q, phi, out, t->red.p, gate_step);
 }
 
-// star = H^-1 rhs (two components), refined in FP32 mode to the CN gate
+// star = H^-1 rhs (two components), refined in FP32 mode to the CN gate; the residual of star and
+// max |rhs| go to RED_CN, RED_RHS
 void tg_helmholtz(gm_tg* t, double dt, const double* rhs, double* star) {
   const int n = t->n;
   const int64_t nn = (int64_t)n * n;
   cudaStream_t st = t->st;
   const double c = 0.5 * dt * t->nu;
-  for (int comp = 0; comp < 2; ++comp) {
-    if (t->precision == 0) fourier_solve<double>(t, 1, c, rhs + comp * nn, star + comp * nn, false);
-    else fourier_solve<float>(t, 1, c, rhs + comp * nn, star + comp * nn, false);
-  }
-  if (t->precision == 1) {
-    for (int sweep = 0; sweep < 6; ++sweep) {
-      TG_CK(cudaMemsetAsync(t->red.p, 0, 2 * sizeof(unsigned long long), st));
+  auto residual = [&](double* r) {
+    gmk::kernel_launch_adjust(1);
+    (t->precision ? k_tg_hres<false> : k_tg_hres<true>)<<<grid_for(2 * nn), PT, 0, st>>>(n, stencil_consts(t, dt), rhs, star,
+                                                                                       r, t->red.p);
+  };
+  if (t->precision == 0) {
+    if (t->sym_dt != dt) {
       gmk::kernel_launch_adjust(1);
-      k_tg_hres<<<grid_for(2 * nn), PT, 0, st>>>(n, t->h, t->nu, 0.5 * dt, rhs, star, t->work.p, t->red.p, t->red.p + 1);
-      unsigned long long v[2];
-      TG_CK(cudaMemcpyAsync(v, t->red.p, sizeof v, cudaMemcpyDeviceToHost, st));
-      TG_CK(cudaStreamSynchronize(st));
-      if (bitsd(v[0]) <= 32 * 2.220446049250313e-16 * std::max(1.0, bitsd(v[1]))) break;
-      for (int comp = 0; comp < 2; ++comp) fourier_solve<float>(t, 1, c, t->work.p + comp * nn, star + comp * nn, true);
+      k_tg_symbol<<<grid_for((int64_t)n * (n / 2 + 1)), PT, 0, st>>>(n, t->s2_64.p, 1, t->h * t->h, c, t->sym_h.p);
+      t->sym_dt = dt;
     }
+    fourier_solve<double>(t, 1, c, rhs, star, false, 1, 0.0);
+    residual(nullptr);
+    return;
   }
+  fourier_solve<float>(t, 1, c, rhs, star, false, 2, 0.0);
+  for (int sweep = 0; sweep < 6; ++sweep) {
+    TG_CK(cudaMemsetAsync(t->red.p, 0, 2 * sizeof(unsigned long long), st));
+    residual(t->work.p);
+    const unsigned long long* v = read_red(t);
+    if (bitsd(v[0]) <= 32 * 2.220446049250313e-16 * std::max(1.0, bitsd(v[1]))) return;  // star is the residual's
+    fourier_solve<float>(t, 1, c, t->work.p, star, true, 2, 0.0);
+  }
+  TG_CK(cudaMemsetAsync(t->red.p, 0, 2 * sizeof(unsigned long long), st));
+  residual(nullptr);
 }
 
-// ab2_cn_step (solver/time_integration.py:7-145) with the periodic operators
-void tg_step(gm_tg* t, double dt, double* max_div) {
+// ab2_cn_step (solver/time_integration.py:7-145) with the periodic operators, queued on the
+// stream; `step` counts from 1 in the call.  The FP64 steps behind a failed CN gate leave the
+// state alone (see k_tg_update), the FP32 mode reads its refinement residuals on the host.
+void tg_step(gm_tg* t, double dt, int step) {
   const int n = t->n;
   const int64_t nn = (int64_t)n * n;
   cudaStream_t st = t->st;
-  const unsigned g2 = (unsigned)((2 * nn + PT - 1) / PT);
+  const double h = t->h;
   auto rhs_kernel = [&](int mode, double alpha, const double* qh, double* out) {
     gmk::kernel_launch_adjust(1);
-    if (t->precision == 1)
-      k_tg_rhs<float><<<g2, PT, 0, st>>>(n, t->h, t->nu, mode, dt, alpha, t->q.p, qh, t->phalf.p, t->hist.p, t->now.p,
-                                         out);
-    else
-      k_tg_rhs<double><<<g2, PT, 0, st>>>(n, t->h, t->nu, mode, dt, alpha, t->q.p, qh, t->phalf.p, t->hist.p,
-                                          t->now.p, out);
+    if (t->precision == 1) {
+      k_tg_rhs<float><<<blocks_of(2 * nn), PT, 0, st>>>(n, h, t->nu, mode, dt, alpha, t->q.p, qh, t->phalf.p, t->hist.p,
+                                                        t->now.p, out);
+      return;
+    }
+    const double e = mode == 1 ? 0.5 * dt : dt;  // the start-up midpoint goes half a step with the full L q
+    const TgRhsC c{-0.25 / h, (mode == 1 ? 1.0 : 0.5) * e * t->nu / (h * h), e / h, e * (1 + alpha), e * alpha};
+    auto* k = mode == 0 ? k_tg_rhs64<0> : mode == 1 ? k_tg_rhs64<1> : k_tg_rhs64<2>;
+    k<<<blocks_of(nn), PT, 0, st>>>(n, c, t->q.p, qh, t->phalf.p, t->hist.p, t->now.p, out, t->red.p);
   };
   const bool first = !t->has_history;
   if (first) {
     rhs_kernel(1, 0.0, nullptr, t->mid.p);
-    tg_project(t, t->mid.p, 0.5 * dt, t->half_q.p, t->phi.p);
+    tg_project(t, t->mid.p, 0.5 * dt, t->half_q.p, t->phi.p, 0);
     rhs_kernel(2, 0.0, t->half_q.p, t->rhs.p);
   } else {
     rhs_kernel(0, dt / (2 * t->prev_dt), nullptr, t->rhs.p);
   }
   tg_helmholtz(t, dt, t->rhs.p, t->star.p);
-  // CN gate: max |H star - rhs| <= 1e-10 max(1, max |rhs|)  (solver/time_integration.py:100-104)
-  TG_CK(cudaMemsetAsync(t->red.p, 0, 5 * sizeof(unsigned long long), st));
+  tg_project(t, t->star.p, dt, t->qn.p, t->phi.p, step);
   gmk::kernel_launch_adjust(1);
-  k_tg_hres<<<grid_for(2 * nn), PT, 0, st>>>(n, t->h, t->nu, 0.5 * dt, t->rhs.p, t->star.p, nullptr, t->red.p,
-                                             t->red.p + 1);
-  unsigned long long v[2];
-  TG_CK(cudaMemcpyAsync(v, t->red.p, sizeof v, cudaMemcpyDeviceToHost, st));
-  TG_CK(cudaStreamSynchronize(st));
-  t->last_cn_residual = bitsd(v[0]);
-  if (!std::isfinite(bitsd(v[0])) || bitsd(v[0]) > 1e-10 * std::max(1.0, bitsd(v[1])))
-    throw TgError(GM_ERUNTIME, "CN momentum solve failed: residual=" + std::to_string(bitsd(v[0])));
-  tg_project(t, t->star.p, dt, t->qn.p, t->phi.p);
-  gmk::kernel_launch_adjust(1);
-  k_tg_defect<<<g2, PT, 0, st>>>(n, t->h, t->nu, 0.5 * dt, t->qn.p, t->rhs.p, t->action.p, t->proj.p);
-  tg_project(t, t->proj.p, dt, t->work.p, t->inc.p);
+  (t->precision ? k_tg_defect<false> : k_tg_defect<true>)<<<grid_for(nn), PT, 0, st>>>(
+      n, stencil_consts(t, dt), t->qn.p, t->rhs.p, t->action.p, t->proj.p, t->red.p);
+  tg_project(t, t->proj.p, dt, nullptr, t->inc.p, 0);
   const double factor = first ? 1.0 : dt / (dt + t->prev_dt);
   gmk::kernel_launch_adjust(1);
-  k_tg_pout<<<grid_for(2 * nn), PT, 0, st>>>(n, t->h, dt, factor, t->phalf.p, t->inc.p, t->action.p, t->rhs.p,
-                                             t->phalf_n.p, t->pout.p, t->red.p + 3);
-  TG_CK(cudaMemsetAsync(t->red.p + 2, 0, sizeof(unsigned long long), st));
-  gmk::kernel_launch_adjust(1);
-  k_tg_div<<<grid_for(nn), PT, 0, st>>>(n, t->h, 1.0, t->qn.p, nullptr, t->red.p + 2);
-  unsigned long long r[2];
-  TG_CK(cudaMemcpyAsync(r, t->red.p + 2, sizeof r, cudaMemcpyDeviceToHost, st));
-  TG_CK(cudaStreamSynchronize(st));
-  *max_div = std::max(*max_div, bitsd(r[0]));
-  t->last_coupled = bitsd(r[1]);
+  (t->precision ? k_tg_pout<false> : k_tg_pout<true>)<<<grid_for(nn), PT, 0, st>>>(
+      n, stencil_consts(t, dt), dt, dt / h, factor, t->phalf.p, t->inc.p, t->action.p, t->rhs.p, t->phalf_n.p, t->pout.p,
+      t->red.p);
+  TG_CK(cudaGetLastError());
+}
+
+void tg_swap(gm_tg* t) {
   std::swap(t->q.p, t->qn.p);
   std::swap(t->phalf.p, t->phalf_n.p);
   std::swap(t->hist.p, t->now.p);
-  t->has_history = true;
-  t->prev_dt = dt;
+}
+
+// n_steps steps; the largest divergence of any of them raises *max_div.  A failed CN gate leaves the
+// state after the last good step.
+void tg_steps(gm_tg* t, double dt, int n_steps, double* max_div) {
+  const bool had = t->has_history;
+  const double prev = t->prev_dt;
+  TG_CK(cudaMemsetAsync(t->red.p, 0, 8 * sizeof(unsigned long long), t->st));
+  const unsigned long long* r = t->host_red;
+  int done = 0, err = 0;
+  for (; done < n_steps && !err; ++done) {
+    tg_step(t, dt, done + 1);
+    tg_swap(t);
+    t->has_history = true;
+    t->prev_dt = dt;
+    if (t->precision == 1 || done + 1 == n_steps || (done + 1) % 64 == 0)
+      err = (int)read_red(t)[RED_ERR];
+  }
+  if (err) {
+    if ((done - (err - 1)) % 2) tg_swap(t);  // step err failed: the state is that after err - 1 steps
+    if (err == 1) { t->has_history = had; t->prev_dt = prev; }
+    throw TgError(GM_ERUNTIME, "CN momentum solve failed: residual=" + std::to_string(bitsd(r[RED_CN])));
+  }
+  *max_div = std::max(*max_div, bitsd(r[RED_DIV]));
 }
 
 int tg_guard(gm_tg* t, const std::function<void()>& f) {
@@ -539,36 +775,51 @@ int gm_tg_create(int32_t n, double nu, int32_t precision, gm_tg** out) {
     std::vector<float> s2f(s2.begin(), s2.end());
     t->s2_32.alloc(n);
     TG_CK(cudaMemcpy(t->s2_32.p, s2f.data(), n * sizeof(float), cudaMemcpyHostToDevice));
-    t->smem = tg_row_smem<double>(n, t->plan.tw_len);
-    t->smem32 = tg_row_smem<float>(n, t->plan.tw_len);
     int optin = 0;
     TG_CK(cudaDeviceGetAttribute(&optin, cudaDevAttrMaxSharedMemoryPerBlockOptin, 0));
-    if (t->smem > (size_t)optin) throw TgError(GM_EVALUE, "grid too large for the row transforms");
+    int dyn = optin;
     // the limit is a process-wide attribute of the kernel shared by every handle: the device
     // maximum, so that a smaller handle created later cannot lower it below a larger one's need
-    for (auto f : {(const void*)k_tg_rows<double, 0>, (const void*)k_tg_rows<double, 1>, (const void*)k_tg_rows<double, 2>,
-                   (const void*)k_tg_rows<float, 0>, (const void*)k_tg_rows<float, 1>, (const void*)k_tg_rows<float, 2>}) {
+    for (auto f : {(const void*)k_tg_rows_fwd<float, LINE_REAL>, (const void*)k_tg_rows_fwd<double, LINE_PAIR>,
+                   (const void*)k_tg_rows_fwd<double, LINE_UV>, (const void*)k_tg_rows_inv<float, LINE_REAL>,
+                   (const void*)k_tg_rows_inv<double, LINE_PAIR>, (const void*)k_tg_rows_inv<double, LINE_UV>,
+                   (const void*)k_tg_cols<float>, (const void*)k_tg_cols<double>}) {
       cudaFuncAttributes fa;
       TG_CK(cudaFuncGetAttributes(&fa, f));
-      const int dyn = optin - (int)fa.sharedSizeBytes;
-      if (t->smem > (size_t)dyn) throw TgError(GM_EVALUE, "grid too large for the row transforms");
-      TG_CK(cudaFuncSetAttribute(f, cudaFuncAttributeMaxDynamicSharedMemorySize, dyn));
+      const int d = optin - (int)fa.sharedSizeBytes;
+      dyn = std::min(dyn, d);
+      TG_CK(cudaFuncSetAttribute(f, cudaFuncAttributeMaxDynamicSharedMemorySize, d));
     }
-    t->threads = std::min(512, std::max(64, ((n / 4 + 31) / 32) * 32));
+    if (tg_smem<double>(n, t->plan.tw_len, 1) > (size_t)dyn) throw TgError(GM_EVALUE, "grid too large for the row transforms");
+    // a thread per radix-8 butterfly of a transform, and up to four transforms a block (64-byte
+    // column pieces in FP64) while a block stays within 512 threads and half of the shared memory
+    t->gt = std::min(512, std::max(32, ((n / 8 + 31) / 32) * 32));
+    for (int d = 0; d < 2; ++d) {
+      auto need = [&](int g) { return d ? tg_smem<double>(n, t->plan.tw_len, g) : tg_smem<float>(n, t->plan.tw_len, g); };
+      for (int g : {2, 4})
+        if (t->gt * g <= 512 && need(g) <= (size_t)dyn) t->gpb[d] = g;
+      t->smem[d] = need(t->gpb[d]);
+    }
     const int64_t nn = (int64_t)n * n;
     for (Buf<double>* b : {&t->q, &t->qn, &t->hist, &t->now, &t->rhs, &t->star, &t->mid, &t->half_q, &t->action,
                            &t->proj, &t->work}) {
       b->alloc(2 * nn);
       TG_CK(cudaMemset(b->p, 0, 2 * nn * sizeof(double)));
     }
-    for (Buf<double>* b : {&t->phalf, &t->phalf_n, &t->pout, &t->phi, &t->inc, &t->div, &t->real64}) {
+    for (Buf<double>* b : {&t->phalf, &t->phalf_n, &t->pout, &t->phi, &t->inc, &t->div}) {
       b->alloc(nn);
       TG_CK(cudaMemset(b->p, 0, nn * sizeof(double)));
     }
-    t->real32.alloc(nn);
-    t->cbuf_a.alloc((size_t)nn * 16);
-    t->cbuf_b.alloc((size_t)nn * 16);
+    t->spec.alloc((size_t)nn * 16);
+    if (precision == 0) {
+      t->sym_p.alloc((size_t)n * (n / 2 + 1));
+      t->sym_h.alloc((size_t)n * (n / 2 + 1));
+      k_tg_symbol<<<grid_for((int64_t)n * (n / 2 + 1)), PT, 0, t->st>>>(n, t->s2_64.p, 0, t->h * t->h, 0.0, t->sym_p.p);
+      gmk::kernel_launch_adjust(1);
+      TG_CK(cudaGetLastError());
+    }
     t->red.alloc(8);
+    TG_CK(cudaMallocHost(&t->host_red, 8 * sizeof(unsigned long long)));
     TG_CK(cudaMemset(t->red.p, 0, 8 * sizeof(unsigned long long)));
   });
   if (rc != GM_OK) { g_tg_create_error = t->err; return rc; }
@@ -619,7 +870,7 @@ int gm_tg_step(gm_tg* t, double dt, int32_t n_steps, double* max_divergence) {
   }
   return tg_guard(t, [&] {
     double md = max_divergence ? *max_divergence : 0.0;
-    for (int s = 0; s < n_steps; ++s) tg_step(t, dt, &md);
+    tg_steps(t, dt, n_steps, &md);
     if (max_divergence) *max_divergence = md;
   });
 }

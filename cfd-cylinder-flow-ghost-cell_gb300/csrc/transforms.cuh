@@ -151,6 +151,24 @@ __device__ __forceinline__ void stage_fixed(const cplx<T>* __restrict__ in, cplx
                                             int nfft, int Ns, unsigned magic, const cplx<T>* __restrict__ tw,
                                             const Grp& G) {
   const int MR = M / R;
+  if (sizeof(T) == 8 && Ns == 1) {
+    // first stage: every twiddle is one.  Leaving the products out takes 4 (R - 1) of a radix-8
+    // butterfly's 80 FP64 instructions, which the FP64 row passes are bound by (the FP64 400x200
+    // step 347 -> 343 us; the FP32 passes are not, and the second copy of the stage cost them 0.6 %)
+    for (int f = 0; f < nfft; ++f) {
+      const cplx<T>* src = in + (size_t)f * M;
+      cplx<T>* dst = out + (size_t)f * M;
+      for (int j = G.tid; j < MR; j += G.n) {
+        cplx<T> v[R];
+#pragma unroll
+        for (int r = 0; r < R; ++r) v[r] = src[j + r * MR];
+        dft_small<T, R>(v, DIR);
+#pragma unroll
+        for (int q = 0; q < R; ++q) dst[j * R + q] = v[q];
+      }
+    }
+    return;
+  }
   for (int f = 0; f < nfft; ++f) {
     const cplx<T>* src = in + (size_t)f * M;
     cplx<T>* dst = out + (size_t)f * M;
