@@ -164,6 +164,9 @@ struct gm_handle {
   DBuf<double> inlet;
   Csrd gf, gp, irr[3];
   DBuf<int32_t> a_nnz;
+  DBuf<NearCell> near_c;       // points next to ghost values (NearCell, NearFace)
+  DBuf<NearFace> near_f;
+  bool forces_read_ghosts = false;  // a force stencil reads a ghost pressure (none does by construction)
   DBuf<int64_t> sp_ptr, sp_col, su_ptr, su_col, sv_ptr, sv_col, d_ui, d_vi, d_pi;
   DBuf<double> sp_val, su_val, sv_val, nwx, nwy, nxx, nyy;
   DBuf<double> surf_part;      // per-point force terms
@@ -936,6 +939,8 @@ void fill_case_dev(gm_handle* h) {
   c.inlet = h->inlet.p;
   c.n_ghost_f = h->gf.n; c.gf_rows = h->gf.rows.p; c.gf_ptr = h->gf.ptr.p; c.gf_col = h->gf.col.p; c.gf_val = h->gf.val.p;
   c.n_ghost_p = h->gp.n; c.gp_rows = h->gp.rows.p; c.gp_ptr = h->gp.ptr.p; c.gp_col = h->gp.col.p; c.gp_val = h->gp.val.p;
+  c.n_near_c = (int)h->near_c.n; c.near_c = h->near_c.p;
+  c.n_near_f = (int)h->near_f.n; c.near_f = h->near_f.p;
   for (int k = 0; k < 3; ++k) {
     c.n_irr[k] = h->irr[k].n; c.irr_rows[k] = h->irr[k].rows.p; c.irr_ptr[k] = h->irr[k].ptr.p;
     c.irr_index[k] = h->irr[k].index.p;
@@ -959,6 +964,36 @@ void fill_case_dev(gm_handle* h) {
   c.fiarea = (float)c.iarea; c.fnu = (float)c.nu; c.fgx = (float)c.gx; c.fgy = (float)c.gy;
 }
 
+// The points that read ghost values (NearCell, NearFace).
+void near_points(const gm::Geometry& g, std::vector<NearCell>& nc, std::vector<NearFace>& nf) {
+  const int nx = g.nx, ny = g.ny;
+  const int32_t vrow0 = (int32_t)g.gu_rows.size();  // v rows follow the u rows in the extension operator
+  auto u = [&](int j, int i) { const int f = j * (nx + 1) + i, r = g.ghost_of_u[f]; return r >= 0 ? r : ~f; };
+  auto v = [&](int j, int i) {
+    const int f = j * nx + i, r = g.ghost_of_v[f];
+    return r >= 0 ? vrow0 + r : ~(int32_t)(g.usize + f);
+  };
+  auto p = [&](int j, int i) { const int k = j * nx + i, r = g.ghost_of_p[k]; return r >= 0 ? r : ~k; };
+  for (int j = 0; j < ny; ++j)
+    for (int i = 0; i < nx; ++i) {
+      if (!g.act_p[(size_t)j * nx + i]) continue;
+      const NearCell c{j * nx + i, {u(j, i + 1), u(j, i), v(j + 1, i), v(j, i)}};
+      if (std::max(std::max(c.code[0], c.code[1]), std::max(c.code[2], c.code[3])) >= 0) nc.push_back(c);
+    }
+  for (int j = 0; j < ny; ++j)
+    for (int i = 1; i <= nx; ++i) {
+      if (!g.act_u[(size_t)j * (nx + 1) + i]) continue;
+      const NearFace f{j * (nx + 1) + i, {p(j, i - 1), i < nx ? p(j, i) : NEAR_OUTLET}};
+      if (std::max(f.code[0], f.code[1]) >= 0) nf.push_back(f);
+    }
+  for (int j = 1; j < ny; ++j)
+    for (int i = 0; i < nx; ++i) {
+      if (!g.act_v[(size_t)j * nx + i]) continue;
+      const NearFace f{(int32_t)(g.usize + (int64_t)j * nx + i), {p(j - 1, i), p(j, i)}};
+      if (std::max(f.code[0], f.code[1]) >= 0) nf.push_back(f);
+    }
+}
+
 void build_class_maps(gm_handle* h) {
   const gm::Geometry& g = h->g;
   std::vector<uint8_t> cu(g.usize), cv(g.vsize), cp(g.psize);
@@ -970,6 +1005,11 @@ void build_class_maps(gm_handle* h) {
     for (int64_t r : h->hs.rows_irr[0]) cu[r] |= CLS_IRREG;
     for (int64_t r : h->hs.rows_irr[1]) cv[r] |= CLS_IRREG;
   }
+  std::vector<NearCell> nc;
+  std::vector<NearFace> nf;
+  near_points(g, nc, nf);
+  for (const NearCell& c : nc) cp[c.cell] |= CLS_NEAR;
+  for (const NearFace& f : nf) (f.face < g.usize ? cu[f.face] : cv[f.face - g.usize]) |= CLS_NEAR;
   std::vector<uint8_t> cf(cu);
   cf.insert(cf.end(), cv.begin(), cv.end());
   if (h->cls_f.n != cf.size()) h->cls_f.alloc(cf.size());
@@ -1550,33 +1590,31 @@ struct SolveCall {  // one monitored solve (the arguments of schur_solve)
 void solve_call(gm_handle* h, const SolveCall& c) {
   schur_solve(h, c.lane, *c.rd, c.kind, 0.0, c.b, c.x, c.res, c.first, c.w2, c.slot);
 }
-SolveCall project_pre(gm_handle* h, double* q, double dt, double* phi, int slot) {
-  cudaStream_t st = h->st;
-  Gate g0 = gate_of(h);
-  launch_set_inlet(h->cd, q, false, st);
-  ghost_faces(h, q, g0);
-  launch_divergence(h->cd, q, h->prhs.p, dt, nullptr, nullptr, 1, g0, st);
+SolveCall project_pre(gm_handle* h, const double* q, double dt, double* phi, int slot, ProjCheck chk) {
+  launch_proj_rhs(h->cd, q, h->prhs.p, dt, chk, h->nchk, gate_of(h), h->st);
   return SolveCall{0, &h->rp, 0, h->prhs.p, phi, h->pres.p, h->pfirst.p, h->pw2.p, slot};
 }
-void project_post(gm_handle* h, double* q, double dt, double* out, double* phi, int slot, int divk) {
+// up to the projected velocity `out` (its ghost values and the divergence check follow in
+// launch_proj_tail)
+void project_post(gm_handle* h, const double* q, double dt, double* out, double* phi, int slot) {
   cudaStream_t st = h->st;
-  Gate g0 = gate_of(h);
   if (h->rec_rhs && !h->capturing && h->rec_count < h->rec_cap) {
     const size_t off = (size_t)h->rec_count * h->Pn;
     CK(cudaMemcpyAsync(h->rec_rhs + off, h->prhs.p, h->Pn * sizeof(double), cudaMemcpyDeviceToDevice, st));
     CK(cudaMemcpyAsync(h->rec_sol + off, phi, h->Pn * sizeof(double), cudaMemcpyDeviceToDevice, st));
     ++h->rec_count;
   }
-  launch_gate_pressure(h->ctl.p, slot, h->nchk, st);
-  ghost_p(h, phi, g0);
-  launch_project_update(h->cd, q, phi, dt, out, nullptr, g0, st);
-  ghost_faces(h, out, g0);
-  launch_divergence(h->cd, out, nullptr, 0.0, nullptr, &h->ctl.p->div_max[divk], 0, g0, st);
-  launch_gate_projection(h->ctl.p, divk, st);
+  launch_proj_update(h->cd, q, phi, dt, out, slot, h->nchk, gate_of(h), st);
 }
-void project(gm_handle* h, double* q, double dt, double* out, double* phi, int slot, int divk) {
-  solve_call(h, project_pre(h, q, dt, phi, slot));
-  project_post(h, q, dt, out, phi, slot, divk);
+// a projection by itself, its gate included (div_max[divk])
+void project(gm_handle* h, const double* q, double dt, double* out, double* phi, int slot, int divk) {
+  solve_call(h, project_pre(h, q, dt, phi, slot, PCHK_NONE));
+  project_post(h, q, dt, out, phi, slot);
+  TailArgs ta{};
+  ta.U = out;
+  ta.divmax = &h->ctl.p->div_max[divk];
+  launch_proj_tail(h->cd, h->rcoef[1], h->rcoef[2], TAIL_PLAIN, ta, gate_of(h), h->st);
+  launch_gate_projection(h->ctl.p, divk, h->st);
 }
 
 // Jacobi tables of the FP32 mode's Helmholtz solves for the current dt: 1 / diagonal per
@@ -1886,19 +1924,17 @@ void step_phase0(gm_handle* h, double dt, int screen, SolveCall calls[2]) {
   cudaStream_t st = h->st;
   phase_mark(h, 0, st);
   Gate g0 = gate_of(h);
-  const size_t keep = offsetof(StepCtl, solve);
-  CK(cudaMemsetAsync(reinterpret_cast<char*>(h->ctl.p) + keep, 0, sizeof(StepCtl) - keep, st));
-  launch_cfl_screen(h->ctl.p, &h->state_max.p[0], &h->state_max.p[1], dt, h->g.dx, h->g.dy, screen, h->counter.p, st);
   const bool first = !h->has_history;
-  // pressure at the previous half step: the stored half pressure, or p at active cells
-  // when there is no history (solver/optimized_ghost_cell.py:256); ghost values for G p
-  if (first) launch_copy_active(h->cls_p.p, h->Pn, h->pout.p, h->phalf.p, g0, st);
-  ghost_p(h, h->phalf.p, g0);
   MomentumArgs ma{};
   ma.U = h->U.p;
   ma.P = h->phalf.p;
   ma.dt = dt;
   if (first) {
+    launch_cfl_screen(h->ctl.p, &h->state_max.p[0], &h->state_max.p[1], dt, h->g.dx, h->g.dy, screen, h->counter.p, st);
+    // pressure at the previous half step: p at active cells when there is no history
+    // (solver/optimized_ghost_cell.py:256); ghost values for G p
+    launch_copy_active(h->cls_p.p, h->Pn, h->pout.p, h->phalf.p, g0, st);
+    ghost_p(h, h->phalf.p, g0);
     ma.mode = 1;
     ma.now = h->now.p;
     ma.out = h->fmid.p;
@@ -1910,16 +1946,18 @@ void step_phase0(gm_handle* h, double dt, int screen, SolveCall calls[2]) {
     ma.out = h->rhs.p;
     momentum(h, ma, g0);
   } else {
+    // the stored half pressure has its ghost values: the previous step's end, or gm_set_history,
+    // filled them; the CFL screen runs in the momentum kernel
     ma.mode = 0;
     ma.alpha = dt / (2 * h->prev_dt);
     ma.prev = h->hist.p;
     ma.now = h->now.p;
     ma.out = h->rhs.p;
-    if (h->precision == 1) {
-      launch_shadow(h->U.p, h->U32.p, h->F, h->phalf.p, h->P32.p, h->Pn, g0, st);
-      ma.U32 = h->U32.p;
-      ma.P32 = h->P32.p;
-    }
+    ma.U32 = h->U32.p;
+    ma.P32 = h->P32.p;
+    ma.state_max = h->state_max.p;
+    ma.counter = h->counter.p;
+    ma.screen = screen;
     momentum(h, ma, g0);
   }
   phase_mark(h, 1, st);
@@ -1935,37 +1973,52 @@ SolveCall step_phase1(gm_handle* h) {
   cudaStream_t st = h->st;
   CK(cudaEventRecord(h->ev_join, h->st2));
   CK(cudaStreamWaitEvent(st, h->ev_join, 0));
-  launch_gate_momentum(h->ctl.p, h->nchk, st);
   phase_mark(h, 2, st);
-  // projection of the CN velocity, defect correction and the pressure increment
-  return project_pre(h, h->star.p, h->step_dt, h->pphi.p, S_P1);
+  // projection of the CN velocity (behind its momentum gate), defect correction and the pressure increment
+  return project_pre(h, h->star.p, h->step_dt, h->pphi.p, S_P1, PCHK_MOMENTUM);
 }
 SolveCall step_phase2(gm_handle* h) {
   cudaStream_t st = h->st;
   const double dt = h->step_dt;
-  project_post(h, h->star.p, dt, h->Unext.p, h->pphi.p, S_P1, 1);
+  project_post(h, h->star.p, dt, h->Unext.p, h->pphi.p, S_P1);
   phase_mark(h, 3, st);
-  launch_defect(h->cd, h->rcoef[1], h->rcoef[2], h->Unext.p, h->rhs.p, h->faction.p, h->fproj.p, gate_of(h), st);
+  TailArgs ta{};
+  ta.U = h->Unext.p;
+  ta.divmax = &h->ctl.p->div_max[1];
+  ta.rhs = h->rhs.p;
+  ta.action = h->faction.p;
+  ta.proj = h->fproj.p;
+  launch_proj_tail(h->cd, h->rcoef[1], h->rcoef[2], TAIL_DEFECT, ta, gate_of(h), st);
   phase_mark(h, 4, st);
-  return project_pre(h, h->fproj.p, dt, h->pinc.p, S_P2);
+  return project_pre(h, h->fproj.p, dt, h->pinc.p, S_P2, PCHK_PROJECTION);
 }
 void step_phase3(gm_handle* h) {
   cudaStream_t st = h->st;
   const double dt = h->step_dt;
   Gate g0 = gate_of(h);
-  project_post(h, h->fproj.p, dt, h->fproj2.p, h->pinc.p, S_P2, 2);
+  project_post(h, h->fproj.p, dt, h->fproj2.p, h->pinc.p, S_P2);
   phase_mark(h, 5, st);
-  // pinc already carries its ghost values: project_post extended it, and the extension rows
-  // read active cells only, so extending it again would rewrite the same values
-  const bool first = !h->has_history;
-  double factor = first ? 1.0 : dt / (dt + h->prev_dt);
-  launch_pressure_out(h->cd, h->phalf.p, h->pinc.p, factor, dt, h->faction.p, h->rhs.p, h->phalf_next.p, h->pout.p,
-                      &h->ctl.p->coupled_max, g0, st);
-  ghost_p(h, h->pout.p, g0);
-  // diagnostics on the new state, forces and the step gates (solver/main.py:383-415)
-  launch_maxabs(h->cd, h->Unext.p, &h->ctl.p->umax, &h->ctl.p->vmax, g0, st);
-  launch_forces(h->cd, h->Unext.p, h->pout.p, h->g.nu * h->g.rho, dt, h->ctl.p, 1, nullptr, g0, st);
-  launch_step_end(h->ctl.p, h->state_max.p, h->ring.p, h->ridx.p, h->counter.p, gm_handle::RING_CAP, st);
+  TailArgs ta{};
+  ta.U = h->fproj2.p;
+  ta.divmax = &h->ctl.p->div_max[2];
+  ta.rhs = h->rhs.p;
+  ta.action = h->faction.p;
+  ta.p = h->phalf.p;
+  ta.inc = h->pinc.p;
+  ta.unew = h->Unext.p;
+  ta.half = h->phalf_next.p;
+  ta.pout = h->pout.p;
+  ta.factor = !h->has_history ? 1.0 : dt / (dt + h->prev_dt);
+  ta.dgx = dt * h->cd.gx;
+  ta.dgy = dt * h->cd.gy;
+  ta.coupled = &h->ctl.p->coupled_max;
+  ta.umax = &h->ctl.p->umax;
+  launch_proj_tail(h->cd, h->rcoef[1], h->rcoef[2], TAIL_PRESSURE, ta, g0, st);
+  // ghost values of the new pressures, forces, the step gates (solver/main.py:383-415), the record
+  if (h->forces_read_ghosts) ghost_p(h, h->pout.p, g0);
+  const StepTail tail{h->pout.p, h->phalf_next.p, h->Unext.p, h->g.nu * h->g.rho, dt, h->state_max.p,
+                      h->ring.p, h->ridx.p, h->counter.p, gm_handle::RING_CAP};
+  launch_step_tail(h->cd, tail, g0, st);
   phase_mark(h, 6, st);
   CK(cudaGetLastError());
 }
@@ -2171,6 +2224,14 @@ void create_device(gm_handle* H) {
   upload_csr(H->irr[0], g.a_rows, g.a_irr, st);
   upload_row_index(H->irr[0], g.a_rows, g.psize, st);
   H->a_nnz.upload(g.a_nnz_row, st);
+  {
+    std::vector<NearCell> nc;
+    std::vector<NearFace> nf;
+    near_points(g, nc, nf);
+    H->near_c.upload(nc, st);
+    H->near_f.upload(nf, st);
+    for (int64_t k : g.surf_p.col) H->forces_read_ghosts = H->forces_read_ghosts || g.ghost_of_p[k] >= 0;
+  }
   H->sp_ptr.upload(g.surf_p.ptr, st); H->sp_col.upload(g.surf_p.col, st); H->sp_val.upload(g.surf_p.val, st);
   H->su_ptr.upload(g.dudn.ptr, st); H->su_col.upload(g.dudn.col, st); H->su_val.upload(g.dudn.val, st);
   H->sv_ptr.upload(g.dvdn.ptr, st); H->sv_col.upload(g.dvdn.col, st); H->sv_val.upload(g.dvdn.val, st);
@@ -2588,6 +2649,7 @@ int gm_set_history(gm_handle* h, int32_t has_history, const double* prev_adv, co
     const double* ph = dev_in(h, 1, half_p, np);
     CK(cudaMemsetAsync(h->phalf.p, 0, h->Pn * sizeof(double), st));
     launch_scatter(ph, h->d_pi.p, np, h->phalf.p, st);
+    ghost_p(h, h->phalf.p, Gate{nullptr, 0, 0});
     CK(cudaStreamSynchronize(st));
     h->has_history = true;
     h->prev_dt = prev_dt;
@@ -2729,7 +2791,7 @@ int gm_apply(gm_handle* h, int32_t op, double param, const double* x, double* y)
       case GM_OP_DIVERGENCE: {
         const double* q = dev_in(h, 0, x, nq);
         unpack_into(q, h->ftmp.p);
-        launch_divergence(h->cd, h->ftmp.p, h->ptmp.p, 0.0, nullptr, nullptr, 0, g0, st);
+        launch_divergence(h->cd, h->ftmp.p, h->ptmp.p, st);
         DevOut o(h, 1, y, np);
         launch_gather(h->ptmp.p, h->d_pi.p, np, o.dev, st);
         o.finish();
@@ -2851,7 +2913,7 @@ int gm_surface_forces(gm_handle* h, const double* u, const double* v, const doub
     const double* pd = dev_in(h, 2, p, g.psize);
     DBuf<double> o6;
     o6.alloc(6);
-    launch_forces(h->cd, h->ftmp.p, pd, mu, 0.0, nullptr, 0, o6.p, Gate{nullptr, 0, 0}, st);
+    launch_forces(h->cd, h->ftmp.p, pd, mu, o6.p, st);
     CK(cudaMemcpyAsync(out, o6.p, 6 * sizeof(double), cudaMemcpyDeviceToHost, st));
     CK(cudaStreamSynchronize(st));
   });

@@ -107,6 +107,7 @@ static int pdl_mode() {
   }
   return mode;
 }
+// A kernel behind a conditional node or a join of two streams is launched plainly.
 template <typename... KArgs, typename... Args>
 static void launch_pdl(void (*kernel)(KArgs...), dim3 grid, dim3 block, size_t smem, cudaStream_t st,
                        Args&&... args) {
@@ -973,6 +974,45 @@ __device__ __forceinline__ void csr_row(const int64_t* __restrict__ col, const d
   }
 }
 
+// ---- the gates of a step (each raises the sticky error word; none clears it) ----
+__device__ void check_momentum(StepCtl* ctl, int nchk) {
+  double r = 0, bm = 0;
+  bool bad = false;
+  for (int s = 0; s < 2; ++s) {
+    const SolveCtl* sc = &ctl->solve[s];
+    double rr = bits2d(sc->rmax[last_check(sc, nchk)]);
+    double bb = bits2d(sc->bmax);
+    if (!(rr <= r)) r = rr;  // propagates NaN
+    if (bb > bm) bm = bb;
+    if (sc->xbad) bad = true;
+  }
+  double thr = 1e-10 * (bm > 1.0 ? bm : 1.0);
+  if (bad || !(r <= thr)) raise_gate(ctl, 2, 2);
+}
+__device__ void check_pressure(StepCtl* ctl, int slot, int nchk) {
+  const SolveCtl* sc = &ctl->solve[slot];
+  int k = last_check(sc, nchk);
+  double linf = bits2d(sc->rmax[k]), bound = bits2d(sc->bound[k]), bm = bits2d(sc->bmax);
+  if (!isfinite(bm)) { raise_gate(ctl, 1, 4); return; }  // solver/pressure_schur.py:33-34
+  double t = 64 * EPS64 * (bm > 1.0 ? bm : 1.0);
+  t = t > 1e-10 ? t : 1e-10;
+  t = bound > t ? bound : t;
+  if (sc->xbad || !(linf <= t)) raise_gate(ctl, 2, 3);
+}
+__device__ __forceinline__ bool projection_ok(const StepCtl* ctl, int k) { return bits2d(ctl->div_max[k]) <= 1e-10; }
+__device__ void check_projection(StepCtl* ctl, int k) {
+  if (!projection_ok(ctl, k)) raise_gate(ctl, 2, 1);
+}
+// CFL screen of solver/main.py:273-278 (screen != 0; < 0: every 100th step by the counter) and the
+// finite-field check of solver/time_integration.py:15-17 on the velocity maxima of the current state
+__device__ void check_cfl(StepCtl* ctl, const unsigned long long* umax, const unsigned long long* vmax, double dt,
+                          double dx, double dy, int screen, const long long* counter) {
+  if (screen < 0) screen = (*counter % 100) == 0;
+  double rate = bits2d(*umax) / dx + bits2d(*vmax) / dy;
+  if (screen && (!isfinite(rate) || dt * rate > 0.5)) raise_gate(ctl, 2, 7);
+  else if (!isfinite(rate)) raise_gate(ctl, 1, 8);
+}
+
 // ---------------------------------------------------------------------------
 // ghost extension rows
 // ---------------------------------------------------------------------------
@@ -980,15 +1020,21 @@ __device__ __forceinline__ void csr_row(const int64_t* __restrict__ col, const d
 // entries are spread over GHOST_LANES lanes, so its loads take one or two rounds instead of a
 // serial chain through L2, and the lanes' partial sums are added in a fixed butterfly order.
 constexpr int GHOST_LANES = 8;
+// Row r by the eight lanes l = 0..7 (r < 0: no row, zero); every lane of the warp calls it.
+__device__ __forceinline__ double ghost_row(const double* __restrict__ f, const int64_t* __restrict__ ptr,
+                                            const int64_t* __restrict__ col, const double* __restrict__ val, int r, int l) {
+  double acc = 0.0;
+  if (r >= 0)
+    for (int64_t e = ptr[r] + l, e1 = ptr[r + 1]; e < e1; e += GHOST_LANES) acc += val[e] * f[col[e]];
+  for (int o = GHOST_LANES / 2; o; o >>= 1) acc += __shfl_xor_sync(0xffffffffu, acc, o);
+  return acc;
+}
 __global__ void k_ghost(double* __restrict__ f, int n, const int64_t* __restrict__ rows, const int64_t* __restrict__ ptr,
                         const int64_t* __restrict__ col, const double* __restrict__ val, Gate gate) {
   if (!gate_open(gate)) return;
   const int t = blockIdx.x * blockDim.x + threadIdx.x;
   const int r = t / GHOST_LANES, l = t % GHOST_LANES;
-  double acc = 0.0;
-  if (r < n)
-    for (int64_t e = ptr[r] + l, e1 = ptr[r + 1]; e < e1; e += GHOST_LANES) acc += val[e] * f[col[e]];
-  for (int o = GHOST_LANES / 2; o; o >>= 1) acc += __shfl_xor_sync(0xffffffffu, acc, o);
+  const double acc = ghost_row(f, ptr, col, val, r < n ? r : -1, l);
   if (r < n && l == 0) f[rows[r]] = acc;
 }
 
@@ -1110,6 +1156,8 @@ __device__ __forceinline__ bool face_of(int64_t t, const Grid& g, int& comp, int
 template <typename T, typename S>
 __global__ void k_momentum(CaseDev c, MomentumArgs a, const S* __restrict__ Us, const S* __restrict__ Ps, Gate gate) {
   if (!gate_open(gate)) return;
+  if (a.state_max && blockIdx.x + threadIdx.x == 0)
+    check_cfl(gate.ctl, a.state_max, a.state_max + 1, a.dt, c.dx, c.dy, a.screen, a.counter);
   const Grid g{c.nx, c.ny, c.usize};
   int64_t t = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
   int comp, j, i;
@@ -1193,9 +1241,11 @@ struct TileGrid {
   __device__ __forceinline__ int p(int j, int i) const { return (j - j0 + 1) * WP + (i - i0 + 1); }
 };
 
+// The FP32 mode converts as it fills the tiles (integer pipe; the halo points twice): a kernel that
+// wrote FP32 copies of the state first took 12 us of the 800x820 step, and its own launch.
 template <typename T, typename S>
-__global__ void __launch_bounds__(MTI * MTJ) k_momentum_tiled(CaseDev c, MomentumArgs a, const S* __restrict__ Us,
-                                                              const S* __restrict__ Ps, Gate gate) {
+__global__ void __launch_bounds__(MTI * MTJ) k_momentum_tiled(CaseDev c, MomentumArgs a, const double* __restrict__ Us,
+                                                              const double* __restrict__ Ps, Gate gate) {
   constexpr int W = TileGrid::W, H = TileGrid::H, WP = TileGrid::WP;
   __shared__ S suv[2 * H * W];
   __shared__ S sp[(MTJ + 1) * WP];
@@ -1204,6 +1254,9 @@ __global__ void __launch_bounds__(MTI * MTJ) k_momentum_tiled(CaseDev c, Momentu
   __shared__ T xu[MTJ * (MTI + 1)];        // Xu at (j0 + r, i0 + q)
   __shared__ T yv[(MTJ + 1) * MTI];        // Yv at (j0 + r, i0 + q)
   if (!gate_open(gate)) return;
+  // a raised screen stops every kernel behind this one, whose outputs are scratch until the step ends
+  if (a.state_max && blockIdx.x + blockIdx.y + threadIdx.x + threadIdx.y == 0)
+    check_cfl(gate.ctl, a.state_max, a.state_max + 1, a.dt, c.dx, c.dy, a.screen, a.counter);
   const int nx = c.nx, ny = c.ny;
   const int j0 = blockIdx.y * MTJ, i0 = blockIdx.x * MTI;
   const int tid = threadIdx.y * MTI + threadIdx.x;
@@ -1213,13 +1266,13 @@ __global__ void __launch_bounds__(MTI * MTJ) k_momentum_tiled(CaseDev c, Momentu
   for (int e = tid; e < H * W; e += MTI * MTJ) {
     const int r = e / W, q = e - r * W;
     const int j = j0 - 1 + r, i = i0 - 1 + q;
-    suv[e] = (j >= 0 && j < ny && i >= 0 && i <= nx) ? Us[g.u(j, i)] : (S)0;
-    suv[H * W + e] = (j >= 0 && j <= ny && i >= 0 && i < nx) ? Us[g.v(j, i)] : (S)0;
+    suv[e] = (j >= 0 && j < ny && i >= 0 && i <= nx) ? cvt_to<S>(Us[g.u(j, i)]) : (S)0;
+    suv[H * W + e] = (j >= 0 && j <= ny && i >= 0 && i < nx) ? cvt_to<S>(Us[g.v(j, i)]) : (S)0;
   }
   for (int e = tid; e < (MTJ + 1) * WP; e += MTI * MTJ) {
     const int r = e / WP, q = e - r * WP;
     const int j = j0 - 1 + r, i = i0 - 1 + q;
-    sp[e] = (j >= 0 && j < ny && i >= 0 && i < nx) ? Ps[g.p(j, i)] : (S)0;
+    sp[e] = (j >= 0 && j < ny && i >= 0 && i < nx) ? cvt_to<S>(Ps[g.p(j, i)]) : (S)0;
   }
   __syncthreads();
   constexpr bool F32 = sizeof(T) == 4;
@@ -1352,15 +1405,17 @@ void launch_momentum_f32(const CaseDev& c, const MomentumArgs& a_in, const Gate&
   MomentumArgs a = a_in;
   a.dt32 = (float)a.dt;
   a.alpha32 = (float)a.alpha;
+  const bool tiled = momentum_tiled(), shadow = a.mode == 0 && !tiled;
+  if (shadow) launch_shadow(a.U, a.U32, c.usize + c.vsize, a.P, a.P32, c.psize, gate, st);
   note_launch();
   kt_mark(3, st);
-  if (a.mode == 0 && a.U32 && a.P32 && momentum_tiled())
-    launch_pdl(k_momentum_tiled<float, float>, dim3(momentum_tiles(c)), dim3(dim3(MTI, MTJ)), 0, st, c, a, a.U32, a.P32, gate);
-  else if (a.mode == 0 && a.U32 && a.P32)
+  if (a.mode == 0 && tiled)
+    launch_pdl(k_momentum_tiled<float, float>, dim3(momentum_tiles(c)), dim3(dim3(MTI, MTJ)), 0, st, c, a, a.U, a.P, gate);
+  else if (shadow)
     launch_pdl(k_momentum<float, float>, dim3(blocks_for(c.usize + c.vsize)), dim3(TPB), 0, st, c, a, a.U32, a.P32, gate);
   else
     launch_pdl(k_momentum<float, double>, dim3(blocks_for(c.usize + c.vsize)), dim3(TPB), 0, st, c, a, a.U, a.P, gate);
-  kt_mark(3, st);
+  kt_mark(3, st, (double)(c.usize + c.vsize) * (8 * 4 + 1) + (double)c.psize * 8);
 }
 
 __global__ void k_advection(CaseDev c, const double* __restrict__ U, double* __restrict__ out, Gate gate) {
@@ -2071,53 +2126,145 @@ void launch_learned_apply(const CaseDev& c, const float* y, const unsigned long 
 // ---------------------------------------------------------------------------
 // projection pieces
 // ---------------------------------------------------------------------------
-// D U at the active cells: its max |.| into divmax and/or, scaled, into out.  The scaled
-// output takes its coefficients sx = idx s, sy = idy s from the host (s = 1/dt or 1), so it
-// costs no more FP64 work than the divergence itself.
-__global__ void k_divergence(CaseDev c, const double* __restrict__ U, double* __restrict__ out, double sx, double sy,
-                             unsigned long long* divmax, int gate_nonfinite, StepCtl* ctl, Gate gate) {
-  if (!gate_open(gate)) return;
+// D U at the active cells (the operator; the projection's kernels are below)
+__global__ void k_divergence(CaseDev c, const double* __restrict__ U, double* __restrict__ out) {
   const Grid g{c.nx, c.ny, c.usize};
-  unsigned long long dm = 0;
-  bool bad = false;
   for (int64_t t = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; t < c.psize; t += (int64_t)gridDim.x * blockDim.x) {
     if (c.cls_p[t] & CLS_ACTIVE) {
       int j = (int)((unsigned)t / (unsigned)c.nx), i = (int)((unsigned)t - (unsigned)j * c.nx);
       const double du = U[g.u(j, i + 1)] - U[g.u(j, i)], dv = U[g.v(j + 1, i)] - U[g.v(j, i)];
-      if (divmax) dm = umax64(dm, absbits(du * c.idx + dv * c.idy));
-      if (out) {
-        const double o = du * sx + dv * sy;
-        out[t] = o;
-        bad = bad || nonfinite_bits(o);
-      }
-    } else if (out) {
+      out[t] = du * c.idx + dv * c.idy;
+    } else {
       out[t] = 0.0;
     }
   }
-  if (gate_nonfinite && bad && ctl) raise_gate(ctl, 1, 4);
-  if (divmax) block_commit_max(dm, divmax);
 }
-void launch_divergence(const CaseDev& c, const double* U, double* out, double scale, SolveCtl* sc,
-                       unsigned long long* divmax, int gate_on_nonfinite, const Gate& gate, cudaStream_t st) {
-  (void)sc;
+void launch_divergence(const CaseDev& c, const double* U, double* out, cudaStream_t st) {
   note_launch();
   kt_mark(6, st);
-  const double s = scale != 0.0 ? 1.0 / scale : 1.0;
-  launch_pdl(k_divergence, dim3(reduce_blocks(c.psize)), dim3(TPB), 0, st, c, U, out, c.idx * s, c.idy * s, divmax, gate_on_nonfinite,
-                                                      gate.ctl, gate);
+  k_divergence<<<reduce_blocks(c.psize), TPB, 0, st>>>(c, U, out);
+  kt_mark(6, st);
+}
+
+// ---- the projection ------------------------------------------------------------------------
+// Each kernel is small (at 800x820 the grid passes take 8-13 us, at 96x48 about 4), so what a
+// projection costs beside its solve is mostly the number of dependent kernels.  The ghost values
+// therefore need none: the few points that read one (CLS_NEAR; about 400 at 800x820) go to the
+// first blocks, eight lanes a ghost row in the order of k_ghost, and the gates sit in the first block
+// of the kernel behind them.  A projection was nine kernels around its solve, now three;
+// with the momentum kernel taking the CFL screen and the step's end one kernel of five, the step went from
+// 259 to 220 us at 96x48, 347 to 309 at 400x200, 924 to 850 (FP64) and 584 to 531 (FP32) at 800x820.
+
+// differences of the near cell's face values, on lane 0 of the warp (all lanes call)
+__device__ __forceinline__ void near_diff(const CaseDev& c, const double* __restrict__ U, const NearCell& nc, double& du,
+                                          double& dv) {
+  const int lane = threadIdx.x & 31, l = lane % GHOST_LANES;
+  const int32_t code = nc.code[lane / GHOST_LANES];
+  double v = ghost_row(U, c.gf_ptr, c.gf_col, c.gf_val, code, l);
+  if (code < 0 && l == 0) {
+    const int f = ~code;
+    v = (f < c.usize && f % (c.nx + 1) == 0) ? c.inlet[f / (c.nx + 1)] : U[f];
+  }
+  const double e = __shfl_sync(0xffffffffu, v, 0), w = __shfl_sync(0xffffffffu, v, GHOST_LANES);
+  const double n = __shfl_sync(0xffffffffu, v, 2 * GHOST_LANES), s = __shfl_sync(0xffffffffu, v, 3 * GHOST_LANES);
+  du = e - w;
+  dv = n - s;
+}
+static inline int near_cell_blocks(const CaseDev& c) { return (c.n_near_c + TPB / 32 - 1) / (TPB / 32); }
+static inline int ghost_blocks(int n) { return (int)blocks_for((int64_t)n * GHOST_LANES); }
+
+__global__ void k_proj_rhs(CaseDev c, const double* __restrict__ U, double* __restrict__ out, double sx, double sy,
+                           int chk, int nchk, int nbn, Gate gate) {
+  if (!gate_open(gate)) return;
+  if (chk && blockIdx.x + threadIdx.x == 0) {
+    if (chk == PCHK_MOMENTUM) check_momentum(gate.ctl, nchk);
+    else check_projection(gate.ctl, 1);
+  }
+  const Grid g{c.nx, c.ny, c.usize};
+  bool bad = false;
+  if ((int)blockIdx.x < nbn) {
+    const int w = (blockIdx.x * TPB + threadIdx.x) >> 5;
+    if (w >= c.n_near_c) return;
+    double du, dv;
+    near_diff(c, U, c.near_c[w], du, dv);
+    if ((threadIdx.x & 31) == 0) {
+      const double o = du * sx + dv * sy;
+      out[c.near_c[w].cell] = o;
+      bad = nonfinite_bits(o);
+    }
+  } else {
+    for (int64_t t = (int64_t)(blockIdx.x - nbn) * TPB + threadIdx.x; t < c.psize; t += (int64_t)(gridDim.x - nbn) * TPB) {
+      const uint8_t k = c.cls_p[t];
+      if (k & CLS_NEAR) continue;
+      double o = 0.0;
+      if (k & CLS_ACTIVE) {
+        const int j = (int)((unsigned)t / (unsigned)c.nx), i = (int)((unsigned)t - (unsigned)j * c.nx);
+        const double uw = i > 0 ? U[g.u(j, i)] : c.inlet[j];
+        const double du = U[g.u(j, i + 1)] - uw, dv = U[g.v(j + 1, i)] - U[g.v(j, i)];
+        o = du * sx + dv * sy;
+        bad = bad || nonfinite_bits(o);
+      }
+      out[t] = o;
+    }
+  }
+  if (bad && gate.ctl) {
+    // the gate in front comes first, whichever thread gets here first
+    if (chk == PCHK_MOMENTUM) check_momentum(gate.ctl, nchk);
+    else if (chk == PCHK_PROJECTION) check_projection(gate.ctl, 1);
+    raise_gate(gate.ctl, 1, 4);
+  }
+}
+void launch_proj_rhs(const CaseDev& c, const double* U, double* out, double dt, ProjCheck chk, int nchk, const Gate& gate,
+                     cudaStream_t st) {
+  const int nbn = near_cell_blocks(c);
+  const double s = 1.0 / dt;
+  note_launch();
+  kt_mark(6, st);
+  const dim3 grid((unsigned)nbn + reduce_blocks(c.psize));
+  const int check = gate.ctl ? (int)chk : 0;
+  if (chk == PCHK_MOMENTUM) k_proj_rhs<<<grid, TPB, 0, st>>>(c, U, out, c.idx * s, c.idy * s, check, nchk, nbn, gate);
+  else launch_pdl(k_proj_rhs, grid, dim3(TPB), 0, st, c, U, out, c.idx * s, c.idy * s, check, nchk, nbn, gate);
   kt_mark(6, st);
 }
 
 // out = q - dt G phi at the active faces, with dgx = dt gx and dgy = dt gy formed on the host:
-// two fused multiply-adds per face (G phi is gx (phi_e - phi_w), at the outlet -2 gx phi_w)
-__global__ void k_project_update(CaseDev c, const double* __restrict__ q, const double* __restrict__ phi, double dgx,
-                                 double dgy, double* __restrict__ out, Gate gate) {
+// two fused multiply-adds per face (G phi is gx (phi_e - phi_w), at the outlet -2 gx phi_w).
+// Blocks: nbf of near faces (16 lanes a face), nbg that fill phi's ghost values, then the grid.
+__global__ void k_proj_update(CaseDev c, const double* __restrict__ q, double* phi, double dgx, double dgy,
+                              double* __restrict__ out, int slot, int nchk, int nbf, int nbg, Gate gate) {
   if (!gate_open(gate)) return;
+  if (gate.ctl && blockIdx.x + threadIdx.x == 0) check_pressure(gate.ctl, slot, nchk);
   const Grid g{c.nx, c.ny, c.usize};
-  int64_t t = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
+  const int b = blockIdx.x;
+  if (b < nbf) {
+    const int lane = threadIdx.x & 31, w = ((b * TPB + threadIdx.x) >> 5) * 2 + (lane >> 4);
+    const bool in = w < c.n_near_f;
+    NearFace nf{0, {NEAR_OUTLET, NEAR_OUTLET}};
+    if (in) nf = c.near_f[w];
+    const int l = lane % GHOST_LANES;
+    const int32_t code = nf.code[(lane >> 3) & 1];
+    double v = ghost_row(phi, c.gp_ptr, c.gp_col, c.gp_val, code, l);
+    if (code < 0 && code != NEAR_OUTLET && l == 0) v = phi[~code];
+    const double hi = __shfl_down_sync(0xffffffffu, v, GHOST_LANES);
+    if (in && (lane & 15) == 0) {
+      const int t = nf.face;
+      if (t >= c.usize) out[t] = fma(dgy, v, fma(-dgy, hi, q[t]));
+      else if (nf.code[1] != NEAR_OUTLET) out[t] = fma(dgx, v, fma(-dgx, hi, q[t]));
+      else out[t] = fma(2.0 * dgx, v, q[t]);
+    }
+    return;
+  }
+  if (b < nbf + nbg) {
+    const int t = (b - nbf) * TPB + threadIdx.x, r = t / GHOST_LANES, l = t % GHOST_LANES;
+    const double v = ghost_row(phi, c.gp_ptr, c.gp_col, c.gp_val, r < c.n_ghost_p ? r : -1, l);
+    if (r < c.n_ghost_p && l == 0) phi[c.gp_rows[r]] = v;
+    return;
+  }
+  const int64_t t = (int64_t)(b - nbf - nbg) * TPB + threadIdx.x;
   int comp, j, i;
   if (!face_of(t, g, comp, j, i)) return;
   const uint8_t cls = comp == 0 ? c.cls_u[t] : c.cls_v[t - c.usize];
+  if (cls & CLS_NEAR) return;
   if (!(cls & CLS_ACTIVE)) {
     out[t] = (comp == 0 && i == 0) ? c.inlet[j] : 0.0;
     return;
@@ -2126,12 +2273,13 @@ __global__ void k_project_update(CaseDev c, const double* __restrict__ q, const 
   else if (i < c.nx) out[t] = fma(dgx, phi[g.p(j, i - 1)], fma(-dgx, phi[g.p(j, i)], q[t]));
   else out[t] = fma(2.0 * dgx, phi[g.p(j, c.nx - 1)], q[t]);
 }
-void launch_project_update(const CaseDev& c, const double* q, const double* phi, double dt, double* out,
-                           const SolveCtl* psolve, const Gate& gate, cudaStream_t st) {
-  (void)psolve;
+void launch_proj_update(const CaseDev& c, const double* q, double* phi, double dt, double* out, int slot, int nchk,
+                        const Gate& gate, cudaStream_t st) {
+  const int nbf = (c.n_near_f + TPB / 16 - 1) / (TPB / 16), nbg = ghost_blocks(c.n_ghost_p);
   note_launch();
   kt_mark(6, st);
-  launch_pdl(k_project_update, dim3(blocks_for(c.usize + c.vsize)), dim3(TPB), 0, st, c, q, phi, dt * c.gx, dt * c.gy, out, gate);
+  k_proj_update<<<(unsigned)(nbf + nbg) + blocks_for(c.usize + c.vsize), TPB, 0, st>>>(c, q, phi, dt * c.gx, dt * c.gy, out,
+                                                                                       slot, nchk, nbf, nbg, gate);
   kt_mark(6, st);
 }
 
@@ -2176,78 +2324,128 @@ __device__ __forceinline__ double helm_action(const CaseDev& c, const ResidualCo
   return fma(rc.cy, xs + xn, fma(rc.ce, xe, fma(cwv, xw, ccv * x[f])));
 }
 
-// Defect correction of the CN velocity (solver/time_integration.py): action = H r and
-// proj = r + (rhs - H r) at the active faces; inlet values and zeros elsewhere.
-__global__ void k_defect(CaseDev c, ResidualCoef rcu, ResidualCoef rcv, const double* __restrict__ r,
-                         const double* __restrict__ rhs, double* __restrict__ action, double* __restrict__ proj,
-                         Gate gate) {
-  if (!gate_open(gate)) return;
-  const Grid g{c.nx, c.ny, c.usize};
-  int64_t t = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
-  int comp, j, i;
-  if (!face_of(t, g, comp, j, i)) return;
-  const uint8_t cls = comp == 0 ? c.cls_u[t] : c.cls_v[t - c.usize];
-  if (!(cls & CLS_ACTIVE)) {
-    action[t] = 0.0;
-    proj[t] = (comp == 0 && i == 0) ? c.inlet[j] : 0.0;
-    return;
+// Block-wide maxima of N words (block_commit_max for several, two barriers in all).
+template <int N>
+__device__ void block_commit_maxes(unsigned long long (&v)[N], unsigned long long* const (&dst)[N]) {
+  __shared__ unsigned long long sm[N][32];
+  const int lane = threadIdx.x & 31, wid = threadIdx.x >> 5;
+#pragma unroll
+  for (int q = 0; q < N; ++q) {
+    v[q] = warp_max_u64(v[q]);
+    if (lane == 0) sm[q][wid] = v[q];
   }
-  const double hr = comp == 0 ? helm_action<1>(c, rcu, r, t, cls) : helm_action<2>(c, rcv, r, t - c.usize, cls);
-  action[t] = hr;
-  proj[t] = r[t] + (rhs[t] - hr);
-}
-void launch_defect(const CaseDev& c, const ResidualCoef& rcu, const ResidualCoef& rcv, const double* result,
-                   const double* rhs, double* action, double* proj, const Gate& gate, cudaStream_t st) {
-  note_launch();
-  kt_mark(7, st);
-  launch_pdl(k_defect, dim3(blocks_for(c.usize + c.vsize)), dim3(TPB), 0, st, c, rcu, rcv, result, rhs, action, proj, gate);
-  kt_mark(7, st);
+  __syncthreads();
+  if (wid < N) {
+    unsigned long long x = 0;
+    unsigned long long* d = nullptr;
+#pragma unroll
+    for (int q = 0; q < N; ++q)
+      if (wid == q) {
+        x = lane < (int)(blockDim.x >> 5) ? sm[q][lane] : 0ull;
+        d = dst[q];
+      }
+    x = warp_max_u64(x);
+    if (lane == 0 && x && d) atomicMax(d, x);
+  }
 }
 
-__global__ void k_pressure_out(CaseDev c, const double* __restrict__ p, const double* __restrict__ inc, double factor,
-                               double dgx, double dgy, const double* __restrict__ action, const double* __restrict__ rhs,
-                               double* __restrict__ half, double* __restrict__ pout, unsigned long long* coupled,
-                               Gate gate) {
+// What follows a projection (TailArgs), one pass over the grids.  Blocks: nbn of near cells, nbg that
+// fill U's ghost values (no other block reads them here: the defect's rows hold active faces only),
+// then the grid.
+//   DEFECT    the defect correction of the CN velocity (solver/time_integration.py): action = H U and
+//             proj = U + (rhs - H U) at the active faces; inlet values and zeros elsewhere
+//   PRESSURE  half = p + inc, pout = half + factor inc, max |action - rhs + dt G inc|, and the maxima of
+//             the new velocity over the whole grids
+template <int KIND>
+__global__ void k_proj_tail(CaseDev c, ResidualCoef rcu, ResidualCoef rcv, TailArgs a, int nbn, int nbg, Gate gate) {
   if (!gate_open(gate)) return;
   const Grid g{c.nx, c.ny, c.usize};
-  int64_t nf = c.usize + c.vsize;
-  unsigned long long cm = 0;
-  for (int64_t t = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; t < nf + c.psize;
-       t += (int64_t)gridDim.x * blockDim.x) {
-  if (t < nf) {
-    int comp, j, i;
-    face_of(t, g, comp, j, i);
-    const uint8_t cls = comp == 0 ? c.cls_u[t] : c.cls_v[t - c.usize];
-    if (cls & CLS_ACTIVE) {
-      // action - rhs + dt G inc, with dgx = dt gx and dgy = dt gy formed on the host
-      const double a0 = action[t] - rhs[t];
-      double r;
-      if (comp == 1) r = fma(-dgy, inc[g.p(j - 1, i)], fma(dgy, inc[g.p(j, i)], a0));
-      else if (i < c.nx) r = fma(-dgx, inc[g.p(j, i - 1)], fma(dgx, inc[g.p(j, i)], a0));
-      else r = fma(-2.0 * dgx, inc[g.p(j, c.nx - 1)], a0);
-      cm = umax64(cm, absbits(r));
+  const int b = blockIdx.x;
+  double* U = a.U;
+  if (b < nbn) {
+    const int w = (b * TPB + threadIdx.x) >> 5;
+    if (w >= c.n_near_c) return;
+    double du, dv;
+    near_diff(c, U, c.near_c[w], du, dv);
+    if ((threadIdx.x & 31) == 0) {
+      const unsigned long long d = absbits(du * c.idx + dv * c.idy);
+      if (d) atomicMax(a.divmax, d);
     }
-  } else {
-    int64_t k = t - nf;
-    if (c.cls_p[k] & CLS_ACTIVE) {
-      double h = p[k] + inc[k];
-      half[k] = h;
-      pout[k] = h + factor * inc[k];
+    return;
+  }
+  if (b < nbn + nbg) {
+    const int t = (b - nbn) * TPB + threadIdx.x, r = t / GHOST_LANES, l = t % GHOST_LANES;
+    const double v = ghost_row(U, c.gf_ptr, c.gf_col, c.gf_val, r < c.n_ghost_f ? r : -1, l);
+    if (r < c.n_ghost_f && l == 0) U[c.gf_rows[r]] = v;
+    return;
+  }
+  const int64_t nf = c.usize + c.vsize, n = KIND == TAIL_PLAIN ? c.psize : nf + c.psize;
+  unsigned long long dm = 0, cm = 0, um = 0, vm = 0;
+  for (int64_t t = (int64_t)(b - nbn - nbg) * TPB + threadIdx.x; t < n; t += (int64_t)(gridDim.x - nbn - nbg) * TPB) {
+    if (KIND == TAIL_PLAIN || t >= nf) {
+      const int64_t k = KIND == TAIL_PLAIN ? t : t - nf;
+      const uint8_t cls = c.cls_p[k];
+      if (!(cls & CLS_ACTIVE)) {
+        if (KIND == TAIL_PRESSURE) a.half[k] = a.pout[k] = 0.0;
+        continue;
+      }
+      if (!(cls & CLS_NEAR)) {
+        const int j = (int)((unsigned)k / (unsigned)c.nx), i = (int)((unsigned)k - (unsigned)j * c.nx);
+        const double du = U[g.u(j, i + 1)] - U[g.u(j, i)], dv = U[g.v(j + 1, i)] - U[g.v(j, i)];
+        dm = umax64(dm, absbits(du * c.idx + dv * c.idy));
+      }
+      if (KIND == TAIL_PRESSURE) {
+        const double h = a.p[k] + a.inc[k];
+        a.half[k] = h;
+        a.pout[k] = h + a.factor * a.inc[k];
+      }
     } else {
-      half[k] = 0.0;
-      pout[k] = 0.0;
+      int comp, j, i;
+      face_of(t, g, comp, j, i);
+      const uint8_t cls = comp == 0 ? c.cls_u[t] : c.cls_v[t - c.usize];
+      if (KIND == TAIL_DEFECT) {
+        if (!(cls & CLS_ACTIVE)) {
+          a.action[t] = 0.0;
+          a.proj[t] = (comp == 0 && i == 0) ? c.inlet[j] : 0.0;
+          continue;
+        }
+        const double hr = comp == 0 ? helm_action<1>(c, rcu, U, t, cls) : helm_action<2>(c, rcv, U, t - c.usize, cls);
+        a.action[t] = hr;
+        a.proj[t] = U[t] + (a.rhs[t] - hr);
+      } else {
+        const unsigned long long x = absbits(a.unew[t]);
+        if (comp == 0) um = umax64(um, x);
+        else vm = umax64(vm, x);
+        if (!(cls & CLS_ACTIVE)) continue;
+        // action - rhs + dt G inc, with dgx = dt gx and dgy = dt gy formed on the host
+        const double a0 = a.action[t] - a.rhs[t];
+        double r;
+        if (comp == 1) r = fma(-a.dgy, a.inc[g.p(j - 1, i)], fma(a.dgy, a.inc[g.p(j, i)], a0));
+        else if (i < c.nx) r = fma(-a.dgx, a.inc[g.p(j, i - 1)], fma(a.dgx, a.inc[g.p(j, i)], a0));
+        else r = fma(-2.0 * a.dgx, a.inc[g.p(j, c.nx - 1)], a0);
+        cm = umax64(cm, absbits(r));
+      }
     }
   }
+  if (KIND == TAIL_PRESSURE) {
+    unsigned long long v[4] = {dm, cm, um, vm};
+    unsigned long long* const d[4] = {a.divmax, a.coupled, a.umax, a.umax + 1};
+    block_commit_maxes<4>(v, d);
+  } else {
+    block_commit_max(dm, a.divmax);
   }
-  block_commit_max(cm, coupled);
 }
-void launch_pressure_out(const CaseDev& c, const double* p, const double* inc, double factor, double dt,
-                         const double* action, const double* rhs, double* half, double* pout,
-                         unsigned long long* coupled, const Gate& gate, cudaStream_t st) {
+void launch_proj_tail(const CaseDev& c, const ResidualCoef& rcu, const ResidualCoef& rcv, ProjTail kind, const TailArgs& a,
+                      const Gate& gate, cudaStream_t st) {
+  const int nbn = near_cell_blocks(c), nbg = kind == TAIL_PRESSURE ? 0 : ghost_blocks(c.n_ghost_f);
+  const int64_t n = kind == TAIL_PLAIN ? c.psize : c.usize + c.vsize + c.psize;
+  // eight blocks an SM (a full one of threads): the passes wait on L2, the reductions are a block's end
+  const dim3 grid((unsigned)(nbn + nbg) + std::min(blocks_for(n), 1216u));
   note_launch();
   kt_mark(7, st);
-  launch_pdl(k_pressure_out, dim3(reduce_blocks(c.usize + c.vsize + c.psize)), dim3(TPB), 0, st, c, p, inc, factor, dt * c.gx, dt * c.gy,
-                                                                          action, rhs, half, pout, coupled, gate);
+  if (kind == TAIL_PLAIN) launch_pdl(k_proj_tail<TAIL_PLAIN>, grid, dim3(TPB), 0, st, c, rcu, rcv, a, nbn, nbg, gate);
+  else if (kind == TAIL_DEFECT) launch_pdl(k_proj_tail<TAIL_DEFECT>, grid, dim3(TPB), 0, st, c, rcu, rcv, a, nbn, nbg, gate);
+  else launch_pdl(k_proj_tail<TAIL_PRESSURE>, grid, dim3(TPB), 0, st, c, rcu, rcv, a, nbn, nbg, gate);
   kt_mark(7, st);
 }
 
@@ -2274,114 +2472,172 @@ void launch_maxabs(const CaseDev& c, const double* U, unsigned long long* umax, 
 // ---------------------------------------------------------------------------
 // surface forces (solver/optimized_ghost_cell.py:280-286) and step gates (solver/main.py:401-415)
 // ---------------------------------------------------------------------------
-__global__ void k_forces(CaseDev c, const double* __restrict__ U, const double* __restrict__ P, double mu, double dt,
-                         StepCtl* ctl, int check_gates, double* out6, Gate gate) {
-  if (!gate_open(gate)) return;
-  // one warp per quadrature point (lanes over the stencil nonzeros), the per-point terms go to
-  // c.surf_part; the last block to finish sums them in a fixed order (deterministic)
-  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5, wpb = blockDim.x >> 5;
-  const int k = blockIdx.x * wpb + warp;
-  if (k < c.n_surf) {
-    double ps = 0, du = 0, dv = 0;
-    for (int64_t e = c.sp_ptr[k] + lane; e < c.sp_ptr[k + 1]; e += 32) ps += c.sp_val[e] * P[c.sp_col[e]];
-    for (int64_t e = c.su_ptr[k] + lane; e < c.su_ptr[k + 1]; e += 32) du += c.su_val[e] * U[c.su_col[e]];
-    for (int64_t e = c.sv_ptr[k] + lane; e < c.sv_ptr[k + 1]; e += 32) dv += c.sv_val[e] * U[c.usize + c.sv_col[e]];
-    ps = warp_sum(ps);
-    du = warp_sum(du);
-    dv = warp_sum(dv);
-    if (lane == 0) {
-      const double nxk = c.nxx[k], nyk = c.nyy[k];
-      const double dn = du * nxk + dv * nyk;
-      double* o = c.surf_part + 4 * (int64_t)k;
-      o[0] = ps * c.nwx[k];
-      o[1] = ps * c.nwy[k];
-      o[2] = mu * (du + nxk * dn);
-      o[3] = mu * (dv + nyk * dn);
-    }
+// One warp a quadrature point (lanes over the stencils' nonzeros, the three rows' loads together):
+// its four force terms to c.surf_part.
+__device__ __forceinline__ void force_point(const CaseDev& c, const double* __restrict__ U, const double* __restrict__ P,
+                                            double mu, int k) {
+  const int lane = threadIdx.x & 31;
+  if (k >= c.n_surf) return;
+  const int64_t p0 = c.sp_ptr[k] + lane, p1 = c.sp_ptr[k + 1], u0 = c.su_ptr[k] + lane, u1 = c.su_ptr[k + 1];
+  const int64_t v0 = c.sv_ptr[k] + lane, v1 = c.sv_ptr[k + 1];
+  double ps = 0, du = 0, dv = 0;
+  for (int64_t e = 0; p0 + e < p1 || u0 + e < u1 || v0 + e < v1; e += 32) {
+    const bool bp = p0 + e < p1, bu = u0 + e < u1, bv = v0 + e < v1;
+    const double xp = bp ? P[c.sp_col[p0 + e]] : 0.0, xu = bu ? U[c.su_col[u0 + e]] : 0.0;
+    const double xv = bv ? U[c.usize + c.sv_col[v0 + e]] : 0.0;
+    if (bp) ps += c.sp_val[p0 + e] * xp;
+    if (bu) du += c.su_val[u0 + e] * xu;
+    if (bv) dv += c.sv_val[v0 + e] * xv;
   }
+  ps = warp_sum(ps);
+  du = warp_sum(du);
+  dv = warp_sum(dv);
+  if (lane == 0) {
+    const double nxk = c.nxx[k], nyk = c.nyy[k];
+    const double dn = du * nxk + dv * nyk;
+    double* o = c.surf_part + 4 * (int64_t)k;
+    o[0] = ps * c.nwx[k];
+    o[1] = ps * c.nwy[k];
+    o[2] = mu * (du + nxk * dn);
+    o[3] = mu * (dv + nyk * dn);
+  }
+}
+// Whether this block is the last of the grid to get here (the others' force terms are visible to it).
+__device__ __forceinline__ bool last_block(unsigned* ticket) {
   __threadfence();
   __syncthreads();
   __shared__ int last;
-  if (threadIdx.x == 0) last = atomicAdd(c.surf_ticket, 1u) == gridDim.x - 1;
+  if (threadIdx.x == 0) last = atomicAdd(ticket, 1u) == gridDim.x - 1;
   __syncthreads();
-  if (!last) return;
+  if (!last) return false;
   __threadfence();
+  return true;
+}
+// The six forces from the point terms, in a fixed order, by the first four warps (w: arc length a
+// point); on every thread after the barrier.
+__device__ __forceinline__ void force_sums(const CaseDev& c, double w, double (&f6)[6]) {
   __shared__ double red[4];
+  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
   if (warp < 4) {
     double acc = 0.0;
+#pragma unroll 4
     for (int q = lane; q < c.n_surf; q += 32) acc += __ldcg(c.surf_part + 4 * (int64_t)q + warp);
     acc = warp_sum(acc);
     if (lane == 0) red[warp] = acc;
   }
   __syncthreads();
+  const double fp[2] = {-red[0], -red[1]}, fv[2] = {red[2] * w, red[3] * w};
+  f6[0] = fp[0] + fv[0]; f6[1] = fp[1] + fv[1];
+  f6[2] = fp[0]; f6[3] = fp[1];
+  f6[4] = fv[0]; f6[5] = fv[1];
+}
+static inline double force_arc(const CaseDev& c) { return 3.141592653589793 * c.D / c.n_surf; }
+constexpr int FORCE_WPB = 8;
+
+__global__ void k_forces(CaseDev c, const double* __restrict__ U, const double* __restrict__ P, double mu, double w,
+                         double* out6) {
+  force_point(c, U, P, mu, (blockIdx.x * blockDim.x + threadIdx.x) >> 5);
+  if (!last_block(c.surf_ticket)) return;
+  double f6[6];
+  force_sums(c, w, f6);
   if (threadIdx.x == 0) {
     *c.surf_ticket = 0u;
-    const double PI = 3.141592653589793;
-    double w = PI * c.D / c.n_surf;
-    double fp[2] = {-red[0], -red[1]};
-    double fv[2] = {red[2] * w, red[3] * w};
-    double f6[6] = {fp[0] + fv[0], fp[1] + fv[1], fp[0], fp[1], fv[0], fv[1]};
-    if (out6)
-      for (int q = 0; q < 6; ++q) out6[q] = f6[q];
-    if (ctl) {
-      for (int q = 0; q < 6; ++q) ctl->forces[q] = f6[q];
-      double denom = ((0.5 * c.rho) * (c.U_ref * c.U_ref)) * c.D;
-      double cd = f6[0] / denom, cl = f6[1] / denom;
-      ctl->cd = cd;
-      ctl->cl = cl;
-      if (check_gates) {
-        if (!isfinite(cd) || !isfinite(cl)) {
-          raise_gate(ctl, 3, 6);
-        } else {
-          double div = bits2d(ctl->div_max[1]);
-          double cfl = dt * (bits2d(ctl->umax) / c.dx + bits2d(ctl->vmax) / c.dy);
-          if (!(div < 1e-10) || !(cfl < 0.5)) raise_gate(ctl, 2, 5);
-        }
-      }
-    }
+    for (int q = 0; q < 6; ++q) out6[q] = f6[q];
   }
 }
-void launch_forces(const CaseDev& c, const double* U, const double* P, double mu, double dt, StepCtl* ctl,
-                   int check_gates, double* out6, const Gate& gate, cudaStream_t st) {
+void launch_forces(const CaseDev& c, const double* U, const double* P, double mu, double* out6, cudaStream_t st) {
   note_launch();
   kt_mark(9, st);
-  const int wpb = 8;
-  launch_pdl(k_forces, dim3((c.n_surf + wpb - 1) / wpb), dim3(32 * wpb), 0, st, c, U, P, mu, dt, ctl, check_gates, out6, gate);
+  k_forces<<<(c.n_surf + FORCE_WPB - 1) / FORCE_WPB, 32 * FORCE_WPB, 0, st>>>(c, U, P, mu, force_arc(c), out6);
   kt_mark(9, st);
 }
 
-__global__ void k_gate_momentum(StepCtl* ctl, int nchk) {
-  if (ctl->err) return;
-  double r = 0, bm = 0;
-  bool bad = false;
-  for (int s = 0; s < 2; ++s) {
-    const SolveCtl* sc = &ctl->solve[s];
-    double rr = bits2d(sc->rmax[last_check(sc, nchk)]);
-    double bb = bits2d(sc->bmax);
-    if (!(rr <= r)) r = rr;  // propagates NaN
-    if (bb > bm) bm = bb;
-    if (sc->xbad) bad = true;
+// The step record: the control block to the ring, the new maxima to the state (a good step), the
+// counters, and the per-step part of the control block cleared for the next step.  One block.
+__device__ void step_end(StepCtl* ctl, const StepTail& a) {
+  __shared__ int slot, err;
+  __syncthreads();
+  if (threadIdx.x == 0) {
+    slot = min(*a.ridx, a.cap - 1);
+    err = *(volatile int*)&ctl->err;
+    if (!err) {
+      a.state_max[0] = ctl->umax;
+      a.state_max[1] = ctl->vmax;
+    }
   }
-  double thr = 1e-10 * (bm > 1.0 ? bm : 1.0);
-  if (bad || !(r <= thr)) raise_gate(ctl, 2, 2);
+  __syncthreads();
+  int* src = reinterpret_cast<int*>(ctl);
+  int* dst = reinterpret_cast<int*>(a.ring + slot);
+  constexpr int N = (int)(sizeof(StepCtl) / sizeof(int)), KEEP = (int)(offsetof(StepCtl, solve) / sizeof(int));
+  for (int i = threadIdx.x; i < N; i += blockDim.x) {
+    dst[i] = src[i];
+    if (!err && i >= KEEP) src[i] = 0;
+  }
+  if (threadIdx.x == 0) {
+    *a.ridx = slot + 1;
+    *a.counter = *a.counter + 1;
+  }
 }
-void launch_gate_momentum(StepCtl* ctl, int nchk, cudaStream_t st) {
+
+// The end of a step (StepTail): nbf blocks of force points, then blocks of both pressures' ghost rows;
+// the last to finish sums the forces, applies the step gates and writes the record.  (Pressure ghost
+// rows, maxima, forces, record and the next step's clearing of the control block were five launches.)
+__global__ void k_step_tail(CaseDev c, StepTail a, double w, double denom, int nbf, int nbg, Gate gate) {
+  StepCtl* ctl = gate.ctl;
+  const bool open = gate_open(gate);
+  if (!open || !projection_ok(ctl, 2)) {  // the same words for every block: all of them leave here
+    if (blockIdx.x == 0) {
+      if (open && threadIdx.x == 0) check_projection(ctl, 2);
+      step_end(ctl, a);
+    }
+    return;
+  }
+  const int b = blockIdx.x;
+  if (b < nbf) {
+    force_point(c, a.U, a.pout, a.mu, (b * blockDim.x + threadIdx.x) >> 5);
+  } else {
+    double* f = b < nbf + nbg ? a.pout : a.half;
+    const int t = (b - nbf - (b < nbf + nbg ? 0 : nbg)) * (int)blockDim.x + threadIdx.x, r = t / GHOST_LANES, l = t % GHOST_LANES;
+    const double v = ghost_row(f, c.gp_ptr, c.gp_col, c.gp_val, r < c.n_ghost_p ? r : -1, l);
+    if (r < c.n_ghost_p && l == 0) f[c.gp_rows[r]] = v;
+  }
+  if (!last_block(c.surf_ticket)) return;
+  double f6[6];
+  force_sums(c, w, f6);
+  // the four quotients on four lanes: one divide's latency instead of four
+  __shared__ double quot[4];
+  if (threadIdx.x < 4) {
+    const double um = bits2d(ctl->umax), vm = bits2d(ctl->vmax);
+    const double num = threadIdx.x == 0 ? f6[0] : threadIdx.x == 1 ? f6[1] : threadIdx.x == 2 ? um : vm;
+    quot[threadIdx.x] = num / (threadIdx.x < 2 ? denom : threadIdx.x == 2 ? c.dx : c.dy);
+  }
+  __syncthreads();
+  if (threadIdx.x == 0) {
+    *c.surf_ticket = 0u;
+    for (int q = 0; q < 6; ++q) ctl->forces[q] = f6[q];
+    const double cd = quot[0], cl = quot[1];
+    ctl->cd = cd;
+    ctl->cl = cl;
+    if (!isfinite(cd) || !isfinite(cl)) {
+      raise_gate(ctl, 3, 6);
+    } else {
+      const double div = bits2d(ctl->div_max[1]), cfl = a.dt * (quot[2] + quot[3]);
+      if (!(div < 1e-10) || !(cfl < 0.5)) raise_gate(ctl, 2, 5);
+    }
+  }
+  step_end(ctl, a);
+}
+void launch_step_tail(const CaseDev& c, const StepTail& a, const Gate& gate, cudaStream_t st) {
+  const int nbf = (c.n_surf + FORCE_WPB - 1) / FORCE_WPB, nbg = ghost_blocks(c.n_ghost_p);
   note_launch();
-  kt_mark(10, st);
-  k_gate_momentum<<<1, 1, 0, st>>>(ctl, nchk);
-  kt_mark(10, st);
+  kt_mark(9, st);
+  launch_pdl(k_step_tail, dim3((unsigned)std::max(1, nbf + 2 * nbg)), dim3(32 * FORCE_WPB), 0, st, c, a, force_arc(c),
+             ((0.5 * c.rho) * (c.U_ref * c.U_ref)) * c.D, nbf, nbg, gate);
+  kt_mark(9, st);
 }
 
 __global__ void k_gate_pressure(StepCtl* ctl, int slot, int nchk) {
-  if (ctl->err) return;
-  const SolveCtl* sc = &ctl->solve[slot];
-  int k = last_check(sc, nchk);
-  double linf = bits2d(sc->rmax[k]), bound = bits2d(sc->bound[k]), bm = bits2d(sc->bmax);
-  if (!isfinite(bm)) { raise_gate(ctl, 1, 4); return; }  // solver/pressure_schur.py:33-34
-  double t = 64 * EPS64 * (bm > 1.0 ? bm : 1.0);
-  t = t > 1e-10 ? t : 1e-10;
-  t = bound > t ? bound : t;
-  if (sc->xbad || !(linf <= t)) raise_gate(ctl, 2, 3);
+  if (!ctl->err) check_pressure(ctl, slot, nchk);
 }
 void launch_gate_pressure(StepCtl* ctl, int slot, int nchk, cudaStream_t st) {
   note_launch();
@@ -2391,9 +2647,7 @@ void launch_gate_pressure(StepCtl* ctl, int slot, int nchk, cudaStream_t st) {
 }
 
 __global__ void k_gate_projection(StepCtl* ctl, int k) {
-  if (ctl->err) return;
-  double d = bits2d(ctl->div_max[k]);
-  if (!(d <= 1e-10)) raise_gate(ctl, 2, 1);
+  if (!ctl->err) check_projection(ctl, k);
 }
 void launch_gate_projection(StepCtl* ctl, int k, cudaStream_t st) {
   note_launch();
@@ -2402,15 +2656,9 @@ void launch_gate_projection(StepCtl* ctl, int k, cudaStream_t st) {
   kt_mark(10, st);
 }
 
-// CFL screen of solver/main.py:273-278 (screen != 0) and the finite-field check of
-// solver/time_integration.py:15-17 on the velocity maxima of the current state.
 __global__ void k_cfl_screen(StepCtl* ctl, const unsigned long long* umax, const unsigned long long* vmax, double dt,
                              double dx, double dy, int screen, const long long* counter) {
-  if (ctl->err) return;
-  if (screen < 0) screen = (*counter % 100) == 0;
-  double rate = bits2d(*umax) / dx + bits2d(*vmax) / dy;
-  if (screen && (!isfinite(rate) || dt * rate > 0.5)) raise_gate(ctl, 2, 7);
-  else if (!isfinite(rate)) raise_gate(ctl, 1, 8);
+  if (!ctl->err) check_cfl(ctl, umax, vmax, dt, dx, dy, screen, counter);
 }
 void launch_cfl_screen(StepCtl* ctl, const unsigned long long* umax, const unsigned long long* vmax, double dt,
                        double dx, double dy, int screen, const long long* counter, cudaStream_t st) {
@@ -2558,34 +2806,6 @@ void launch_refine_decide(StepCtl* ctl, int slot, int nchk, cudaGraphConditional
   note_launch();
   kt_mark(10, st);
   k_refine_decide<<<1, 1, 0, st>>>(ctl, slot, nchk, cond);
-  kt_mark(10, st);
-}
-
-__global__ void k_step_end(StepCtl* ctl, unsigned long long* state_max, StepCtl* ring, int* ridx, long long* counter,
-                           int cap) {
-  __shared__ int slot;
-  if (threadIdx.x == 0) {
-    slot = min(*ridx, cap - 1);
-    if (!ctl->err) {
-      state_max[0] = ctl->umax;
-      state_max[1] = ctl->vmax;
-    }
-  }
-  __syncthreads();
-  const int* src = reinterpret_cast<const int*>(ctl);
-  int* dst = reinterpret_cast<int*>(ring + slot);
-  for (int i = threadIdx.x; i < (int)(sizeof(StepCtl) / sizeof(int)); i += blockDim.x) dst[i] = src[i];
-  __syncthreads();
-  if (threadIdx.x == 0) {
-    *ridx = slot + 1;
-    *counter = *counter + 1;
-  }
-}
-void launch_step_end(StepCtl* ctl, unsigned long long* state_max, StepCtl* ring, int* ridx, long long* counter,
-                     int cap, cudaStream_t st) {
-  note_launch();
-  kt_mark(10, st);
-  k_step_end<<<1, 128, 0, st>>>(ctl, state_max, ring, ridx, counter, cap);
   kt_mark(10, st);
 }
 

@@ -17,7 +17,8 @@
 namespace gmk {
 
 // class bits of every grid point
-enum : uint8_t { CLS_ACTIVE = 1, CLS_IRREG = 2, CLS_GHOST = 4 };
+// (CLS_NEAR: an active cell with a ghost face, an active face with a ghost pressure cell)
+enum : uint8_t { CLS_ACTIVE = 1, CLS_IRREG = 2, CLS_GHOST = 4, CLS_NEAR = 8 };
 
 // Residual checks of one solve: check 0 after the first application of the
 // inverse, check k after refinement sweep k.  Plain FP64 runs at most 2 sweeps (as
@@ -171,6 +172,17 @@ __device__ __forceinline__ void raise_gate(StepCtl* ctl, int err_class, int gate
   if (atomicCAS(&ctl->err, 0, err_class) == 0) ctl->gate = gate;
 }
 
+// The points whose stencil reads ghost values.  The projection kernels form those values from
+// their extension rows as they go (code >= 0: the row), so no kernel has to fill them first;
+// the other operands are read from the grid (code < 0: ~index).
+struct NearCell {             // an active pressure cell: east, west, north, south face
+  int32_t cell, code[4];
+};
+struct NearFace {             // an active face: the pressure cells below (i - 1 or j - 1) and above it
+  int32_t face, code[2];      // code[1] NEAR_OUTLET: the outlet face, which has no upper cell
+};
+static constexpr int32_t NEAR_OUTLET = INT32_MIN;
+
 // Static geometry of one case on the device.
 struct CaseDev {
   int nx, ny;
@@ -188,6 +200,8 @@ struct CaseDev {
   const int64_t* gf_rows; const int64_t* gf_ptr; const int64_t* gf_col; const double* gf_val;
   int n_ghost_p;
   const int64_t* gp_rows; const int64_t* gp_ptr; const int64_t* gp_col; const double* gp_val;
+  int n_near_c, n_near_f;
+  const NearCell* near_c; const NearFace* near_f;
   // irregular rows: pressure A (p grid), Helmholtz u (u grid), v (v grid)
   int n_irr[3];
   const int64_t* irr_rows[3]; const int64_t* irr_ptr[3]; const int64_t* irr_col[3]; const double* irr_val[3];
@@ -471,11 +485,15 @@ struct MomentumArgs {
   const double* prev;     // previous advection (mode 0)
   double* now;            // advection output (modes 0, 1)
   double* out;            // rhs (modes 0, 2) or midpoint (mode 1)
-  const float* U32;       // FP32 copies of U and P for the stencils (FP32 mode, mode 0)
-  const float* P32;
+  float* U32;             // FP32 copies of U and P, filled and read by the one-thread-per-face
+  float* P32;             // kernel (FP32 mode, mode 0)
   double dt, alpha;
   float dt32, alpha32;    // FP32 copies (set by the FP32 launcher)
   int mode;
+  // mode 0: the CFL screen of k_cfl_screen, made by the first block (state_max nullptr: none)
+  const unsigned long long* state_max;
+  const long long* counter;
+  int screen;
 };
 void launch_momentum(const CaseDev& c, const MomentumArgs& a, const Gate& gate, cudaStream_t st);
 // same with the stencil arithmetic in FP32 (outputs and q + increment in FP64); in mode 0 the
@@ -491,35 +509,55 @@ void launch_diffusion(const CaseDev& c, const double* U, double* out, bool with_
                       cudaStream_t st);  // hdt==0: L U (+offset); else U - hdt*L U (H matvec)
 void launch_gradient(const CaseDev& c, const double* P, double* out, const Gate& gate, cudaStream_t st);
 
-// divergence at active p cells of an unpacked face grid: out = div / scale (div when scale is 0),
-// max|div| -> *divmax (if divmax); a non-finite out raises the gate error when
-// gate_on_nonfinite is set; sc is unused
-void launch_divergence(const CaseDev& c, const double* U, double* out, double scale, SolveCtl* sc,
-                       unsigned long long* divmax, int gate_on_nonfinite, const Gate& gate, cudaStream_t st);
-
-// out = q - dt * G phi on active faces (phi grid ghost-filled); pressure gate of slot checked first
-void launch_project_update(const CaseDev& c, const double* q, const double* phi, double dt, double* out,
-                           const SolveCtl* psolve, const Gate& gate, cudaStream_t st);
-
-// action = H result; proj = result + (rhs - action), H = I - c L of the CN solves with the
-// residual's coefficients (rcu: u faces, rcv: v faces)
-void launch_defect(const CaseDev& c, const ResidualCoef& rcu, const ResidualCoef& rcv, const double* result,
-                   const double* rhs, double* action, double* proj, const Gate& gate, cudaStream_t st);
-
-// half = p + inc; out = half + factor*inc (active p); coupled = max|action - rhs + dt G inc|
-void launch_pressure_out(const CaseDev& c, const double* p, const double* inc, double factor, double dt,
-                         const double* action, const double* rhs, double* half, double* pout,
-                         unsigned long long* coupled, const Gate& gate, cudaStream_t st);
+// divergence at active p cells of an unpacked face grid
+void launch_divergence(const CaseDev& c, const double* U, double* out, cudaStream_t st);
 
 void launch_maxabs(const CaseDev& c, const double* U, unsigned long long* umax, unsigned long long* vmax,
                    const Gate& gate, cudaStream_t st);
 
-// forces and coefficients; raises the force/step gates
-void launch_forces(const CaseDev& c, const double* U, const double* P, double mu, double dt, StepCtl* ctl,
-                   int check_gates, double* out6, const Gate& gate, cudaStream_t st);
+// fx, fy and their pressure and viscous parts
+void launch_forces(const CaseDev& c, const double* U, const double* P, double mu, double* out6, cudaStream_t st);
 
-// CN momentum gate (after both Helmholtz solves), nchk residual checks per solve
-void launch_gate_momentum(StepCtl* ctl, int nchk, cudaStream_t st);
+// The projection in three kernels around its pressure solve, with the gates between them folded in
+// (each gate is evaluated by the first block of the kernel behind it):
+//   launch_proj_rhs     out = div(U) scale at the active cells, from active and inlet values alone
+//   launch_proj_update  out = q - dt G phi, and the ghost values of phi
+//   launch_proj_tail    the largest |div U|, with by TAIL_*: the ghost values of U (PLAIN, DEFECT), the
+//                       defect of the CN velocity U (DEFECT), the new pressures, the coupled residual
+//                       and the maxima of the new velocity (PRESSURE)
+enum ProjCheck { PCHK_NONE = 0, PCHK_MOMENTUM = 1, PCHK_PROJECTION = 2 };  // PROJECTION: of div_max[1]
+enum ProjTail { TAIL_PLAIN = 0, TAIL_DEFECT = 1, TAIL_PRESSURE = 2 };
+struct TailArgs {
+  double* U;                                  // the projected velocity
+  unsigned long long* divmax;
+  const double* rhs;                          // DEFECT, PRESSURE
+  double *action, *proj;                      // DEFECT (out); PRESSURE reads action
+  const double *p, *inc, *unew;               // PRESSURE
+  double *half, *pout;
+  double factor, dgx, dgy;
+  unsigned long long *coupled, *umax;         // umax: max |u|, then max |v|
+};
+void launch_proj_rhs(const CaseDev& c, const double* U, double* out, double dt, ProjCheck chk, int nchk, const Gate& gate,
+                     cudaStream_t st);
+void launch_proj_update(const CaseDev& c, const double* q, double* phi, double dt, double* out, int slot, int nchk,
+                        const Gate& gate, cudaStream_t st);
+void launch_proj_tail(const CaseDev& c, const ResidualCoef& rcu, const ResidualCoef& rcv, ProjTail kind, const TailArgs& a,
+                      const Gate& gate, cudaStream_t st);
+// The end of a step: the gate of the second projection, the ghost values of the two new pressures, the
+// surface forces with the step gates, and the step record: if no gate failed the new state's
+// velocity maxima become the persistent ones, the control block is appended to ring[*ridx], the
+// step counter advances, and the per-step part of the control block is cleared for the next step.
+struct StepTail {
+  double *pout, *half;
+  const double* U;
+  double mu, dt;
+  unsigned long long* state_max;
+  StepCtl* ring;
+  int* ridx;
+  long long* counter;
+  int cap;
+};
+void launch_step_tail(const CaseDev& c, const StepTail& a, const Gate& gate, cudaStream_t st);
 // projection divergence gate on div_max[k]
 void launch_gate_projection(StepCtl* ctl, int k, cudaStream_t st);
 // CFL screen: dt*(umax/dx + vmax/dy) > 0.5 -> error (values from a previous maxabs);
@@ -538,11 +576,6 @@ void launch_schur_column(const double* first, const RectView& view, int rank, co
 // Refinement loop decision for a graph WHILE node: if check sc->k exceeded the inner
 // target and another check is allowed, advance sc->k and set the condition to 1.
 void launch_refine_decide(StepCtl* ctl, int slot, int nchk, cudaGraphConditionalHandle cond, cudaStream_t st);
-// end of a step: if no gate failed, the new state's velocity maxima become the persistent
-// ones; the step's control block is appended to ring[*ridx] and the step counter advances
-void launch_step_end(StepCtl* ctl, unsigned long long* state_max, StepCtl* ring, int* ridx, long long* counter,
-                     int cap, cudaStream_t st);
-
 // zero/copy helpers
 void launch_copy_active(const uint8_t* cls, int64_t n, const double* src, double* dst, const Gate& gate,
                         cudaStream_t st);
