@@ -118,6 +118,11 @@ struct RectDev {
   int mcount = 0;             // distinct points read by the C rows
   DBuf<int64_t> mcols;        // their field-grid flat indices
   DBuf<double> mmat;          // M = S^{-1} C, rank x mcount
+  // GMRES in the boundary rows' space (pressure, plain FP64; CompactGmres)
+  DBuf<double> cgK;
+  DBuf<int32_t> cgrow;
+  DBuf<int64_t> cgfield;
+  CompactGmres compact{};
   // band solve of the Schur term (pivots, decay factors, band work array)
   DBuf<double> bpiv, phi, psi, band;
   DBuf<float> bpiv32, phi32, psi32, band32;
@@ -191,6 +196,7 @@ struct gm_handle {
   // directions Z (m), the refinement correction and reduction scratch
   static constexpr int GMRES_M = 50;
   DBuf<double> gV, gZ, gdx, gpart, gdots, gcoef;
+  DBuf<double> gC, gcout;  // CompactGmres: v0, z0, E e; the cycle's result
   // FGMRES with its control on the device: state, scalars, and one instantiated graph per
   // (right-hand side, solution) pair it has solved for
   DBuf<GmresDev> gdev;
@@ -853,6 +859,24 @@ void build_schur(gm_handle* h, RectDev& rd, const std::vector<int64_t>& rows, co
   CK(cudaMemcpyAsync(hs.data(), S.p, hs.size() * sizeof(double), cudaMemcpyDeviceToHost, st));
   CK(cudaStreamSynchronize(st));
   for (int i = 0; i < n; ++i) hs[(size_t)i * n + i] += 1.0;
+  if (&rd == &h->rp && h->g.pressure_solver == 1 && h->precision == 0) {
+    // A T^-1 on the active boundary rows: their block of I + C T^-1 E
+    std::vector<int32_t> act;
+    std::vector<int64_t> field;
+    for (int i = 0; i < n; ++i)
+      if (h->g.act_p[frows[i]]) { act.push_back(i); field.push_back(frows[i]); }
+    const int na = (int)act.size();
+    if (compact_gmres_fits(na)) {
+      std::vector<double> K((size_t)na * na);
+      for (int i = 0; i < na; ++i)
+        for (int k = 0; k < na; ++k) K[(size_t)i * na + k] = hs[(size_t)act[i] * n + act[k]];
+      rd.cgK.upload(K, st);
+      rd.cgrow.upload(act, st);
+      rd.cgfield.upload(field, st);
+      CK(cudaStreamSynchronize(st));
+      rd.compact = CompactGmres{na, rd.cgK.p, rd.cgrow.p, rd.cgfield.p, rd.cptr.p, rd.ccol.p, rd.cval.p};
+    }
+  }
   std::vector<int> piv(n);
   if (!gm::lu_factor(n, hs.data(), piv.data())) throw GateError(GM_ERUNTIME, "Singular boundary Schur matrix");
   std::vector<double> inv((size_t)n * n);
@@ -1235,18 +1259,12 @@ void schur_solve_graph(gm_handle* h, int lane, RectDev& rd, int kind, double hc,
 // cycle (whose residual is b itself, the distribution the network was trained on) is
 // preconditioned by T^-1 + s net; every later direction by T^-1 alone (a flexible
 // preconditioner may change from one direction to the next).
+void gmres_arrays(gm_handle* h, bool compact);
 int fgmres(gm_handle* h, const double* b, double* x, int& iterations, bool learned) {
   const int m = gm_handle::GMRES_M;
   const int64_t n = h->Pn;
   cudaStream_t st = h->st;
-  if (!h->gV.p) {
-    h->gV.alloc((size_t)(m + 1) * n);
-    h->gZ.alloc((size_t)m * n);
-    h->gdx.alloc(n);
-    h->gpart.alloc((size_t)multidot_blocks(n) * 64);
-    h->gdots.alloc(64);
-    h->gcoef.alloc(64);
-  }
+  gmres_arrays(h, false);
   RectDev& rd = h->rp;
   const Gate open{nullptr, 0, 0};
   double* V = h->gV.p;
@@ -1416,11 +1434,25 @@ gm_handle::GmresExec& gmres_graph(gm_handle* h, const double* b, double* x) {
   add_conditional(st, cyc, cudaGraphCondTypeWhile, &cycle_body);
   CK(cudaStreamBeginCaptureToGraph(sb1, cycle_body, nullptr, nullptr, 0, cudaStreamCaptureModeThreadLocal));
   const long long c1 = kernel_launch_count();
+  long long per_step = 0;
+  const CompactGmres& cg = rd.compact;
   // V0 = (b - A x) / ||b - A x||
-  launch_apply_pressure(h->cd, h->rcoef[0], x, vec(V, 1), open, sb1);
-  CK(cudaMemcpyAsync(vec(V, 0), b, n * sizeof(double), cudaMemcpyDeviceToDevice, sb1));
-  launch_multiaxpy(vec(V, 1), n, 1, h->gone.p, -1.0, 1.0, vec(V, 0), n, sb1);
-  launch_multidot(vec(V, 0), n, 1, vec(V, 0), n, h->gpart.p, h->gbeta.p, sb1);
+  double* v0 = cg.n ? h->gC.p : vec(V, 0);
+  double* v1 = cg.n ? vec(v0, 1) : vec(V, 1);
+  launch_apply_pressure(h->cd, h->rcoef[0], x, v1, open, sb1);
+  CK(cudaMemcpyAsync(v0, b, n * sizeof(double), cudaMemcpyDeviceToDevice, sb1));
+  launch_multiaxpy(v1, n, 1, h->gone.p, -1.0, 1.0, v0, n, sb1);
+  launch_multidot(v0, n, 1, v0, n, h->gpart.p, h->gbeta.p, sb1);
+  if (cg.n) {
+    double* e = vec(v0, 2);
+    launch_cg_offnorm(h->cd, v0, h->gpart.p, sb1);
+    launch_cg_begin(h->gdev.p, h->gbeta.p, sb1);
+    launch_gm_scale(v0, n, h->gdev.p, sb1);
+    plain_inverse<double, double, double>(rd.tt, rd.view, v0, true, h->spectral.p, v1, nullptr, nullptr, open, sb1);
+    launch_cg_cycle(h->cd, cg, v0, v1, h->gpart.p, h->gdev.p, cyc, h->gcout.p, sb1);
+    launch_cg_combine(h->cd, cg, v1, h->gcout.p, x, e, sb1);
+    plain_inverse<double, double, double>(rd.tt, rd.view, e, true, h->spectral.p, x, rd.view.cls, x, open, sb1);
+  } else {
   GmresHandles hs{};
   hs.count = m;
   cudaGraph_t cyc_graph;
@@ -1428,7 +1460,6 @@ gm_handle::GmresExec& gmres_graph(gm_handle* h, const double* b, double* x) {
   for (int j = 0; j < m; ++j) CK(cudaGraphConditionalHandleCreate(&hs.step[j], cyc_graph, 0, 0));
   launch_gm_cycle_begin(h->gdev.p, h->gbeta.p, hs, sb1);
   launch_gm_scale(vec(V, 0), n, h->gdev.p, sb1);
-  long long per_step = 0;
   for (int j = 0; j < m; ++j) {
     cudaGraph_t step_body;
     add_conditional(sb1, hs.step[j], cudaGraphCondTypeIf, &step_body);
@@ -1453,6 +1484,7 @@ gm_handle::GmresExec& gmres_graph(gm_handle* h, const double* b, double* x) {
   // y = R^{-1} g, x += Z y
   launch_gm_cycle_end(h->gdev.p, h->gy.p, h->gnv.p, cyc, sb1);
   launch_multiaxpy_dev(Z, n, h->gnv.p, h->gy.p, x, n, sb1);
+  }
   ge.per_step = per_step;
   ge.per_cycle = kernel_launch_count() - c1 - (long long)m * per_step;
   cudaGraph_t done1;
@@ -1471,17 +1503,30 @@ gm_handle::GmresExec& gmres_graph(gm_handle* h, const double* b, double* x) {
   return h->gexec.back();
 }
 
-int fgmres_device(gm_handle* h, const double* b, double* x, int& iterations) {
-  if (!h->gV.p) {
-    const int m = gm_handle::GMRES_M;
-    const int64_t n = h->Pn;
-    h->gV.alloc((size_t)(m + 1) * n);
-    h->gZ.alloc((size_t)m * n);
+// GMRES work arrays: the grid iteration's basis (2 GMRES_M + 1 vectors) only where it runs
+void gmres_arrays(gm_handle* h, bool compact) {
+  const int m = gm_handle::GMRES_M;
+  const int64_t n = h->Pn;
+  if (!h->gdx.p) {
     h->gdx.alloc(n);
     h->gpart.alloc((size_t)multidot_blocks(n) * 64);
     h->gdots.alloc(64);
     h->gcoef.alloc(64);
   }
+  if (compact) {
+    if (!h->gC.p) {
+      h->gC.alloc(3 * n);
+      h->gC.zero(h->st);  // the third stays zero off the boundary rows
+      h->gcout.alloc(h->rp.compact.n + 1);
+    }
+  } else if (!h->gV.p) {
+    h->gV.alloc((size_t)(m + 1) * n);
+    h->gZ.alloc((size_t)m * n);
+  }
+}
+
+int fgmres_device(gm_handle* h, const double* b, double* x, int& iterations) {
+  gmres_arrays(h, h->rp.compact.n > 0);
   gm_handle::GmresExec& ge = gmres_graph(h, b, x);
   CK(cudaGraphLaunch(ge.exec, h->st));
   int r[5];

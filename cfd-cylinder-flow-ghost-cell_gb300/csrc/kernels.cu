@@ -622,6 +622,9 @@ template <typename T, typename TI, typename TO>
 __global__ void k_xpass_multi(const __grid_constant__ ArgPack<XpassArgs<T, TI, TO>> p);
 template <typename T, int L>
 __global__ void k_ysolve_multi(const __grid_constant__ ArgPack<YsolveArgs<T>> p);
+__global__ void k_cg_cycle(CompactGmres g, const double* __restrict__ v0, const double* __restrict__ z0,
+                           const double* __restrict__ part, int npart, GmresDev* gd, cudaGraphConditionalHandle cycle,
+                           double* __restrict__ out);
 
 // Opts the transform kernels into the large dynamic shared memory carve-out; returns the
 // dynamic bytes every one of them may use (the opt-in limit minus their static shared memory).
@@ -659,6 +662,7 @@ int configure_kernels(int smem_optin) {
   d = std::min(d, allow_dynamic_smem(k_ysolve_multi<float, 4>, smem_optin));
   d = std::min(d, allow_dynamic_smem(k_ysolve_multi<float, 8>, smem_optin));
   d = std::min(d, allow_dynamic_smem(k_ysolve_multi<float, 16>, smem_optin));
+  d = std::min(d, allow_dynamic_smem(k_cg_cycle, smem_optin));
   return d;
 }
 
@@ -2684,6 +2688,7 @@ __global__ void k_gm_init(GmresDev* gd, const double* __restrict__ bn2, cudaGrap
   gd->stop = 0;
   gd->cycle = 0;
   gd->jend = -1;
+  gd->polish = 0;
   cudaGraphSetConditional(cycle, 1u);
 }
 // beta = ||b - A x||; the cycle's first step runs while beta > tol
@@ -2792,6 +2797,281 @@ void launch_multiaxpy_dev(const double* V, int64_t ld, const int* nv, const doub
                           cudaStream_t st) {
   note_launch();
   k_multiaxpy_dev<<<reduce_blocks(n), TPB, 0, st>>>(V, ld, nv, coef, y, n);
+}
+
+// ---- FGMRES in the boundary rows' space (CompactGmres) ----------------------------------------
+// An Arnoldi step over the grid is a rectangle inverse, the operator and two Gram-Schmidt passes over
+// up to 50 grid vectors, some 15 kernels: 146 us at 512x256, 18 steps a solve.  With right
+// preconditioning by T^-1 the operator is v -> v + E C T^-1 v, so in the coordinates (alpha, d) it is
+// alpha' = alpha, d' = alpha G + K d with G = C T^-1 r / |r| and K formed with the boundary Schur matrix
+// at set-up.  r / |r| and E are orthonormal, so the dot products, the rotations and the iterates are
+// those of the grid iteration up to rounding.  V y = c v_0 + E e, so x takes c z_0 (z_0 = T^-1 v_0, formed as
+// the grid iteration forms it, gives G as well) and T^-1 E e: two inverses a cycle.  A cycle is then some 15 kernels, of which k_cg_cycle does all Arnoldi
+// steps on one cluster of eight SMs: the product with K by slices of rows (exchanged through distributed
+// shared memory, one cluster barrier a step), Gram-Schmidt and rotations by every SM on its own copy.
+// The model takes T^-1 as exact where the grid iteration sees the rounding of A T^-1, which left x with
+// the direct solver's error (3e-12 against 2e-13 at 400x200).  A converged solve therefore runs one more,
+// uncounted cycle on its true residual to CG_POLISH of it, after which x is nearer the exact solution
+// than the grid iteration's.  FP32 preconditioning is not linear to 1e-12, so that mode keeps the grid iteration, and so do
+// bodies with more rows than one SM's shared memory holds vectors of (CG_ROWS).  At 512x256 (58
+// rows, 15-18 steps a solve) a time step took 5.3 ms, now 1.3.
+constexpr int CG_CTAS = 8, CG_TPB = 256, CG_ROWS = 448;
+constexpr int CG_M = GmresDev::M;
+bool compact_gmres_fits(int n) { return n > 0 && n <= CG_ROWS; }
+static size_t cg_smem(int n) {
+  // V (M + 1 vectors), two copies of the exchanged vector, H, cs, sn, g, y, the step's coefficients, scratch
+  return ((size_t)(CG_M + 1 + 2) * (n + 1) + CG_M * CG_M + 6 * (CG_M + 2) + 64) * sizeof(double);
+}
+
+// (k_gm_cycle_begin, and the correcting cycle's start)
+constexpr double CG_POLISH = 0.02;
+__global__ void k_cg_begin(GmresDev* gd, const double* __restrict__ beta2) {
+  const double beta = sqrt(beta2[0]);
+  gd->jend = -1;
+  const bool go = gd->polish ? beta > 0.0 && isfinite(beta) : beta > gd->tol;
+  if (!go) {
+    if (!gd->polish) gd->converged = isfinite(beta) ? 1 : 0;
+    gd->stop = 1;
+    gd->hscale = 1.0;
+    return;
+  }
+  gd->g[0] = beta;
+  gd->hscale = 1.0 / beta;
+  gd->ptol = CG_POLISH * beta;
+}
+void launch_cg_begin(GmresDev* gd, const double* beta2, cudaStream_t st) {
+  note_launch();
+  k_cg_begin<<<1, 1, 0, st>>>(gd, beta2);
+}
+__global__ void k_cg_offnorm(CaseDev c, const double* __restrict__ r, double* __restrict__ part) {
+  __shared__ double red[TPB / 32];
+  double acc = 0.0;
+  for (int64_t t = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; t < c.psize; t += (int64_t)gridDim.x * blockDim.x)
+    if (!(c.cls_p[t] & CLS_IRREG)) acc += r[t] * r[t];
+  acc = warp_sum(acc);
+  if ((threadIdx.x & 31) == 0) red[threadIdx.x >> 5] = acc;
+  __syncthreads();
+  if (threadIdx.x == 0) {
+    double s = 0.0;
+    for (int q = 0; q < TPB / 32; ++q) s += red[q];
+    part[blockIdx.x] = s;
+  }
+}
+void launch_cg_offnorm(const CaseDev& c, const double* r, double* part, cudaStream_t st) {
+  note_launch();
+  kt_mark(6, st);
+  k_cg_offnorm<<<reduce_blocks(c.psize), TPB, 0, st>>>(c, r, part);
+  kt_mark(6, st, (double)c.psize * 9);
+}
+
+__device__ __forceinline__ void cluster_sync_all() {
+  asm volatile("barrier.cluster.arrive.release.aligned;\nbarrier.cluster.wait.acquire.aligned;" ::: "memory");
+}
+__device__ __forceinline__ void cluster_store(double* local, unsigned rank, double v) {  // to the same place in CTA `rank`
+  unsigned a = (unsigned)__cvta_generic_to_shared(local), r;
+  asm("mapa.shared::cluster.u32 %0, %1, %2;" : "=r"(r) : "r"(a), "r"(rank));
+  asm volatile("st.shared::cluster.f64 [%0], %1;" ::"r"(r), "d"(v) : "memory");
+}
+
+__global__ void __launch_bounds__(CG_TPB) k_cg_cycle(CompactGmres g, const double* __restrict__ v0, const double* __restrict__ z0,
+                                                     const double* __restrict__ part, int npart, GmresDev* gd,
+                                                     cudaGraphConditionalHandle cycle, double* __restrict__ out) {
+  extern __shared__ __align__(16) unsigned char smem_raw[];
+  const int n = g.n, n1 = n + 1, tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
+  constexpr int NW = CG_TPB / 32;
+  double* V = reinterpret_cast<double*>(smem_raw);      // V_i at i n1: d (n values), then alpha
+  double* wx = V + (size_t)(CG_M + 1) * n1;              // the exchanged vector, two copies by step parity
+  double* H = wx + 2 * (size_t)n1;                       // rotated columns: H[i M + j]
+  double* cs = H + CG_M * CG_M;
+  double* sn = cs + CG_M + 2;
+  double* gv = sn + CG_M + 2;
+  double* y = gv + CG_M + 2;
+  double* hc = y + CG_M + 2;                             // the step's column
+  double* cf = hc + CG_M + 2;                            // a pass's coefficients
+  double* sc = cf + CG_M + 2;                            // scratch: warp sums, broadcast scalars
+  unsigned rank;
+  asm("mov.u32 %0, %%cluster_ctarank;" : "=r"(rank));
+  const int slice = (n + CG_CTAS - 1) / CG_CTAS, ra = min(n, (int)rank * slice), rb = min(n, ra + slice);
+  // block-wide sum of one value a thread, the same for every thread (two barriers)
+  auto total = [&](double v) {
+    v = warp_sum(v);
+    __syncthreads();
+    if (lane == 0) sc[warp] = v;
+    __syncthreads();
+    double s = 0.0;
+#pragma unroll
+    for (int q = 0; q < NW; ++q) s += sc[q];
+    return s;
+  };
+  double acc = 0.0;
+  for (int q = tid; q < npart; q += CG_TPB) acc += part[q];
+  // k_cg_begin has decided whether the cycle runs; v0 is scaled
+  const bool polish = gd->polish != 0;
+  const double alpha0 = sqrt(total(acc)) * gd->hscale, tol = polish ? gd->ptol : gd->tol;
+  int jend = -1, its = 0, converged = 0;
+  const bool stop = gd->stop != 0;
+  if (!stop) {
+    for (int k = tid; k < n; k += CG_TPB) V[k] = v0[g.field[k]];
+    if (tid == 0) {
+      V[n] = alpha0;
+      gv[0] = gd->g[0];
+    }
+    // K times the boundary part of `v` by rows of this CTA's slice, to every CTA's `w`; the barrier in
+    // front of the first call makes the clusters' shared memory ready for remote stores
+    auto product = [&](const double* v, double* w) {
+      for (int r = ra + warp; r < rb; r += NW) {
+        double s = 0.0;
+        for (int k = lane; k < n; k += 32) s += g.K[(size_t)r * n + k] * v[k];
+        s = warp_sum(s);
+        if (lane < CG_CTAS) cluster_store(w + r, lane, s);
+      }
+      cluster_sync_all();
+    };
+    cluster_sync_all();
+    product(V, wx + n1);
+    // G = (C z0 - (K - I) d0) / alpha0 by this thread's rows, kept in registers (n <= 2 CG_TPB)
+    const double ia = alpha0 > 0.0 ? 1.0 / alpha0 : 0.0;
+    double G[2] = {0.0, 0.0};
+#pragma unroll
+    for (int u = 0; u < 2; ++u) {
+      const int k = tid + u * CG_TPB;
+      if (k < n) {
+        const int r = g.crow[k];
+        double s = 0.0;
+        for (int64_t e = g.cptr[r]; e < g.cptr[r + 1]; ++e) s += g.cval[e] * z0[g.ccol[e]];
+        G[u] = (s - (wx[n1 + k] - V[k])) * ia;
+      }
+    }
+    for (int j = 0; j < CG_M; ++j) {
+      const double* v = V + (size_t)j * n1;
+      double* w = wx + (size_t)(j & 1) * n1;
+      __syncthreads();
+      if (tid == 0) w[n] = v[n];
+      product(v, w);
+      const double alpha = v[n];
+#pragma unroll
+      for (int u = 0; u < 2; ++u) {
+        const int k = tid + u * CG_TPB;
+        if (k < n) w[k] += alpha * G[u];
+      }
+      __syncthreads();
+      // two classical Gram-Schmidt passes against V_0..V_j, then the norm
+      for (int pass = 0; pass < 2; ++pass) {
+        for (int i = warp; i <= j; i += NW) {
+          const double* vi = V + (size_t)i * n1;
+          double s = 0.0;
+          for (int k = lane; k < n1; k += 32) s += vi[k] * w[k];
+          s = warp_sum(s);
+          if (lane == 0) {
+            cf[i] = s;
+            hc[i] = pass ? hc[i] + s : s;
+          }
+        }
+        __syncthreads();
+        for (int k = tid; k < n1; k += CG_TPB) {
+          double s0 = 0.0, s1 = 0.0;
+          int i = 0;
+          for (; i + 1 <= j; i += 2) {
+            s0 += cf[i] * V[(size_t)i * n1 + k];
+            s1 += cf[i + 1] * V[(size_t)(i + 1) * n1 + k];
+          }
+          if (i <= j) s0 += cf[i] * V[(size_t)i * n1 + k];
+          w[k] -= s0 + s1;
+        }
+        __syncthreads();
+      }
+      acc = 0.0;
+      for (int k = tid; k < n1; k += CG_TPB) acc += w[k] * w[k];
+      const double hn = sqrt(total(acc)), scale = hn > 0 ? 1.0 / hn : 1.0;
+      for (int k = tid; k < n1; k += CG_TPB) V[(size_t)(j + 1) * n1 + k] = w[k] * scale;
+      // the rotations of k_gm_step_end
+      if (tid == 0) {
+        hc[j + 1] = hn;
+        for (int i = 0; i < j; ++i) {
+          const double a = cs[i] * hc[i] + sn[i] * hc[i + 1];
+          hc[i + 1] = -sn[i] * hc[i] + cs[i] * hc[i + 1];
+          H[i * CG_M + j] = a;
+        }
+        const double den = hypot(hc[j], hc[j + 1]);
+        cs[j] = den > 0 ? hc[j] / den : 1.0;
+        sn[j] = den > 0 ? hc[j + 1] / den : 0.0;
+        H[j * CG_M + j] = den;
+        gv[j + 1] = -sn[j] * gv[j];
+        gv[j] = cs[j] * gv[j];
+      }
+      __syncthreads();
+      ++its;
+      jend = j;
+      const double r = gv[j + 1];
+      if (!isfinite(r)) break;
+      if (fabs(r) <= tol) { converged = 1; break; }
+    }
+  }
+  // no CTA leaves (or ends) while another may still store into its shared memory: the last exchange
+  // is behind every CTA's last cluster barrier, so none can
+  if (rank != 0) return;
+  if (tid == 0) {
+    for (int i = jend; i >= 0; --i) {
+      double a = gv[i];
+      for (int k = i + 1; k <= jend; ++k) a -= H[i * CG_M + k] * y[k];
+      y[i] = a / H[i * CG_M + i];
+    }
+    gd->jend = jend;
+    gd->cycle += 1;
+    bool go = false;
+    if (!polish) {
+      gd->iterations += its;
+      if (converged) gd->converged = 1;
+      go = jend >= 0 && !stop && (converged || gd->cycle < 100);
+      if (go && converged) gd->polish = 1;
+    }
+    cudaGraphSetConditional(cycle, go ? 1u : 0u);
+  }
+  __syncthreads();
+  double f = 0.0;  // the factor of v0
+  if (jend >= 0 && alpha0 > 0.0) {
+    for (int i = 0; i <= jend; ++i) f += y[i] * V[(size_t)i * n1 + n];
+    f /= alpha0;
+  }
+  for (int k = tid; k < n; k += CG_TPB) {
+    double s = 0.0;
+    for (int i = 0; i <= jend; ++i) s += y[i] * V[(size_t)i * n1 + k];
+    out[1 + k] = jend >= 0 ? s - f * V[k] : 0.0;
+  }
+  if (tid == 0) out[0] = f;
+}
+void launch_cg_cycle(const CaseDev& c, const CompactGmres& g, const double* v0, const double* z0, const double* part,
+                     GmresDev* gd, cudaGraphConditionalHandle cycle, double* out, cudaStream_t st) {
+  note_launch();
+  kt_mark(6, st);
+  cudaLaunchConfig_t cfg{};
+  cfg.gridDim = dim3(CG_CTAS);
+  cfg.blockDim = dim3(CG_TPB);
+  cfg.dynamicSmemBytes = cg_smem(g.n);
+  cfg.stream = st;
+  cudaLaunchAttribute at[1];
+  at[0].id = cudaLaunchAttributeClusterDimension;
+  at[0].val.clusterDim.x = CG_CTAS;
+  at[0].val.clusterDim.y = at[0].val.clusterDim.z = 1;
+  cfg.attrs = at;
+  cfg.numAttrs = 1;
+  cudaLaunchKernelEx(&cfg, k_cg_cycle, g, v0, z0, part, (int)reduce_blocks(c.psize), gd, cycle, out);
+  kt_mark(6, st);
+}
+
+__global__ void k_cg_combine(CaseDev c, CompactGmres g, const double* __restrict__ z0, const double* __restrict__ out,
+                             double* __restrict__ x, double* __restrict__ e) {
+  const double f = out[0];
+  for (int64_t t = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; t < c.psize; t += (int64_t)gridDim.x * blockDim.x)
+    if (c.cls_p[t] & CLS_ACTIVE) x[t] += f * z0[t];
+  for (int k = blockIdx.x * blockDim.x + threadIdx.x; k < g.n; k += gridDim.x * blockDim.x) e[g.field[k]] = out[1 + k];
+}
+void launch_cg_combine(const CaseDev& c, const CompactGmres& g, const double* z0, const double* out, double* x, double* e,
+                       cudaStream_t st) {
+  note_launch();
+  kt_mark(6, st);
+  k_cg_combine<<<reduce_blocks(c.psize), TPB, 0, st>>>(c, g, z0, out, x, e);
+  kt_mark(6, st, (double)c.psize * 25);
 }
 
 __global__ void k_refine_decide(StepCtl* ctl, int slot, int nchk, cudaGraphConditionalHandle cond) {

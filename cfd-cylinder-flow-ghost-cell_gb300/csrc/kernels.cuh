@@ -281,6 +281,8 @@ struct GmresDev {             // the state of one solve, in device memory
   double cs[M], sn[M], g[M + 1], y[M];
   double tol, hscale;         // stop tolerance; scale of the next basis vector
   int jend, cycle, iterations, converged, stop;
+  int polish;                  // CompactGmres: this cycle corrects the rounding of T^-1 (its tolerance: ptol)
+  double ptol;
 };
 struct GmresHandles {         // the conditions of the Arnoldi-step IF nodes of a cycle (count <= M)
   cudaGraphConditionalHandle step[GmresDev::M];
@@ -296,6 +298,31 @@ void launch_gm_step_end(GmresDev* gd, int j, const double* d1, const double* d2,
 void launch_gm_cycle_end(GmresDev* gd, double* y, int* nv, cudaGraphConditionalHandle cycle, cudaStream_t st);
 void launch_multiaxpy_dev(const double* V, int64_t ld, const int* nv, const double* coef, double* y, int64_t n,
                           cudaStream_t st);
+
+// ---- the same iteration in the boundary rows' space (plain FP64, kernels.cu) ----
+// The operator A T^-1 that GMRES works on is the identity outside the rows where A differs from the
+// rectangle operator T (the irregular active rows E, n of them), so every Krylov vector is
+// alpha r / |r| + E d: r the cycle's first residual off E, and values on E.
+struct CompactGmres {
+  int n;                       // rows of E; 0: not built
+  const double* K;             // n x n: E^T A T^-1 E
+  const int32_t* crow;         // their rows in the boundary matrix C = A - T (cptr, ccol, cval)
+  const int64_t* field;        // their grid indices
+  const int64_t* cptr; const int64_t* ccol; const double* cval;
+};
+bool compact_gmres_fits(int n);
+// beta = ||r||: whether the cycle runs, the scale of v0 and, in the correcting cycle, its tolerance
+void launch_cg_begin(GmresDev* gd, const double* beta2, cudaStream_t st);
+// block partials of |r|^2 off E
+void launch_cg_offnorm(const CaseDev& c, const double* r, double* part, cudaStream_t st);
+// One restart cycle from the first basis vector v0 (scaled by gd->hscale, part: of the residual
+// before) and z0 = T^-1 v0: V y = out[0] v0 + E out[1..].  Sets the cycle condition as
+// launch_gm_cycle_end does.
+void launch_cg_cycle(const CaseDev& c, const CompactGmres& g, const double* v0, const double* z0, const double* part,
+                     GmresDev* gd, cudaGraphConditionalHandle cycle, double* out, cudaStream_t st);
+// x += out[0] z0 at the active cells, and out[1..] to the rows E of e (zero elsewhere)
+void launch_cg_combine(const CaseDev& c, const CompactGmres& g, const double* z0, const double* out, double* x, double* e,
+                       cudaStream_t st);
 
 // ---- tensor-core row transforms of the FP32 mode (rowgemm.cu) ---------------
 // Transform matrices of the pressure rectangle in split TF32 (both directions) with their TMA
