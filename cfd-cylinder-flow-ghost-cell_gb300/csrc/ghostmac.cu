@@ -241,6 +241,13 @@ struct gm_handle {
   long long body_nodes_slot[5] = {0, 0, 0, 0, 0};  // kernels per refinement sweep of each solve slot
   bool use_graphs = true;
   bool capturing = false;
+  // A step graph holds a fixed number of gated refinement sweeps for each solve slot and no loop: a
+  // conditional node costs 8 us even when its body does not run and 4 more per pass (a kernel node 1.2),
+  // 25 us of a 220 us step in FP64, which needs no sweep, and about 50 in the FP32 mode.  A solve that
+  // needs more than its slot's stops the steps behind it (ERR_SWEEPS); the host adds one and repeats
+  // the step.  FP64 starts with none, the FP32 mode with the one that it always needs.
+  bool loops = true;  // captures as WHILE nodes (batches, whose cases the host cannot repeat alone; cut-cell)
+  int sweeps[5] = {0, 0, 0, 0, 0};
   // launch-by-launch steps decide every refinement sweep on the host (one synchronisation
   // per sweep) instead of launching all sweeps gated: then every launched kernel does work,
   // which per-kernel timing and profiling need (environment GHOSTMAC_HOST_REFINE=1)
@@ -263,8 +270,7 @@ struct gm_handle {
     cudaGraphExec_t exec = nullptr;
     const double* key[6] = {};
     double dt = 0;
-    long long outer_nodes = 0;     // kernel nodes outside the refinement loops
-    long long body_nodes[5] = {};  // kernel nodes of one refinement sweep, per solve slot
+    long long nodes = 0;  // kernel nodes
   } graphs[2];
   bool has_history = false;
   bool host_only = false;
@@ -1586,13 +1592,17 @@ void gmres_monitored(gm_handle* h, const double* b, double* x, double* res, int 
 
 // One solve A x = b with the FFT + boundary Schur inverse and refinement sweeps to the
 // reference's residual target (solver/pressure_schur.py:16-72, direct branch).
+// refinement sweeps launched for a slot
+int sweeps_of(const gm_handle* h, int slot) {
+  return h->capturing && !h->loops ? std::min(h->sweeps[slot], h->nchk - 1) : h->nchk - 1;
+}
 void schur_solve(gm_handle* h, int lane, RectDev& rd, int kind, double hc, const double* b, double* x, double* res,
                  double* first, double* w2, int slot) {
   if (kind == 0 && h->g.pressure_solver == 1) {
     gmres_monitored(h, b, x, res, slot);
     return;
   }
-  if (h->capturing) {
+  if (h->capturing && h->loops) {
     schur_solve_graph(h, lane, rd, kind, hc, b, x, res, first, w2, slot);
     return;
   }
@@ -1600,11 +1610,15 @@ void schur_solve(gm_handle* h, int lane, RectDev& rd, int kind, double hc, const
   SolveCtl* sc = &h->ctl.p->solve[slot];
   const bool f32 = h->precision == 1;
   void* resb = f32 ? (void*)(kind == 0 ? h->pres32.p : h->fres32.p) : (void*)res;
-  for (int sweep = 0; sweep < h->nchk; ++sweep) {
+  const int last = sweeps_of(h, slot);
+  for (int sweep = 0; sweep <= last; ++sweep) {
     Gate gt = gate_of(h, slot, sweep);
+    h->sweep_marking = h->phase_on && h->capturing && slot == S_P1 && sweep == 0;
     apply_inverse(h, lane, rd, kind, sweep == 0 ? (const void*)b : (const void*)resb, sweep > 0 && f32, x, sweep > 0,
                   first, w2, gt, st);
     launch_residual(h->cd, h->rcoef[kind], kind, b, x, resb, f32, sc, sweep, sweep == 0, gt, st);
+    if (h->sweep_marking) sweep_mark(h, 8, st);
+    h->sweep_marking = false;
     if (h->host_refine && sweep + 1 < h->nchk) {
       // the rule of k_refine_decide, read back on the host
       SolveCtl hs;
@@ -1636,7 +1650,7 @@ void solve_call(gm_handle* h, const SolveCall& c) {
   schur_solve(h, c.lane, *c.rd, c.kind, 0.0, c.b, c.x, c.res, c.first, c.w2, c.slot);
 }
 SolveCall project_pre(gm_handle* h, const double* q, double dt, double* phi, int slot, ProjCheck chk) {
-  launch_proj_rhs(h->cd, q, h->prhs.p, dt, chk, h->nchk, gate_of(h), h->st);
+  launch_proj_rhs(h->cd, q, h->prhs.p, dt, chk, h->nchk, sweeps_of(h, S_HELM_U), sweeps_of(h, S_HELM_V), gate_of(h), h->st);
   return SolveCall{0, &h->rp, 0, h->prhs.p, phi, h->pres.p, h->pfirst.p, h->pw2.p, slot};
 }
 // up to the projected velocity `out` (its ghost values and the divergence check follow in
@@ -1649,7 +1663,7 @@ void project_post(gm_handle* h, const double* q, double dt, double* out, double*
     CK(cudaMemcpyAsync(h->rec_sol + off, phi, h->Pn * sizeof(double), cudaMemcpyDeviceToDevice, st));
     ++h->rec_count;
   }
-  launch_proj_update(h->cd, q, phi, dt, out, slot, h->nchk, gate_of(h), st);
+  launch_proj_update(h->cd, q, phi, dt, out, slot, h->nchk, sweeps_of(h, slot), !(h->capturing && h->loops), gate_of(h), st);
 }
 // a projection by itself, its gate included (div_max[divk])
 void project(gm_handle* h, const double* q, double dt, double* out, double* phi, int slot, int divk) {
@@ -2098,29 +2112,25 @@ cudaGraphExec_t step_graph(gm_handle* h, double dt) {
                                : (!h->graphs[1].exec || h->graphs[1].dt != dt ? &h->graphs[1] : &h->graphs[0]);
   if (slot->exec) { cudaGraphExecDestroy(slot->exec); slot->exec = nullptr; }
   const long long c0 = kernel_launch_count();
-  long long body_total = 0;
-  std::fill(h->body_nodes_slot, h->body_nodes_slot + 5, 0LL);
   h->capturing = true;
+  h->loops = false;
   cudaGraph_t g = nullptr;
   CK(cudaStreamBeginCapture(h->st, cudaStreamCaptureModeThreadLocal));
   try {
     step_once(h, dt, -1);
   } catch (...) {
     h->capturing = false;
+    h->loops = true;
     cudaStreamEndCapture(h->st, &g);
     if (g) cudaGraphDestroy(g);
     cudaGetLastError();
     throw;
   }
   h->capturing = false;
+  h->loops = true;
   CK(cudaStreamEndCapture(h->st, &g));
-  const long long captured = kernel_launch_count() - c0;
-  kernel_launch_adjust(-captured);
-  for (int q = 0; q < 5; ++q) {
-    body_total += h->body_nodes_slot[q];
-    slot->body_nodes[q] = h->body_nodes_slot[q];
-  }
-  slot->outer_nodes = captured - body_total;
+  slot->nodes = kernel_launch_count() - c0;
+  kernel_launch_adjust(-slot->nodes);
   cudaGraphExec_t ex = nullptr;
   cudaError_t e = cudaGraphInstantiate(&ex, g, 0);
   cudaGraphDestroy(g);
@@ -2299,6 +2309,7 @@ void create_device(gm_handle* H) {
   H->spectral.alloc(std::max<int64_t>(H->Pn, (int64_t)g.ny * g.nx));
   H->spectral_b.alloc(H->spectral.n);
   if (H->precision == 1) {
+    std::fill(H->sweeps, H->sweeps + 5, 1);
     H->spectral32.alloc(H->spectral.n);
     H->spectral32_b.alloc(H->spectral.n);
     H->pres32.alloc(H->Pn);
@@ -2383,16 +2394,21 @@ void step_loop(gm_handle* h, double dt, int32_t n_steps, int64_t first_step_inde
       cudaGetLastError();
       int good = 0;
       while (good < batch && h->host_ring[good].err == 0) ++good;
-      if (!direct) {
-        // kernel nodes the replays executed: outer nodes + one sweep body per refinement iteration
-        const gm_handle::StepGraph& gr = h->graphs[0].exec ? h->graphs[0] : h->graphs[1];
-        long long nodes = 0;
-        for (int k = 0; k < batch; ++k) {
-          const StepCtl& c = h->host_ring[k];
-          nodes += gr.outer_nodes;
-          for (int sl = 0; sl < 5; ++sl) nodes += gr.body_nodes[sl] * c.solve[sl].k;
-        }
-        kernel_launch_adjust(nodes);
+      if (!direct) kernel_launch_adjust(batch * (h->graphs[0].exec ? h->graphs[0] : h->graphs[1]).nodes);
+      if (good < batch && h->host_ring[good].err == ERR_SWEEPS) {
+        // a solve of step s + good needs one sweep more than the graph holds: back to the state before
+        // that step, and on from there with graphs that have it
+        for (int k = 0; k < good; ++k)
+          if (diag) fill_diag(h, h->host_ring[k], start_time + (s + k + 1) * dt, dt, false, &diag[s + k]);
+        if ((batch - good) % 2) swap_state(h);
+        ++h->sweeps[h->host_ring[good].gate];
+        for (auto& gr : h->graphs)
+          if (gr.exec) { cudaGraphExecDestroy(gr.exec); gr.exec = nullptr; }
+        s += good;
+        counter = first_step_index + s;
+        CK(cudaMemsetAsync(h->ctl.p, 0, sizeof(StepCtl), st));
+        CK(cudaMemcpyAsync(h->counter.p, &counter, sizeof counter, cudaMemcpyHostToDevice, st));
+        continue;
       }
       for (int k = 0; k < std::min(batch, good + 1); ++k)
         if (diag) fill_diag(h, h->host_ring[k], start_time + (s + k + 1) * dt, dt, first && k == 0, &diag[s + k]);

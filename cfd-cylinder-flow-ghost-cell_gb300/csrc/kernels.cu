@@ -979,7 +979,14 @@ __device__ __forceinline__ void csr_row(const int64_t* __restrict__ col, const d
 }
 
 // ---- the gates of a step (each raises the sticky error word; none clears it) ----
-__device__ void check_momentum(StepCtl* ctl, int nchk) {
+// whether the solve's checks ended within the sweeps that were launched for it
+__device__ __forceinline__ bool sweeps_done(StepCtl* ctl, int slot, int nchk, int sweeps) {
+  if (sweeps >= nchk - 1 || last_check(&ctl->solve[slot], nchk) <= sweeps) return true;
+  raise_gate(ctl, ERR_SWEEPS, slot);
+  return false;
+}
+__device__ void check_momentum(StepCtl* ctl, int nchk, int sweeps_u, int sweeps_v) {
+  if (!sweeps_done(ctl, S_HELM_U, nchk, sweeps_u) || !sweeps_done(ctl, S_HELM_V, nchk, sweeps_v)) return;
   double r = 0, bm = 0;
   bool bad = false;
   for (int s = 0; s < 2; ++s) {
@@ -993,7 +1000,8 @@ __device__ void check_momentum(StepCtl* ctl, int nchk) {
   double thr = 1e-10 * (bm > 1.0 ? bm : 1.0);
   if (bad || !(r <= thr)) raise_gate(ctl, 2, 2);
 }
-__device__ void check_pressure(StepCtl* ctl, int slot, int nchk) {
+__device__ void check_pressure(StepCtl* ctl, int slot, int nchk, int sweeps) {
+  if (!sweeps_done(ctl, slot, nchk, sweeps)) return;
   const SolveCtl* sc = &ctl->solve[slot];
   int k = last_check(sc, nchk);
   double linf = bits2d(sc->rmax[k]), bound = bits2d(sc->bound[k]), bm = bits2d(sc->bmax);
@@ -2178,10 +2186,10 @@ static inline int near_cell_blocks(const CaseDev& c) { return (c.n_near_c + TPB 
 static inline int ghost_blocks(int n) { return (int)blocks_for((int64_t)n * GHOST_LANES); }
 
 __global__ void k_proj_rhs(CaseDev c, const double* __restrict__ U, double* __restrict__ out, double sx, double sy,
-                           int chk, int nchk, int nbn, Gate gate) {
+                           int chk, int nchk, int sweeps_u, int sweeps_v, int nbn, Gate gate) {
   if (!gate_open(gate)) return;
   if (chk && blockIdx.x + threadIdx.x == 0) {
-    if (chk == PCHK_MOMENTUM) check_momentum(gate.ctl, nchk);
+    if (chk == PCHK_MOMENTUM) check_momentum(gate.ctl, nchk, sweeps_u, sweeps_v);
     else check_projection(gate.ctl, 1);
   }
   const Grid g{c.nx, c.ny, c.usize};
@@ -2213,21 +2221,22 @@ __global__ void k_proj_rhs(CaseDev c, const double* __restrict__ U, double* __re
   }
   if (bad && gate.ctl) {
     // the gate in front comes first, whichever thread gets here first
-    if (chk == PCHK_MOMENTUM) check_momentum(gate.ctl, nchk);
+    if (chk == PCHK_MOMENTUM) check_momentum(gate.ctl, nchk, sweeps_u, sweeps_v);
     else if (chk == PCHK_PROJECTION) check_projection(gate.ctl, 1);
     raise_gate(gate.ctl, 1, 4);
   }
 }
-void launch_proj_rhs(const CaseDev& c, const double* U, double* out, double dt, ProjCheck chk, int nchk, const Gate& gate,
-                     cudaStream_t st) {
+void launch_proj_rhs(const CaseDev& c, const double* U, double* out, double dt, ProjCheck chk, int nchk, int sweeps_u,
+                     int sweeps_v, const Gate& gate, cudaStream_t st) {
   const int nbn = near_cell_blocks(c);
   const double s = 1.0 / dt;
   note_launch();
   kt_mark(6, st);
   const dim3 grid((unsigned)nbn + reduce_blocks(c.psize));
   const int check = gate.ctl ? (int)chk : 0;
-  if (chk == PCHK_MOMENTUM) k_proj_rhs<<<grid, TPB, 0, st>>>(c, U, out, c.idx * s, c.idy * s, check, nchk, nbn, gate);
-  else launch_pdl(k_proj_rhs, grid, dim3(TPB), 0, st, c, U, out, c.idx * s, c.idy * s, check, nchk, nbn, gate);
+  if (chk == PCHK_MOMENTUM) k_proj_rhs<<<grid, TPB, 0, st>>>(c, U, out, c.idx * s, c.idy * s, check, nchk, sweeps_u,
+                                                           sweeps_v, nbn, gate);
+  else launch_pdl(k_proj_rhs, grid, dim3(TPB), 0, st, c, U, out, c.idx * s, c.idy * s, check, nchk, sweeps_u, sweeps_v, nbn, gate);
   kt_mark(6, st);
 }
 
@@ -2235,9 +2244,9 @@ void launch_proj_rhs(const CaseDev& c, const double* U, double* out, double dt, 
 // two fused multiply-adds per face (G phi is gx (phi_e - phi_w), at the outlet -2 gx phi_w).
 // Blocks: nbf of near faces (16 lanes a face), nbg that fill phi's ghost values, then the grid.
 __global__ void k_proj_update(CaseDev c, const double* __restrict__ q, double* phi, double dgx, double dgy,
-                              double* __restrict__ out, int slot, int nchk, int nbf, int nbg, Gate gate) {
+                              double* __restrict__ out, int slot, int nchk, int sweeps, int nbf, int nbg, Gate gate) {
   if (!gate_open(gate)) return;
-  if (gate.ctl && blockIdx.x + threadIdx.x == 0) check_pressure(gate.ctl, slot, nchk);
+  if (gate.ctl && blockIdx.x + threadIdx.x == 0) check_pressure(gate.ctl, slot, nchk, sweeps);
   const Grid g{c.nx, c.ny, c.usize};
   const int b = blockIdx.x;
   if (b < nbf) {
@@ -2278,12 +2287,14 @@ __global__ void k_proj_update(CaseDev c, const double* __restrict__ q, double* p
   else out[t] = fma(2.0 * dgx, phi[g.p(j, c.nx - 1)], q[t]);
 }
 void launch_proj_update(const CaseDev& c, const double* q, double* phi, double dt, double* out, int slot, int nchk,
-                        const Gate& gate, cudaStream_t st) {
+                        int sweeps, bool pdl, const Gate& gate, cudaStream_t st) {
   const int nbf = (c.n_near_f + TPB / 16 - 1) / (TPB / 16), nbg = ghost_blocks(c.n_ghost_p);
+  const dim3 grid((unsigned)(nbf + nbg) + blocks_for(c.usize + c.vsize));
+  const double dgx = dt * c.gx, dgy = dt * c.gy;
   note_launch();
   kt_mark(6, st);
-  k_proj_update<<<(unsigned)(nbf + nbg) + blocks_for(c.usize + c.vsize), TPB, 0, st>>>(c, q, phi, dt * c.gx, dt * c.gy, out,
-                                                                                       slot, nchk, nbf, nbg, gate);
+  if (pdl) launch_pdl(k_proj_update, grid, dim3(TPB), 0, st, c, q, phi, dgx, dgy, out, slot, nchk, sweeps, nbf, nbg, gate);
+  else k_proj_update<<<grid, TPB, 0, st>>>(c, q, phi, dgx, dgy, out, slot, nchk, sweeps, nbf, nbg, gate);
   kt_mark(6, st);
 }
 
@@ -2641,7 +2652,7 @@ void launch_step_tail(const CaseDev& c, const StepTail& a, const Gate& gate, cud
 }
 
 __global__ void k_gate_pressure(StepCtl* ctl, int slot, int nchk) {
-  if (!ctl->err) check_pressure(ctl, slot, nchk);
+  if (!ctl->err) check_pressure(ctl, slot, nchk, nchk - 1);
 }
 void launch_gate_pressure(StepCtl* ctl, int slot, int nchk, cudaStream_t st) {
   note_launch();

@@ -51,6 +51,10 @@ struct StepCtl {
   double cd, cl;
 };
 
+// Error class of a step whose graph holds fewer refinement sweeps than a solve needed (the gate word
+// is the solve's slot): the host captures one more for that slot and runs the step again.
+static constexpr int ERR_SWEEPS = 100;
+
 enum Slot { S_HELM_U = 0, S_HELM_V = 1, S_P0 = 2, S_P1 = 3, S_P2 = 4 };
 
 __device__ __forceinline__ unsigned long long dbits(double v) { return __double_as_longlong(v); }
@@ -564,10 +568,12 @@ struct TailArgs {
   double factor, dgx, dgy;
   unsigned long long *coupled, *umax;         // umax: max |u|, then max |v|
 };
-void launch_proj_rhs(const CaseDev& c, const double* U, double* out, double dt, ProjCheck chk, int nchk, const Gate& gate,
-                     cudaStream_t st);
+// sweeps: those launched for the solve(s) the gate is behind (ERR_SWEEPS when they needed more;
+// nchk - 1: all of them); pdl: the kernel in front is an ordinary one of the same stream
+void launch_proj_rhs(const CaseDev& c, const double* U, double* out, double dt, ProjCheck chk, int nchk, int sweeps_u,
+                     int sweeps_v, const Gate& gate, cudaStream_t st);
 void launch_proj_update(const CaseDev& c, const double* q, double* phi, double dt, double* out, int slot, int nchk,
-                        const Gate& gate, cudaStream_t st);
+                        int sweeps, bool pdl, const Gate& gate, cudaStream_t st);
 void launch_proj_tail(const CaseDev& c, const ResidualCoef& rcu, const ResidualCoef& rcv, ProjTail kind, const TailArgs& a,
                       const Gate& gate, cudaStream_t st);
 // The end of a step: the gate of the second projection, the ghost values of the two new pressures, the
