@@ -238,7 +238,6 @@ struct gm_handle {
   cudaEvent_t ev_fork = nullptr, ev_join = nullptr;
   DBuf<double> spectral_b;
   DBuf<float> spectral32_b;
-  long long body_nodes_slot[5] = {0, 0, 0, 0, 0};  // kernels per refinement sweep of each solve slot
   bool use_graphs = true;
   bool capturing = false;
   // A step graph holds a fixed number of gated refinement sweeps for each solve slot and no loop: a
@@ -246,7 +245,7 @@ struct gm_handle {
   // 25 us of a 220 us step in FP64, which needs no sweep, and about 50 in the FP32 mode.  A solve that
   // needs more than its slot's stops the steps behind it (ERR_SWEEPS); the host adds one and repeats
   // the step.  FP64 starts with none, the FP32 mode with the one that it always needs.
-  bool loops = true;  // captures as WHILE nodes (batches, whose cases the host cannot repeat alone; cut-cell)
+  bool loops = true;  // captures as WHILE nodes (the cut-cell step)
   int sweeps[5] = {0, 0, 0, 0, 0};
   // launch-by-launch steps decide every refinement sweep on the host (one synchronisation
   // per sweep) instead of launching all sweeps gated: then every launched kernel does work,
@@ -1247,11 +1246,9 @@ void schur_solve_graph(gm_handle* h, int lane, RectDev& rd, int kind, double hc,
   cudaGraph_t body = cp.conditional.phGraph_out[0];
   CK(cudaStreamUpdateCaptureDependencies(st, &cnode, nullptr, 1, cudaStreamSetCaptureDependencies));
   CK(cudaStreamBeginCaptureToGraph(body_st, body, nullptr, nullptr, 0, cudaStreamCaptureModeRelaxed));
-  long long c0 = kernel_launch_count();
   apply_inverse(h, lane, rd, kind, resb, f32, x, true, first, w2, g0, body_st);
   launch_residual(h->cd, h->rcoef[kind], kind, b, x, resb, f32, sc, -1, false, g0, body_st);
   launch_refine_decide(h->ctl.p, slot, h->nchk, cond, body_st);
-  h->body_nodes_slot[slot] = kernel_launch_count() - c0;
   CK(cudaStreamEndCapture(body_st, &body));
 }
 
@@ -3099,8 +3096,7 @@ struct gm_batch {
     std::vector<const double*> key;
     std::vector<long long> gens;
     double dt = 0;
-    std::vector<long long> outer;               // per-case kernel nodes outside the refinement loops
-    std::vector<std::array<long long, 5>> body;  // per-case kernel nodes of one sweep, per solve slot
+    std::vector<long long> outer;  // kernel nodes of a case's own branch
     long long group_outer = 0;                          // case-indexed solves: nodes outside the loops
     std::vector<std::array<long long, 5>> group_body;   // and per group, one sweep per solve slot
   } graphs[2];
@@ -3507,8 +3503,11 @@ std::vector<const double*> batch_key(gm_batch* b) {
 
 gm_batch::Graph& batch_graph(gm_batch* b, double dt) {
   std::vector<const double*> key = batch_key(b);
-  std::vector<long long> gens;
-  for (gm_handle* h : b->cases) gens.push_back(h->helm_gen);
+  std::vector<long long> gens;  // what else a captured step depends on: Helmholtz tables, sweeps
+  for (gm_handle* h : b->cases) {
+    gens.push_back(h->helm_gen);
+    gens.insert(gens.end(), h->sweeps, h->sweeps + 5);
+  }
   for (auto& gr : b->graphs)
     if (gr.exec && gr.dt == dt && gr.key == key && gr.gens == gens) return gr;
   gm_batch::Graph* slot = !b->graphs[0].exec ? &b->graphs[0] : (!b->graphs[1].exec ? &b->graphs[1] : nullptr);
@@ -3518,7 +3517,6 @@ gm_batch::Graph& batch_graph(gm_batch* b, double dt) {
     slot->exec = nullptr;
   }
   slot->outer.assign(b->cases.size(), 0);
-  slot->body.assign(b->cases.size(), std::array<long long, 5>{});
   slot->group_outer = 0;
   slot->group_body.clear();
   batch_shapes(b);
@@ -3531,7 +3529,6 @@ gm_batch::Graph& batch_graph(gm_batch* b, double dt) {
       for (size_t c = 0; c < b->cases.size(); ++c) {
         gm_handle* h = b->cases[c];
         CK(cudaStreamWaitEvent(h->st, b->fork, 0));
-        std::fill(h->body_nodes_slot, h->body_nodes_slot + 5, 0LL);
         h->capturing = true;
       }
       const long long c0 = kernel_launch_count();
@@ -3548,23 +3545,18 @@ gm_batch::Graph& batch_graph(gm_batch* b, double dt) {
       gm_handle* h = b->cases[c];
       CK(cudaStreamWaitEvent(h->st, b->fork, 0));
       const long long c0 = kernel_launch_count();
-      std::fill(h->body_nodes_slot, h->body_nodes_slot + 5, 0LL);
       h->capturing = true;
+      h->loops = false;
       step_once(h, dt, -1);
       h->capturing = false;
-      const long long captured = kernel_launch_count() - c0;
-      kernel_launch_adjust(-captured);
-      long long body_total = 0;
-      for (int q = 0; q < 5; ++q) {
-        slot->body[c][q] = h->body_nodes_slot[q];
-        body_total += h->body_nodes_slot[q];
-      }
-      slot->outer[c] = captured - body_total;
+      h->loops = true;
+      slot->outer[c] = kernel_launch_count() - c0;
+      kernel_launch_adjust(-slot->outer[c]);
       CK(cudaEventRecord(b->join[c], h->st));
       CK(cudaStreamWaitEvent(b->root, b->join[c], 0));
     }
   } catch (...) {
-    for (gm_handle* h : b->cases) h->capturing = false;
+    for (gm_handle* h : b->cases) { h->capturing = false; h->loops = true; }
     cudaStreamEndCapture(b->root, &g);
     if (g) cudaGraphDestroy(g);
     cudaGetLastError();
@@ -3680,16 +3672,40 @@ int gm_batch_step(gm_batch* b, double dt, int32_t n_steps, int64_t first_step_in
         int good = 0;
         while (good < batch && h->host_ring[good].err == 0) ++good;
         const double t0 = start_times ? start_times[c] : 0.0;
+        if (steady) nodes += batch * (b->graphs[0].exec ? b->graphs[0] : b->graphs[1]).outer[c];
+        if (good < batch && h->host_ring[good].err == ERR_SWEEPS) {
+          // a solve needs a sweep more than the graph holds: this case goes back to the state before
+          // that step and takes the rest of the graph batch alone (the same kernels, so the same
+          // values), the next graph holds the sweep
+          for (int k = 0; k < good; ++k)
+            if (diag) fill_diag(h, h->host_ring[k], t0 + (s + k + 1) * dt, dt, false, &diag[(size_t)c * n_steps + s + k]);
+          if ((batch - good) % 2) swap_state(h);
+          ++h->sweeps[h->host_ring[good].gate];
+          std::vector<gm_step_diag> rest(batch - good);
+          int done = 0;
+          try {
+            step_loop(h, dt, batch - good, first_step_index + s + good, t0 + (s + good) * dt, rest.data(), {});
+            done = batch - good;
+          } catch (const GateError& e) {
+            while (done < batch - good && rest[done].status == 0) ++done;
+            if (first_error == GM_OK) {
+              first_error = e.cls;
+              b->err = "case " + std::to_string(c) + ": gate " + std::to_string(rest[done].gate) + " failed at step " +
+                       std::to_string(first_step_index + s + good + done);
+            }
+          }
+          if (diag) std::copy(rest.begin(), rest.begin() + std::min(batch - good, done + 1), &diag[(size_t)c * n_steps + s + good]);
+          if (steps_done) steps_done[c] = s + good + done;
+          // a graph batch that follows expects a clear control block and its own counter
+          CK(cudaMemsetAsync(h->ctl.p, 0, sizeof(StepCtl), h->st));
+          const long long next = first_step_index + s + batch;
+          CK(cudaMemcpyAsync(h->counter.p, &next, sizeof next, cudaMemcpyHostToDevice, h->st));
+          CK(cudaStreamSynchronize(h->st));
+          continue;
+        }
         for (int k = 0; k < std::min(batch, good + 1); ++k)
           if (diag) fill_diag(h, h->host_ring[k], t0 + (s + k + 1) * dt, dt, first && k == 0,
                               &diag[(size_t)c * n_steps + s + k]);
-        if (steady) {
-          const gm_batch::Graph& gr = b->graphs[0].exec ? b->graphs[0] : b->graphs[1];
-          for (int k = 0; k < batch; ++k) {
-            nodes += gr.outer[c];
-            for (int sl = 0; sl < 5; ++sl) nodes += gr.body[c][sl] * h->host_ring[k].solve[sl].k;
-          }
-        }
         if (steps_done) steps_done[c] = s + good;
         if (good > 0) { h->has_history = true; h->prev_dt = dt; }
         if (good < batch) {
