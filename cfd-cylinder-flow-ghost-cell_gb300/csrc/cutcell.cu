@@ -20,9 +20,8 @@
 //                merging, covered faces zero, and the packed output (or the CN operator
 //                x - dt/2 a for GMRES)
 // The CN system is solved by GMRES(30) without a preconditioner (scipy.sparse.linalg.gmres of
-// solver/time_integration.py:99-101, rtol 1e-12, atol 1e-13) with its control on the device:
-// one WHILE node per restart cycle, one IF node per Arnoldi step, two classical Gram-Schmidt
-// passes.  The three pressure solves per step use the pressure-only handle of ghostmac.cu
+// solver/time_integration.py:99-101, rtol 1e-12, atol 1e-13) with its control on the device, over
+// an operator on packed vectors that takes one pass (k_cn_eval, k_cn_apply).  The three pressure solves per step use the pressure-only handle of ghostmac.cu
 // over the cut-cell Poisson operator (internal.hpp).  One step is one CUDA graph.
 #include <cuda_runtime.h>
 
@@ -172,37 +171,49 @@ struct CcDiagDev {
   double res_linf, res_l2;     // the legacy step's pressure residual b - A phi (unscaled rows)
 };
 
+// (row, column) of flat index t on a grid of n columns, in 32 bits (faces are fewer than 2^31): a 64-bit
+// division by a run-time value costs some 80 instructions, more than most of these kernels' arithmetic
+struct RowCol { int j, i; };
+__device__ __forceinline__ RowCol row_col(int64_t t, int n) {
+  const unsigned q = (unsigned)t / (unsigned)n;
+  return {(int)q, (int)((unsigned)t - q * (unsigned)n)};
+}
+
 // field value c of the concatenated face grid, with the inlet column from `inl` when given
 __device__ __forceinline__ double fld(const CcGeo& g, const double* __restrict__ X, const double* __restrict__ inl,
                                       int64_t c) {
-  if (inl && c < g.usize && c % (g.nx + 1) == 0) return inl[c / (g.nx + 1)];
+  if (inl && c < g.usize) {
+    const auto [j, i] = row_col(c, g.nx + 1);
+    if (i == 0) return inl[j];
+  }
   return X[c];
 }
 
-__device__ __forceinline__ void atomic_max_abs(unsigned long long* out, double v) {
-  atomicMax(out, (unsigned long long)__double_as_longlong(fabs(v)));
+// Maxima of |v| run on the bits (non-negative doubles order like them, a NaN above all): integer
+// comparisons keep the FP64 pipe, 1/64 of the FP32 rate, for the arithmetic.
+using MaxBits = unsigned long long;
+__device__ __forceinline__ MaxBits max_abs(MaxBits m, double v) {
+  const MaxBits b = (MaxBits)__double_as_longlong(v) & 0x7fffffffffffffffull;
+  return b > m ? b : m;
 }
-
-// the block's maximum |m| (a NaN stays visible) committed with one atomic: warp maxima, then
-// the first warp over the block's warps
-__device__ __forceinline__ void block_commit_max_abs(double m, unsigned long long* out) {
-  __shared__ double wm[32];
-  for (int o = 16; o; o >>= 1) {
-    const double q = __shfl_down_sync(0xffffffffu, m, o);
-    m = (q != q) ? q : fmax(m, q);
-  }
+// the block's maximum committed with one atomic: warp maxima, then the first warp over the block's warps
+__device__ __forceinline__ void block_commit_max(MaxBits m, unsigned long long* out) {
+  __shared__ MaxBits wm[32];
+  auto warp_max = [](MaxBits v) {
+    for (int o = 16; o; o >>= 1) {
+      const MaxBits q = __shfl_xor_sync(0xffffffffu, v, o);
+      v = q > v ? q : v;
+    }
+    return v;
+  };
+  m = warp_max(m);
   const int lane = threadIdx.x & 31, w = threadIdx.x >> 5;
   __syncthreads();  // an earlier call's readers are done with wm
   if (lane == 0) wm[w] = m;
   __syncthreads();
   if (w == 0) {
-    const int nw = (blockDim.x + 31) >> 5;
-    m = lane < nw ? wm[lane] : 0.0;
-    for (int o = 16; o; o >>= 1) {
-      const double q = __shfl_down_sync(0xffffffffu, m, o);
-      m = (q != q) ? q : fmax(m, q);
-    }
-    if (lane == 0) atomic_max_abs(out, m);
+    m = warp_max(lane < (int)((blockDim.x + 31) >> 5) ? wm[lane] : 0);
+    if (lane == 0) atomicMax(out, m);
   }
 }
 
@@ -231,7 +242,7 @@ __global__ void k_cc_flux(CcGeo g, const double* __restrict__ X, const double* _
   const int nx = g.nx, ny = g.ny;
   const int64_t t = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
   if (t >= (int64_t)(ny + 1) * (nx + 1)) return;
-  const int j = (int)(t / (nx + 1)), i = (int)(t % (nx + 1));
+  const auto [j, i] = row_col(t, nx + 1);
   const double* V = X + g.usize;
   auto U = [&](int jj, int ii) -> double {
     const int64_t f = (int64_t)jj * (nx + 1) + ii;
@@ -325,7 +336,7 @@ template <bool ADV>
 __device__ __forceinline__ double rhs_base(const CcGeo& g, const CcFlux& F, const double* __restrict__ X, int64_t f) {
   const int nx = g.nx, ny = g.ny;
   if (f < g.usize) {
-    const int j = (int)(f / (nx + 1)), i = (int)(f % (nx + 1));
+    const auto [j, i] = row_col(f, nx + 1);
     if (i >= 1 && i < nx)
       return (F.xx[(int64_t)j * nx + i] - F.xx[(int64_t)j * nx + i - 1]) + (F.xy[f + nx + 1] - F.xy[f]);
     if (i == nx) {
@@ -339,7 +350,7 @@ __device__ __forceinline__ double rhs_base(const CcGeo& g, const CcFlux& F, cons
     return 0.0;
   }
   const int64_t c = f - g.usize;
-  const int j = (int)(c / nx), i = (int)(c % nx);
+  const auto [j, i] = row_col(c, nx);
   if (j >= 1 && j < ny)
     return (F.yx[(int64_t)j * (nx + 1) + i + 1] - F.yx[(int64_t)j * (nx + 1) + i]) + (F.yy[c] - F.yy[c - nx]);
   return 0.0;
@@ -431,7 +442,7 @@ __global__ void k_cc_divrhs(CcGeo g, const double* __restrict__ X, const double*
   if (c >= g.psize) return;
   if (g.cell_type[c] == -1) { B[c] = 0.0; return; }
   const int nx = g.nx;
-  const int j = (int)(c / nx), i = (int)(c % nx);
+  const auto [j, i] = row_col(c, nx);
   const int64_t fu = (int64_t)j * (nx + 1) + i;
   const double uw = (i == 0 && inl) ? inl[j] : X[fu];
   const double* V = X + g.usize;
@@ -447,46 +458,57 @@ __global__ void k_cc_scale_rhs(CcGeo g, double* __restrict__ B) {
   B[c] = g.cell_type[c] == -1 ? 0.0 : B[c] * g.ikappa[c];
 }
 
-// corrector (solver/cut_cell_solver.py:740-753), packed output; sx = dt / (rho dx), sy = dt / (rho dy)
+// corrector (solver/cut_cell_solver.py:740-753), packed output; sx = dt / (rho dx), sy = dt / (rho dy).
+// With a residual: also the predicted divergence dt/rho max_fluid |res| / kappa (:721-722; the residual
+// of the row-scaled system already carries the 1 / kappa).
 __global__ void k_cc_correct(CcGeo g, const double* __restrict__ X, const double* __restrict__ phi, double sx,
-                             double sy, double* __restrict__ Y) {
-  const int64_t f = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
-  if (f >= g.F) return;
+                             double sy, double* __restrict__ Y, const double* __restrict__ res, double scale,
+                             unsigned long long* out) {
   const int nx = g.nx, ny = g.ny;
-  double r = 0.0;
-  if (f < g.usize) {
-    const int j = (int)(f / (nx + 1)), i = (int)(f % (nx + 1));
-    const int64_t c = (int64_t)j * nx + i;
-    if (i >= 1 && i < nx) r = g.ax[f] > 0.0 ? X[f] - sx * (phi[c] - phi[c - 1]) : 0.0;
-    else if (i == nx) r = X[f] + (2.0 * sx) * phi[c - 1];
-  } else {
-    const int64_t c = f - g.usize;
-    const int j = (int)(c / nx);
-    if (j >= 1 && j < ny) r = g.ay[c] > 0.0 ? X[f] - sy * (phi[c] - phi[c - nx]) : 0.0;
+  MaxBits m = 0;
+  for (int64_t f = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; f < g.F; f += (int64_t)gridDim.x * blockDim.x) {
+    double r = 0.0;
+    if (f < g.usize) {
+      const auto [j, i] = row_col(f, nx + 1);
+      const int64_t c = (int64_t)j * nx + i;
+      if (i >= 1 && i < nx) r = g.ax[f] > 0.0 ? X[f] - sx * (phi[c] - phi[c - 1]) : 0.0;
+      else if (i == nx) r = X[f] + (2.0 * sx) * phi[c - 1];
+    } else {
+      const int64_t c = f - g.usize;
+      const int j = row_col(c, nx).j;
+      if (j >= 1 && j < ny) r = g.ay[c] > 0.0 ? X[f] - sy * (phi[c] - phi[c - nx]) : 0.0;
+    }
+    Y[f] = (g.flags[f] & F_ACTIVE) ? r : 0.0;
+    if (res && f < g.psize && g.cell_type[f] != -1) m = max_abs(m, scale * res[f]);
   }
-  Y[f] = (g.flags[f] & F_ACTIVE) ? r : 0.0;
+  if (res) block_commit_max(m, out);
 }
 
-// pressure gradient / rho on the unknown faces (advance_ab2_cn's gradient,
-// solver/cut_cell_solver.py:979-984); gx = 1 / (rho dx), gy = 1 / (rho dy)
-__global__ void k_cc_grad(CcGeo g, const double* __restrict__ P, double gx, double gy, double* __restrict__ Y) {
-  const int64_t f = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
-  if (f >= g.F) return;
+// pressure gradient / rho at face f (advance_ab2_cn's gradient, solver/cut_cell_solver.py:979-984), zero on
+// faces that are not unknown; gx = 1 / (rho dx), gy = 1 / (rho dy)
+__device__ __forceinline__ double face_grad(const CcGeo& g, const double* __restrict__ P, double gx, double gy, int64_t f) {
+  if (!(g.flags[f] & F_ACTIVE)) return 0.0;
   const int nx = g.nx, ny = g.ny;
-  double r = 0.0;
   if (f < g.usize) {
-    const int j = (int)(f / (nx + 1)), i = (int)(f % (nx + 1));
+    const auto [j, i] = row_col(f, nx + 1);
     const int64_t c = (int64_t)j * nx + i;
-    if (i >= 1 && i < nx) r = (P[c] - P[c - 1]) * gx;
-    else if (i == nx) r = -2.0 * P[c - 1] * gx;
-  } else {
-    const int64_t c = f - g.usize;
-    const int j = (int)(c / nx);
-    if (j >= 1 && j < ny) r = (P[c] - P[c - nx]) * gy;
+    if (i >= 1 && i < nx) return (P[c] - P[c - 1]) * gx;
+    return i == nx ? -2.0 * P[c - 1] * gx : 0.0;
   }
-  Y[f] = (g.flags[f] & F_ACTIVE) ? r : 0.0;
+  const int64_t c = f - g.usize;
+  const int j = row_col(c, nx).j;
+  return j >= 1 && j < ny ? (P[c] - P[c - nx]) * gy : 0.0;
 }
 
+// face f of the unpacked field: inlet column, packed values on the unknown faces, zero elsewhere
+__device__ __forceinline__ double unpacked(const CcGeo& g, const double* __restrict__ X, const double* __restrict__ inl,
+                                           int64_t f) {
+  if (f < g.usize) {
+    const auto [j, i] = row_col(f, g.nx + 1);
+    if (i == 0) return inl[j];
+  }
+  return (g.flags[f] & F_ACTIVE) ? X[f] : 0.0;
+}
 // pack (X = masked U) and unpack (U = X with the inlet column)
 __global__ void k_cc_pack(CcGeo g, const double* __restrict__ U, double* __restrict__ X) {
   const int64_t f = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
@@ -496,81 +518,49 @@ __global__ void k_cc_unpack(CcGeo g, const double* __restrict__ X, const double*
                             double* __restrict__ U) {
   const int64_t f = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
   if (f >= g.F) return;
-  if (f < g.usize && f % (g.nx + 1) == 0) U[f] = inl[f / (g.nx + 1)];
-  else U[f] = (g.flags[f] & F_ACTIVE) ? X[f] : 0.0;
+  U[f] = unpacked(g, X, inl, f);
 }
 
-// ---- vector steps of solver/time_integration.py:7-145 -------------------------------------
-// op 0: out = a + s0 ((b + c) - d)            midpoint start-up
-// op 1: out = (1 + s0) a - s0 b               AB2 advection
-// op 2: out = (a + s0 ((b + 0.5 c) - d)) + s1 e   CN right-hand side
-// op 3: out = a + (b - c)                     projected result plus the momentum defect
-__global__ void k_cc_vec(int op, int64_t n, const double* __restrict__ a, const double* __restrict__ b,
-                         const double* __restrict__ c, const double* __restrict__ d, const double* __restrict__ e,
-                         double s0, double s1, double* __restrict__ out) {
-  const int64_t t = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
-  if (t >= n) return;
-  double r;
-  if (op == 0) r = a[t] + s0 * ((b[t] + c[t]) - d[t]);
-  else if (op == 1) r = (1 + s0) * a[t] - s0 * b[t];
-  else if (op == 2) r = (a[t] + s0 * ((b[t] + 0.5 * c[t]) - d[t])) + s1 * e[t];
-  else r = a[t] + (b[t] - c[t]);
-  out[t] = r;
-}
-// half = p + inc; out = half + factor inc
-__global__ void k_cc_pressure_out(int64_t n, const double* __restrict__ p, const double* __restrict__ inc,
-                                  double factor, double* __restrict__ half, double* __restrict__ out) {
-  const int64_t t = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
-  if (t >= n) return;
-  const double h = p[t] + inc[t];
-  half[t] = h;
-  out[t] = h + factor * inc[t];
-}
 // max |a - b| (b may be null), max |(a - b) + s c| with c set
 __global__ void k_cc_maxdiff(int64_t n, const double* __restrict__ a, const double* __restrict__ b,
                              const double* __restrict__ c, double s, unsigned long long* out) {
-  double m = 0.0;
+  MaxBits m = 0;
   for (int64_t t = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; t < n; t += (int64_t)gridDim.x * blockDim.x) {
     double v = b ? a[t] - b[t] : a[t];
     if (c) v = v + s * c[t];
-    m = fmax(m, fabs(v));
-    if (v != v) m = v;  // keep a NaN visible
+    m = max_abs(m, v);
   }
-  block_commit_max_abs(m, out);
+  block_commit_max(m, out);
 }
 // predicted divergence dt/rho max_fluid |res| / kappa (solver/cut_cell_solver.py:721-722); the
 // residual of the row-scaled system already carries the 1 / kappa
 __global__ void k_cc_pdiv(CcGeo g, const double* __restrict__ res, double scale, unsigned long long* out) {
-  double m = 0.0;
+  MaxBits m = 0;
   for (int64_t c = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; c < g.psize; c += (int64_t)gridDim.x * blockDim.x)
-    if (g.cell_type[c] != -1) {
-      const double v = scale * fabs(res[c]);
-      m = (v != v) ? v : fmax(m, v);
-    }
-  block_commit_max_abs(m, out);
+    if (g.cell_type[c] != -1) m = max_abs(m, scale * res[c]);
+  block_commit_max(m, out);
 }
 // step gate quantities of solver/main.py:416-424: max_fluid |flux divergence| / kappa, max |u|, max |v|
 __global__ void k_cc_stepmax(CcGeo g, const double* __restrict__ U, unsigned long long* divmax,
                              unsigned long long* umax, unsigned long long* vmax) {
   const int nx = g.nx;
-  double dm = 0.0, um = 0.0, vm = 0.0;
+  MaxBits dm = 0, um = 0, vm = 0;
   const double* V = U + g.usize;
   for (int64_t f = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; f < g.F; f += (int64_t)gridDim.x * blockDim.x) {
-    if (f < g.usize) um = fmax(um, fabs(U[f]));
-    else vm = fmax(vm, fabs(U[f]));
+    if (f < g.usize) um = max_abs(um, U[f]);
+    else vm = max_abs(vm, U[f]);
     if (f < g.psize && g.cell_type[f] != -1) {
       const int64_t c = f;
-      const int j = (int)(c / nx), i = (int)(c % nx);
+      const auto [j, i] = row_col(c, nx);
       const int64_t fu = (int64_t)j * (nx + 1) + i;
       const double d = (g.ax[fu + 1] * U[fu + 1] - g.ax[fu] * U[fu]) * g.idx +
                        (g.ay[c + nx] * V[c + nx] - g.ay[c] * V[c]) * g.idy;
-      const double v = fabs(d) * g.ikappa[c];
-      dm = (v != v) ? v : fmax(dm, v);
+      dm = max_abs(dm, d * g.ikappa[c]);
     }
   }
-  block_commit_max_abs(dm, divmax);
-  block_commit_max_abs(um, umax);
-  block_commit_max_abs(vm, vmax);
+  block_commit_max(dm, divmax);
+  block_commit_max(um, umax);
+  block_commit_max(vm, vmax);
 }
 
 // The legacy predictor (advance_momentum_predictor, solver/cut_cell_solver.py:1017-1033) and
@@ -587,11 +577,12 @@ __global__ void k_cc_legacy_pred(CcGeo g, const double* __restrict__ U, const do
   double s = ab2 ? U[f] + dt * ((1 + alpha) * a - alpha * prev[f]) : U[f] + dt * a;
   prev[f] = a;
   if (f < g.usize) {
-    if (f % (g.nx + 1) == 0) s = inl[f / (g.nx + 1)];
+    const auto [j, i] = row_col(f, g.nx + 1);
+    if (i == 0) s = inl[j];
     if (g.ax[f] == 0.0) s = 0.0;
   } else {
     const int64_t c = f - g.usize;
-    const int j = (int)(c / g.nx);
+    const int j = row_col(c, g.nx).j;
     if (g.ay[c] == 0.0 || j == 0 || j == g.ny) s = 0.0;
   }
   star[f] = s;
@@ -651,44 +642,41 @@ __global__ void k_cc_resnorm_fold(const double* __restrict__ part, int nb, doubl
   }
 }
 
-// fixed-order block sum of one value per thread (blockDim a power of two <= 1024)
+// fixed-order block sum of one value per thread, the same in every thread (at most 32 warps)
 __device__ double block_sum(double v, double* sh) {
-  const int tid = threadIdx.x;
-  sh[tid] = v;
+  for (int o = 16; o; o >>= 1) v += __shfl_xor_sync(0xffffffffu, v, o);
+  if ((threadIdx.x & 31) == 0) sh[threadIdx.x >> 5] = v;
   __syncthreads();
-  for (int s = blockDim.x / 2; s > 0; s >>= 1) {
-    if (tid < s) sh[tid] = sh[tid] + sh[tid + s];
-    __syncthreads();
-  }
-  const double r = sh[0];
+  v = (int)(threadIdx.x & 31) < (int)(blockDim.x >> 5) ? sh[threadIdx.x & 31] : 0.0;
+  for (int o = 16; o; o >>= 1) v += __shfl_xor_sync(0xffffffffu, v, o);
   __syncthreads();
-  return r;
+  return v;
 }
 
-// mu (rate . field) at every wall Gauss point, one warp each: the wall shear stress of the
-// forces (the same warp dot product as the forces kernel's, so the same values)
-__global__ void k_cc_wall_tau(CcWall w, const double* __restrict__ U, double mu, double* __restrict__ tau) {
+// mu (rate . field) at every wall Gauss point and the pressure at every surface point, one warp each
+__global__ void k_cc_wall_points(gmi::SurfaceCsr S, CcWall w, const double* __restrict__ U, const double* __restrict__ P,
+                                 double mu, double* __restrict__ tau, double* __restrict__ pb) {
   const int lane = threadIdx.x & 31;
   const int k = (int)(((int64_t)blockIdx.x * blockDim.x + threadIdx.x) >> 5);
-  if (k >= w.n) return;  // whole warps leave together
-  const double acc = warp_row_dot(w.ptr, w.col, w.val, k, CcGeo{}, U, nullptr, lane);
-  if (lane == 0) tau[k] = mu * acc;
+  if (k >= w.n + S.n) return;  // whole warps leave together
+  const bool wall = k < w.n;
+  const double acc = wall ? warp_row_dot(w.ptr, w.col, w.val, k, CcGeo{}, U, nullptr, lane)
+                          : warp_row_dot(S.ptr, S.col, S.val, k - w.n, CcGeo{}, P, nullptr, lane);
+  if (lane == 0) {
+    if (wall) tau[k] = mu * acc;
+    else pb[k - w.n] = acc;
+  }
 }
 
 // Forces on the true circle (extract_true_surface_forces, solver/cut_cell_solver.py:755-765):
 // pressure from the point reconstruction with its mean removed, shear mu (rate . field) at
 // the wall Gauss points.  One block; out = fx, fy, fx_p, fy_p, fx_v, fy_v.
-__global__ void k_cc_forces(gmi::SurfaceCsr S, CcWall w, const double* __restrict__ P,
-                            const double* __restrict__ tau, double* __restrict__ pb, double* __restrict__ out) {
+__global__ void k_cc_forces(gmi::SurfaceCsr S, CcWall w, const double* __restrict__ tau, const double* __restrict__ pb,
+                            double* __restrict__ out) {
   __shared__ double sh[CC_FORCE_THREADS];
   const int tid = threadIdx.x, nt = blockDim.x;
   double s = 0.0;
-  for (int k = tid; k < S.n; k += nt) {
-    double acc = 0.0;
-    for (int64_t e = S.ptr[k]; e < S.ptr[k + 1]; ++e) acc += S.val[e] * P[S.col[e]];
-    pb[k] = acc;
-    s += acc;
-  }
+  for (int k = tid; k < S.n; k += nt) s += pb[k];
   const double mean = block_sum(s, sh) / S.n;
   double px = 0.0, py = 0.0;
   for (int k = tid; k < S.n; k += nt) {
@@ -696,14 +684,13 @@ __global__ void k_cc_forces(gmi::SurfaceCsr S, CcWall w, const double* __restric
     px += d * S.nwx[k];
     py += d * S.nwy[k];
   }
-  const double fxp = -block_sum(px, sh), fyp = -block_sum(py, sh);
   double vx = 0.0, vy = 0.0;
-  const int lane = tid & 31, warp = tid >> 5, nwarp = nt >> 5;
-  if (lane == 0)
-    for (int k = warp; k < w.n; k += nwarp) {
-      vx += tau[k] * w.tx[k] * w.ds[k];
-      vy += tau[k] * w.ty[k] * w.ds[k];
-    }
+  for (int k = tid; k < w.n; k += nt) {
+    const double t = tau[k] * w.ds[k];
+    vx += t * w.tx[k];
+    vy += t * w.ty[k];
+  }
+  const double fxp = -block_sum(px, sh), fyp = -block_sum(py, sh);
   const double fxv = block_sum(vx, sh), fyv = block_sum(vy, sh);
   if (tid == 0) {
     out[0] = fxp + fxv;
@@ -724,7 +711,7 @@ __global__ void k_cc_divstats(CcGeo g, const double* __restrict__ U, double* __r
   double mdiv = 0.0, sq = 0.0, cnt = 0.0, mflux = 0.0;
   for (int64_t c = threadIdx.x; c < g.psize; c += blockDim.x) {
     if (g.cell_type[c] == -1) continue;
-    const int j = (int)(c / nx), i = (int)(c % nx);
+    const auto [j, i] = row_col(c, nx);
     const int64_t fu = (int64_t)j * (nx + 1) + i;
     const double fx = g.ax[fu + 1] * g.dy * U[fu + 1] - g.ax[fu] * g.dy * U[fu];
     const double fy = g.ay[c + nx] * g.dx * V[c + nx] - g.ay[c] * g.dx * V[c];
@@ -759,148 +746,479 @@ __global__ void k_cc_divstats(CcGeo g, const double* __restrict__ U, double* __r
   }
 }
 
-// ---- Gram-Schmidt of the CN GMRES -------------------------------------------------------
-// Two classical passes per Arnoldi step with the basis read once per pass: k_gs_dot forms the
-// partial dots V^T w; k_gs_pass<NV, NORM> reduces the previous partials to the coefficients
-// (every block in the same fixed order, so all blocks hold identical values), subtracts V c
-// from w and, in the same sweep, forms the partials of the next pass (V^T w) or of |w|^2.
-// One block per SM; NV (the basis size, a compile-time constant per Arnoldi step) keeps the
-// accumulators in registers.
-constexpr int GS_BLOCKS = 152;
-constexpr int GS_THREADS = 512;
-constexpr int GS_MAXV = 32;
+// ---- the viscous operator of the CN step --------------------------------------------------
+// L x on packed vectors (zero on faces that are not unknown; the inlet's part is the constant vector
+// `offset`).  By flux arrays it is three kernels (k_cc_flux, k_cc_fix, k_cc_rhs: 45 us at 800x410, four
+// arrays through L2 and three launches); as an operator on packed vectors it is one pass, because
+// every face near the body is one sparse row formed at set-up (curved fluxes, wall shear, covered
+// transfers and merging are linear), and every other face is a five-point stencil: the constant one
+// where apertures and volumes are full, the structured one at the channel's edges.  16 us with the vector
+// step behind it at 800x410; the FP64 pipe is the bound (5 multiply-adds a regular face).
+struct CnOp {
+  const uint8_t* cls;    // per face: CN_ZERO, CN_REGULAR, CN_EDGE or CN_ROW
+  int n_row;             // rows near the body
+  const int32_t* face;
+  const int64_t* ptr;
+  const int32_t* col;
+  const double* val;
+  double kx, ky;         // nu / dx^2, nu / dy^2 of the regular faces
+  double rnu;
+  int slip;
+};
+enum : uint8_t { CN_ZERO = 0, CN_REGULAR = 1, CN_EDGE = 2, CN_ROW = 3 };
 
-template <int NV>
-__device__ __forceinline__ void gs_block_partials(double (&acc)[NV], double* __restrict__ part) {
-  __shared__ double red[GS_THREADS / 32][NV];
+// (L x)(f) of a face at the channel's edge, or with apertures or a volume of its own
+__device__ double cn_edge(const CcGeo& g, const CnOp& L, const double* __restrict__ X, int64_t f) {
+  if (!(g.flags[f] & F_FLUID) || (g.flags[f] & F_SOLID)) return 0.0;
+  const int nx = g.nx, ny = g.ny;
+  double r = 0.0;
+  if (f < g.usize) {
+    const auto [j, i] = row_col(f, nx + 1);
+    const int64_t c = (int64_t)j * nx + i;
+    if (i == 0) return 0.0;
+    const double fs = j == 0 ? (L.slip ? 0.0 : X[f] * (2.0 * g.cxy[f])) : (X[f] - X[f - nx - 1]) * g.cxy[f];
+    const double fn = j == ny - 1 ? (L.slip ? 0.0 : -(X[f] * (2.0 * g.cxy[f + nx + 1])))
+                                  : (X[f + nx + 1] - X[f]) * g.cxy[f + nx + 1];
+    const double fw = (X[f] - X[f - 1]) * g.cxx[c - 1];
+    r = i == nx ? 0.5 * (fn - fs) - fw : ((X[f + 1] - X[f]) * g.cxx[c] - fw) + (fn - fs);
+  } else {
+    const int64_t c = f - g.usize;
+    const auto [j, i] = row_col(c, nx);
+    if (j == 0 || j == ny) return 0.0;
+    const int64_t t = (int64_t)j * (nx + 1) + i;
+    const double fw = i == 0 ? X[f] * (2.0 * g.cyx[t]) : (X[f] - X[f - 1]) * g.cyx[t];
+    const double fe = i + 1 == nx ? 0.0 : (X[f + 1] - X[f]) * g.cyx[t + 1];
+    r = (fe - fw) + ((X[f + nx] - X[f]) * g.cyy[c] - (X[f] - X[f - nx]) * g.cyy[c - nx]);
+  }
+  return L.rnu * r * g.ivol_rho[f];
+}
+
+// the stencil of H on regular faces: H x = c x - x_w (west + east) - y (south + north)
+struct CnH {
+  double hdt, c, x, y;
+};
+inline CnH cn_h(const CnOp& L, double hdt) { return {hdt, 1.0 + 2.0 * (hdt * L.kx + hdt * L.ky), hdt * L.kx, hdt * L.ky}; }
+
+// Every face once over the whole grid of threads: f(face, x, value), value = L x (H = false) or
+// s (x - hdt L x) (H = true, the stencil h holding the factor s); faces that are not unknown report 0, 0.  The rows near the body, a warp
+// each (its lane 0 reports), go to blocks of their own: their chain of loads would otherwise come on
+// top of those warps' share of the sweep.
+template <bool H, class Fn>
+__device__ __forceinline__ void cn_sweep(const CcGeo& g, const CnOp& L, const double* __restrict__ X, const CnH& h, double s,
+                                         Fn&& fn) {
+  const int lane = threadIdx.x & 31, nw = blockDim.x >> 5;
+  const int rb = min((L.n_row + nw - 1) / nw, (int)(gridDim.x / 4));  // at least one when there are rows (gridDim >= 4)
+  if ((int)blockIdx.x < rb) {
+    for (int r = blockIdx.x * nw + (threadIdx.x >> 5); r < L.n_row; r += rb * nw) {
+      double a = 0.0;
+      for (int64_t e = L.ptr[r] + lane, e1 = L.ptr[r + 1]; e < e1; e += 32) a += L.val[e] * X[L.col[e]];
+      for (int o = 16; o; o >>= 1) a += __shfl_xor_sync(0xffffffffu, a, o);
+      if (lane == 0) {
+        const int64_t f = L.face[r];
+        const double x = X[f];
+        fn(f, x, H ? s * (x - h.hdt * a) : a);
+      }
+    }
+    return;
+  }
+  for (int64_t f = (int64_t)(blockIdx.x - rb) * blockDim.x + threadIdx.x; f < g.F; f += (int64_t)(gridDim.x - rb) * blockDim.x) {
+    const uint8_t k = L.cls[f];
+    if (k == CN_ROW) continue;
+    double x = 0.0, v = 0.0;
+    if (k == CN_REGULAR) {
+      const int up = f < g.usize ? g.nx + 1 : g.nx;
+      x = X[f];
+      const double ew = X[f - 1] + X[f + 1], ns = X[f - up] + X[f + up];
+      if (H) v = (h.c * x - h.x * ew) - h.y * ns;
+      else v = L.kx * (ew - 2.0 * x) + L.ky * (ns - 2.0 * x);
+    } else if (k == CN_EDGE) {
+      x = X[f];
+      const double a = cn_edge(g, L, X, f);
+      v = H ? s * (x - h.hdt * a) : a;
+    }
+    fn(f, x, v);
+  }
+}
+
+// The vector steps around the operator (solver/time_integration.py:7-145), one pass each:
+// CN_MID     out = x + dt ((a + d) - grad p), d = L x + offset      (projected midpoint start-up; dt is its half step)
+// CN_RHS     out = (x + dt ((e + d / 2) - grad p)) + hdt offset, out2 = x (the first iterate),
+//            e = (1 + s) a - s b (AB2) or a (b null); max |out|
+// CN_CHECK   max |H x - a|
+// CN_ACTION  out = H x, out2 = x + (a - H x)                           (projected result plus the momentum defect)
+// CN_H       out = H x; CN_L: out = L x + offset
+enum CnMode { CN_MID, CN_RHS, CN_CHECK, CN_ACTION, CN_H, CN_L };
+struct CnEval {
+  const double *x, *a, *b, *offset, *p;
+  double dt, hdt, s, gx, gy;
+  CnH h;
+  double *out, *out2;
+  unsigned long long* mx;
+};
+template <int MODE>
+__global__ void k_cn_eval(CcGeo g, CnOp L, CnEval e) {
+  constexpr bool H = MODE == CN_CHECK || MODE == CN_ACTION || MODE == CN_H;
+  MaxBits m = 0;
+  cn_sweep<H>(g, L, e.x, e.h, 1.0, [&](int64_t f, double x, double v) {
+    if (MODE == CN_MID || MODE == CN_RHS) {
+      const double d = v + e.offset[f], gp = face_grad(g, e.p, e.gx, e.gy, f);
+      if (MODE == CN_MID) e.out[f] = x + e.dt * ((e.a[f] + d) - gp);
+      else {
+        const double ex = e.b ? (1 + e.s) * e.a[f] - e.s * e.b[f] : e.a[f];
+        const double r = (x + e.dt * ((ex + 0.5 * d) - gp)) + e.hdt * e.offset[f];
+        e.out[f] = r;
+        e.out2[f] = x;
+        m = max_abs(m, r);
+      }
+    } else if (MODE == CN_CHECK) {
+      m = max_abs(m, v - e.a[f]);
+    } else if (MODE == CN_ACTION) {
+      e.out[f] = v;
+      e.out2[f] = x + (e.a[f] - v);
+    } else {
+      e.out[f] = MODE == CN_L ? v + e.offset[f] : v;
+    }
+  });
+  if (MODE == CN_RHS || MODE == CN_CHECK) block_commit_max(m, e.mx);
+}
+
+// ---- GMRES(30) of the CN system ---------------------------------------------------------------
+// H x = b from x0 = x (solver/time_integration.py:99-101: rtol 1e-12, atol 1e-13, restart 30, at most
+// 100 cycles), no preconditioner, two classical Gram-Schmidt passes, Givens rotations.  An Arnoldi
+// step is three kernels: k_cn_apply (operator and the first pass's dots while w is in registers),
+// k_cn_pass<false> (first update, second pass's dots) and k_cn_pass<true> (second update, |w|^2).  The
+// last block of the third to finish holds the whole column, so it does the rotations, the
+// convergence test and the next scale: basis vectors stay unscaled in memory (v_i = sc[i] V_i), the
+// scales enter the coefficients.  A step is bound by the FP64 pipe (some 6 + 3 nv multiply-adds a
+// face) and the basis in L2.
+// A step graph holds `steps` Arnoldi steps, each gated by `go`, and no conditional node (8 us each
+// even when its body does not run: 30 of them and the loop were 250 of 590 us).  A system that needs
+// more stops the step (ERR_SWEEPS) before any state is written and the host repeats it with more;
+// beyond 30 the cycle runs in a WHILE node.  At 800x410 (5 Arnoldi steps) the solve took 588 us, now 306;
+// one block of 512 threads an SM, as two cost 12 us more (twice the sums to fold).
+constexpr int CN_BLOCKS = 152;
+constexpr int CN_THREADS = 512;
+constexpr int CN_M = 30;
+constexpr int CN_SHORT = 5;  // gate word of ERR_SWEEPS when the Arnoldi steps did not suffice (below: solve slots)
+struct CnDev {
+  double H[CN_M * CN_M];     // R of the rotated Hessenberg matrix, row i column j at i M + j
+  double cs[CN_M], sn[CN_M], g[CN_M + 1], sc[CN_M + 1], d1[CN_M], coef[CN_M];
+  double tol;
+  int jend, cycle, its, converged, go, nv;
+  unsigned ticket;
+};
+
+// Block sums of NA values a thread, value i of this block to part[i CN_BLOCKS + block].  An FP64 warp
+// instruction occupies the pipe for 16 cycles, so the sums take as few as they can: up to four values
+// go through shared memory to a warp each (21 additions a value instead of 5 a warp and value); for
+// more, lanes exchange halves of their values (about NA + 5 additions a warp instead of 5 NA).
+template <int NA>
+__device__ __forceinline__ void cn_partials_few(double (&acc)[NA], double* __restrict__ part) {
+  __shared__ double red[NA][CN_THREADS];
   const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
 #pragma unroll
-  for (int i = 0; i < NV; ++i) {
-    double a = acc[i];
-    for (int o = 16; o; o >>= 1) a += __shfl_xor_sync(0xffffffffu, a, o);
-    if (lane == 0) red[warp][i] = a;
-  }
+  for (int i = 0; i < NA; ++i) red[i][threadIdx.x] = acc[i];
   __syncthreads();
-  for (int i = threadIdx.x; i < NV; i += blockDim.x) {
-    double a = 0.0;
-    for (int q = 0; q < GS_THREADS / 32; ++q) a += red[q][i];
-    part[(int64_t)blockIdx.x * GS_MAXV + i] = a;
-  }
+  if (warp >= NA) return;
+  double a[4] = {0.0, 0.0, 0.0, 0.0};
+#pragma unroll
+  for (int q = 0; q < CN_THREADS / 32; ++q) a[q & 3] += red[warp][32 * q + lane];
+  double v = (a[0] + a[1]) + (a[2] + a[3]);
+  for (int o = 16; o; o >>= 1) v += __shfl_xor_sync(0xffffffffu, v, o);
+  if (lane == 0) part[(int64_t)warp * CN_BLOCKS + blockIdx.x] = v;
 }
-
-// coefficients c_i = sum over blocks of part[b][i], in a fixed order
-template <int NV>
-__device__ __forceinline__ void gs_coefficients(const double* __restrict__ part, double* cf) {
+template <int NA>
+__device__ __forceinline__ void cn_partials(double (&acc)[NA], int na, double* __restrict__ part) {
+  if constexpr (NA <= 4) {
+    cn_partials_few(acc, part);
+    return;
+  }
+  __shared__ double red[NA][CN_THREADS / 32];
+  constexpr int K = NA > 16 ? 5 : NA > 8 ? 4 : NA > 4 ? 3 : NA > 2 ? 2 : NA > 1 ? 1 : 0;  // 2^K >= NA
   const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
-  if (warp < NV) {
-    double a = 0.0;
-    for (int b = lane; b < GS_BLOCKS; b += 32) a += part[(int64_t)b * GS_MAXV + warp];
-    for (int o = 16; o; o >>= 1) a += __shfl_xor_sync(0xffffffffu, a, o);
-    if (lane == 0) cf[warp] = a;
+#pragma unroll
+  for (int k = 0; k < 5; ++k) {
+    const int o = 16 >> k, half = k < K ? 1 << (K - 1 - k) : 0;  // lane bit o takes the upper half of the values
+    const bool up = (lane & o) != 0;
+#pragma unroll
+    for (int i = 0; i < (k < K ? half : 1); ++i) {
+      if (i < NA) {
+        const bool pair = k < K && i + half < NA;
+        const double other = pair ? acc[pair ? i + half : 0] : acc[i];
+        const double send = pair && !up ? other : acc[i], keep = pair && up ? other : acc[i];
+        acc[i] = keep + __shfl_xor_sync(0xffffffffu, send, o);
+      }
+    }
   }
+  const int i = lane >> (5 - K);
+  if ((lane & ((1 << (5 - K)) - 1)) == 0 && i < NA) red[i][warp] = acc[0];
   __syncthreads();
+  for (int q = threadIdx.x; q < na; q += CN_THREADS) {
+    double a = 0.0;
+    for (int w = 0; w < CN_THREADS / 32; ++w) a += red[q][w];
+    part[(int64_t)q * CN_BLOCKS + blockIdx.x] = a;
+  }
+}
+// sum over the blocks of value i, by one warp in a fixed order
+__device__ __forceinline__ double cn_fold(const double* part, int i, int lane) {
+  double a = 0.0;
+  for (int b = lane; b < CN_BLOCKS; b += 32) a += __ldcg(part + (int64_t)i * CN_BLOCKS + b);
+  for (int o = 16; o; o >>= 1) a += __shfl_xor_sync(0xffffffffu, a, o);
+  return a;
+}
+// whether this block is the last of the grid to get here; what the others wrote before is then visible
+__device__ __forceinline__ bool cn_last_block(CnDev* gd) {
+  __shared__ int last;
+  __threadfence();
+  __syncthreads();
+  if (threadIdx.x == 0) last = atomicAdd(&gd->ticket, 1u) == gridDim.x - 1;
+  __syncthreads();
+  if (last) __threadfence();
+  return last != 0;
 }
 
+// V_0 = b - H x, and the start of a cycle
+__global__ void __launch_bounds__(CN_THREADS) k_cn_start(CcGeo g, CnOp L, const double* __restrict__ x, CnH h,
+                                                         const double* __restrict__ b, double* __restrict__ V,
+                                                         double* part, CnDev* gd, int first) {
+  double acc[2] = {0.0, 0.0};
+  cn_sweep<true>(g, L, x, h, 1.0, [&](int64_t f, double, double v) {
+    const double bf = b[f], r = bf - v;
+    V[f] = r;
+    acc[0] += r * r;
+    acc[1] += bf * bf;
+  });
+  cn_partials(acc, 2, part);
+  if (!cn_last_block(gd)) return;
+  if (threadIdx.x >= 32) return;
+  const double r2 = cn_fold(part, 0, threadIdx.x), b2 = cn_fold(part, 1, threadIdx.x);
+  if (threadIdx.x != 0) return;
+  const double beta = sqrt(r2), tol = fmax(1e-12 * sqrt(b2), 1e-13);
+  if (first) gd->cycle = gd->its = gd->converged = 0;
+  const bool go = beta > tol;
+  if (!go) gd->converged = isfinite(beta) ? 1 : 0;
+  gd->tol = tol;
+  gd->jend = -1;
+  gd->nv = 0;
+  gd->sc[0] = 1.0 / beta;
+  gd->g[0] = beta;
+  gd->go = go ? 1 : 0;
+  gd->ticket = 0;
+}
+
+// w = H v_j (v_j = sc[j] V_j, nv = j + 1) and the partial dots of the unscaled basis with w
 template <int NV>
-__global__ void __launch_bounds__(GS_THREADS) k_gs_dot(const double* __restrict__ V, int64_t n,
-                                                       const double* __restrict__ w, double* __restrict__ part) {
+__global__ void __launch_bounds__(CN_THREADS, 1) k_cn_apply(CcGeo g, CnOp L, const double* __restrict__ V, int nv,
+                                                             CnH h, double* __restrict__ w, double* __restrict__ part,
+                                                             const CnDev* __restrict__ gd) {
+  asm volatile("griddepcontrol.wait;" ::: "memory");
+  if (!gd->go) return;
+  const int64_t n = g.F;
+  __shared__ CnH hs;
+  const double s = gd->sc[nv - 1];
+  if (threadIdx.x == 0) hs = CnH{h.hdt, s * h.c, s * h.x, s * h.y};
+  __syncthreads();
   double acc[NV];
 #pragma unroll
   for (int i = 0; i < NV; ++i) acc[i] = 0.0;
-  for (int64_t t = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; t < n; t += (int64_t)gridDim.x * blockDim.x) {
-    const double wt = w[t];
+  cn_sweep<true>(g, L, V + (int64_t)(nv - 1) * n, hs, s, [&](int64_t f, double, double y) {
+    w[f] = y;
+    const double* p = V + f;
 #pragma unroll
-    for (int i = 0; i < NV; ++i) acc[i] += V[(int64_t)i * n + t] * wt;
-  }
-  gs_block_partials<NV>(acc, part);
+    for (int i = 0; i < NV; ++i, p += n)
+      if (NV <= 8 || i < nv) acc[i] += *p * y;
+  });
+  cn_partials(acc, nv, part);
 }
 
-// w -= V c (c from part_in); then part_out = partials of V^T w (NORM = false) or of |w|^2
-// (NORM = true, one value per block); block 0 stores c for the Hessenberg column
+// w -= V c, c from the partials of the previous kernel; then the partials of V^T w (NORM = false) or of
+// |w|^2 and the end of the Arnoldi step (NORM = true).  ctl is set on the last step that the graph
+// holds when it may be followed by more.
 template <int NV, bool NORM>
-__global__ void __launch_bounds__(GS_THREADS) k_gs_pass(const double* __restrict__ V, int64_t n,
-                                                        const double* __restrict__ part_in, double* __restrict__ w,
-                                                        double* __restrict__ part_out, double* __restrict__ coef) {
-  __shared__ double cf[NV];
-  gs_coefficients<NV>(part_in, cf);
-  if (blockIdx.x == 0)
-    for (int i = threadIdx.x; i < NV; i += blockDim.x) coef[i] = cf[i];
+__global__ void __launch_bounds__(CN_THREADS, 1) k_cn_pass(const double* __restrict__ V, int64_t n, int nv,
+                                                            const double* __restrict__ part_in, double* __restrict__ w,
+                                                            double* part_out, CnDev* gd, int last_step, StepCtl* ctl) {
+  asm volatile("griddepcontrol.wait;" ::: "memory");
+  if (!gd->go) return;
+  __shared__ double cf[NV], ck[NV];  // coefficients in the scaled and in the unscaled basis
+  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+  for (int i = warp; i < nv; i += CN_THREADS / 32) {
+    const double s = gd->sc[i], c = s * cn_fold(part_in, i, lane);
+    if (lane == 0) { cf[i] = c; ck[i] = s * c; }
+  }
+  __syncthreads();
+  if (!NORM && blockIdx.x == 0 && threadIdx.x < nv) gd->d1[threadIdx.x] = cf[threadIdx.x];
   constexpr int NA = NORM ? 1 : NV;
   double acc[NA];
 #pragma unroll
   for (int i = 0; i < NA; ++i) acc[i] = 0.0;
-  for (int64_t t = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; t < n; t += (int64_t)gridDim.x * blockDim.x) {
-    double v[NV];
+  for (int64_t t = (int64_t)blockIdx.x * CN_THREADS + threadIdx.x; t < n; t += (int64_t)CN_BLOCKS * CN_THREADS) {
+    double v[NV <= 8 ? NV : 1];  // wider bases are read twice (the second time from L1)
     double s = 0.0;
+    const double* p = V + t;
 #pragma unroll
-    for (int i = 0; i < NV; ++i) {
-      v[i] = V[(int64_t)i * n + t];
-      s += cf[i] * v[i];
-    }
+    for (int i = 0; i < NV; ++i, p += n)
+      if (NV <= 8 || i < nv) {
+        const double vi = *p;
+        if (NV <= 8) v[NV <= 8 ? i : 0] = vi;
+        s += ck[i] * vi;
+      }
     const double wt = w[t] - s;
     w[t] = wt;
     if (NORM) acc[0] += wt * wt;
     else {
+      p = V + t;
 #pragma unroll
-      for (int i = 0; i < NA; ++i) acc[i] += v[i] * wt;
+      for (int i = 0; i < NA; ++i, p += n)
+        if (NV <= 8 || i < nv) acc[i] += (NV <= 8 ? v[NV <= 8 ? i : 0] : *p) * wt;
     }
   }
-  gs_block_partials<NA>(acc, part_out);
-}
-
-// V0 = b - w with the partials of |V0|^2 (the residual that starts a restart cycle)
-__global__ void __launch_bounds__(GS_THREADS) k_gs_residual(const double* __restrict__ b, const double* __restrict__ w,
-                                                            int64_t n, double* __restrict__ r,
-                                                            double* __restrict__ part) {
-  double acc[1] = {0.0};
-  for (int64_t t = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; t < n; t += (int64_t)gridDim.x * blockDim.x) {
-    const double v = b[t] - w[t];
-    r[t] = v;
-    acc[0] += v * v;
+  cn_partials(acc, NORM ? 1 : nv, part_out);
+  if (!NORM) return;
+  if (!cn_last_block(gd)) return;
+  if (threadIdx.x >= 32) return;
+  // the end of Arnoldi step j (one warp): column j of H, the rotations, the residual estimate
+  const int j = nv - 1;
+  __shared__ double hc[CN_M + 1], cs[CN_M], sn[CN_M];
+  const double w2 = cn_fold(part_out, 0, lane);
+  if (lane < nv) hc[lane] = __ldcg(&gd->d1[lane]) + cf[lane];
+  if (lane < j) { cs[lane] = gd->cs[lane]; sn[lane] = gd->sn[lane]; }
+  __syncwarp();
+  __shared__ int stop;
+  if (lane == 0) {
+    const double h = sqrt(w2);
+    double below = h;
+    for (int i = 0; i < j; ++i) {
+      const double a = cs[i] * hc[i] + sn[i] * hc[i + 1];
+      hc[i + 1] = -sn[i] * hc[i] + cs[i] * hc[i + 1];
+      hc[i] = a;
+    }
+    const double den = hypot(hc[j], below), inv = 1.0 / den, c = den > 0 ? hc[j] * inv : 1.0, s = den > 0 ? below * inv : 0.0;
+    hc[j] = den;
+    gd->cs[j] = c;
+    gd->sn[j] = s;
+    const double gj = gd->g[j], r = -s * gj;
+    gd->g[j + 1] = r;
+    gd->g[j] = c * gj;
+    gd->sc[j + 1] = h > 0 ? 1.0 / h : 1.0;
+    gd->its += 1;
+    gd->jend = j;
+    bool go = true;
+    if (!isfinite(r)) go = false;
+    else if (fabs(r) <= gd->tol) { gd->converged = 1; go = false; }
+    const bool more = go && last_step && ctl;
+    if (more) raise_gate(ctl, ERR_SWEEPS, CN_SHORT);
+    if (go && last_step) go = false;
+    gd->go = go ? 1 : 0;
+    gd->ticket = 0;
+    stop = !go && !more;
   }
-  gs_block_partials<1>(acc, part);
+  __syncwarp();
+  if (lane <= j) gd->H[lane * CN_M + j] = hc[lane];
+  __syncwarp();
+  if (!stop) return;
+  // y = R^-1 g (lane i keeps g_i), as coefficients of the unscaled basis
+  double gi = lane <= j ? gd->g[lane] : 0.0;
+  for (int k = j; k >= 0; --k) {
+    const double hik = lane <= k ? gd->H[lane * CN_M + k] : 1.0;
+    const double yk = __shfl_sync(0xffffffffu, gi / hik, k);
+    if (lane < k) gi -= hik * yk;
+    else if (lane == k) gd->coef[k] = yk * gd->sc[k];
+  }
+  if (lane == 0) gd->nv = nv;
 }
 
-// the sum of one partial per block, in a fixed order, into out[0]
-__global__ void k_gs_sum(const double* __restrict__ part, double* __restrict__ out) {
-  double a = 0.0;
-  for (int b = threadIdx.x; b < GS_BLOCKS; b += 32) a += part[(int64_t)b * GS_MAXV];
-  for (int o = 16; o; o >>= 1) a += __shfl_xor_sync(0xffffffffu, a, o);
-  if (threadIdx.x == 0) out[0] = a;
+// x += V coef
+__global__ void k_cn_combine(const double* __restrict__ V, int64_t n, const CnDev* __restrict__ gd, double* __restrict__ x) {
+  const int nv = gd->nv;
+  if (nv == 0) return;
+  __shared__ double cf[CN_M];
+  if (threadIdx.x < nv) cf[threadIdx.x] = gd->coef[threadIdx.x];
+  __syncthreads();
+  for (int64_t t = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; t < n; t += (int64_t)gridDim.x * blockDim.x) {
+    double a = 0.0;
+#pragma unroll 4
+    for (int i = 0; i < nv; ++i) a += cf[i] * V[(int64_t)i * n + t];
+    x[t] += a;
+  }
+}
+// the next restart cycle runs while not converged, a step was taken and fewer than 100 cycles ran
+__global__ void k_cn_cycle(CnDev* gd, cudaGraphConditionalHandle cycle) {
+  const bool go = gd->jend >= 0 && !gd->converged && ++gd->cycle < 100;
+  cudaGraphSetConditional(cycle, go ? 1u : 0u);
 }
 
 template <int NV>
-void gs_step_nv(const double* V, int64_t n, double* w, double* part1, double* part2, double* d1, double* d2,
-                cudaStream_t st) {
+void cn_arnoldi_nv(const CcGeo& g, const CnOp& L, double* V, int nv, const CnH& h, double* part1, double* part2, CnDev* gd,
+                   int last_step, StepCtl* ctl, cudaStream_t st) {
+  double* w = V + (int64_t)nv * g.F;
   counted();
-  k_gs_dot<NV><<<GS_BLOCKS, GS_THREADS, 0, st>>>(V, n, w, part1);
+  launch_pdl_ext(k_cn_apply<NV>, dim3(CN_BLOCKS), dim3(CN_THREADS), 0, st, g, L, V, nv, h, w, part1, gd);
   counted();
-  k_gs_pass<NV, false><<<GS_BLOCKS, GS_THREADS, 0, st>>>(V, n, part1, w, part2, d1);
+  launch_pdl_ext(k_cn_pass<NV, false>, dim3(CN_BLOCKS), dim3(CN_THREADS), 0, st, V, g.F, nv, part1, w, part2, gd, 0, nullptr);
   counted();
-  k_gs_pass<NV, true><<<GS_BLOCKS, GS_THREADS, 0, st>>>(V, n, part2, w, part1, d2);
+  launch_pdl_ext(k_cn_pass<NV, true>, dim3(CN_BLOCKS), dim3(CN_THREADS), 0, st, V, g.F, nv, part2, w, part1, gd, last_step, ctl);
+}
+// Arnoldi step nv - 1.  Up to eight basis vectors the kernels keep a face's values in registers; beyond
+// (steps that few systems reach) the size is rounded up and the vectors are read again.
+void cn_arnoldi(const CcGeo& g, const CnOp& L, double* V, int nv, const CnH& h, double* part1, double* part2, CnDev* gd,
+                int last_step, StepCtl* ctl, cudaStream_t st) {
+#define CN_CASE(K) if (nv <= K) return cn_arnoldi_nv<K>(g, L, V, nv, h, part1, part2, gd, last_step, ctl, st)
+  CN_CASE(1); CN_CASE(2); CN_CASE(3); CN_CASE(4); CN_CASE(5); CN_CASE(6); CN_CASE(7); CN_CASE(8);
+  CN_CASE(12); CN_CASE(20); CN_CASE(CN_M);
+#undef CN_CASE
 }
 
-// both Gram-Schmidt passes of Arnoldi step j (basis V_0..V_j) on w; d1, d2 the coefficients,
-// |w|^2 into wn2.  Up to 12 basis vectors the fused passes keep their values in registers;
-// beyond that (steps that converged problems rarely reach) the separate dot / update kernels
-// (part1 then holds multidot_blocks(n) x 64 partials).
-void gs_step(int nv, const double* V, int64_t n, double* w, double* part1, double* part2, double* d1, double* d2,
-             double* wn2, cudaStream_t st) {
-  switch (nv) {
-#define GS_CASE(K) case K: gs_step_nv<K>(V, n, w, part1, part2, d1, d2, st); break;
-    GS_CASE(1) GS_CASE(2) GS_CASE(3) GS_CASE(4) GS_CASE(5) GS_CASE(6) GS_CASE(7) GS_CASE(8) GS_CASE(9)
-    GS_CASE(10) GS_CASE(11) GS_CASE(12)
-#undef GS_CASE
-    default:
-      launch_multidot(V, n, nv, w, n, part1, d1, st);
-      launch_multiaxpy(V, n, nv, d1, -1.0, 1.0, w, n, st);
-      launch_multidot(V, n, nv, w, n, part1, d2, st);
-      launch_multiaxpy(V, n, nv, d2, -1.0, 1.0, w, n, st);
-      launch_multidot(w, n, 1, w, n, part1, wn2, st);
-      return;
+// ---- the end of a step ------------------------------------------------------------------------
+// Pressure (half = p + inc, next = half + factor inc), unpacked velocity, advection history, the
+// coupled residual max |(H q - rhs) + dt grad inc| and the gate quantities of solver/main.py:416-424
+// (max_fluid |flux divergence| / kappa, max |u|, max |v|) in one pass; nothing is written when a solve
+// ran out of its graph's sweeps or Arnoldi steps (the host repeats the step).
+struct CcEnd {
+  const double *q, *inl, *now, *action, *rhs, *p, *inc;
+  double factor, dt, gx, gy;
+  double *U, *prev_adv, *half, *P;
+  const int* err;
+  CcDiagDev* d;
+};
+__global__ void k_cc_step_end(CcGeo g, CcEnd e) {
+  if (*e.err == ERR_SWEEPS) return;
+  const int nx = g.nx;
+  MaxBits dm = 0, um = 0, vm = 0, cm = 0;
+  for (int64_t f = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; f < g.F; f += (int64_t)gridDim.x * blockDim.x) {
+    const bool isu = f < g.usize;
+    const auto [fj, fi] = row_col(isu ? f : f - g.usize, isu ? nx + 1 : nx);
+    const bool act = (g.flags[f] & F_ACTIVE) != 0;
+    const double u = isu && fi == 0 ? e.inl[fj] : act ? e.q[f] : 0.0;
+    e.U[f] = u;
+    if (isu) um = max_abs(um, u);
+    else vm = max_abs(vm, u);
+    e.prev_adv[f] = e.now[f];
+    // (face_grad of inc)
+    double gp = 0.0;
+    if (act) {
+      const int64_t c = isu ? (int64_t)fj * nx + fi : f - g.usize;
+      if (isu) gp = fi == 0 ? 0.0 : fi < nx ? (e.inc[c] - e.inc[c - 1]) * e.gx : -2.0 * e.inc[c - 1] * e.gx;
+      else if (fj >= 1 && fj < g.ny) gp = (e.inc[c] - e.inc[c - nx]) * e.gy;
+    }
+    cm = max_abs(cm, (e.action[f] - e.rhs[f]) + e.dt * gp);
+    // the cell east of a u face: this thread has its west face, the packed field the others
+    if (isu && fi < nx) {
+      const int64_t c = (int64_t)fj * nx + fi, fv = g.usize + c;
+      if (g.cell_type[c] != -1) {
+        auto val = [&](int64_t t) { return (g.flags[t] & F_ACTIVE) ? e.q[t] : 0.0; };
+        const double d = (g.ax[f + 1] * val(f + 1) - g.ax[f] * u) * g.idx + (g.ay[c + nx] * val(fv + nx) - g.ay[c] * val(fv)) * g.idy;
+        dm = max_abs(dm, d * g.ikappa[c]);
+      }
+      const double inc = e.inc[c], h = e.p[c] + inc;
+      e.half[c] = h;
+      e.P[c] = h + e.factor * inc;
+    }
   }
-  counted();
-  k_gs_sum<<<1, 32, 0, st>>>(part1, wn2);
+  block_commit_max(cm, &e.d->coupled);
+  block_commit_max(dm, &e.d->divmax);
+  block_commit_max(um, &e.d->umax);
+  block_commit_max(vm, &e.d->vmax);
 }
 
 }  // namespace
@@ -938,11 +1256,11 @@ struct gm_cc {
   CcFix fix{};
   CcWall wall{};
   // state: U (unpacked face grid), P; history
-  Buf<double> U, Pst, prev_adv, halfp, halfp_next;
+  Buf<double> U, Pst, prev_adv, halfp;
   bool has_history = false;
   double prev_dt = 0;
   // work vectors (face grid) and pressure-grid work
-  Buf<double> q0, now, d0, gp, mid, halfq, expl, offset, dq, rhs, star, w, result, action, tmp, zero, Rw;
+  Buf<double> q0, now, mid, halfq, expl, offset, rhs, star, w, result, action, tmp, zero;
   Buf<double> fxx, fxy, fyx, fyy;
   Buf<double> B, phi, inc, pb, io_f, io_p;
   // the legacy predictor: advective and viscous accelerations, scratch, previous acceleration,
@@ -952,11 +1270,16 @@ struct gm_cc {
   bool l_has_prev = false;
   double l_prev_dt = 0;
   CcFlux flux{};
-  // GMRES(30)
-  static constexpr int GM_M = 30;
-  Buf<double> V, gpart, gpart2, gd1, gd2, gwn, gbeta, gbn, gy, gone;
-  Buf<int> gnv;
-  Buf<GmresDev> gdev;
+  // the CN operator on packed vectors and its GMRES(30)
+  Buf<uint8_t> ncls;
+  Buf<int32_t> nface, ncol;
+  Buf<int64_t> nptr;
+  Buf<double> nval;
+  CnOp cn{};
+  bool offset_stale = true;  // the inlet changed since offset was formed
+  int cn_steps = 6;          // Arnoldi steps that a step graph holds; above CN_M: restart cycles in a WHILE node
+  Buf<double> V, gpart, gpart2;
+  Buf<CnDev> gdev;
   // per-step diagnostics
   Buf<CcDiagDev> diag;
   CcDiagDev* host_diag = nullptr;
@@ -965,7 +1288,7 @@ struct gm_cc {
     cudaGraphExec_t exec = nullptr;
     double dt = 0, prev_dt = 0;
     bool hist = false;
-    long long outer = 0, per_step = 0, per_cycle = 0;
+    long long outer = 0, per_cycle = 0;
   };
   Graph graphs[3];
   int next_graph = 0;
@@ -1020,23 +1343,6 @@ void momentum(gm_cc* c, bool adv, const double* X, const double* inl, double nu,
   else k_cc_rhs<false><<<nblk(c->F), CC_TPB, 0, st>>>(c->geo, c->flux, c->wall, X, shear ? 1 : 0, hdt, mode, Y, Rout);
 }
 
-void vec(gm_cc* c, int op, int64_t n, const double* a, const double* b, const double* cc, const double* d,
-         const double* e, double s0, double s1, double* out, cudaStream_t st) {
-  counted();
-  k_cc_vec<<<nblk(n), CC_TPB, 0, st>>>(op, n, a, b, cc, d, e, s0, s1, out);
-}
-
-void grad(gm_cc* c, const double* P, double* Y, cudaStream_t st) {
-  counted();
-  k_cc_grad<<<nblk(c->F), CC_TPB, 0, st>>>(c->geo, P, 1.0 / (c->rho * c->dx), 1.0 / (c->rho * c->dy), Y);
-}
-
-void maxdiff(gm_cc* c, int64_t n, const double* a, const double* b, const double* cc, double s, unsigned long long* out,
-             cudaStream_t st) {
-  counted();
-  k_cc_maxdiff<<<std::min<unsigned>(nblk(n), 1216), CC_TPB, 0, st>>>(n, a, b, cc, s, out);
-}
-
 // project(q, step) of advance_ab2_cn (solver/cut_cell_solver.py:993-1002): q -> out (packed),
 // phi; slot selects the control block entry and the predicted-divergence record
 void project(gm_cc* c, const double* q, double step, double* out, double* phi, int slot, int rec, cudaStream_t st) {
@@ -1044,26 +1350,37 @@ void project(gm_cc* c, const double* q, double step, double* out, double* phi, i
   k_cc_divrhs<<<nblk(c->psize), CC_TPB, 0, st>>>(c->geo, q, c->inlet.p, c->rho / step, c->B.p);
   gmi::pressure_solve(c->P, c->B.p, phi, slot);
   counted();
-  k_cc_pdiv<<<std::min<unsigned>(nblk(c->psize), 1216), CC_TPB, 0, st>>>(c->geo, gmi::pressure_residual(c->P),
-                                                                        step / c->rho, &c->diag.p->pdiv[rec]);
-  counted();
-  k_cc_correct<<<nblk(c->F), CC_TPB, 0, st>>>(c->geo, q, phi, (step / c->rho) / c->dx, (step / c->rho) / c->dy, out);
+  k_cc_correct<<<std::min<unsigned>(nblk(c->F), 1216), CC_TPB, 0, st>>>(
+      c->geo, q, phi, (step / c->rho) / c->dx, (step / c->rho) / c->dy, out, gmi::pressure_residual(c->P), step / c->rho,
+      &c->diag.p->pdiv[rec]);
 }
 
-// forces on the circle into diag->forces: the wall shear of every Gauss point (one warp each),
+// forces on the circle into diag->forces: the wall shear and pressure of every point (one warp each),
 // then the one-block sums
 void forces(gm_cc* c, const double* U, const double* P, double mu, cudaStream_t st) {
-  if (c->wall.n > 0) {
+  const gmi::SurfaceCsr S = gmi::surface(c->P);
+  if (c->wall.n + S.n > 0) {
     counted();
-    k_cc_wall_tau<<<nblk((int64_t)c->wall.n * 32, 256), 256, 0, st>>>(c->wall, U, mu, c->ftau.p);
+    k_cc_wall_points<<<nblk((int64_t)(c->wall.n + S.n) * 32, 256), 256, 0, st>>>(S, c->wall, U, P, mu, c->ftau.p, c->pb.p);
   }
   counted();
-  k_cc_forces<<<1, CC_FORCE_THREADS, 0, st>>>(gmi::surface(c->P), c->wall, P, c->ftau.p, c->pb.p, c->diag.p->forces);
+  k_cc_forces<<<1, CC_FORCE_THREADS, 0, st>>>(S, c->wall, c->ftau.p, c->pb.p, c->diag.p->forces);
 }
 
-// H x = x - dt/2 L x on packed vectors (L the viscous operator without the inlet)
-void hmatvec(gm_cc* c, const double* x, double dt, double* y, cudaStream_t st) {
-  momentum(c, false, x, nullptr, c->nu, 1, 0.5 * dt, y, nullptr, st);
+template <int MODE>
+void cn_eval(gm_cc* c, CnEval e, cudaStream_t st) {
+  e.offset = c->offset.p;
+  e.h = cn_h(c->cn, e.hdt);
+  e.gx = 1.0 / (c->rho * c->dx);
+  e.gy = 1.0 / (c->rho * c->dy);
+  counted();
+  k_cn_eval<MODE><<<std::max(4u, std::min<unsigned>(nblk(c->F), 1216)), CC_TPB, 0, st>>>(c->geo, c->cn, e);
+}
+// the inlet's part of the viscous operator, by the flux arrays (mode 0 of momentum on the zero vector)
+void refresh_offset(gm_cc* c) {
+  if (!c->offset_stale) return;
+  momentum(c, false, c->zero.p, c->inlet.p, c->nu, 0, 0.0, c->offset.p, nullptr, c->st);
+  c->offset_stale = false;
 }
 
 cudaGraphNode_t add_cond(cudaStream_t st, cudaGraphConditionalHandle cond, cudaGraphConditionalNodeType type,
@@ -1085,68 +1402,43 @@ cudaGraphNode_t add_cond(cudaStream_t st, cudaGraphConditionalHandle cond, cudaG
   return node;
 }
 
-// GMRES(30) for H x = b from x0 = x, captured on st (solver/time_integration.py:99-101:
-// rtol 1e-12, atol 1e-13, restart 30, at most 100 cycles)
+// the CN solve (see k_cn_start), captured on st: x holds the first iterate and the solution
 void gmres(gm_cc* c, const double* b, double* x, double dt, gm_cc::Graph& gr, cudaStream_t st) {
-  const int m = gm_cc::GM_M;
-  const int64_t n = c->F;
-  double* V = c->V.p;
-  auto vec_i = [&](int i) { return V + (int64_t)i * n; };
-  cudaStream_t sb1 = gmi::body_stream(c->P, 0), sb2 = gmi::body_stream(c->P, 1);
-  counted();
-  k_gs_dot<1><<<GS_BLOCKS, GS_THREADS, 0, st>>>(b, n, b, c->gpart.p);
-  counted();
-  k_gs_sum<<<1, 32, 0, st>>>(c->gpart.p, c->gbn.p);
+  const CnH h = cn_h(c->cn, 0.5 * dt);
+  auto cycle = [&](int first, int steps, StepCtl* ctl, cudaStream_t s) {
+    counted();
+    k_cn_start<<<CN_BLOCKS, CN_THREADS, 0, s>>>(c->geo, c->cn, x, h, b, c->V.p, c->gpart.p, c->gdev.p, first);
+    for (int nv = 1; nv <= steps; ++nv)
+      cn_arnoldi(c->geo, c->cn, c->V.p, nv, h, c->gpart.p, c->gpart2.p, c->gdev.p, nv == steps, ctl, s);
+    counted();
+    k_cn_combine<<<std::min<unsigned>(nblk(c->F), 1216), CC_TPB, 0, s>>>(c->V.p, c->F, c->gdev.p, x);
+  };
+  if (c->cn_steps <= CN_M) {
+    cycle(1, c->cn_steps, gmi::control(c->P), st);
+    return;
+  }
+  CCK(cudaMemsetAsync(&c->gdev.p->jend, 0, sizeof(CnDev) - offsetof(CnDev, jend), st));
   cudaStreamCaptureStatus cs;
   cudaGraph_t top;
   CCK(cudaStreamGetCaptureInfo(st, &cs, nullptr, &top, nullptr, nullptr, nullptr));
   cudaGraphConditionalHandle cyc;
-  CCK(cudaGraphConditionalHandleCreate(&cyc, top, 0, 0));
-  launch_gm_init(c->gdev.p, c->gbn.p, cyc, st, 1e-12, 1e-13);
-  cudaGraph_t cycle_body;
-  add_cond(st, cyc, cudaGraphCondTypeWhile, &cycle_body);
-  CCK(cudaStreamBeginCaptureToGraph(sb1, cycle_body, nullptr, nullptr, 0, cudaStreamCaptureModeThreadLocal));
+  CCK(cudaGraphConditionalHandleCreate(&cyc, top, 1, cudaGraphCondAssignDefault));
+  cudaGraph_t body;
+  add_cond(st, cyc, cudaGraphCondTypeWhile, &body);
+  cudaStream_t sb = gmi::body_stream(c->P, 0);
+  CCK(cudaStreamBeginCaptureToGraph(sb, body, nullptr, nullptr, 0, cudaStreamCaptureModeThreadLocal));
   const long long c1 = kernel_launch_count();
-  hmatvec(c, x, dt, vec_i(1), sb1);
+  cycle(0, CN_M, nullptr, sb);
   counted();
-  k_gs_residual<<<GS_BLOCKS, GS_THREADS, 0, sb1>>>(b, vec_i(1), n, vec_i(0), c->gpart.p);
-  counted();
-  k_gs_sum<<<1, 32, 0, sb1>>>(c->gpart.p, c->gbeta.p);
-  GmresHandles hs{};
-  hs.count = m;
-  cudaGraph_t cyc_graph;
-  CCK(cudaStreamGetCaptureInfo(sb1, &cs, nullptr, &cyc_graph, nullptr, nullptr, nullptr));
-  for (int j = 0; j < m; ++j) CCK(cudaGraphConditionalHandleCreate(&hs.step[j], cyc_graph, 0, 0));
-  launch_gm_cycle_begin(c->gdev.p, c->gbeta.p, hs, sb1);
-  launch_gm_scale(vec_i(0), n, c->gdev.p, sb1);
-  long long per_step = 0;
-  for (int j = 0; j < m; ++j) {
-    cudaGraph_t step_body;
-    add_cond(sb1, hs.step[j], cudaGraphCondTypeIf, &step_body);
-    CCK(cudaStreamBeginCaptureToGraph(sb2, step_body, nullptr, nullptr, 0, cudaStreamCaptureModeThreadLocal));
-    const long long c2 = kernel_launch_count();
-    double* wv = vec_i(j + 1);
-    hmatvec(c, vec_i(j), dt, wv, sb2);
-    gs_step(j + 1, V, n, wv, c->gpart.p, c->gpart2.p, c->gd1.p, c->gd2.p, c->gwn.p, sb2);
-    launch_gm_step_end(c->gdev.p, j, c->gd1.p, c->gd2.p, c->gwn.p, j + 1 < m ? hs.step[j + 1] : hs.step[0],
-                       j + 1 < m, sb2);
-    launch_gm_scale(wv, n, c->gdev.p, sb2);
-    per_step = kernel_launch_count() - c2;
-    cudaGraph_t done;
-    CCK(cudaStreamEndCapture(sb2, &done));
-  }
-  launch_gm_cycle_end(c->gdev.p, c->gy.p, c->gnv.p, cyc, sb1);
-  launch_multiaxpy_dev(V, n, c->gnv.p, c->gy.p, x, n, sb1);
-  gr.per_step = per_step;
-  gr.per_cycle = kernel_launch_count() - c1 - (long long)m * per_step;
-  cudaGraph_t done1;
-  CCK(cudaStreamEndCapture(sb1, &done1));
+  k_cn_cycle<<<1, 1, 0, sb>>>(c->gdev.p, cyc);
+  gr.per_cycle = kernel_launch_count() - c1;
+  cudaGraph_t done;
+  CCK(cudaStreamEndCapture(sb, &done));
 }
 
 // One AB2/CN step (advance_ab2_cn, solver/cut_cell_solver.py:959-1015, with ab2_cn_step,
 // solver/time_integration.py:7-145), captured on st.
 void step_body(gm_cc* c, double dt, gm_cc::Graph& gr, cudaStream_t st) {
-  const int64_t F = c->F, Pn = c->psize;
   const double* inl = c->inlet.p;
   auto mark = [&](int k) {
     // inside a capture an event record node needs the external flag (a plain record only
@@ -1156,51 +1448,57 @@ void step_body(gm_cc* c, double dt, gm_cc::Graph& gr, cudaStream_t st) {
   mark(0);
   CCK(cudaMemsetAsync(c->diag.p, 0, offsetof(CcDiagDev, forces), st));
   counted();
-  k_cc_pack<<<nblk(F), CC_TPB, 0, st>>>(c->geo, c->U.p, c->q0.p);
+  k_cc_pack<<<nblk(c->F), CC_TPB, 0, st>>>(c->geo, c->U.p, c->q0.p);
   momentum(c, true, c->q0.p, inl, 0.0, 0, 0.0, c->now.p, nullptr, st);
   mark(1);
   const double* pressure = c->has_history ? c->halfp.p : c->Pst.p;
+  CnEval e{};
+  e.x = c->q0.p;
+  e.p = pressure;
+  e.hdt = 0.5 * dt;
   if (!c->has_history) {
     // projected midpoint start-up
-    momentum(c, false, c->q0.p, inl, c->nu, 0, 0.0, c->d0.p, nullptr, st);
-    grad(c, pressure, c->gp.p, st);
-    vec(c, 0, F, c->q0.p, c->now.p, c->d0.p, c->gp.p, nullptr, 0.5 * dt, 0.0, c->mid.p, st);
+    e.a = c->now.p;
+    e.dt = 0.5 * dt;
+    e.out = c->mid.p;
+    cn_eval<CN_MID>(c, e, st);
     project(c, c->mid.p, 0.5 * dt, c->halfq.p, c->phi.p, S_P0, 0, st);
     momentum(c, true, c->halfq.p, inl, 0.0, 0, 0.0, c->expl.p, nullptr, st);
+    e.a = c->expl.p;
   } else {
-    vec(c, 1, F, c->now.p, c->prev_adv.p, nullptr, nullptr, nullptr, dt / (2 * c->prev_dt), 0.0, c->expl.p, st);
+    e.a = c->now.p;
+    e.b = c->prev_adv.p;
+    e.s = dt / (2 * c->prev_dt);
   }
-  momentum(c, false, c->zero.p, inl, c->nu, 0, 0.0, c->offset.p, nullptr, st);
-  momentum(c, false, c->q0.p, inl, c->nu, 0, 0.0, c->dq.p, nullptr, st);
-  grad(c, pressure, c->gp.p, st);
-  vec(c, 2, F, c->q0.p, c->expl.p, c->dq.p, c->gp.p, c->offset.p, dt, 0.5 * dt, c->rhs.p, st);
-  maxdiff(c, F, c->rhs.p, nullptr, nullptr, 0.0, &c->diag.p->rhs_max, st);
-  CCK(cudaMemcpyAsync(c->star.p, c->q0.p, F * sizeof(double), cudaMemcpyDeviceToDevice, st));
+  e.dt = dt;
+  e.out = c->rhs.p;
+  e.out2 = c->star.p;
+  e.mx = &c->diag.p->rhs_max;
+  cn_eval<CN_RHS>(c, e, st);
   mark(2);
   gmres(c, c->rhs.p, c->star.p, dt, gr, st);
   mark(3);
-  hmatvec(c, c->star.p, dt, c->w.p, st);
-  maxdiff(c, F, c->w.p, c->rhs.p, nullptr, 0.0, &c->diag.p->mres, st);
+  CnEval r{};
+  r.x = c->star.p;
+  r.a = c->rhs.p;
+  r.hdt = 0.5 * dt;
+  r.mx = &c->diag.p->mres;
+  cn_eval<CN_CHECK>(c, r, st);
   mark(4);
   project(c, c->star.p, dt, c->result.p, c->phi.p, S_P1, 1, st);
   mark(5);
-  hmatvec(c, c->result.p, dt, c->action.p, st);
-  vec(c, 3, F, c->result.p, c->rhs.p, c->action.p, nullptr, nullptr, 0.0, 0.0, c->tmp.p, st);
+  r.x = c->result.p;
+  r.out = c->action.p;
+  r.out2 = c->tmp.p;
+  cn_eval<CN_ACTION>(c, r, st);
   mark(6);
   project(c, c->tmp.p, dt, c->w.p, c->inc.p, S_P2, 2, st);
   mark(7);
-  const double factor = c->has_history ? dt / (dt + c->prev_dt) : 1.0;
+  CcEnd n{c->result.p, inl, c->now.p, c->action.p, c->rhs.p, pressure, c->inc.p,
+          c->has_history ? dt / (dt + c->prev_dt) : 1.0, dt, 1.0 / (c->rho * c->dx), 1.0 / (c->rho * c->dy),
+          c->U.p, c->prev_adv.p, c->halfp.p, c->Pst.p, &gmi::control(c->P)->err, c->diag.p};
   counted();
-  k_cc_pressure_out<<<nblk(Pn), CC_TPB, 0, st>>>(Pn, pressure, c->inc.p, factor, c->halfp_next.p, c->Pst.p);
-  grad(c, c->inc.p, c->gp.p, st);
-  maxdiff(c, F, c->action.p, c->rhs.p, c->gp.p, dt, &c->diag.p->coupled, st);
-  CCK(cudaMemcpyAsync(c->halfp.p, c->halfp_next.p, Pn * sizeof(double), cudaMemcpyDeviceToDevice, st));
-  CCK(cudaMemcpyAsync(c->prev_adv.p, c->now.p, F * sizeof(double), cudaMemcpyDeviceToDevice, st));
-  counted();
-  k_cc_unpack<<<nblk(F), CC_TPB, 0, st>>>(c->geo, c->result.p, inl, c->U.p);
-  counted();
-  k_cc_stepmax<<<std::min<unsigned>(nblk(F), 1216), CC_TPB, 0, st>>>(c->geo, c->U.p, &c->diag.p->divmax,
-                                                                      &c->diag.p->umax, &c->diag.p->vmax);
+  k_cc_step_end<<<std::min<unsigned>(nblk(c->F), 1216), CC_TPB, 0, st>>>(c->geo, n);
   forces(c, c->U.p, c->Pst.p, c->nu * c->rho, st);
   mark(8);
 }
@@ -1211,6 +1509,7 @@ gm_cc::Graph& step_graph(gm_cc* c, double dt) {
   gm_cc::Graph& gr = c->graphs[c->next_graph];
   c->next_graph = (c->next_graph + 1) % 3;
   if (gr.exec) { cudaGraphExecDestroy(gr.exec); gr.exec = nullptr; }
+  gr.per_cycle = 0;
   cudaStream_t st = c->st;
   const long long c0 = kernel_launch_count();
   gmi::set_capturing(c->P, true);
@@ -1229,7 +1528,7 @@ gm_cc::Graph& step_graph(gm_cc* c, double dt) {
   CCK(cudaStreamEndCapture(st, &g));
   const long long captured = kernel_launch_count() - c0;
   kernel_launch_adjust(-captured);
-  gr.outer = captured - (long long)gm_cc::GM_M * gr.per_step - gr.per_cycle;
+  gr.outer = captured - gr.per_cycle;
   cudaGraphExec_t ex = nullptr;
   cudaError_t e = cudaGraphInstantiate(&ex, g, 0);
   cudaGraphDestroy(g);
@@ -1306,7 +1605,7 @@ void initial_state(gm_cc* c, const std::vector<double>& inlet, const int32_t* ce
                                                                         1.0 / c->rho, &c->diag.p->pdiv[1]);
   counted();
   k_cc_correct<<<nblk(c->F), CC_TPB, 0, st>>>(c->geo, c->U.p, c->phi.p, (1.0 / c->rho) / c->dx, (1.0 / c->rho) / c->dy,
-                                             c->tmp.p);
+                                             c->tmp.p, nullptr, 0.0, nullptr);
   counted();
   k_cc_unpack<<<nblk(c->F), CC_TPB, 0, st>>>(c->geo, c->tmp.p, c->inlet.p, c->U.p);
   CCK(cudaMemsetAsync(c->Pst.p, 0, c->psize * sizeof(double), st));
@@ -1322,6 +1621,148 @@ void initial_state(gm_cc* c, const std::vector<double>& inlet, const int32_t* ce
       std::snprintf(pbuf, sizeof pbuf, "Pressure residual exceeds divergence budget: %g", pd);
       throw CcFail(GM_ERUNTIME, pbuf);
     }
+}
+
+// Tables of the CN operator (CnOp): the class of every face, and the sparse rows of L = (viscous
+// acceleration) of the unknown faces near the body -- those with a curved flux among their four, wall
+// shear, covered transfers or a merge -- composed from the same pieces in the order of k_cc_fix and k_cc_rhs.
+// Columns that are not unknown hold zero in packed vectors and are left out.
+void build_cn(gm_cc* C, const gm_cc_config* cfg, const std::vector<uint8_t>& fl, const std::vector<double>& vr,
+              const std::vector<int32_t>& mof, const std::vector<int64_t>& ms, const std::vector<int64_t>& mm,
+              const std::vector<double>& mv, const std::vector<int64_t>& tgt, const std::vector<int64_t>& tptr,
+              const std::vector<int32_t>& tk, const std::vector<int64_t>& own, const std::vector<int64_t>& optr,
+              const std::vector<int64_t>& odon, const std::vector<int64_t>& donors, const std::vector<uint8_t>& dfam,
+              const std::vector<int64_t>& dface, const std::vector<int64_t>& dptr, const std::vector<int64_t>& dcol,
+              const std::vector<double>& dval) {
+  const int nx = C->nx, ny = C->ny, nu1 = nx + 1;
+  const int64_t us = C->usize, F = C->F;
+  const double dx = C->dx, dy = C->dy, rnu = C->rho * C->nu;
+  using Row = std::map<int64_t, double>;
+  std::array<std::map<int64_t, int64_t>, 4> over;  // curved faces of each family: row of the tables
+  for (size_t r = 0; r < dface.size(); ++r) over[dfam[r]][dface[r]] = (int64_t)r;
+  std::map<int64_t, int64_t> tof, oof, don;
+  for (size_t t = 0; t < tgt.size(); ++t) tof[tgt[t]] = (int64_t)t;
+  for (size_t o = 0; o < own.size(); ++o) oof[own[o]] = (int64_t)o;
+  for (int64_t d : donors) don[d] = 1;
+  const double dydx = dy / dx, dxdy = dx / dy;
+  // flux `idx` of a family (0 F_xx, 1 F_xy, 2 F_yx, 3 F_yy) times s, added to a row
+  auto flux = [&](int fam, int64_t idx, double s, Row& row) {
+    auto it = over[fam].find(idx);
+    if (it != over[fam].end()) {
+      for (int64_t e = dptr[it->second]; e < dptr[it->second + 1]; ++e) row[dcol[e]] += s * (rnu * dval[e]);
+      return;
+    }
+    auto u = [&](int j, int i, double w) { row[(int64_t)j * nu1 + i] += s * w; };
+    auto v = [&](int j, int i, double w) { row[us + (int64_t)j * nx + i] += s * w; };
+    if (fam == 0 || fam == 3) {
+      const int j = (int)(idx / nx), i = (int)(idx % nx);
+      if (fam == 0) {
+        const double w = rnu * (cfg->ax_mid[idx] * dydx);
+        u(j, i + 1, w); u(j, i, -w);
+      } else {
+        const double w = rnu * (cfg->ay_mid[idx] * dxdy);
+        v(j + 1, i, w); v(j, i, -w);
+      }
+      return;
+    }
+    const int j = (int)(idx / nu1), i = (int)(idx % nu1);
+    if (fam == 1) {
+      const double w = rnu * (cfg->ay_u[idx] * dxdy);
+      if (j == 0) { if (!C->slip) u(0, i, 2.0 * w); }
+      else if (j == ny) { if (!C->slip) u(ny - 1, i, -2.0 * w); }
+      else { u(j, i, w); u(j - 1, i, -w); }
+    } else {
+      const double w = rnu * (cfg->ax_v[idx] * dydx);
+      if (i == 0) v(j, 0, 2.0 * w);
+      else if (i < nx) { v(j, i, w); v(j, i - 1, -w); }
+    }
+  };
+  // the four fluxes of face f (family, index, sign), none on the faces without a flux balance
+  struct Part { int fam; int64_t idx; double s; };
+  auto parts = [&](int64_t f) {
+    std::vector<Part> p;
+    if (f < us) {
+      const int j = (int)(f / nu1), i = (int)(f % nu1);
+      const int64_t c = (int64_t)j * nx + i;
+      if (i >= 1 && i < nx) p = {{0, c, 1.0}, {0, c - 1, -1.0}, {1, f + nu1, 1.0}, {1, f, -1.0}};
+      else if (i == nx) p = {{0, c - 1, -1.0}, {1, f + nu1, 0.5}, {1, f, -0.5}};
+    } else {
+      const int64_t c = f - us;
+      const int j = (int)(c / nx), i = (int)(c % nx);
+      const int64_t t = (int64_t)j * nu1 + i;
+      if (j >= 1 && j < ny) p = {{2, t + 1, 1.0}, {2, t, -1.0}, {3, c, 1.0}, {3, c - nx, -1.0}};
+    }
+    return p;
+  };
+  auto walled = [&](int64_t f, double s, Row& row) {
+    for (const Part& p : parts(f)) flux(p.fam, p.idx, s * p.s, row);
+    auto t = tof.find(f);
+    if (t == tof.end() || rnu == 0.0) return;
+    for (int64_t q = tptr[t->second]; q < tptr[t->second + 1]; ++q) {
+      const int k = tk[q];
+      const double w = s * (-rnu) * (f < us ? cfg->wall_tx[k] : cfg->wall_ty[k]) * cfg->wall_ds[k];
+      for (int64_t e = cfg->wall_rate.ptr[k]; e < cfg->wall_rate.ptr[k + 1]; ++e)
+        row[cfg->wall_rate.col[e]] += w * cfg->wall_rate.val[e];
+    }
+  };
+  auto full = [&](int64_t f, double s, Row& row) {
+    if (don.count(f)) return;
+    walled(f, s, row);
+    auto o = oof.find(f);
+    if (o != oof.end())
+      for (int64_t q = optr[o->second]; q < optr[o->second + 1]; ++q) walled(odon[q], s, row);
+  };
+  std::vector<uint8_t> cls(F, CN_ZERO);
+  std::vector<int32_t> face, col;
+  std::vector<int64_t> ptr{0};
+  std::vector<double> val;
+  const double iv = 1.0 / (C->rho * dx * dy);
+  for (int64_t f = 0; f < F; ++f) {
+    if (!(fl[f] & F_ACTIVE)) continue;
+    const std::vector<Part> ps = parts(f);
+    bool row = mof[f] >= 0 || (fl[f] & F_AUX), reg = (fl[f] & F_FLUID) && !(fl[f] & F_SOLID) && ps.size() == 4;
+    for (const Part& p : ps) {
+      row = row || over[p.fam].count(p.idx);
+      const double a = p.fam == 0 ? cfg->ax_mid[p.idx] : p.fam == 1 ? cfg->ay_u[p.idx] : p.fam == 2 ? cfg->ax_v[p.idx] : cfg->ay_mid[p.idx];
+      reg = reg && a == 1.0;
+    }
+    if (row) {
+      cls[f] = CN_ROW;
+      Row r;
+      if (fl[f] & F_SOLID) {}
+      else if (mof[f] >= 0) {
+        full(ms[mof[f]], mv[mof[f]], r);
+        full(mm[mof[f]], mv[mof[f]], r);
+      } else if (fl[f] & F_FLUID) full(f, vr[f], r);
+      face.push_back((int32_t)f);
+      for (const auto& kv : r)
+        if (fl[kv.first] & F_ACTIVE) {
+          col.push_back((int32_t)kv.first);
+          val.push_back(kv.second);
+        }
+      ptr.push_back((int64_t)col.size());
+      continue;
+    }
+    // regular: full apertures and volume, all four fluxes between two faces of its own grid
+    if (f < us) {
+      const int j = (int)(f / nu1);
+      reg = reg && j >= 1 && j + 1 < ny;
+    } else {
+      const int i = (int)((f - us) % nx);
+      reg = reg && i >= 1 && i + 1 < nx;
+    }
+    reg = reg && std::fabs(vr[f] / iv - 1.0) <= 1e-15;
+    cls[f] = reg ? CN_REGULAR : CN_EDGE;
+  }
+  cudaStream_t st = C->st;
+  C->ncls.upload(cls, st);
+  C->nface.upload(face, st);
+  C->nptr.upload(ptr, st);
+  C->ncol.upload(col, st);
+  C->nval.upload(val, st);
+  CCK(cudaStreamSynchronize(st));
+  C->cn = CnOp{C->ncls.p, (int)face.size(), C->nface.p, C->nptr.p, C->ncol.p, C->nval.p,
+               rnu * dydx * iv, rnu * dxdy * iv, rnu, C->slip};
 }
 
 template <typename T>
@@ -1581,29 +2022,25 @@ int gm_cc_create(const gm_cc_config* cfg, gm_cc** out) {
     W.n_aux = (int)aux_face.size(); W.aux_face = C->aux_face.p; W.aux_tgt = C->aux_tgt.p; W.aux_own = C->aux_own.p;
     W.aux_don = C->aux_don.p;
     // state and work arrays
-    for (Buf<double>* b : {&C->U, &C->prev_adv, &C->q0, &C->now, &C->d0, &C->gp, &C->mid, &C->halfq, &C->expl,
-                           &C->offset, &C->dq, &C->rhs, &C->star, &C->w, &C->result, &C->action, &C->tmp, &C->zero,
-                           &C->Rw, &C->la, &C->ld, &C->lr, &C->lprev, &C->lstar}) {
+    for (Buf<double>* b : {&C->U, &C->prev_adv, &C->q0, &C->now, &C->mid, &C->halfq, &C->expl,
+                           &C->offset, &C->rhs, &C->star, &C->w, &C->result, &C->action, &C->tmp, &C->zero,
+                           &C->la, &C->ld, &C->lr, &C->lprev, &C->lstar}) {
       b->alloc(F);
       b->zero(st);
     }
-    for (Buf<double>* b : {&C->Pst, &C->halfp, &C->halfp_next, &C->B, &C->phi, &C->inc}) {
+    for (Buf<double>* b : {&C->Pst, &C->halfp, &C->B, &C->phi, &C->inc}) {
       b->alloc(Pn);
       b->zero(st);
     }
     C->fxx.alloc(Pn); C->fyy.alloc(Pn); C->fxy.alloc(nvert); C->fyx.alloc(nvert);
     C->flux = CcFlux{C->fxx.p, C->fxy.p, C->fyx.p, C->fyy.p};
     C->pb.alloc(std::max(1, gmi::surface(C->P).n));
-    const int m = gm_cc::GM_M;
-    C->V.alloc((size_t)(m + 1) * F);
-    C->gpart.alloc(std::max<size_t>((size_t)GS_BLOCKS * GS_MAXV, (size_t)multidot_blocks(F) * 64));
-    C->gpart2.alloc((size_t)GS_BLOCKS * GS_MAXV);
-    for (Buf<double>* b : {&C->gd1, &C->gd2, &C->gy}) b->alloc(64);
-    for (Buf<double>* b : {&C->gwn, &C->gbeta, &C->gbn, &C->gone}) b->alloc(1);
-    C->gnv.alloc(1);
+    C->V.alloc((size_t)(CN_M + 1) * F);
+    C->gpart.alloc((size_t)CN_BLOCKS * CN_M);
+    C->gpart2.alloc((size_t)CN_BLOCKS * CN_M);
     C->gdev.alloc(1);
-    const double one = 1.0;
-    CCK(cudaMemcpyAsync(C->gone.p, &one, sizeof one, cudaMemcpyHostToDevice, st));
+    CCK(cudaMemsetAsync(C->gdev.p, 0, sizeof(CnDev), st));
+    build_cn(C, cfg, fl, vr, mof, ms, mm, mv, tgt, tptr, tk, own, optr, odon, donors, dfam, dface, dptr, dcol, dval);
     C->lres.alloc(2 * CC_RES_BLOCKS);
     C->ftau.alloc(std::max<int64_t>(1, nw));
     C->diag.alloc(1);
@@ -1692,6 +2129,7 @@ int gm_cc_set_inlet(gm_cc* c, const double* u_inlet) {
   if (!c || !u_inlet) return GM_EVALUE;
   return guarded(c, [&] {
     copy_in(c->inlet.p, u_inlet, c->ny, c->st);
+    c->offset_stale = true;
     CCK(cudaStreamSynchronize(c->st));
   });
 }
@@ -1743,21 +2181,32 @@ int gm_cc_step(gm_cc* c, double dt, int32_t n_steps, double start_time, gm_cc_st
   return guarded(c, [&] {
     cudaStream_t st = c->st;
     for (int32_t k = 0; k < n_steps; ++k) {
+      refresh_offset(c);
       gm_cc::Graph& gr = step_graph(c, dt);
       CCK(cudaMemsetAsync(gmi::control(c->P), 0, sizeof(StepCtl), st));
       CCK(cudaGraphLaunch(gr.exec, st));
-      int r[5];
+      int r[4];
       CCK(cudaMemcpyAsync(r, &c->gdev.p->jend, sizeof r, cudaMemcpyDeviceToHost, st));
       CCK(cudaMemcpyAsync(c->host_diag, c->diag.p, sizeof(CcDiagDev), cudaMemcpyDeviceToHost, st));
       std::string m;
       const int prc = gmi::check(c->P, "cut-cell step", m);  // synchronises the stream
       const int cycles = r[1], its = r[2], converged = r[3];
+      kernel_launch_adjust(gr.outer + (long long)cycles * gr.per_cycle);
+      if (prc == ERR_SWEEPS) {
+        // a solve needs more than the graph holds; the state is as before the step: once more with more
+        const int what = gmi::failed_gate(c->P);
+        if (what == CN_SHORT) c->cn_steps = c->cn_steps < CN_M ? std::min(c->cn_steps + 4, CN_M) : CN_M + 1;
+        else gmi::add_sweep(c->P, what);
+        for (auto& g : c->graphs)
+          if (g.exec) { cudaGraphExecDestroy(g.exec); g.exec = nullptr; }
+        --k;
+        continue;
+      }
       if (c->phase_on)
         for (int q = 0; q < gm_cc::NPHASE; ++q) {
           float ms = 0.f;
           c->phase_ms[q] = cudaEventElapsedTime(&ms, c->pev[q], c->pev[q + 1]) == cudaSuccess ? ms : 0.0;
         }
-      kernel_launch_adjust(gr.outer + (long long)cycles * gr.per_cycle + (long long)its * gr.per_step);
       const CcDiagDev& d = *c->host_diag;
       gm_cc_step_diag out{};
       out.time = start_time + (k + 1) * dt;
@@ -1932,14 +2381,24 @@ int gm_cc_apply(gm_cc* c, int32_t op, double param, const double* x, double* y, 
       case GM_CC_OP_ADVECTION:
       case GM_CC_OP_DIFFUSION: {
         scatter(x, c->tmp.p);
-        const bool adv = op == GM_CC_OP_ADVECTION;
-        momentum(c, adv, c->tmp.p, c->inlet.p, adv ? 0.0 : c->nu, 0, 0.0, c->w.p, nullptr, st);
+        if (op == GM_CC_OP_ADVECTION) momentum(c, true, c->tmp.p, c->inlet.p, 0.0, 0, 0.0, c->w.p, nullptr, st);
+        else {
+          refresh_offset(c);
+          CnEval e{};
+          e.x = c->tmp.p;
+          e.out = c->w.p;
+          cn_eval<CN_L>(c, e, st);
+        }
         gather(c->w.p, y);
         break;
       }
       case GM_CC_OP_H_MATVEC: {
         scatter(x, c->tmp.p);
-        hmatvec(c, c->tmp.p, param, c->w.p, st);
+        CnEval e{};
+        e.x = c->tmp.p;
+        e.hdt = 0.5 * param;
+        e.out = c->w.p;
+        cn_eval<CN_H>(c, e, st);
         gather(c->w.p, y);
         break;
       }

@@ -245,7 +245,7 @@ struct gm_handle {
   // 25 us of a 220 us step in FP64, which needs no sweep, and about 50 in the FP32 mode.  A solve that
   // needs more than its slot's stops the steps behind it (ERR_SWEEPS); the host adds one and repeats
   // the step.  FP64 starts with none, the FP32 mode with the one that it always needs.
-  bool loops = true;  // captures as WHILE nodes (the cut-cell step)
+  bool looped = false;  // the solves of this capture are the loops of a batch group
   int sweeps[5] = {0, 0, 0, 0, 0};
   // launch-by-launch steps decide every refinement sweep on the host (one synchronisation
   // per sweep) instead of launching all sweeps gated: then every launched kernel does work,
@@ -1210,48 +1210,6 @@ void apply_inverse(gm_handle* h, int lane, RectDev& rd, int kind, const void* r,
   }
 }
 
-// The same solve while the step is being captured into a CUDA graph: the refinement
-// sweeps form a WHILE conditional node whose body runs only while the residual check
-// exceeds the target, so no sweep kernel launches when none is needed.
-void schur_solve_graph(gm_handle* h, int lane, RectDev& rd, int kind, double hc, const double* b, double* x,
-                       double* res, double* first, double* w2, int slot) {
-  cudaStream_t st = lane == 0 ? h->st : h->st2;
-  cudaStream_t body_st = lane == 0 ? h->st_body : h->st2_body;
-  SolveCtl* sc = &h->ctl.p->solve[slot];
-  Gate g0 = gate_of(h, slot, 0);
-  const bool f32 = h->precision == 1;
-  void* resb = f32 ? (void*)(kind == 0 ? h->pres32.p : h->fres32.p) : (void*)res;
-  (void)hc;
-  h->sweep_marking = h->phase_on && slot == S_P1;
-  apply_inverse(h, lane, rd, kind, b, false, x, false, first, w2, g0, st);
-  launch_residual(h->cd, h->rcoef[kind], kind, b, x, resb, f32, sc, 0, true, g0, st);
-  sweep_mark(h, 8, st);
-  h->sweep_marking = false;
-  cudaStreamCaptureStatus cs;
-  cudaGraph_t graph;
-  const cudaGraphNode_t* deps = nullptr;
-  size_t nd = 0;
-  CK(cudaStreamGetCaptureInfo(st, &cs, nullptr, &graph, nullptr, nullptr, nullptr));
-  cudaGraphConditionalHandle cond;
-  CK(cudaGraphConditionalHandleCreate(&cond, graph, 0, 0));
-  launch_refine_decide(h->ctl.p, slot, h->nchk, cond, st);
-  CK(cudaStreamGetCaptureInfo(st, &cs, nullptr, &graph, &deps, nullptr, &nd));
-  cudaGraphNodeParams cp{};
-  cp.type = cudaGraphNodeTypeConditional;
-  cp.conditional.handle = cond;
-  cp.conditional.type = cudaGraphCondTypeWhile;
-  cp.conditional.size = 1;
-  cudaGraphNode_t cnode;
-  CK(cudaGraphAddNode(&cnode, graph, deps, nullptr, nd, &cp));
-  cudaGraph_t body = cp.conditional.phGraph_out[0];
-  CK(cudaStreamUpdateCaptureDependencies(st, &cnode, nullptr, 1, cudaStreamSetCaptureDependencies));
-  CK(cudaStreamBeginCaptureToGraph(body_st, body, nullptr, nullptr, 0, cudaStreamCaptureModeRelaxed));
-  apply_inverse(h, lane, rd, kind, resb, f32, x, true, first, w2, g0, body_st);
-  launch_residual(h->cd, h->rcoef[kind], kind, b, x, resb, f32, sc, -1, false, g0, body_st);
-  launch_refine_decide(h->ctl.p, slot, h->nchk, cond, body_st);
-  CK(cudaStreamEndCapture(body_st, &body));
-}
-
 // Flexible GMRES(50) for A x = b on the pressure grid, right-preconditioned by the separable
 // rectangle inverse (no boundary term) -- solver/pressure_schur.py:20-41 with
 // gmres(rtol=atol=1e-12, restart=50, maxiter=100): at most 100 restart cycles, convergence
@@ -1591,16 +1549,12 @@ void gmres_monitored(gm_handle* h, const double* b, double* x, double* res, int 
 // reference's residual target (solver/pressure_schur.py:16-72, direct branch).
 // refinement sweeps launched for a slot
 int sweeps_of(const gm_handle* h, int slot) {
-  return h->capturing && !h->loops ? std::min(h->sweeps[slot], h->nchk - 1) : h->nchk - 1;
+  return h->capturing && !h->looped ? std::min(h->sweeps[slot], h->nchk - 1) : h->nchk - 1;
 }
 void schur_solve(gm_handle* h, int lane, RectDev& rd, int kind, double hc, const double* b, double* x, double* res,
                  double* first, double* w2, int slot) {
   if (kind == 0 && h->g.pressure_solver == 1) {
     gmres_monitored(h, b, x, res, slot);
-    return;
-  }
-  if (h->capturing && h->loops) {
-    schur_solve_graph(h, lane, rd, kind, hc, b, x, res, first, w2, slot);
     return;
   }
   cudaStream_t st = lane == 0 ? h->st : h->st2;
@@ -1617,7 +1571,7 @@ void schur_solve(gm_handle* h, int lane, RectDev& rd, int kind, double hc, const
     if (h->sweep_marking) sweep_mark(h, 8, st);
     h->sweep_marking = false;
     if (h->host_refine && sweep + 1 < h->nchk) {
-      // the rule of k_refine_decide, read back on the host
+      // sweep_needed's rule, read back on the host
       SolveCtl hs;
       CK(cudaMemcpyAsync(&hs, sc, sizeof hs, cudaMemcpyDeviceToHost, st));
       int err = 0;
@@ -1660,7 +1614,7 @@ void project_post(gm_handle* h, const double* q, double dt, double* out, double*
     CK(cudaMemcpyAsync(h->rec_sol + off, phi, h->Pn * sizeof(double), cudaMemcpyDeviceToDevice, st));
     ++h->rec_count;
   }
-  launch_proj_update(h->cd, q, phi, dt, out, slot, h->nchk, sweeps_of(h, slot), !(h->capturing && h->loops), gate_of(h), st);
+  launch_proj_update(h->cd, q, phi, dt, out, slot, h->nchk, sweeps_of(h, slot), !h->looped, gate_of(h), st);
 }
 // a projection by itself, its gate included (div_max[divk])
 void project(gm_handle* h, const double* q, double dt, double* out, double* phi, int slot, int divk) {
@@ -2110,21 +2064,18 @@ cudaGraphExec_t step_graph(gm_handle* h, double dt) {
   if (slot->exec) { cudaGraphExecDestroy(slot->exec); slot->exec = nullptr; }
   const long long c0 = kernel_launch_count();
   h->capturing = true;
-  h->loops = false;
   cudaGraph_t g = nullptr;
   CK(cudaStreamBeginCapture(h->st, cudaStreamCaptureModeThreadLocal));
   try {
     step_once(h, dt, -1);
   } catch (...) {
     h->capturing = false;
-    h->loops = true;
     cudaStreamEndCapture(h->st, &g);
     if (g) cudaGraphDestroy(g);
     cudaGetLastError();
     throw;
   }
   h->capturing = false;
-  h->loops = true;
   CK(cudaStreamEndCapture(h->st, &g));
   slot->nodes = kernel_launch_count() - c0;
   kernel_launch_adjust(-slot->nodes);
@@ -2927,7 +2878,7 @@ int gm_pressure_solve(gm_handle* h, const double* rhs, double* phi, gm_solve_inf
     launch_scatter(b, h->d_pi.p, np, h->prhs.p, st);
     CK(cudaMemsetAsync(h->ctl.p, 0, sizeof(StepCtl), st));
     schur_solve(h, 0, h->rp, 0, 0.0, h->prhs.p, h->pphi.p, h->pres.p, h->pfirst.p, h->pw2.p, S_P1);
-    launch_gate_pressure(h->ctl.p, S_P1, h->nchk, st);
+    launch_gate_pressure(h->ctl.p, S_P1, h->nchk, h->nchk - 1, st);
     CK(cudaMemcpyAsync(h->host_ctl, h->ctl.p, sizeof(StepCtl), cudaMemcpyDeviceToHost, st));
     CK(cudaStreamSynchronize(st));
     solve_info_from(h, S_P1, info);
@@ -3529,14 +3480,14 @@ gm_batch::Graph& batch_graph(gm_batch* b, double dt) {
       for (size_t c = 0; c < b->cases.size(); ++c) {
         gm_handle* h = b->cases[c];
         CK(cudaStreamWaitEvent(h->st, b->fork, 0));
-        h->capturing = true;
+        h->capturing = h->looped = true;
       }
       const long long c0 = kernel_launch_count();
       capture_grouped_step(b, dt, *slot);
       kernel_launch_adjust(-(kernel_launch_count() - c0));
       for (size_t c = 0; c < b->cases.size(); ++c) {
         gm_handle* h = b->cases[c];
-        h->capturing = false;
+        h->capturing = h->looped = false;
         CK(cudaEventRecord(b->join[c], h->st));
         CK(cudaStreamWaitEvent(b->root, b->join[c], 0));
       }
@@ -3546,17 +3497,15 @@ gm_batch::Graph& batch_graph(gm_batch* b, double dt) {
       CK(cudaStreamWaitEvent(h->st, b->fork, 0));
       const long long c0 = kernel_launch_count();
       h->capturing = true;
-      h->loops = false;
       step_once(h, dt, -1);
       h->capturing = false;
-      h->loops = true;
       slot->outer[c] = kernel_launch_count() - c0;
       kernel_launch_adjust(-slot->outer[c]);
       CK(cudaEventRecord(b->join[c], h->st));
       CK(cudaStreamWaitEvent(b->root, b->join[c], 0));
     }
   } catch (...) {
-    for (gm_handle* h : b->cases) { h->capturing = false; h->loops = true; }
+    for (gm_handle* h : b->cases) h->capturing = h->looped = false;
     cudaStreamEndCapture(b->root, &g);
     if (g) cudaGraphDestroy(g);
     cudaGetLastError();
@@ -3780,7 +3729,7 @@ void set_capturing(gm_handle* h, bool on) { h->capturing = on; }
 
 void pressure_solve(gm_handle* h, const double* b, double* x, int slot) {
   schur_solve(h, 0, h->rp, 0, 0.0, b, x, h->pres.p, h->pfirst.p, h->pw2.p, slot);
-  launch_gate_pressure(h->ctl.p, slot, h->nchk, h->st);
+  launch_gate_pressure(h->ctl.p, slot, h->nchk, sweeps_of(h, slot), h->st);
 }
 
 const double* pressure_residual(gm_handle* h) { return h->pres.p; }
@@ -3791,6 +3740,9 @@ int check(gm_handle* h, const char* where, std::string& err) {
   if (rc != GM_OK) err = h->err;
   return rc;
 }
+
+int failed_gate(const gm_handle* h) { return h->host_ctl->gate; }
+void add_sweep(gm_handle* h, int slot) { ++h->sweeps[slot]; }
 
 int64_t schur_rank(const gm_handle* h) { return h->rp.rank; }
 

@@ -26,10 +26,10 @@ int pressure_create(gm::Geometry&& g, gm_handle** out, std::string& err);
 void pressure_destroy(gm_handle* h);
 const gm::Geometry& geometry(const gm_handle* h);
 cudaStream_t stream(gm_handle* h);
-// streams that capture the bodies of conditional graph nodes (two nesting levels)
+// streams that capture the bodies of conditional graph nodes
 cudaStream_t body_stream(gm_handle* h, int level);
-// while set, pressure_solve records its refinement sweeps as a WHILE node of the graph being
-// captured on stream(h)
+// while set, pressure_solve records as many gated refinement sweeps as its slot holds (a solve that needs
+// more raises gmk::ERR_SWEEPS with the slot as the gate word)
 void set_capturing(gm_handle* h, bool on);
 // Monitored solve of A x = b (full pressure grids on the device, inactive cells ignored in b
 // and zero in x) in control slot `slot` (gmk::S_P0..S_P2), then its pressure gate.
@@ -39,6 +39,8 @@ const double* pressure_residual(gm_handle* h);
 gmk::StepCtl* control(gm_handle* h);
 // GM_OK or the class of a failed gate / CUDA error recorded in the control block (message in err)
 int check(gm_handle* h, const char* where, std::string& err);
+int failed_gate(const gm_handle* h);       // the gate word that check read
+void add_sweep(gm_handle* h, int slot);    // one more sweep in graphs captured from here on
 int64_t schur_rank(const gm_handle* h);
 // surface point-pressure reconstruction (rows = quadrature points, columns = pressure cells)
 struct SurfaceCsr {

@@ -1522,6 +1522,7 @@ __device__ __forceinline__ void residual_body(const CaseDev& c, const ResidualCo
   double* res64 = reinterpret_cast<double*>(res_out);
   float* res32 = reinterpret_cast<float*>(res_out);
   unsigned long long rm = 0, bm = 0, bd = 0, xb = 0;
+  unsigned long long full = 0;  // largest |A| |x| + |b| over rows with five entries: scaling by their (2 nnz + 2) eps is monotonic
   double rs = 0.0, bs = 0.0;
   float rs32 = 0.0f;  // RES_F32: sum of the stored FP32 residuals squared (diagnostics only)
   float bs32 = 0.0f;  // RES_F32: sum of the right-hand side squared in FP32 (diagnostics only)
@@ -1608,7 +1609,11 @@ __device__ __forceinline__ void residual_body(const CaseDev& c, const ResidualCo
       res64[f] = r;
       rs += r * r;
     }
-    if (KIND == 0 && !RES_F32) bd = umax64(bd, dbits((2.0 * nnz + 2.0) * EPS64 * (aabs + absd(bv))));
+    if (KIND == 0 && !RES_F32) {
+      const double ab = aabs + absd(bv);
+      if (nnz == 5) full = umax64(full, dbits(ab));
+      else bd = umax64(bd, dbits((2.0 * nnz + 2.0) * EPS64 * ab));
+    }
     if (BOUND32)
       bd32 = fmaxf(bd32, (2.0f * (float)nnz + 2.0f) * 2.220446049250313e-16f * (aabs32 + fabsf(f64_to_f32i(bv))));
     if (first) {
@@ -1625,7 +1630,7 @@ __device__ __forceinline__ void residual_body(const CaseDev& c, const ResidualCo
   block_commit_max(rm, &sc->rmax[check]);
   if constexpr (RES_F32) block_commit_sum_f32(rs32, &sc->rsq[check]);
   else block_commit_sum(rs, &sc->rsq[check]);
-  if (KIND == 0 && !RES_F32) block_commit_max(bd, &sc->bound[check]);
+  if (KIND == 0 && !RES_F32) block_commit_max(umax64(bd, dbits((2.0 * 5 + 2.0) * EPS64 * bits2d(full))), &sc->bound[check]);
   // the FP32 bound times 1 + 2^-20 (above its own rounding), as an FP64 value; non-negative
   // doubles order like their bits
   if (BOUND32) block_commit_max(dbits(f32_to_f64i(bd32 * 1.00000095367431640625f)), &sc->bound[check]);
@@ -2651,13 +2656,13 @@ void launch_step_tail(const CaseDev& c, const StepTail& a, const Gate& gate, cud
   kt_mark(9, st);
 }
 
-__global__ void k_gate_pressure(StepCtl* ctl, int slot, int nchk) {
-  if (!ctl->err) check_pressure(ctl, slot, nchk, nchk - 1);
+__global__ void k_gate_pressure(StepCtl* ctl, int slot, int nchk, int sweeps) {
+  if (!ctl->err) check_pressure(ctl, slot, nchk, sweeps);
 }
-void launch_gate_pressure(StepCtl* ctl, int slot, int nchk, cudaStream_t st) {
+void launch_gate_pressure(StepCtl* ctl, int slot, int nchk, int sweeps, cudaStream_t st) {
   note_launch();
   kt_mark(10, st);
-  k_gate_pressure<<<1, 1, 0, st>>>(ctl, slot, nchk);
+  k_gate_pressure<<<1, 1, 0, st>>>(ctl, slot, nchk, sweeps);
   kt_mark(10, st);
 }
 
@@ -3083,21 +3088,6 @@ void launch_cg_combine(const CaseDev& c, const CompactGmres& g, const double* z0
   kt_mark(6, st);
   k_cg_combine<<<reduce_blocks(c.psize), TPB, 0, st>>>(c, g, z0, out, x, e);
   kt_mark(6, st, (double)c.psize * 25);
-}
-
-__global__ void k_refine_decide(StepCtl* ctl, int slot, int nchk, cudaGraphConditionalHandle cond) {
-  SolveCtl* sc = &ctl->solve[slot];
-  int k = sc->k;
-  bool need = false;
-  if (!ctl->err) need = bits2d(sc->rmax[k]) > inner_target(sc) && k + 1 < nchk;
-  if (need) sc->k = k + 1;
-  cudaGraphSetConditional(cond, need ? 1u : 0u);
-}
-void launch_refine_decide(StepCtl* ctl, int slot, int nchk, cudaGraphConditionalHandle cond, cudaStream_t st) {
-  note_launch();
-  kt_mark(10, st);
-  k_refine_decide<<<1, 1, 0, st>>>(ctl, slot, nchk, cond);
-  kt_mark(10, st);
 }
 
 __global__ void k_copy_active(const uint8_t* __restrict__ cls, int64_t n, const double* __restrict__ src,

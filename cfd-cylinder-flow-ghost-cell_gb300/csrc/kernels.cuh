@@ -447,7 +447,7 @@ void launch_ghost(double* field, int n, const int64_t* rows, const int64_t* ptr,
 
 // residual of the operator of kind (0 pressure A, 1 Helmholtz u, 2 Helmholtz v)
 // res = b - Op x on active points; reductions into sc at check index `check`
-// (check < 0: the index sc->k maintained by launch_refine_decide)
+// (check < 0: the index sc->k maintained by launch_refine_decide_multi)
 // Host-formed coefficients of the regular rows of one operator: A x at a point is
 //   cc[ic][jc] x + cw[ic] x_west + ce x_east + cy (x_south + x_north)
 // with ic = 0 first column, 1 interior, 2 last column and jc = 0 wall row, 1 interior.
@@ -598,7 +598,7 @@ void launch_gate_projection(StepCtl* ctl, int k, cudaStream_t st);
 void launch_cfl_screen(StepCtl* ctl, const unsigned long long* umax, const unsigned long long* vmax, double dt,
                        double dx, double dy, int screen, const long long* counter, cudaStream_t st);
 
-void launch_gate_pressure(StepCtl* ctl, int slot, int nchk, cudaStream_t st);
+void launch_gate_pressure(StepCtl* ctl, int slot, int nchk, int sweeps, cudaStream_t st);
 // dst[k] = src[idx[k]] and dst[idx[k]] = src[k]
 void launch_gather(const double* src, const int64_t* idx, int64_t n, double* dst, cudaStream_t st);
 void launch_scatter(const double* src, const int64_t* idx, int64_t n, double* dst, cudaStream_t st);
@@ -606,9 +606,6 @@ void launch_scatter(const double* src, const int64_t* idx, int64_t n, double* ds
 void launch_schur_column(const double* first, const RectView& view, int rank, const int64_t* c_ptr,
                          const int64_t* c_col, const double* c_val, double* S, int col, cudaStream_t st);
 
-// Refinement loop decision for a graph WHILE node: if check sc->k exceeded the inner
-// target and another check is allowed, advance sc->k and set the condition to 1.
-void launch_refine_decide(StepCtl* ctl, int slot, int nchk, cudaGraphConditionalHandle cond, cudaStream_t st);
 // zero/copy helpers
 void launch_copy_active(const uint8_t* cls, int64_t n, const double* src, double* dst, const Gate& gate,
                         cudaStream_t st);
