@@ -32,6 +32,7 @@
 
 namespace gmk {
 void kernel_launch_adjust(long long delta);  // the library's launch counter (kernels.cu)
+int pdl_mode_ext();
 }
 
 namespace {
@@ -116,6 +117,61 @@ __device__ __forceinline__ T lap_p(const S* f, int n, int j, int i, T h, T nu) {
   return ((fE - fW) + (fN - fS)) / (h * h);
 }
 
+// ---- a step's control words -----------------------------------------------------------------
+// Reductions (bits of non-negative doubles), the step whose gate failed (RED_ERR, from 1) and, when it
+// failed because a solve needed more refinement sweeps than were queued, that solve's slot + 1
+// (RED_SHORT); then the residual of every check of every refined solve (FP32 mode).
+enum : int { RED_CN = 0, RED_RHS = 1, RED_DIV = 2, RED_COUPLED = 3, RED_SHORT = 4, RED_ERR = 5, RED_W = 8 };
+enum : int { SLOT_START = 0, SLOT_CN = 1, SLOT_P1 = 2, SLOT_P2 = 3, NSLOT = 4, SLOT_CHECKS = 9, RED_N = RED_W + NSLOT * SLOT_CHECKS };
+// Whether an earlier gate of this call failed: the state writers of the steps queued behind it return.
+__device__ __forceinline__ bool tg_failed(const unsigned long long* red) {
+  return *(const volatile unsigned long long*)(red + RED_ERR) != 0;
+}
+// A kernel launched as a programmatic dependent starts before its predecessor ends; every kernel of this
+// file waits for it here before it reads anything.
+__device__ __forceinline__ void tg_wait() { asm volatile("griddepcontrol.wait;" ::: "memory"); }
+// Whether check k of a refined solve is above its target: max |r| <= 32 eps max(1, max |b|) for the CN
+// solve, max |r| step <= 1e-11 for a pressure.  A check that did not run holds zero.
+__device__ __forceinline__ bool tg_above(const unsigned long long* red, int slot, int k, double step) {
+  const double r = __longlong_as_double((long long)*(const volatile unsigned long long*)(red + RED_W + slot * SLOT_CHECKS + k));
+  if (slot != SLOT_CN) return !(r * step <= 1e-11);
+  const double b = __longlong_as_double((long long)*(const volatile unsigned long long*)(red + RED_RHS));
+  return !(r <= 32 * 2.220446049250313e-16 * (b > 1.0 ? b : 1.0));
+}
+// The FP32 mode queues a fixed number of refinement sweeps for each solve; the kernels of a sweep run
+// while the check `k` before it (k < 0: none) is above the target.
+struct TgGate {
+  const unsigned long long* red;  // null: always open
+  int slot, k;
+  double step;
+};
+__device__ __forceinline__ bool tg_open(const TgGate& g) {
+  tg_wait();
+  if (!g.red) return true;
+  return !tg_failed(g.red) && (g.k < 0 || tg_above(g.red, g.slot, g.k, g.step));
+}
+// The solve's residual is still above the target after all sweeps that were queued (`held`; the largest
+// number that the mode takes, `most`, never falls short): the step fails and the host repeats it.
+struct TgHeld {
+  int slot, held, most;  // slot < 0: none
+  double step;
+};
+__device__ __forceinline__ bool tg_short(unsigned long long* red, const TgHeld& h, int step_index) {
+  if (h.slot < 0 || h.held >= h.most || !tg_above(red, h.slot, h.held, h.step)) return false;
+  if (blockIdx.x == 0 && threadIdx.x == 0) {
+    red[RED_SHORT] = (unsigned long long)h.slot + 1;
+    red[RED_ERR] = (unsigned long long)step_index;
+  }
+  return true;
+}
+// a / b for a divisor known in advance (rb = 1 / b, correctly rounded): one multiplication and two fused
+// multiply-adds give the correctly rounded quotient (Brisebarre, Muller and Raina, IEEE Trans. Computers
+// 53, 2004), a third of a divide's FP64 instructions and the same bits
+__device__ __forceinline__ double div_by(double a, double b, double rb) {
+  const double q = a * rb;
+  return fma(fma(-q, b, a), rb, q);
+}
+
 // ---- kernels ------------------------------------------------------------------------------
 // AB2/CN right-hand sides (solver/time_integration.py:20-67): mode 0 AB2, mode 1 start-up
 // midpoint, mode 2 start-up CN right-hand side from the half-step velocity
@@ -123,9 +179,15 @@ __device__ __forceinline__ T lap_p(const S* f, int n, int j, int i, T h, T nu) {
 template <typename T>
 __global__ void k_tg_rhs(int n, double h, double nu, int mode, double dt, double alpha, const double* __restrict__ q,
                          const double* __restrict__ qh, const double* __restrict__ p, const double* __restrict__ prev,
-                         double* __restrict__ now, double* __restrict__ out) {
+                         double* __restrict__ now, double* __restrict__ out, unsigned long long* red, TgHeld start,
+                         int step_index) {
+  tg_wait();
+  if (tg_failed(red) || (mode == 2 && tg_short(red, start, step_index))) return;
   const int nn = n * n;
   const int t = blockIdx.x * blockDim.x + threadIdx.x;
+  // this step's words; the previous step's kernels have read theirs (mode 2 follows the start-up solve)
+  if (mode != 2 && t < NSLOT * SLOT_CHECKS) red[RED_W + t] = 0;
+  if (mode != 2 && t == 0) red[RED_RHS] = 0;
   if (t >= 2 * nn) return;
   const int comp = t >= nn, k = t - comp * nn, j = k / n, i = k - j * n;
   const double* u = q;
@@ -159,12 +221,6 @@ __global__ void k_tg_rhs(int n, double h, double nu, int mode, double dt, double
 
 // ---- FP64 stencils: 1/h and the products of the step formed on the host (GB300 issues FP64 at
 // 1/64 of the FP32 rate and a divide costs about seven instructions) --------------------------
-// A step's reductions and its failed-gate word (bits of non-negative doubles).
-enum : int { RED_CN = 0, RED_RHS = 1, RED_DIV = 2, RED_COUPLED = 3, RED_PRES = 4, RED_ERR = 5 };
-// Whether an earlier gate of this call failed: the state writers of the steps queued behind it return.
-__device__ __forceinline__ bool tg_failed(const unsigned long long* red) {
-  return *(const volatile unsigned long long*)(red + RED_ERR) != 0;
-}
 __device__ __forceinline__ double lap4(const double* __restrict__ f, int n, int j, int i, int k, double c) {
   const double e = f[i + 1 < n ? k + 1 : k + 1 - n], w = f[i > 0 ? k - 1 : k - 1 + n];
   const double u = f[j + 1 < n ? k + n : k + n - n * n], d = f[j > 0 ? k - n : k - n + n * n];
@@ -182,6 +238,7 @@ template <int MODE>
 __global__ void k_tg_rhs64(int n, TgRhsC c, const double* __restrict__ q, const double* __restrict__ qh,
                            const double* __restrict__ p, const double* __restrict__ prev, double* __restrict__ now,
                            double* __restrict__ out, unsigned long long* red) {
+  tg_wait();
   if (tg_failed(red)) return;
   const int nn = n * n, k = blockIdx.x * blockDim.x + threadIdx.x;
   if (k == 0) red[RED_CN] = red[RED_RHS] = 0;  // this step's; the previous step's were read by its gate
@@ -229,56 +286,58 @@ __global__ void k_tg_rhs64(int n, TgRhsC c, const double* __restrict__ q, const 
 // another last bit of these stencils moves by 4e-8 in 20 steps, and its small grids gain little.
 struct TgC {
   double h, nu, hdt;     // with divides: spacing, viscosity, dt / 2
-  double ih, kh;         // P64: 1 / h, dt nu / (2 h^2)
+  double hh, ihh;        // h^2 and its reciprocal
+  double ih, kh;         // 1 / h; P64: dt nu / (2 h^2)
 };
+// nu L at a point (lap_p in FP64) with div_by for its divides
+__device__ __forceinline__ double lap_d(const TgC& g, const double* f, int n, int j, int i) {
+  const int ip = wrapi(i + 1, n), im = wrapi(i - 1, n), jp = wrapi(j + 1, n), jm = wrapi(j - 1, n);
+  const double c = f[j * n + i], h = g.h, nu = g.nu;
+  const double fE = div_by(nu * (f[j * n + ip] - c), h, g.ih) * h, fW = div_by(nu * (c - f[j * n + im]), h, g.ih) * h;
+  const double fN = div_by(nu * (f[jp * n + i] - c), h, g.ih) * h, fS = div_by(nu * (c - f[jm * n + i]), h, g.ih) * h;
+  return div_by((fE - fW) + (fN - fS), g.hh, g.ihh);
+}
 template <bool P64>
 __device__ __forceinline__ double helm_p(const TgC& c, const double* __restrict__ f, int n, int j, int i, int k, double x) {
   if (P64) return fma(-c.kh, lap4(f, n, j, i, k, x), x);
-  return x - c.hdt * lap_p<double>(f, n, j, i, c.h, c.nu);
+  return x - c.hdt * lap_d(c, f, n, j, i);
 }
 __device__ __forceinline__ double div_sum(const double* __restrict__ q, int n, int j, int i, int k) {
   const int nn = n * n;
   return q[i + 1 < n ? k + 1 : k + 1 - n] - q[k] + q[nn + (j + 1 < n ? k + n : k + n - nn)] - q[nn + k];
 }
 
-// r = b - H x (H = I - dt/2 nu L) with max |r| and max |b|
+// max |b - H x| (H = I - dt/2 nu L) and max |b|
 template <bool P64>
 __global__ void k_tg_hres(int n, TgC c, const double* __restrict__ b, const double* __restrict__ x,
-                          double* __restrict__ r, unsigned long long* red) {
+                          unsigned long long* rmax, unsigned long long* bmax, TgGate gate) {
+  if (!tg_open(gate)) return;
   const int nn = n * n;
   unsigned long long rm = 0, bm = 0;
   for (int t = blockIdx.x * blockDim.x + threadIdx.x; t < 2 * nn; t += gridDim.x * blockDim.x) {
     const int comp = t >= nn, k = t - comp * nn, j = k / n, i = k - j * n;
     const double bv = b[t], rv = bv - helm_p<P64>(c, x + comp * nn, n, j, i, k, x[t]);
-    if (r) r[t] = rv;
     rm = max(rm, absbits_(rv));
     bm = max(bm, absbits_(bv));
   }
-  commit_max(rm, red + RED_CN);
-  commit_max(bm, red + RED_RHS);
+  commit_max(rm, rmax);
+  if (bmax) commit_max(bm, bmax);
 }
 
-// FP32 mode: d = div(q) / step on the cell grid
-__global__ void k_tg_div(int n, double h, double inv_step, const double* __restrict__ q, double* __restrict__ d) {
-  const int nn = n * n;
-  for (int k = blockIdx.x * blockDim.x + threadIdx.x; k < nn; k += gridDim.x * blockDim.x) {
-    const int j = k / n, i = k - j * n;
-    d[k] = div_sum(q, n, j, i, k) / h * inv_step;
-  }
+// FP32 mode: (A phi)(k) with A = div grad (periodic 5-point / h^2)
+__device__ __forceinline__ double pres_p(const TgC& c, const double* __restrict__ x, int n, int j, int i, int k) {
+  return div_by(((x[j * n + wrapi(i + 1, n)] - x[k]) - (x[k] - x[j * n + wrapi(i - 1, n)]) +
+                 (x[wrapi(j + 1, n) * n + i] - x[k]) - (x[k] - x[wrapi(j - 1, n) * n + i])), c.hh, c.ihh);
 }
-
-// FP32 mode: r = b - A phi with A = div grad (periodic 5-point / h^2), max |r|
-__global__ void k_tg_pres(int n, double h, const double* __restrict__ b, const double* __restrict__ x,
-                          double* __restrict__ r, unsigned long long* rmax) {
+// max |b - A phi|
+__global__ void k_tg_pres(int n, TgC c, const double* __restrict__ b, const double* __restrict__ x,
+                          unsigned long long* rmax, TgGate gate) {
+  if (!tg_open(gate)) return;
   const int nn = n * n;
   unsigned long long rm = 0;
   for (int k = blockIdx.x * blockDim.x + threadIdx.x; k < nn; k += gridDim.x * blockDim.x) {
     const int j = k / n, i = k - j * n;
-    const double ax = ((x[j * n + wrapi(i + 1, n)] - x[k]) - (x[k] - x[j * n + wrapi(i - 1, n)]) +
-                       (x[wrapi(j + 1, n) * n + i] - x[k]) - (x[k] - x[wrapi(j - 1, n) * n + i])) / (h * h);
-    const double rv = b[k] - ax;
-    r[k] = rv;
-    rm = max(rm, absbits_(rv));
+    rm = max(rm, absbits_(b[k] - pres_p(c, x, n, j, i, k)));
   }
   commit_max(rm, rmax);
 }
@@ -290,12 +349,20 @@ __global__ void k_tg_pres(int n, double h, const double* __restrict__ b, const d
 template <bool P64>
 __global__ void k_tg_update(int n, TgC c, double step, double kg, const double* __restrict__ q,
                             const double* __restrict__ phi, double* __restrict__ out, unsigned long long* red,
-                            int gate_step) {
+                            int gate_step, TgHeld cn) {
+  tg_wait();
   if (gate_step > 0) {
-    if (tg_failed(red)) return;
-    const double r = __longlong_as_double((long long)red[RED_CN]), b = __longlong_as_double((long long)red[RED_RHS]);
+    if (tg_failed(red) || (!P64 && tg_short(red, cn, gate_step))) return;
+    int last = 0;  // FP32 mode: the last check that ran
+    if (!P64)
+      while (last < cn.held && tg_above(red, SLOT_CN, last, 0.0)) ++last;
+    const double r = __longlong_as_double((long long)red[P64 ? RED_CN : RED_W + SLOT_CN * SLOT_CHECKS + last]);
+    const double b = __longlong_as_double((long long)red[RED_RHS]);
     if (!(r <= 1e-10 * (b > 1.0 ? b : 1.0)) || !isfinite(r)) {
-      if (blockIdx.x == 0 && threadIdx.x == 0) red[RED_ERR] = (unsigned long long)gate_step;
+      if (blockIdx.x == 0 && threadIdx.x == 0) {
+        if (!P64) red[RED_CN] = dbits_(r);
+        red[RED_ERR] = (unsigned long long)gate_step;
+      }
       return;
     }
   }
@@ -304,16 +371,18 @@ __global__ void k_tg_update(int n, TgC c, double step, double kg, const double* 
   const int j = k / n, i = k - j * n;
   const double f = phi[k];
   const double gu = f - phi[i > 0 ? k - 1 : k - 1 + n], gv = f - phi[j > 0 ? k - n : k - n + nn];
-  out[k] = P64 ? fma(-kg, gu, q[k]) : q[k] - step * (gu / c.h);
-  out[nn + k] = P64 ? fma(-kg, gv, q[nn + k]) : q[nn + k] - step * (gv / c.h);
+  out[k] = P64 ? fma(-kg, gu, q[k]) : q[k] - step * div_by(gu, c.h, c.ih);
+  out[nn + k] = P64 ? fma(-kg, gv, q[nn + k]) : q[nn + k] - step * div_by(gv, c.h, c.ih);
 }
 
 // action = H result, proj = result + (rhs - action)   (solver/time_integration.py:107-113), and
 // the largest |div result|
 template <bool P64>
 __global__ void k_tg_defect(int n, TgC c, const double* __restrict__ res, const double* __restrict__ rhs,
-                            double* __restrict__ action, double* __restrict__ proj, unsigned long long* red) {
-  if (tg_failed(red)) return;
+                            double* __restrict__ action, double* __restrict__ proj, unsigned long long* red, TgHeld p1,
+                            int step_index) {
+  tg_wait();
+  if (tg_failed(red) || (!P64 && tg_short(red, p1, step_index))) return;
   const int nn = n * n;
   unsigned long long m = 0;
   for (int k = blockIdx.x * blockDim.x + threadIdx.x; k < nn; k += gridDim.x * blockDim.x) {
@@ -326,7 +395,7 @@ __global__ void k_tg_defect(int n, TgC c, const double* __restrict__ res, const 
       proj[t] = x + (rhs[t] - a);
     }
     const double d = div_sum(res, n, j, i, k);
-    m = max(m, absbits_(P64 ? d * c.ih : d / c.h));
+    m = max(m, absbits_(P64 ? d * c.ih : div_by(d, c.h, c.ih)));
   }
   commit_max(m, red + RED_DIV);
 }
@@ -336,8 +405,9 @@ template <bool P64>
 __global__ void k_tg_pout(int n, TgC c, double dt, double kg, double factor, const double* __restrict__ p,
                           const double* __restrict__ inc, const double* __restrict__ action,
                           const double* __restrict__ rhs, double* __restrict__ half, double* __restrict__ pout,
-                          unsigned long long* red) {
-  if (tg_failed(red)) return;
+                          unsigned long long* red, TgHeld p2, int step_index) {
+  tg_wait();
+  if (tg_failed(red) || (!P64 && tg_short(red, p2, step_index))) return;
   const int nn = n * n;
   unsigned long long m = 0;
   for (int k = blockIdx.x * blockDim.x + threadIdx.x; k < nn; k += gridDim.x * blockDim.x) {
@@ -345,8 +415,8 @@ __global__ void k_tg_pout(int n, TgC c, double dt, double kg, double factor, con
     const double f = inc[k];
     const double gu = f - inc[i > 0 ? k - 1 : k - 1 + n], gv = f - inc[j > 0 ? k - n : k - n + nn];
     const double au = action[k] - rhs[k], av = action[nn + k] - rhs[nn + k];
-    m = max(m, absbits_(P64 ? fma(kg, gu, au) : au + dt * (gu / c.h)));
-    m = max(m, absbits_(P64 ? fma(kg, gv, av) : av + dt * (gv / c.h)));
+    m = max(m, absbits_(P64 ? fma(kg, gu, au) : au + dt * div_by(gu, c.h, c.ih)));
+    m = max(m, absbits_(P64 ? fma(kg, gv, av) : av + dt * div_by(gv, c.h, c.ih)));
     const double hv = p[k] + f;
     half[k] = hv;
     pout[k] = hv + factor * f;
@@ -370,7 +440,18 @@ __global__ void k_tg_pout(int n, TgC c, double dt, double kg, double factor, con
 // (8 8 8 2) the column pass takes 150 us for u + i v and 77 for a pressure (0.80 and 0.77 of the pipe's
 // rate), row passes 82-87 and 47-54; a solve of seven kernels with transposes took 366 us a field,
 // now 186 a pressure and 319 both components
-enum : int { LINE_REAL = 0, LINE_PAIR = 1, LINE_UV = 2 };
+// and, forward in the FP32 mode (one real row each):
+//   LINE_DIV   div(q) / step, stored on the way (the right-hand side of a pressure)
+//   LINE_PRES  the residual b - A x of a pressure, its maximum on the way: a check of the refinement and
+//   LINE_HRES  the first pass of the sweep behind it in one kernel; of the CN solve
+enum : int { LINE_REAL = 0, LINE_PAIR = 1, LINE_UV = 2, LINE_DIV = 3, LINE_PRES = 4, LINE_HRES = 5 };
+struct TgRow {
+  TgC c;
+  double s;              // LINE_DIV: 1 / step
+  double* d;             // LINE_DIV: the stored right-hand side
+  const double* x;       // LINE_PRES, LINE_HRES: the iterate
+  unsigned long long *rmax, *bmax;
+};
 
 // A block holds gpb groups of gt threads, each with two length-n buffers (pad entries apart, so that
 // a quarter warp's column loads touch distinct banks), behind the plan's twiddles.
@@ -394,7 +475,8 @@ __device__ __forceinline__ cplx<T>* tg_stage(const FftPlan& plan, const cplx<T>*
 // two components (LINE_UV).
 template <typename T, int LINE>
 __global__ void k_tg_rows_fwd(int n, FftPlan plan, const cplx<T>* __restrict__ tw_g, const double* __restrict__ in,
-                              cplx<T>* __restrict__ S, int pitch, double s, int gt, int gpb) {
+                              cplx<T>* __restrict__ S, int pitch, double s, int gt, int gpb, TgRow rw, TgGate gate) {
+  if (!tg_open(gate)) return;
   extern __shared__ __align__(16) unsigned char smem_raw[];
   cplx<T>* base = tg_stage<T>(plan, tw_g, smem_raw);
   const int grp = threadIdx.x / gt, tid = threadIdx.x - grp * gt, nn = n * n;
@@ -409,6 +491,26 @@ __global__ void k_tg_rows_fwd(int n, FftPlan plan, const cplx<T>* __restrict__ t
   } else if (LINE == LINE_UV) {
     const double* src = in + (size_t)row * n;
     for (int e = tid; e < n; e += gt) a[e] = {(T)src[e], (T)src[nn + e]};
+  } else if (LINE == LINE_DIV) {
+    for (int e = tid; e < n; e += gt) {
+      const int k = row * n + e;
+      const double d = div_by(div_sum(in, n, row, e, k), rw.c.h, rw.c.ih) * rw.s;
+      rw.d[k] = d;
+      a[e] = {(T)d, (T)0};
+    }
+  } else if (LINE == LINE_PRES || LINE == LINE_HRES) {
+    const double* src = in + (size_t)blockIdx.y * nn;
+    const double* x = rw.x + (size_t)blockIdx.y * nn;
+    unsigned long long rm = 0, bm = 0;
+    for (int e = tid; e < n; e += gt) {
+      const int k = row * n + e;
+      const double bv = src[k], r = bv - (LINE == LINE_PRES ? pres_p(rw.c, x, n, row, e, k) : helm_p<false>(rw.c, x, n, row, e, k, x[k]));
+      a[e] = {(T)r, (T)0};
+      rm = max(rm, absbits_(r));
+      bm = max(bm, absbits_(bv));
+    }
+    commit_max(rm, rw.rmax);
+    if (LINE == LINE_HRES && rw.bmax) commit_max(bm, rw.bmax);
   } else {
     const bool two = row + 1 < n;
     for (int e = tid; e < n; e += gt) {
@@ -438,7 +540,8 @@ __global__ void k_tg_rows_fwd(int n, FftPlan plan, const cplx<T>* __restrict__ t
 template <typename T>
 __global__ void k_tg_cols(int n, FftPlan plan, const cplx<T>* __restrict__ tw_g, cplx<T>* __restrict__ S, int pitch,
                           int ncols, const double* __restrict__ f, const T* __restrict__ s2, int kind, T hh2, T coef,
-                          int gt, int gpb) {
+                          int gt, int gpb, TgGate gate) {
+  if (!tg_open(gate)) return;
   extern __shared__ __align__(16) unsigned char smem_raw[];
   cplx<T>* base = tg_stage<T>(plan, tw_g, smem_raw);
   const int stride = 2 * n + tg_pad<T>(gpb), c0 = blockIdx.x * gpb;
@@ -483,7 +586,8 @@ __global__ void k_tg_cols(int n, FftPlan plan, const cplx<T>* __restrict__ tw_g,
 // Rows inverse: the real parts (LINE_PAIR: two rows, LINE_UV: both components) times scale, FP64.
 template <typename T, int LINE>
 __global__ void k_tg_rows_inv(int n, FftPlan plan, const cplx<T>* __restrict__ tw_g, const cplx<T>* __restrict__ S,
-                              int pitch, double* __restrict__ out, T scale, int accumulate, int gt, int gpb) {
+                              int pitch, double* __restrict__ out, T scale, int accumulate, int gt, int gpb, TgGate gate) {
+  if (!tg_open(gate)) return;
   extern __shared__ __align__(16) unsigned char smem_raw[];
   cplx<T>* base = tg_stage<T>(plan, tw_g, smem_raw);
   const int grp = threadIdx.x / gt, tid = threadIdx.x - grp * gt, nn = n * n;
@@ -521,6 +625,7 @@ __global__ void k_tg_rows_inv(int n, FftPlan plan, const cplx<T>* __restrict__ t
 
 // FP64 symbol tables (n x (n / 2 + 1)): the factor of each mode
 __global__ void k_tg_symbol(int n, const double* __restrict__ s2, int kind, double hh2, double coef, double* __restrict__ f) {
+  tg_wait();
   const int nh = n / 2 + 1;
   for (int t = blockIdx.x * blockDim.x + threadIdx.x; t < n * nh; t += gridDim.x * blockDim.x) {
     const int l = t / nh, k = t - l * nh;
@@ -541,13 +646,17 @@ struct gm_tg {
   FftPlan plan{};
   int gt = 32, gpb[2] = {1, 1};  // threads per transform, transforms per block (FP32, FP64)
   size_t smem[2] = {0, 0};
-  Buf<double> q, qn, hist, now, rhs, star, mid, half_q, action, proj, phalf, phalf_n, pout, phi, inc, div, work;
+  Buf<double> q, qn, hist, now, rhs, star, mid, half_q, action, proj, phalf, phalf_n, pout, phi, inc, div;
   Buf<double> tw64, s2_64, sym_p, sym_h;  // FP64 symbol tables of the pressure and the CN operator (for sym_dt)
   Buf<float> tw32, s2_32;
   double sym_dt = 0;
   Buf<unsigned char> spec;            // the spectrum: n x n complex FP64, or two of FP32
   Buf<unsigned long long> red;        // RED_*
-  unsigned long long* host_red = nullptr;  // its page-locked copy (a pageable one costs the FP32 refinement's read-backs a staging copy each)
+  unsigned long long* host_red = nullptr;  // its page-locked copy
+  // FP32 mode: refinement sweeps queued for each solve.  A read-back per check held the stream for some
+  // 20 us, six to eight times a step; now the steps of a call queue behind each other, a step that needs
+  // one sweep more than is held leaves its state alone, and the host repeats it with the sweep.
+  int held[NSLOT] = {1, 1, 1, 1};
   ~gm_tg() { if (host_red) cudaFreeHost(host_red); }
   bool has_history = false;
   double prev_dt = 0;
@@ -555,30 +664,56 @@ struct gm_tg {
 
 namespace {
 
-// One solve: kind 0 Poisson, 1 Helmholtz (coef = dt nu / 2).
-//   FP32: x (+)= S^-1 b for `fields` cell grids of n n values.
+template <typename... K, typename... A>
+void tg_launch(void (*kernel)(K...), dim3 grid, dim3 block, size_t smem, cudaStream_t st, A... args) {
+  cudaLaunchConfig_t cfg{};
+  cfg.gridDim = grid;
+  cfg.blockDim = block;
+  cfg.dynamicSmemBytes = smem;
+  cfg.stream = st;
+  cudaLaunchAttribute at[1];
+  at[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+  at[0].val.programmaticStreamSerializationAllowed = gmk::pdl_mode_ext();
+  cfg.attrs = at;
+  cfg.numAttrs = 1;
+  gmk::kernel_launch_adjust(1);
+  cudaLaunchKernelEx(&cfg, kernel, args...);
+}
+
+unsigned blocks_of(int64_t n) { return (unsigned)((n + PT - 1) / PT); }
+TgC stencil_consts(const gm_tg* t, double dt) {
+  const double hh = t->h * t->h;
+  return TgC{t->h, t->nu, 0.5 * dt, hh, 1.0 / hh, 1.0 / t->h, 0.5 * dt * t->nu / hh};
+}
+// refinement sweeps at most: CN 6 (then a last check), pressure 8 (none behind the last)
+int most_of(int slot) { return slot == SLOT_CN ? 6 : 8; }
+TgHeld held_of(const gm_tg* t, int slot, double step) {
+  return t->precision ? TgHeld{slot, t->held[slot], most_of(slot), step} : TgHeld{-1, 0, 0, 0.0};
+}
+
+// One application of a solve: kind 0 Poisson, 1 Helmholtz (coef = dt nu / 2), the forward rows as LINE:
+//   FP32: x (+)= S^-1 of `fields` cell grids of n n values.
 //   FP64: kind 0 takes the velocity b and solves for s div(b); kind 1 takes both components.
-template <typename T>
-void fourier_solve(gm_tg* t, int kind, double coef, const double* b, double* x, bool accumulate, int fields, double s) {
+// first gates the forward rows, rest the other two kernels.
+template <typename T, int LINE>
+void fourier_solve(gm_tg* t, int kind, double coef, const double* b, double* x, bool accumulate, int fields, double s,
+                   const TgRow& rw, const TgGate& first, const TgGate& rest) {
   constexpr bool D = sizeof(T) == 8;
-  const int n = t->n, gt = t->gt, gpb = t->gpb[D], thr = gt * gpb;
+  constexpr int INV = D ? LINE : LINE_REAL;
+  const int n = t->n, gt = t->gt, gpb = t->gpb[D];
+  const dim3 thr((unsigned)(gt * gpb));
   const size_t sm = t->smem[D];
   cudaStream_t st = t->st;
   const cplx<T>* tw = D ? (const cplx<T>*)t->tw64.p : (const cplx<T>*)t->tw32.p;
   const T* s2 = D ? (const T*)t->s2_64.p : (const T*)t->s2_32.p;
   cplx<T>* S = reinterpret_cast<cplx<T>*>(t->spec.p);
-  const T scale = (T)((D && kind == 0 ? 0.5 : 1.0) / ((double)n * n));
-  const int pair = D && kind == 0, ncols = pair ? n / 2 + 1 : n, lines = pair ? (n + 1) / 2 : n;
+  const T scale = (T)((LINE == LINE_PAIR ? 0.5 : 1.0) / ((double)n * n));
+  const int ncols = LINE == LINE_PAIR ? n / 2 + 1 : n, lines = LINE == LINE_PAIR ? (n + 1) / 2 : n;
   const dim3 gr((unsigned)((lines + gpb - 1) / gpb), (unsigned)fields), gc((unsigned)((ncols + gpb - 1) / gpb), (unsigned)fields);
   const double* f = kind == 0 ? t->sym_p.p : t->sym_h.p;
-  gmk::kernel_launch_adjust(3);
-  if constexpr (!D) k_tg_rows_fwd<T, LINE_REAL><<<gr, thr, sm, st>>>(n, t->plan, tw, b, S, n, 0.0, gt, gpb);
-  else if (pair) k_tg_rows_fwd<T, LINE_PAIR><<<gr, thr, sm, st>>>(n, t->plan, tw, b, S, ncols, s, gt, gpb);
-  else k_tg_rows_fwd<T, LINE_UV><<<gr, thr, sm, st>>>(n, t->plan, tw, b, S, n, 0.0, gt, gpb);
-  k_tg_cols<T><<<gc, thr, sm, st>>>(n, t->plan, tw, S, ncols, ncols, f, s2, kind, (T)(t->h * t->h), (T)coef, gt, gpb);
-  if constexpr (!D) k_tg_rows_inv<T, LINE_REAL><<<gr, thr, sm, st>>>(n, t->plan, tw, S, n, x, scale, accumulate ? 1 : 0, gt, gpb);
-  else if (pair) k_tg_rows_inv<T, LINE_PAIR><<<gr, thr, sm, st>>>(n, t->plan, tw, S, ncols, x, scale, 0, gt, gpb);
-  else k_tg_rows_inv<T, LINE_UV><<<gr, thr, sm, st>>>(n, t->plan, tw, S, n, x, scale, 0, gt, gpb);
+  tg_launch(k_tg_rows_fwd<T, LINE>, gr, thr, sm, st, n, t->plan, tw, b, S, ncols, s, gt, gpb, rw, first);
+  tg_launch(k_tg_cols<T>, gc, thr, sm, st, n, t->plan, tw, S, ncols, ncols, f, s2, kind, (T)(t->h * t->h), (T)coef, gt, gpb, rest);
+  tg_launch(k_tg_rows_inv<T, INV>, gr, thr, sm, st, n, t->plan, tw, (const cplx<T>*)S, ncols, x, scale, accumulate ? 1 : 0, gt, gpb, rest);
   TG_CK(cudaGetLastError());
 }
 
@@ -593,110 +728,100 @@ double bitsd(unsigned long long b) {
   return d;
 }
 
-unsigned blocks_of(int64_t n) { return (unsigned)((n + PT - 1) / PT); }
-TgC stencil_consts(const gm_tg* t, double dt) {
-  return TgC{t->h, t->nu, 0.5 * dt, 1.0 / t->h, 0.5 * dt * t->nu / (t->h * t->h)};
+// The FP32 solve of a slot with its held refinement sweeps: the residual that sweep k transforms is check
+// k - 1, so a sweep is three kernels; a last check follows the last sweep.
+template <int FIRST, int RES>
+void refined_solve(gm_tg* t, int slot, double coef, const double* b, const double* rhs, double* x, double dt, double step) {
+  const int fields = slot == SLOT_CN ? 2 : 1, kind = slot == SLOT_CN ? 1 : 0, held = std::min(t->held[slot], most_of(slot));
+  unsigned long long* w = t->red.p + RED_W + slot * SLOT_CHECKS;
+  unsigned long long* bmax = slot == SLOT_CN ? t->red.p + RED_RHS : nullptr;
+  const TgC c = stencil_consts(t, dt);
+  auto gate = [&](int k) { return TgGate{t->red.p, slot, k, step}; };
+  TgRow rw{c, 1.0 / step, t->div.p, x, nullptr, nullptr};
+  fourier_solve<float, FIRST>(t, kind, coef, b, x, false, fields, 0.0, rw, gate(-1), gate(-1));
+  for (int k = 1; k <= held; ++k) {
+    rw.rmax = w + k - 1;
+    rw.bmax = k == 1 ? bmax : nullptr;
+    fourier_solve<float, RES>(t, kind, coef, rhs, x, true, fields, 0.0, rw, gate(k - 2), gate(k - 1));
+  }
+  if (slot != SLOT_CN && held >= most_of(slot)) return;
+  const int64_t nn = (int64_t)t->n * t->n;
+  if (slot == SLOT_CN)
+    tg_launch(k_tg_hres<false>, dim3(grid_for(2 * nn)), dim3(PT), 0, t->st, t->n, c, rhs, (const double*)x, w + held,
+              held == 0 ? bmax : nullptr, gate(held - 1));
+  else
+    tg_launch(k_tg_pres, dim3(grid_for(nn)), dim3(PT), 0, t->st, t->n, c, rhs, (const double*)x, w + held, gate(held - 1));
 }
 
 // project(q, step): phi = A^-1 (div q / step), out = q - step grad phi (refined in FP32 mode
 // until the projected divergence max |step (b - A phi)| is below 1e-11)
-void tg_project(gm_tg* t, const double* q, double step, double* out, double* phi, int gate_step) {
-  const int n = t->n;
-  const int64_t nn = (int64_t)n * n;
-  cudaStream_t st = t->st;
-  if (t->precision == 0) {
-    fourier_solve<double>(t, 0, 0.0, q, phi, false, 1, 1.0 / (t->h * step));
-  } else {
-    gmk::kernel_launch_adjust(1);
-    k_tg_div<<<grid_for(nn), PT, 0, st>>>(n, t->h, 1.0 / step, q, t->div.p);
-    fourier_solve<float>(t, 0, 0.0, t->div.p, phi, false, 1, 0.0);
-    for (int sweep = 0; sweep < 8; ++sweep) {
-      TG_CK(cudaMemsetAsync(t->red.p + RED_PRES, 0, sizeof(unsigned long long), st));
-      gmk::kernel_launch_adjust(1);
-      k_tg_pres<<<grid_for(nn), PT, 0, st>>>(n, t->h, t->div.p, phi, t->work.p, t->red.p + RED_PRES);
-      if (bitsd(read_red(t)[RED_PRES]) * step <= 1e-11) break;
-      fourier_solve<float>(t, 0, 0.0, t->work.p, phi, true, 1, 0.0);
-    }
-  }
+void tg_project(gm_tg* t, const double* q, double step, double* out, double* phi, int slot, int gate_step) {
+  if (t->precision == 0)
+    fourier_solve<double, LINE_PAIR>(t, 0, 0.0, q, phi, false, 1, 1.0 / (t->h * step), TgRow{}, TgGate{}, TgGate{});
+  else
+    refined_solve<LINE_DIV, LINE_PRES>(t, slot, 0.0, q, t->div.p, phi, 0.0, step);
   if (!out) return;
-  gmk::kernel_launch_adjust(1);
-  (t->precision ? k_tg_update<false> : k_tg_update<true>)<<<blocks_of(nn), PT, 0, st>>>(n, stencil_consts(t, 0.0), step,
-                                                                                    step / t->h, q, phi, out, t->red.p, gate_step);
+  tg_launch(t->precision ? k_tg_update<false> : k_tg_update<true>, dim3(blocks_of((int64_t)t->n * t->n)), dim3(PT), 0, t->st, t->n,
+            stencil_consts(t, 0.0), step, step / t->h, q, (const double*)phi, out, t->red.p, gate_step, held_of(t, SLOT_CN, 0.0));
 }
 
-// star = H^-1 rhs (two components), refined in FP32 mode to the CN gate; the residual of star and
-// max |rhs| go to RED_CN, RED_RHS
+// star = H^-1 rhs (two components), refined in FP32 mode to the CN gate
 void tg_helmholtz(gm_tg* t, double dt, const double* rhs, double* star) {
   const int n = t->n;
   const int64_t nn = (int64_t)n * n;
-  cudaStream_t st = t->st;
   const double c = 0.5 * dt * t->nu;
-  auto residual = [&](double* r) {
-    gmk::kernel_launch_adjust(1);
-    (t->precision ? k_tg_hres<false> : k_tg_hres<true>)<<<grid_for(2 * nn), PT, 0, st>>>(n, stencil_consts(t, dt), rhs, star,
-                                                                                       r, t->red.p);
-  };
-  if (t->precision == 0) {
-    if (t->sym_dt != dt) {
-      gmk::kernel_launch_adjust(1);
-      k_tg_symbol<<<grid_for((int64_t)n * (n / 2 + 1)), PT, 0, st>>>(n, t->s2_64.p, 1, t->h * t->h, c, t->sym_h.p);
-      t->sym_dt = dt;
-    }
-    fourier_solve<double>(t, 1, c, rhs, star, false, 1, 0.0);
-    residual(nullptr);
+  if (t->precision) {
+    refined_solve<LINE_REAL, LINE_HRES>(t, SLOT_CN, c, rhs, rhs, star, dt, 1.0);
     return;
   }
-  fourier_solve<float>(t, 1, c, rhs, star, false, 2, 0.0);
-  for (int sweep = 0; sweep < 6; ++sweep) {
-    TG_CK(cudaMemsetAsync(t->red.p, 0, 2 * sizeof(unsigned long long), st));
-    residual(t->work.p);
-    const unsigned long long* v = read_red(t);
-    if (bitsd(v[0]) <= 32 * 2.220446049250313e-16 * std::max(1.0, bitsd(v[1]))) return;  // star is the residual's
-    fourier_solve<float>(t, 1, c, t->work.p, star, true, 2, 0.0);
+  if (t->sym_dt != dt) {
+    tg_launch(k_tg_symbol, dim3(grid_for((int64_t)n * (n / 2 + 1))), dim3(PT), 0, t->st, n, (const double*)t->s2_64.p, 1,
+              t->h * t->h, c, t->sym_h.p);
+    t->sym_dt = dt;
   }
-  TG_CK(cudaMemsetAsync(t->red.p, 0, 2 * sizeof(unsigned long long), st));
-  residual(nullptr);
+  fourier_solve<double, LINE_UV>(t, 1, c, rhs, star, false, 1, 0.0, TgRow{}, TgGate{}, TgGate{});
+  tg_launch(k_tg_hres<true>, dim3(grid_for(2 * nn)), dim3(PT), 0, t->st, n, stencil_consts(t, dt), rhs, (const double*)star,
+            t->red.p + RED_CN, t->red.p + RED_RHS, TgGate{});
 }
 
 // ab2_cn_step (solver/time_integration.py:7-145) with the periodic operators, queued on the
-// stream; `step` counts from 1 in the call.  The FP64 steps behind a failed CN gate leave the
-// state alone (see k_tg_update), the FP32 mode reads its refinement residuals on the host.
+// stream; `step` counts from 1 in the call.  The steps behind a failed gate leave the state alone
+// (see k_tg_update).
 void tg_step(gm_tg* t, double dt, int step) {
   const int n = t->n;
   const int64_t nn = (int64_t)n * n;
   cudaStream_t st = t->st;
   const double h = t->h;
   auto rhs_kernel = [&](int mode, double alpha, const double* qh, double* out) {
-    gmk::kernel_launch_adjust(1);
     if (t->precision == 1) {
-      k_tg_rhs<float><<<blocks_of(2 * nn), PT, 0, st>>>(n, h, t->nu, mode, dt, alpha, t->q.p, qh, t->phalf.p, t->hist.p,
-                                                        t->now.p, out);
+      tg_launch(k_tg_rhs<float>, dim3(blocks_of(2 * nn)), dim3(PT), 0, st, n, h, t->nu, mode, dt, alpha, (const double*)t->q.p, qh,
+                (const double*)t->phalf.p, (const double*)t->hist.p, t->now.p, out, t->red.p, held_of(t, SLOT_START, 0.5 * dt), step);
       return;
     }
     const double e = mode == 1 ? 0.5 * dt : dt;  // the start-up midpoint goes half a step with the full L q
     const TgRhsC c{-0.25 / h, (mode == 1 ? 1.0 : 0.5) * e * t->nu / (h * h), e / h, e * (1 + alpha), e * alpha};
     auto* k = mode == 0 ? k_tg_rhs64<0> : mode == 1 ? k_tg_rhs64<1> : k_tg_rhs64<2>;
-    k<<<blocks_of(nn), PT, 0, st>>>(n, c, t->q.p, qh, t->phalf.p, t->hist.p, t->now.p, out, t->red.p);
+    tg_launch(k, dim3(blocks_of(nn)), dim3(PT), 0, st, n, c, (const double*)t->q.p, qh, (const double*)t->phalf.p,
+              (const double*)t->hist.p, t->now.p, out, t->red.p);
   };
   const bool first = !t->has_history;
   if (first) {
     rhs_kernel(1, 0.0, nullptr, t->mid.p);
-    tg_project(t, t->mid.p, 0.5 * dt, t->half_q.p, t->phi.p, 0);
+    tg_project(t, t->mid.p, 0.5 * dt, t->half_q.p, t->phi.p, SLOT_START, 0);
     rhs_kernel(2, 0.0, t->half_q.p, t->rhs.p);
   } else {
     rhs_kernel(0, dt / (2 * t->prev_dt), nullptr, t->rhs.p);
   }
   tg_helmholtz(t, dt, t->rhs.p, t->star.p);
-  tg_project(t, t->star.p, dt, t->qn.p, t->phi.p, step);
-  gmk::kernel_launch_adjust(1);
-  (t->precision ? k_tg_defect<false> : k_tg_defect<true>)<<<grid_for(nn), PT, 0, st>>>(
-      n, stencil_consts(t, dt), t->qn.p, t->rhs.p, t->action.p, t->proj.p, t->red.p);
-  tg_project(t, t->proj.p, dt, nullptr, t->inc.p, 0);
+  tg_project(t, t->star.p, dt, t->qn.p, t->phi.p, SLOT_P1, step);
+  const bool f32 = t->precision != 0;
+  tg_launch(f32 ? k_tg_defect<false> : k_tg_defect<true>, dim3(grid_for(nn)), dim3(PT), 0, st, n, stencil_consts(t, dt),
+            (const double*)t->qn.p, (const double*)t->rhs.p, t->action.p, t->proj.p, t->red.p, held_of(t, SLOT_P1, dt), step);
+  tg_project(t, t->proj.p, dt, nullptr, t->inc.p, SLOT_P2, 0);
   const double factor = first ? 1.0 : dt / (dt + t->prev_dt);
-  gmk::kernel_launch_adjust(1);
-  (t->precision ? k_tg_pout<false> : k_tg_pout<true>)<<<grid_for(nn), PT, 0, st>>>(
-      n, stencil_consts(t, dt), dt, dt / h, factor, t->phalf.p, t->inc.p, t->action.p, t->rhs.p, t->phalf_n.p, t->pout.p,
-      t->red.p);
+  tg_launch(f32 ? k_tg_pout<false> : k_tg_pout<true>, dim3(grid_for(nn)), dim3(PT), 0, st, n, stencil_consts(t, dt), dt, dt / h,
+            factor, (const double*)t->phalf.p, (const double*)t->inc.p, (const double*)t->action.p, (const double*)t->rhs.p,
+            t->phalf_n.p, t->pout.p, t->red.p, held_of(t, SLOT_P2, dt), step);
   TG_CK(cudaGetLastError());
 }
 
@@ -711,21 +836,24 @@ void tg_swap(gm_tg* t) {
 void tg_steps(gm_tg* t, double dt, int n_steps, double* max_div) {
   const bool had = t->has_history;
   const double prev = t->prev_dt;
-  TG_CK(cudaMemsetAsync(t->red.p, 0, 8 * sizeof(unsigned long long), t->st));
+  TG_CK(cudaMemsetAsync(t->red.p, 0, RED_N * sizeof(unsigned long long), t->st));
   const unsigned long long* r = t->host_red;
-  int done = 0, err = 0;
-  for (; done < n_steps && !err; ++done) {
+  for (int done = 0; done < n_steps;) {
     tg_step(t, dt, done + 1);
     tg_swap(t);
     t->has_history = true;
     t->prev_dt = dt;
-    if (t->precision == 1 || done + 1 == n_steps || (done + 1) % 64 == 0)
-      err = (int)read_red(t)[RED_ERR];
-  }
-  if (err) {
+    ++done;
+    if (done != n_steps && done % 64 != 0) continue;
+    const int err = (int)read_red(t)[RED_ERR];
+    if (!err) continue;
     if ((done - (err - 1)) % 2) tg_swap(t);  // step err failed: the state is that after err - 1 steps
     if (err == 1) { t->has_history = had; t->prev_dt = prev; }
-    throw TgError(GM_ERUNTIME, "CN momentum solve failed: residual=" + std::to_string(bitsd(r[RED_CN])));
+    const int slot = (int)r[RED_SHORT] - 1;
+    if (slot < 0) throw TgError(GM_ERUNTIME, "CN momentum solve failed: residual=" + std::to_string(bitsd(r[RED_CN])));
+    ++t->held[slot];
+    done = err - 1;
+    TG_CK(cudaMemsetAsync(t->red.p + RED_SHORT, 0, 2 * sizeof(unsigned long long), t->st));
   }
   *max_div = std::max(*max_div, bitsd(r[RED_DIV]));
 }
@@ -780,7 +908,9 @@ int gm_tg_create(int32_t n, double nu, int32_t precision, gm_tg** out) {
     int dyn = optin;
     // the limit is a process-wide attribute of the kernel shared by every handle: the device
     // maximum, so that a smaller handle created later cannot lower it below a larger one's need
-    for (auto f : {(const void*)k_tg_rows_fwd<float, LINE_REAL>, (const void*)k_tg_rows_fwd<double, LINE_PAIR>,
+    for (auto f : {(const void*)k_tg_rows_fwd<float, LINE_REAL>, (const void*)k_tg_rows_fwd<float, LINE_DIV>,
+                   (const void*)k_tg_rows_fwd<float, LINE_PRES>, (const void*)k_tg_rows_fwd<float, LINE_HRES>,
+                   (const void*)k_tg_rows_fwd<double, LINE_PAIR>,
                    (const void*)k_tg_rows_fwd<double, LINE_UV>, (const void*)k_tg_rows_inv<float, LINE_REAL>,
                    (const void*)k_tg_rows_inv<double, LINE_PAIR>, (const void*)k_tg_rows_inv<double, LINE_UV>,
                    (const void*)k_tg_cols<float>, (const void*)k_tg_cols<double>}) {
@@ -802,7 +932,7 @@ int gm_tg_create(int32_t n, double nu, int32_t precision, gm_tg** out) {
     }
     const int64_t nn = (int64_t)n * n;
     for (Buf<double>* b : {&t->q, &t->qn, &t->hist, &t->now, &t->rhs, &t->star, &t->mid, &t->half_q, &t->action,
-                           &t->proj, &t->work}) {
+                           &t->proj}) {
       b->alloc(2 * nn);
       TG_CK(cudaMemset(b->p, 0, 2 * nn * sizeof(double)));
     }
@@ -818,9 +948,9 @@ int gm_tg_create(int32_t n, double nu, int32_t precision, gm_tg** out) {
       gmk::kernel_launch_adjust(1);
       TG_CK(cudaGetLastError());
     }
-    t->red.alloc(8);
+    t->red.alloc(RED_N);
     TG_CK(cudaMallocHost(&t->host_red, 8 * sizeof(unsigned long long)));
-    TG_CK(cudaMemset(t->red.p, 0, 8 * sizeof(unsigned long long)));
+    TG_CK(cudaMemset(t->red.p, 0, RED_N * sizeof(unsigned long long)));
   });
   if (rc != GM_OK) { g_tg_create_error = t->err; return rc; }
   *out = t.release();
