@@ -439,7 +439,7 @@ __global__ void k_tg_pout(int n, TgC c, double dt, double kg, double factor, con
 // these a pressure solve takes half and a CN solve half of the one-row form's work.  At 1024^2
 // (8 8 8 2) the column pass takes 150 us for u + i v and 77 for a pressure (0.80 and 0.77 of the pipe's
 // rate), row passes 82-87 and 47-54; a solve of seven kernels with transposes took 366 us a field,
-// now 186 a pressure and 319 both components
+// 186 a pressure and 319 both components with four transforms a block (3 % less with one, see gm_tg_create)
 // and, forward in the FP32 mode (one real row each):
 //   LINE_DIV   div(q) / step, stored on the way (the right-hand side of a pressure)
 //   LINE_PRES  the residual b - A x of a pressure, its maximum on the way: a check of the refinement and
@@ -644,7 +644,7 @@ struct gm_tg {
   std::string err;
   cudaStream_t st = nullptr;
   FftPlan plan{};
-  int gt = 32, gpb[2] = {1, 1};  // threads per transform, transforms per block (FP32, FP64)
+  int gt[2] = {32, 32}, gpb[2] = {1, 1};  // threads per transform, transforms per block (FP32, FP64)
   size_t smem[2] = {0, 0};
   Buf<double> q, qn, hist, now, rhs, star, mid, half_q, action, proj, phalf, phalf_n, pout, phi, inc, div;
   Buf<double> tw64, s2_64, sym_p, sym_h;  // FP64 symbol tables of the pressure and the CN operator (for sym_dt)
@@ -700,7 +700,7 @@ void fourier_solve(gm_tg* t, int kind, double coef, const double* b, double* x, 
                    const TgRow& rw, const TgGate& first, const TgGate& rest) {
   constexpr bool D = sizeof(T) == 8;
   constexpr int INV = D ? LINE : LINE_REAL;
-  const int n = t->n, gt = t->gt, gpb = t->gpb[D];
+  const int n = t->n, gt = t->gt[D], gpb = t->gpb[D];
   const dim3 thr((unsigned)(gt * gpb));
   const size_t sm = t->smem[D];
   cudaStream_t st = t->st;
@@ -921,13 +921,23 @@ int gm_tg_create(int32_t n, double nu, int32_t precision, gm_tg** out) {
       TG_CK(cudaFuncSetAttribute(f, cudaFuncAttributeMaxDynamicSharedMemorySize, d));
     }
     if (tg_smem<double>(n, t->plan.tw_len, 1) > (size_t)dyn) throw TgError(GM_EVALUE, "grid too large for the row transforms");
-    // a thread per radix-8 butterfly of a transform, and up to four transforms a block (64-byte
-    // column pieces in FP64) while a block stays within 512 threads and half of the shared memory
-    t->gt = std::min(512, std::max(32, ((n / 8 + 31) / 32) * 32));
+    // Threads of a transform and transforms of a block, by sweeps of both over n = 128..4096 (us a step).
+    // FP64: one transform a block (smaller blocks spread evenly over the SMs; column accesses of 16 bytes
+    // cost less than that gains: n = 512 328 -> 257, 700 1074 -> 796, 1024 884 -> 853, 2048 3550 -> 3272
+    // against four or two) with a thread per radix-4 butterfly, 128 to 256 but no more than n / 2
+    // (n = 250: 32 threads 232, 64 147, 128 135; 2048: 256 3272, 512 3452).
+    // FP32: powers of two from 512 a thread per radix-8 butterfly and four transforms (512: 417 against
+    // 430 with 128 x 2); else some 128 threads, as one warp a transform leaves the chip idle (250:
+    // 32 x 4 248, 128 x 2 191) or a thread per radix-5 butterfly (700: 96 x 4 1062, 192 x 2 946), two a block.
+    auto r32 = [](int v) { return std::max(32, (v + 31) / 32 * 32); };
+    const bool octal = n >= 512 && (n & (n - 1)) == 0;
+    t->gt[1] = std::max(r32(n / 8), std::min(r32(n / 2), std::max(128, std::min(256, r32(n / 4)))));
+    t->gt[0] = octal ? r32(n / 8) : std::min(r32(n / 2), std::max(128, r32(n / 5)));
     for (int d = 0; d < 2; ++d) {
+      t->gt[d] = std::min(512, t->gt[d]);
       auto need = [&](int g) { return d ? tg_smem<double>(n, t->plan.tw_len, g) : tg_smem<float>(n, t->plan.tw_len, g); };
-      for (int g : {2, 4})
-        if (t->gt * g <= 512 && need(g) <= (size_t)dyn) t->gpb[d] = g;
+      for (int g = 2; d == 0 && g <= (octal ? 4 : 2); g *= 2)
+        if (t->gt[d] * g <= 512 && need(g) <= (size_t)dyn) t->gpb[d] = g;
       t->smem[d] = need(t->gpb[d]);
     }
     const int64_t nn = (int64_t)n * n;
@@ -975,7 +985,7 @@ int gm_tg_set_state(gm_tg* t, const double* q, const double* p) {
     const int64_t nn = (int64_t)t->n * t->n;
     TG_CK(cudaMemcpyAsync(t->q.p, q, 2 * nn * sizeof(double), cudaMemcpyDefault, t->st));
     TG_CK(cudaMemcpyAsync(t->phalf.p, p, nn * sizeof(double), cudaMemcpyDefault, t->st));
-    TG_CK(cudaMemcpyAsync(t->pout.p, p, nn * sizeof(double), cudaMemcpyDefault, t->st));
+    TG_CK(cudaMemcpyAsync(t->pout.p, t->phalf.p, nn * sizeof(double), cudaMemcpyDeviceToDevice, t->st));
     TG_CK(cudaStreamSynchronize(t->st));
     t->has_history = false;
     t->prev_dt = 0;
