@@ -1512,19 +1512,19 @@ gm_cc::Graph& step_graph(gm_cc* c, double dt) {
   gr.per_cycle = 0;
   cudaStream_t st = c->st;
   const long long c0 = kernel_launch_count();
-  gmi::set_capturing(c->P, true);
+  gmi::hold_sweeps(c->P, true);
   cudaGraph_t g = nullptr;
   CCK(cudaStreamBeginCapture(st, cudaStreamCaptureModeThreadLocal));
   try {
     step_body(c, dt, gr, st);
   } catch (...) {
-    gmi::set_capturing(c->P, false);
+    gmi::hold_sweeps(c->P, false);
     cudaStreamEndCapture(st, &g);
     if (g) cudaGraphDestroy(g);
     cudaGetLastError();
     throw;
   }
-  gmi::set_capturing(c->P, false);
+  gmi::hold_sweeps(c->P, false);
   CCK(cudaStreamEndCapture(st, &g));
   const long long captured = kernel_launch_count() - c0;
   kernel_launch_adjust(-captured);
@@ -2493,7 +2493,7 @@ struct gm_poisson {
   Buf<double> b, x;
   Buf<double> ikappa;
   Buf<int32_t> cell_type;
-  // the legacy loop's device scratch and per-step records (four forces and the residual bits)
+  // the legacy loop's device scratch and per-step records (see gml::forces)
   Buf<double> lscratch, lrec;
   cudaEvent_t ev_in = nullptr, ev_out = nullptr;
 };
@@ -2580,44 +2580,50 @@ int gm_poisson_legacy_step(gm_poisson* p, gm_legacy_state* s, double dt, int32_t
     CCK(cudaStreamWaitEvent(st, p->ev_in, 0));
     const size_t need = gml::scratch_doubles(*s);
     if (p->lscratch.n < need) p->lscratch.alloc(need);
-    if (p->lrec.n < (size_t)n_steps * 5) p->lrec.alloc((size_t)n_steps * 5);
-    CcGeo g{};
-    g.psize = p->psize;
-    g.cell_type = p->cell_type.p;
-    g.ikappa = p->ikappa.p;
-    std::vector<double> rec((size_t)n_steps * 5);
-    for (int32_t k = 0; k < n_steps; ++k) {
-      double* r = p->lrec.p + (size_t)k * 5;
-      gml::predict(*s, dt, p->lscratch.p, st);
-      if (s->centered) {  // the loop keeps the AB2 history before its pressure solve (solver/main.py:320)
-        s->has_prev = 1;
-        s->prev_dt = dt;
+    constexpr int NR = 6;  // a step's record (gml::forces)
+    if (p->lrec.n < (size_t)n_steps * NR) p->lrec.alloc((size_t)n_steps * NR);
+    StepCtl* ctl = gmi::control(p->P);
+    CCK(cudaMemsetAsync(ctl, 0, sizeof(StepCtl), st));
+    CCK(cudaMemsetAsync(p->lrec.p, 0, (size_t)n_steps * NR * sizeof(double), st));
+    std::vector<double> rec((size_t)n_steps * NR);
+    // All steps queue behind each other: a failed pressure gate stops the kernels behind it, and a solve
+    // that needs more refinement sweeps than are held (FP64 starts with none) goes on from there with one
+    // more.  With a read-back a step and two idle sweeps a solve a step took 229 us at 350x213, now 154.
+    bool predicted = false;
+    for (int32_t k = 0; k < n_steps;) {
+      for (; k < n_steps; ++k) {
+        if (!predicted) {
+          gml::predict(*s, dt, p->lscratch.p, p->cell_type.p, p->ikappa.p, &ctl->err, st);
+          if (s->centered) {  // the loop keeps the AB2 history before its pressure solve (solver/main.py:320)
+            s->has_prev = 1;
+            s->prev_dt = dt;
+          }
+          CCK(cudaMemsetAsync(ctl->solve, 0, sizeof ctl->solve, st));
+        }
+        predicted = false;
+        gmi::hold_sweeps(p->P, true);
+        gmi::pressure_solve(p->P, s->rhs, s->phi, S_P1);
+        gmi::hold_sweeps(p->P, false);
+        gml::correct(*s, dt, p->lscratch.p, &ctl->err, st);
+        gml::forces(*s, p->lscratch.p, p->lrec.p + (size_t)k * NR, ctl, S_P1, gmi::checks(p->P), st);
       }
-      counted();
-      k_cc_scale_rhs<<<nblk(p->psize), CC_TPB, 0, st>>>(g, s->rhs);
-      CCK(cudaMemsetAsync(gmi::control(p->P), 0, sizeof(StepCtl), st));
-      CCK(cudaMemsetAsync(r + 4, 0, sizeof(double), st));
-      gmi::pressure_solve(p->P, s->rhs, s->phi, S_P1);
-      counted();
-      k_cc_maxdiff<<<std::min<unsigned>(nblk(p->psize), 1216), CC_TPB, 0, st>>>(
-          p->psize, gmi::pressure_residual(p->P), nullptr, nullptr, 0.0, reinterpret_cast<unsigned long long*>(r + 4));
+      CCK(cudaMemcpyAsync(rec.data(), p->lrec.p, rec.size() * sizeof(double), cudaMemcpyDeviceToHost, st));
+      CCK(cudaGetLastError());
       std::string m;
       const int rc = gmi::check(p->P, "pressure solve", m);  // synchronises the stream
-      if (rc != GM_OK) throw CcFail(rc, m);
-      gml::correct(*s, dt, p->lscratch.p, st);
-      gml::forces(*s, p->lscratch.p, r, st);
+      if (rc == GM_OK) break;
+      if (rc != ERR_SWEEPS) throw CcFail(rc, m);
+      gmi::add_sweep(p->P, gmi::failed_gate(p->P));
+      for (k = 0; k < n_steps && rec[(size_t)k * NR + 5] != 0.0; ++k) {}
+      CCK(cudaMemsetAsync(ctl, 0, sizeof(StepCtl), st));
+      predicted = true;
     }
-    CCK(cudaMemcpyAsync(rec.data(), p->lrec.p, rec.size() * sizeof(double), cudaMemcpyDeviceToHost, st));
-    CCK(cudaGetLastError());
-    CCK(cudaStreamSynchronize(st));
     CCK(cudaEventRecord(p->ev_out, st));
     CCK(cudaStreamWaitEvent(cs, p->ev_out, 0));
     if (diag)
       for (int32_t k = 0; k < n_steps; ++k) {
-        for (int q = 0; q < 4; ++q) diag[k].forces[q] = rec[(size_t)k * 5 + q];
-        unsigned long long bits;
-        std::memcpy(&bits, &rec[(size_t)k * 5 + 4], sizeof bits);
-        diag[k].pressure_residual_linf = bits_to_double(bits);
+        for (int q = 0; q < 4; ++q) diag[k].forces[q] = rec[(size_t)k * NR + q];
+        diag[k].pressure_residual_linf = rec[(size_t)k * NR + 4];
       }
   } catch (const CcFail& e) {
     p->err = e.msg;

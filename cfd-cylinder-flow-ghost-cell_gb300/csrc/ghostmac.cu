@@ -3725,7 +3725,8 @@ void pressure_destroy(gm_handle* h) { gm_destroy(h); }
 const gm::Geometry& geometry(const gm_handle* h) { return h->g; }
 cudaStream_t stream(gm_handle* h) { return h->st; }
 cudaStream_t body_stream(gm_handle* h, int level) { return level == 0 ? h->st_body : h->st2_body; }
-void set_capturing(gm_handle* h, bool on) { h->capturing = on; }
+void hold_sweeps(gm_handle* h, bool on) { h->capturing = on; }
+int checks(const gm_handle* h) { return h->nchk; }
 
 void pressure_solve(gm_handle* h, const double* b, double* x, int slot) {
   schur_solve(h, 0, h->rp, 0, 0.0, b, x, h->pres.p, h->pfirst.p, h->pw2.p, slot);

@@ -28,9 +28,10 @@ const gm::Geometry& geometry(const gm_handle* h);
 cudaStream_t stream(gm_handle* h);
 // streams that capture the bodies of conditional graph nodes
 cudaStream_t body_stream(gm_handle* h, int level);
-// while set, pressure_solve records as many gated refinement sweeps as its slot holds (a solve that needs
-// more raises gmk::ERR_SWEEPS with the slot as the gate word)
-void set_capturing(gm_handle* h, bool on);
+// while set, pressure_solve queues (or records) as many gated refinement sweeps as its slot holds; a solve
+// that needs more raises gmk::ERR_SWEEPS with the slot as the gate word
+void hold_sweeps(gm_handle* h, bool on);
+int checks(const gm_handle* h);            // residual checks of a solve at most
 // Monitored solve of A x = b (full pressure grids on the device, inactive cells ignored in b
 // and zero in x) in control slot `slot` (gmk::S_P0..S_P2), then its pressure gate.
 void pressure_solve(gm_handle* h, const double* b, double* x, int slot);
@@ -60,12 +61,16 @@ SurfaceCsr surface(const gm_handle* h);
 namespace gml {
 // doubles of device scratch the calls below need
 size_t scratch_doubles(const gm_legacy_state& s);
+// Every call returns once *err is set (device memory; null: never).
 // u*, v* (predictor_rhs_cpp), ghost velocities, the AB2 step (centred), ghost velocities, and
-// the Poisson right-hand side into s.rhs
-void predict(const gm_legacy_state& s, double dt, double* scratch, cudaStream_t st);
+// the Poisson right-hand side into s.rhs, in the row scaling of the pressure system
+void predict(const gm_legacy_state& s, double dt, double* scratch, const int32_t* cell_type, const double* ikappa,
+             const int* err, cudaStream_t st);
 // the corrector (with the ghost-cell branch's ghost velocities and boundary faces), then
 // p = phi (centred) or p += phi
-void correct(const gm_legacy_state& s, double dt, double* scratch, cudaStream_t st);
-// the step's forces (fx_p, fy_p, fx_v, fy_v) into out[0..3] (device)
-void forces(const gm_legacy_state& s, double* scratch, double* out, cudaStream_t st);
+void correct(const gm_legacy_state& s, double dt, double* scratch, const int* err, cudaStream_t st);
+// the step's record: forces (fx_p, fy_p, fx_v, fy_v), the bits of max |residual| of the solve in `slot`, and
+// 1, into out[0..5] (device)
+void forces(const gm_legacy_state& s, double* scratch, double* out, const gmk::StepCtl* ctl, int slot, int nchk,
+            cudaStream_t st);
 }  // namespace gml

@@ -25,6 +25,7 @@
 #include <vector>
 
 #include "../../include/ghostmac.h"
+#include "exactdiv.cuh"
 #include "internal.hpp"
 
 namespace gmk {
@@ -33,8 +34,30 @@ void kernel_launch_adjust(long long delta);  // the library's launch counter (ke
 void gm_internal_set_error(const char* msg);  // defined in ghostmac.cu
 
 namespace {
+using gmk::div_by;
 
 constexpr int LT = 256;
+
+// Steps of the legacy loop queue behind each other without a host check between them: every kernel that
+// writes the state returns once the control block's sticky error word is set (null: no control block).
+__device__ __forceinline__ bool stopped(const int* err) { return err && *(const volatile int*)err != 0; }
+// (row, column), in 32 bits where the index allows it
+struct RowCol { int j, i; };
+__device__ __forceinline__ RowCol row_col(long long t, int n) {
+  if (t >> 32) return {(int)(t / n), (int)(t % n)};
+  const unsigned q = (unsigned)t / (unsigned)n;
+  return {(int)q, (int)((unsigned)t - q * (unsigned)n)};
+}
+// spacings and their reciprocals: the predictor's six divides a face, all by constants, were two thirds
+// of its FP64 instructions (17 us a component at 350x213)
+struct Spacing {
+  double dx, dy, dx2, dy2, rho, idx, idy, idx2, idy2, irho;
+};
+Spacing spacing_of(double dx, double dy, double rho) {
+  using gmk::reciprocal_of;
+  return {dx, dy, dx * dx, dy * dy, rho, reciprocal_of(dx), reciprocal_of(dy), reciprocal_of(dx * dx), reciprocal_of(dy * dy),
+          reciprocal_of(rho)};
+}
 
 #define P_(j, i) p[(size_t)(j) * nx + (i)]
 #define M_(j, i) mask[(size_t)(j) * nx + (i)]
@@ -44,89 +67,125 @@ constexpr int LT = 256;
 #define VS_(j, i) vs[(size_t)(j) * nx + (i)]
 #define PHI_(j, i) phi[(size_t)(j) * nx + (i)]
 
+// (a - 2 b + c) / h^2; 2 b is exact, so the fused form rounds as the two operations do.  (So do the factors
+// 1/2 and 1/4 of the transport terms, which are taken out of the products and quotients.)
+__device__ __forceinline__ double second_difference(double a, double b, double c, double hh, double ihh) {
+  return div_by(__fma_rn(-2.0, b, a) + c, hh, ihh);
+}
+struct PredictArgs {
+  const double *u, *v, *p, *inlet;  // p null: zero
+  const uint8_t* mask;
+  int nx, ny;
+  Spacing h;
+  double dt, nu;
+  int slip, centered;
+};
 // u* on every vertical face (bindings.cpp:98-139): interior faces by the predictor, the inlet
 // column from the inlet profile, the outlet column from the previous u
-__global__ void k_predict_u(const double* __restrict__ u, const double* __restrict__ v, double* __restrict__ us,
-                            const double* __restrict__ p, const uint8_t* __restrict__ mask,
-                            const double* __restrict__ inlet, int nx, int ny, double dx, double dy, double dx2,
-                            double dy2, double dt, double nu, double rho, int slip, int centered) {
-  const long long t = (long long)blockIdx.x * blockDim.x + threadIdx.x;
-  if (t >= (long long)ny * (nx + 1)) return;
-  const int j = (int)(t / (nx + 1)), i = (int)(t - (long long)j * (nx + 1));
-  if (i == 0) { US_(j, 0) = inlet[j]; return; }
-  if (i == nx) { US_(j, nx) = U_(j, nx - 1); return; }
-  if (M_(j, i - 1) || M_(j, i)) { US_(j, i) = 0.0; return; }
+__device__ __forceinline__ double predict_u(const PredictArgs& a, int j, int i) {
+  const double *u = a.u, *v = a.v, *p = a.p;
+  const uint8_t* mask = a.mask;
+  const int nx = a.nx, ny = a.ny, slip = a.slip;
+  const Spacing& h = a.h;
+  if (i == 0) return a.inlet[j];
+  if (i == nx) return U_(j, nx - 1);
+  if (M_(j, i - 1) || M_(j, i)) return 0.0;
   const double uc = U_(j, i);
-  const double vavg = 0.25 * (V_(j, i - 1) + V_(j, i) + V_(j + 1, i - 1) + V_(j + 1, i));
   double ub, ut;
   if (j == 0) ub = slip ? uc : -uc;
   else ub = (M_(j - 1, i - 1) && M_(j - 1, i)) ? -uc : U_(j - 1, i);
   if (j == ny - 1) ut = slip ? uc : -uc;
   else ut = (M_(j + 1, i - 1) && M_(j + 1, i)) ? -uc : U_(j + 1, i);
-  const double lap = (U_(j, i + 1) - 2.0 * uc + U_(j, i - 1)) / dx2 + (ut - 2.0 * uc + ub) / dy2;
-  const double dpdx = (P_(j, i) - P_(j, i - 1)) / dx;
+  const double lap = second_difference(U_(j, i + 1), uc, U_(j, i - 1), h.dx2, h.idx2) + second_difference(ut, uc, ub, h.dy2, h.idy2);
   double conv;
-  if (centered) {
-    const double e = .5 * (uc + U_(j, i + 1)), w = .5 * (uc + U_(j, i - 1));
-    conv = (e * e - w * w) / dx +
-           .25 * ((uc + ut) * (V_(j + 1, i - 1) + V_(j + 1, i)) - (uc + ub) * (V_(j, i - 1) + V_(j, i))) / dy;
+  if (a.centered) {
+    const double e = uc + U_(j, i + 1), w = uc + U_(j, i - 1);
+    conv = .25 * (div_by(e * e - w * w, h.dx, h.idx) +
+                  div_by((uc + ut) * (V_(j + 1, i - 1) + V_(j + 1, i)) - (uc + ub) * (V_(j, i - 1) + V_(j, i)), h.dy, h.idy));
   } else {
-    const double dudx = (uc > 0.0) ? (uc - U_(j, i - 1)) / dx : (U_(j, i + 1) - uc) / dx;
-    const double dudy = (vavg > 0.0) ? (uc - ub) / dy : (ut - uc) / dy;
+    const double vavg = 0.25 * (V_(j, i - 1) + V_(j, i) + V_(j + 1, i - 1) + V_(j + 1, i));
+    const double dudx = div_by((uc > 0.0) ? uc - U_(j, i - 1) : U_(j, i + 1) - uc, h.dx, h.idx);
+    const double dudy = div_by((vavg > 0.0) ? uc - ub : ut - uc, h.dy, h.idy);
     conv = uc * dudx + vavg * dudy;
   }
-  US_(j, i) = uc + dt * (-conv + nu * lap - dpdx / rho);
+  double r = -conv + a.nu * lap;
+  if (p) r = r - div_by(div_by(P_(j, i) - P_(j, i - 1), h.dx, h.idx), h.rho, h.irho);
+  return uc + a.dt * r;
 }
 
 // v* on every horizontal face (bindings.cpp:142-193): walls zero
-__global__ void k_predict_v(const double* __restrict__ u, const double* __restrict__ v, double* __restrict__ vs,
-                            const double* __restrict__ p, const uint8_t* __restrict__ mask, int nx, int ny,
-                            double dx, double dy, double dx2, double dy2, double dt, double nu, double rho,
-                            int centered) {
-  const long long t = (long long)blockIdx.x * blockDim.x + threadIdx.x;
-  if (t >= (long long)(ny + 1) * nx) return;
-  const int j = (int)(t / nx), i = (int)(t - (long long)j * nx);
-  if (j == 0 || j == ny) { VS_(j, i) = 0.0; return; }
-  if (M_(j - 1, i) || M_(j, i)) { VS_(j, i) = 0.0; return; }
+__device__ __forceinline__ double predict_v(const PredictArgs& a, int j, int i) {
+  const double *u = a.u, *v = a.v, *p = a.p;
+  const uint8_t* mask = a.mask;
+  const int nx = a.nx, ny = a.ny;
+  const Spacing& h = a.h;
+  if (j == 0 || j == ny) return 0.0;
+  if (M_(j - 1, i) || M_(j, i)) return 0.0;
   const double vc = V_(j, i);
-  const double uavg = 0.25 * (U_(j - 1, i) + U_(j, i) + U_(j - 1, i + 1) + U_(j, i + 1));
   double vl, vr;
   if (i == 0) vl = -vc;
   else vl = (M_(j - 1, i - 1) && M_(j, i - 1)) ? -vc : V_(j, i - 1);
   if (i == nx - 1) vr = vc;
   else vr = (M_(j - 1, i + 1) && M_(j, i + 1)) ? -vc : V_(j, i + 1);
-  const double lap = (vr - 2.0 * vc + vl) / dx2 + (V_(j + 1, i) - 2.0 * vc + V_(j - 1, i)) / dy2;
-  const double dpdy = (P_(j, i) - P_(j - 1, i)) / dy;
+  const double lap = second_difference(vr, vc, vl, h.dx2, h.idx2) + second_difference(V_(j + 1, i), vc, V_(j - 1, i), h.dy2, h.idy2);
   double conv;
-  if (centered) {
-    const double n = .5 * (vc + V_(j + 1, i)), s = .5 * (vc + V_(j - 1, i));
-    conv = (n * n - s * s) / dy +
-           .25 * ((vc + vr) * (U_(j - 1, i + 1) + U_(j, i + 1)) - (vc + vl) * (U_(j - 1, i) + U_(j, i))) / dx;
+  if (a.centered) {
+    const double n = vc + V_(j + 1, i), s = vc + V_(j - 1, i);
+    conv = .25 * (div_by(n * n - s * s, h.dy, h.idy) +
+                  div_by((vc + vr) * (U_(j - 1, i + 1) + U_(j, i + 1)) - (vc + vl) * (U_(j - 1, i) + U_(j, i)), h.dx, h.idx));
   } else {
-    const double dvdx = (uavg > 0.0) ? (vc - vl) / dx : (vr - vc) / dx;
-    const double dvdy = (vc > 0.0) ? (vc - V_(j - 1, i)) / dy : (V_(j + 1, i) - vc) / dy;
+    const double uavg = 0.25 * (U_(j - 1, i) + U_(j, i) + U_(j - 1, i + 1) + U_(j, i + 1));
+    const double dvdx = div_by((uavg > 0.0) ? vc - vl : vr - vc, h.dx, h.idx);
+    const double dvdy = div_by((vc > 0.0) ? vc - V_(j - 1, i) : V_(j + 1, i) - vc, h.dy, h.idy);
     conv = uavg * dvdx + vc * dvdy;
   }
-  VS_(j, i) = vc + dt * (-conv + nu * lap - dpdy / rho);
+  double r = -conv + a.nu * lap;
+  if (p) r = r - div_by(div_by(P_(j, i) - P_(j - 1, i), h.dy, h.idy), h.rho, h.irho);
+  return vc + a.dt * r;
+}
+
+// The predictor on every face, with the loop's AB2 step on the interior faces (solver/main.py:315-322)
+// behind it when ab2 >= 0: d = (u* - u) / dt, u* += dt alpha (d - d_prev) when a previous step exists
+// (ab2 = 1), d_prev = d.  The FP64 pipe is the bound; predictor and AB2 in three kernels took 40 us at
+// 350x213, 17 as one with divides by known divisors.
+__global__ void k_predict(PredictArgs a, double* __restrict__ us, double* __restrict__ vs, int ab2, double idt,
+                          double dt_alpha, double* __restrict__ pdu, double* __restrict__ pdv, const int* err) {
+  if (stopped(err)) return;
+  const int nx = a.nx, ny = a.ny;
+  const long long t = (long long)blockIdx.x * blockDim.x + threadIdx.x;
+  const long long nu_ = (long long)ny * (nx + 1);
+  if (t >= nu_ + (long long)(ny + 1) * nx) return;
+  const bool isu = t < nu_;
+  const long long f = isu ? t : t - nu_;
+  const auto [j, i] = row_col(f, isu ? nx + 1 : nx);
+  double s = isu ? predict_u(a, j, i) : predict_v(a, j, i);
+  if (ab2 >= 0 && (isu ? i >= 1 && i < nx : j >= 1 && j < ny)) {
+    const double d = div_by(s - (isu ? a.u : a.v)[f], a.dt, idt);
+    double* prev = isu ? pdu : pdv;
+    if (ab2) s = s + dt_alpha * (d - prev[f]);
+    prev[f] = d;
+  }
+  (isu ? us : vs)[f] = s;
 }
 
 // Poisson right-hand side rho/dt div u* on the fluid cells (bindings.cpp:201-215)
 __global__ void k_poisson_rhs(const double* __restrict__ us, const double* __restrict__ vs,
-                              const uint8_t* __restrict__ mask, double* __restrict__ rhs, int nx, int ny, double dx,
-                              double dy, double inv_dt) {
+                              const uint8_t* __restrict__ mask, double* __restrict__ rhs, int nx, int ny,
+                              Spacing h, double inv_dt) {
   const long long t = (long long)blockIdx.x * blockDim.x + threadIdx.x;
   if (t >= (long long)ny * nx) return;
   const int j = (int)(t / nx), i = (int)(t - (long long)j * nx);
   if (M_(j, i)) { rhs[t] = 0.0; return; }
-  const double div = (US_(j, i + 1) - US_(j, i)) / dx + (VS_(j + 1, i) - VS_(j, i)) / dy;
+  const double div = div_by(US_(j, i + 1) - US_(j, i), h.dx, h.idx) + div_by(VS_(j + 1, i) - VS_(j, i), h.dy, h.idy);
   rhs[t] = inv_dt * div;
 }
 
-// The legacy loop's AB2 step on the interior faces (solver/main.py:315-322): d = (u* - u) / dt,
+// The same AB2 step by itself (the ghost-cell branch sets its ghost faces in between): d = (u* - u) / dt,
 // u* += dt alpha (d - d_prev) when a previous step exists, d_prev = d
 __global__ void k_ab2(const double* __restrict__ u, const double* __restrict__ v, double* __restrict__ us,
                       double* __restrict__ vs, double* __restrict__ pdu, double* __restrict__ pdv, int nx, int ny,
-                      double dt, double dt_alpha, int has_prev) {
+                      double dt, double dt_alpha, int has_prev, const int* err) {
+  if (stopped(err)) return;
   const long long t = (long long)blockIdx.x * blockDim.x + threadIdx.x;
   const long long nu_ = (long long)ny * (nx + 1), nv_ = (long long)(ny + 1) * nx;
   if (t < nu_) {
@@ -146,15 +205,19 @@ __global__ void k_ab2(const double* __restrict__ u, const double* __restrict__ v
 }
 
 // the recomputed Poisson right-hand side of the legacy loop (solver/main.py:337-339):
-// rho/dt ((u*_e - u*_w)/dx + (v*_n - v*_s)/dy), zero on masked cells
+// rho/dt ((u*_e - u*_w)/dx + (v*_n - v*_s)/dy), zero on masked cells; with cell_type in the row
+// scaling of the pressure system (1 / kappa on cut cells, zero on covered ones)
 __global__ void k_legacy_rhs(const double* __restrict__ us, const double* __restrict__ vs,
-                             const uint8_t* __restrict__ mask, double* __restrict__ rhs, int nx, int ny, double dx,
-                             double dy, double rho_dt) {
+                             const uint8_t* __restrict__ mask, double* __restrict__ rhs, int nx, int ny, Spacing h,
+                             double rho_dt, const int32_t* __restrict__ cell_type, const double* __restrict__ ikappa,
+                             const int* err) {
+  if (stopped(err)) return;
   const long long t = (long long)blockIdx.x * blockDim.x + threadIdx.x;
   if (t >= (long long)ny * nx) return;
-  const int j = (int)(t / nx), i = (int)(t - (long long)j * nx);
-  if (M_(j, i)) { rhs[t] = 0.0; return; }
-  rhs[t] = rho_dt * ((US_(j, i + 1) - US_(j, i)) / dx + (VS_(j + 1, i) - VS_(j, i)) / dy);
+  const auto [j, i] = row_col(t, nx);
+  if (M_(j, i) || (cell_type && cell_type[t] == -1)) { rhs[t] = 0.0; return; }
+  const double r = rho_dt * (div_by(US_(j, i + 1) - US_(j, i), h.dx, h.idx) + div_by(VS_(j + 1, i) - VS_(j, i), h.dy, h.idy));
+  rhs[t] = cell_type ? r * ikappa[t] : r;
 }
 
 // ---- the legacy loop's ghost-cell branch (solver/ghost_cell.py:32-234, solver/main.py:347-370) --
@@ -164,7 +227,8 @@ __global__ void k_legacy_rhs(const double* __restrict__ us, const double* __rest
 // the faces into levels (a face is one level above every earlier ghost face it reads), the old
 // values are saved first, and each level is one launch.
 __global__ void k_ghost_save(const double* __restrict__ f, long long nf, const long long* __restrict__ target,
-                             long long n, double* __restrict__ snap) {
+                             long long n, double* __restrict__ snap, const int* err) {
+  if (stopped(err)) return;
   const long long g = (long long)blockIdx.x * blockDim.x + threadIdx.x;
   if (g < n) {
     const long long t = target[g];
@@ -176,7 +240,8 @@ __global__ void k_ghost_level(double* __restrict__ f, long long nf, const long l
                               const long long* __restrict__ src, const int* __restrict__ snap_of,
                               const double* __restrict__ w, const double* __restrict__ gamma,
                               const int* __restrict__ level, long long n, int lvl, const double* __restrict__ snap,
-                              double wall) {
+                              double wall, const int* err) {
+  if (stopped(err)) return;
   const long long g = (long long)blockIdx.x * blockDim.x + threadIdx.x;
   if (g >= n || level[g] != lvl) return;
   const long long t = target[g];
@@ -200,7 +265,8 @@ __global__ void k_ghost_level(double* __restrict__ f, long long nf, const long l
 __global__ void k_ghost_correct(double* __restrict__ u, double* __restrict__ v, const double* __restrict__ us,
                                 const double* __restrict__ vs, const double* __restrict__ phi,
                                 const uint8_t* __restrict__ mask, const double* __restrict__ inlet, int nx, int ny,
-                                double dx, double dy, double dt_over_rho) {
+                                double dx, double dy, double dt_over_rho, const int* err) {
+  if (stopped(err)) return;
   const long long t = (long long)blockIdx.x * blockDim.x + threadIdx.x;
   const long long nu_ = (long long)ny * (nx + 1);
   if (t < nu_) {
@@ -225,11 +291,14 @@ __global__ void k_ghost_correct(double* __restrict__ u, double* __restrict__ v, 
     V_(j, i) = val;
   }
 }
-// faces between a fluid and a masked cell keep u* (solver/main.py:368-370)
+// faces between a fluid and a masked cell keep u* (solver/main.py:368-370); the pressure update
 __global__ void k_ghost_boundary(double* __restrict__ u, double* __restrict__ v, const double* __restrict__ us,
-                                 const double* __restrict__ vs, const uint8_t* __restrict__ mask, int nx, int ny) {
+                                 const double* __restrict__ vs, const uint8_t* __restrict__ mask, int nx, int ny, double* __restrict__ p,
+                                 const double* __restrict__ phi, int add, const int* err) {
+  if (stopped(err)) return;
   const long long t = (long long)blockIdx.x * blockDim.x + threadIdx.x;
   const long long nu_ = (long long)ny * (nx + 1);
+  if (p && t < (long long)ny * nx) p[t] = add ? p[t] + phi[t] : phi[t];
   if (t < nu_) {
     const int j = (int)(t / (nx + 1)), i = (int)(t - (long long)j * (nx + 1));
     if (i >= 1 && i <= nx - 1 && M_(j, i - 1) != M_(j, i)) U_(j, i) = US_(j, i);
@@ -239,6 +308,20 @@ __global__ void k_ghost_boundary(double* __restrict__ u, double* __restrict__ v,
     if (j >= 1 && j <= ny - 1 && M_(j - 1, i) != M_(j, i)) V_(j, i) = VS_(j, i);
   }
 }
+
+// A step's record behind its four forces: max |residual| of the pressure solve's last check (out[4], its bits)
+// and a mark that the step is complete (out[5]).
+struct StepRecord {
+  const gmk::StepCtl* ctl;  // null: no record
+  int slot, nchk;
+  __device__ const int* err() const { return ctl ? &ctl->err : nullptr; }
+  __device__ void close(double* out) const {
+    if (!ctl) return;
+    const gmk::SolveCtl* sc = &ctl->solve[slot];
+    out[4] = gmk::bits2d(sc->rmax[gmk::last_check(sc, nchk)]);
+    out[5] = 1.0;
+  }
+};
 
 // bilinear value of a staggered field at (y, x): the linear RegularGridInterpolator of the
 // reference (solver/ghost_cell.py:199-201), zero outside the grid
@@ -260,7 +343,8 @@ __device__ double grid_linear(const double* __restrict__ f, int nxf, int nyf, do
 // fixed order; out = fx_p, fy_p, fx_v, fy_v
 __global__ void k_ghost_forces(const double* __restrict__ u, const double* __restrict__ v, const double* __restrict__ p,
                                int nx, int ny, double dx, double dy, double xc, double yc, double radius, int n,
-                               double mu, double* __restrict__ out) {
+                               double mu, double* __restrict__ out, StepRecord rec) {
+  if (stopped(rec.err())) return;
   __shared__ double sh[4][256];
   double ax = 0.0, ay = 0.0, bx = 0.0, by = 0.0;
   const double eps = 1e-4 * dx;
@@ -294,30 +378,34 @@ __global__ void k_ghost_forces(const double* __restrict__ u, const double* __res
     out[1] = -sh[1][0] * ds;
     out[2] = sh[2][0] * ds;
     out[3] = sh[3][0] * ds;
+    rec.close(out);
   }
 }
 
-// u = u* - dt/rho d phi/dx, v = v* - dt/rho d phi/dy (bindings.cpp:248-281)
+// u = u* - dt/rho d phi/dx, v = v* - dt/rho d phi/dy (bindings.cpp:248-281); with p also the loop's pressure
+// update, p = phi (add = 0) or p += phi
 __global__ void k_correct(double* __restrict__ u, double* __restrict__ v, const double* __restrict__ us,
                           const double* __restrict__ vs, const double* __restrict__ phi,
                           const uint8_t* __restrict__ mask, const double* __restrict__ inlet, int nx, int ny,
-                          double dx, double dy, double dt_over_rho) {
+                          Spacing h, double dt_over_rho, double* __restrict__ p, int add, const int* err) {
+  if (stopped(err)) return;
   const long long t = (long long)blockIdx.x * blockDim.x + threadIdx.x;
   const long long nu_ = (long long)ny * (nx + 1);
+  if (p && t < (long long)ny * nx) p[t] = add ? p[t] + phi[t] : phi[t];
   if (t < nu_) {
-    const int j = (int)(t / (nx + 1)), i = (int)(t - (long long)j * (nx + 1));
+    const auto [j, i] = row_col(t, nx + 1);
     if (i == 0) U_(j, 0) = inlet[j];
-    else if (i == nx) U_(j, nx) = US_(j, nx) + dt_over_rho * 2.0 * PHI_(j, nx - 1) / dx;
+    else if (i == nx) U_(j, nx) = US_(j, nx) + div_by(dt_over_rho * 2.0 * PHI_(j, nx - 1), h.dx, h.idx);
     else if (M_(j, i - 1) || M_(j, i)) U_(j, i) = 0.0;
-    else U_(j, i) = US_(j, i) - dt_over_rho * (PHI_(j, i) - PHI_(j, i - 1)) / dx;
+    else U_(j, i) = US_(j, i) - div_by(dt_over_rho * (PHI_(j, i) - PHI_(j, i - 1)), h.dx, h.idx);
     return;
   }
   const long long r = t - nu_;
   if (r >= (long long)(ny + 1) * nx) return;
-  const int j = (int)(r / nx), i = (int)(r - (long long)j * nx);
+  const auto [j, i] = row_col(r, nx);
   if (j == 0 || j == ny) V_(j, i) = 0.0;
   else if (M_(j - 1, i) || M_(j, i)) V_(j, i) = 0.0;
-  else V_(j, i) = VS_(j, i) - dt_over_rho * (PHI_(j, i) - PHI_(j - 1, i)) / dy;
+  else V_(j, i) = VS_(j, i) - div_by(dt_over_rho * (PHI_(j, i) - PHI_(j - 1, i)), h.dy, h.idy);
 }
 
 template <int NF>
@@ -409,25 +497,30 @@ __global__ void k_div_part(const double* __restrict__ u, const double* __restric
 // per-field sums of the block partials (one block of LT threads: thread t adds the partials of
 // blocks t, t + LT, ... in order, then a tree in a fixed order; the same sums every run); the
 // maximum of the divergence after them when nmax is set
-__global__ void k_fold(const double* __restrict__ part, int nblocks, int nf, int nmax, double* __restrict__ out) {
-  __shared__ double sh[LT];
-  const int nout = nf + (nmax ? 1 : 0);
-  for (int f = 0; f < nout; ++f) {
-    const bool is_max = f == nf;
-    double a = 0.0;
-    for (int b = threadIdx.x; b < nblocks; b += blockDim.x) {
-      const double v = is_max ? part[(size_t)nblocks * nf + b] : part[(size_t)b * nf + f];
-      a = is_max ? fmax(a, v) : a + v;
+__global__ void k_fold(const double* __restrict__ part, int nblocks, int nmax, double* __restrict__ out, StepRecord rec) {
+  if (stopped(rec.err())) return;
+  constexpr int NF = 4;
+  __shared__ double sh[NF + 1][LT];
+  double a[NF + 1] = {0.0, 0.0, 0.0, 0.0, 0.0};
+  for (int b = threadIdx.x; b < nblocks; b += LT) {
+#pragma unroll
+    for (int f = 0; f < NF; ++f) a[f] = a[f] + part[(size_t)b * NF + f];
+    if (nmax) a[NF] = fmax(a[NF], part[(size_t)nblocks * NF + b]);
+  }
+#pragma unroll
+  for (int f = 0; f <= NF; ++f) sh[f][threadIdx.x] = a[f];
+  __syncthreads();
+  for (int k = LT / 2; k > 0; k >>= 1) {
+    if ((int)threadIdx.x < k) {
+#pragma unroll
+      for (int f = 0; f < NF; ++f) sh[f][threadIdx.x] = sh[f][threadIdx.x] + sh[f][threadIdx.x + k];
+      sh[NF][threadIdx.x] = fmax(sh[NF][threadIdx.x], sh[NF][threadIdx.x + k]);
     }
-    sh[threadIdx.x] = a;
     __syncthreads();
-    for (int k = blockDim.x / 2; k > 0; k >>= 1) {
-      if ((int)threadIdx.x < k)
-        sh[threadIdx.x] = is_max ? fmax(sh[threadIdx.x], sh[threadIdx.x + k]) : sh[threadIdx.x] + sh[threadIdx.x + k];
-      __syncthreads();
-    }
-    if (threadIdx.x == 0) out[f] = sh[0];
-    __syncthreads();
+  }
+  if (threadIdx.x == 0) {
+    for (int f = 0; f < NF + (nmax ? 1 : 0); ++f) out[f] = sh[f][0];
+    rec.close(out);
   }
 }
 
@@ -537,21 +630,15 @@ int cuda_fail(cudaError_t e) {
 }
 unsigned blocks(long long n) { return (unsigned)((n + LT - 1) / LT); }
 
-// p = phi (c = 0) or p += phi (c = 1)
-__global__ void k_pupdate(double* __restrict__ p, const double* __restrict__ phi, long long n, int add) {
-  const long long t = (long long)blockIdx.x * blockDim.x + threadIdx.x;
-  if (t < n) p[t] = add ? p[t] + phi[t] : phi[t];
-}
-
-void ghost_pass(const gm_legacy_state& s, int k, double* field, double* snap, cudaStream_t st) {
+void ghost_pass(const gm_legacy_state& s, int k, double* field, double* snap, const int* err, cudaStream_t st) {
   const long long n = s.n_ghost[k];
   if (n <= 0) return;
   const long long nf = k == 0 ? (long long)s.ny * (s.nx + 1) : (long long)(s.ny + 1) * s.nx;
   const long long* tg = reinterpret_cast<const long long*>(s.target[k]);
-  k_ghost_save<<<blocks(n), LT, 0, st>>>(field, nf, tg, n, snap);
+  k_ghost_save<<<blocks(n), LT, 0, st>>>(field, nf, tg, n, snap, err);
   for (int l = 0; l < s.n_levels[k]; ++l)
     k_ghost_level<<<blocks(n), LT, 0, st>>>(field, nf, tg, reinterpret_cast<const long long*>(s.src[k]), s.snap_of[k],
-                                            s.weights[k], s.gamma[k], s.level[k], n, l, snap, 0.0);
+                                            s.weights[k], s.gamma[k], s.level[k], n, l, snap, 0.0, err);
   gmk::kernel_launch_adjust(1 + s.n_levels[k]);
 }
 
@@ -565,63 +652,62 @@ size_t scratch_doubles(const gm_legacy_state& s) {
   return (size_t)(ng + (long long)blocks(nP) * 4 + 16);
 }
 
-void predict(const gm_legacy_state& s, double dt, double* scratch, cudaStream_t st) {
+void predict(const gm_legacy_state& s, double dt, double* scratch, const int32_t* cell_type, const double* ikappa,
+             const int* err, cudaStream_t st) {
   const int nx = s.nx, ny = s.ny;
   const long long nU = (long long)ny * (nx + 1), nV = (long long)(ny + 1) * nx, nP = (long long)ny * nx;
-  const double* pin = s.centered ? s.zero_p : s.p;
-  k_predict_u<<<blocks(nU), LT, 0, st>>>(s.u, s.v, s.u_star, pin, s.mask, s.inlet, nx, ny, s.dx, s.dy, s.dx * s.dx,
-                                         s.dy * s.dy, dt, s.nu, s.rho, s.slip_walls ? 1 : 0, s.centered ? 1 : 0);
-  k_predict_v<<<blocks(nV), LT, 0, st>>>(s.u, s.v, s.v_star, pin, s.mask, nx, ny, s.dx, s.dy, s.dx * s.dx,
-                                         s.dy * s.dy, dt, s.nu, s.rho, s.centered ? 1 : 0);
-  gmk::kernel_launch_adjust(2);
+  const PredictArgs a{s.u, s.v, s.centered ? nullptr : s.p, s.inlet, s.mask, nx, ny, spacing_of(s.dx, s.dy, s.rho), dt, s.nu,
+                      s.slip_walls ? 1 : 0, s.centered ? 1 : 0};
+  const bool hp = s.has_prev != 0;
+  const double dta = hp ? dt * (dt / (2 * s.prev_dt)) : 0.0;
+  k_predict<<<blocks(nU + nV), LT, 0, st>>>(a, s.u_star, s.v_star, s.ghost || !s.centered ? -1 : hp ? 1 : 0, gmk::reciprocal_of(dt), dta,
+                                            s.prev_du, s.prev_dv, err);
+  gmk::kernel_launch_adjust(1);
   if (s.ghost) {
-    ghost_pass(s, 0, s.u_star, scratch, st);
-    ghost_pass(s, 1, s.v_star, scratch, st);
-  }
-  if (s.centered) {
-    const bool hp = s.has_prev != 0;
-    k_ab2<<<blocks(nU + nV), LT, 0, st>>>(s.u, s.v, s.u_star, s.v_star, s.prev_du, s.prev_dv, nx, ny, dt,
-                                          hp ? dt * (dt / (2 * s.prev_dt)) : 0.0, hp ? 1 : 0);
-    gmk::kernel_launch_adjust(1);
-    if (s.ghost) {
-      ghost_pass(s, 0, s.u_star, scratch, st);
-      ghost_pass(s, 1, s.v_star, scratch, st);
+    ghost_pass(s, 0, s.u_star, scratch, err, st);
+    ghost_pass(s, 1, s.v_star, scratch, err, st);
+    if (s.centered) {
+      k_ab2<<<blocks(nU + nV), LT, 0, st>>>(s.u, s.v, s.u_star, s.v_star, s.prev_du, s.prev_dv, nx, ny, dt, dta, hp ? 1 : 0, err);
+      gmk::kernel_launch_adjust(1);
+      ghost_pass(s, 0, s.u_star, scratch, err, st);
+      ghost_pass(s, 1, s.v_star, scratch, err, st);
     }
   }
-  k_legacy_rhs<<<blocks(nP), LT, 0, st>>>(s.u_star, s.v_star, s.mask, s.rhs, nx, ny, s.dx, s.dy, s.rho / dt);
+  k_legacy_rhs<<<blocks(nP), LT, 0, st>>>(s.u_star, s.v_star, s.mask, s.rhs, nx, ny, a.h, s.rho / dt, cell_type, ikappa, err);
   gmk::kernel_launch_adjust(1);
 }
 
-void correct(const gm_legacy_state& s, double dt, double* scratch, cudaStream_t st) {
+void correct(const gm_legacy_state& s, double dt, double* scratch, const int* err, cudaStream_t st) {
   const int nx = s.nx, ny = s.ny;
-  const long long n = (long long)ny * (nx + 1) + (long long)(ny + 1) * nx, nP = (long long)ny * nx;
+  const long long n = (long long)ny * (nx + 1) + (long long)(ny + 1) * nx;
   if (s.ghost) {
     k_ghost_correct<<<blocks(n), LT, 0, st>>>(s.u, s.v, s.u_star, s.v_star, s.phi, s.mask, s.inlet, nx, ny, s.dx,
-                                              s.dy, dt / s.rho);
-    gmk::kernel_launch_adjust(1);
-    ghost_pass(s, 0, s.u, scratch, st);
-    ghost_pass(s, 1, s.v, scratch, st);
-    k_ghost_boundary<<<blocks(n), LT, 0, st>>>(s.u, s.v, s.u_star, s.v_star, s.mask, nx, ny);
+                                              s.dy, dt / s.rho, err);
+    ghost_pass(s, 0, s.u, scratch, err, st);
+    ghost_pass(s, 1, s.v, scratch, err, st);
+    k_ghost_boundary<<<blocks(n), LT, 0, st>>>(s.u, s.v, s.u_star, s.v_star, s.mask, nx, ny, s.p, s.phi, s.centered ? 0 : 1, err);
+    gmk::kernel_launch_adjust(2);
   } else {
-    k_correct<<<blocks(n), LT, 0, st>>>(s.u, s.v, s.u_star, s.v_star, s.phi, s.mask, s.inlet, nx, ny, s.dx, s.dy,
-                                        dt / s.rho);
+    k_correct<<<blocks(n), LT, 0, st>>>(s.u, s.v, s.u_star, s.v_star, s.phi, s.mask, s.inlet, nx, ny,
+                                        spacing_of(s.dx, s.dy, s.rho), dt / s.rho, s.p, s.centered ? 0 : 1, err);
+    gmk::kernel_launch_adjust(1);
   }
-  k_pupdate<<<blocks(nP), LT, 0, st>>>(s.p, s.phi, nP, s.centered ? 0 : 1);
-  gmk::kernel_launch_adjust(2);
 }
 
-void forces(const gm_legacy_state& s, double* scratch, double* out, cudaStream_t st) {
+void forces(const gm_legacy_state& s, double* scratch, double* out, const gmk::StepCtl* ctl, int slot, int nchk,
+            cudaStream_t st) {
   const int nx = s.nx, ny = s.ny;
   const double mu = s.nu * s.rho;
+  const StepRecord rec{ctl, slot, nchk};
   if (s.ghost) {
-    k_ghost_forces<<<1, 256, 0, st>>>(s.u, s.v, s.p, nx, ny, s.dx, s.dy, s.xc, s.yc, s.radius, s.n_theta, mu, out);
+    k_ghost_forces<<<1, 256, 0, st>>>(s.u, s.v, s.p, nx, ny, s.dx, s.dy, s.xc, s.yc, s.radius, s.n_theta, mu, out, rec);
     gmk::kernel_launch_adjust(1);
     return;
   }
   const unsigned nb = blocks((long long)ny * nx);
-  double* part = scratch + std::max<long long>(s.ghost ? std::max(s.n_ghost[0], s.n_ghost[1]) : 0, 1);
+  double* part = scratch + 1;
   k_forces_part<<<nb, LT, 0, st>>>(s.u, s.v, s.p, s.mask, nx, ny, s.dx, s.dy, mu, part);
-  k_fold<<<1, LT, 0, st>>>(part, (int)nb, 4, 0, out);
+  k_fold<<<1, LT, 0, st>>>(part, (int)nb, 0, out, rec);
   gmk::kernel_launch_adjust(2);
 }
 
@@ -646,16 +732,14 @@ int gm_mac_predictor_rhs(const double* u, const double* v, double* u_star, doubl
   double* extra = nullptr;
   if (cudaError_t e = sg.begin(0, &extra)) return cuda_fail(e);
   cudaStream_t st = sg.st;
-  k_predict_u<<<blocks((long long)nU), LT, 0, st>>>(sg.dev<double>(iu), sg.dev<double>(iv), sg.dev<double>(ius),
-                                                    sg.dev<double>(ip), sg.dev<uint8_t>(im), sg.dev<double>(ii), nx,
-                                                    ny, dx, dy, dx * dx, dy * dy, dt, nu, rho, slip_walls ? 1 : 0,
-                                                    centered ? 1 : 0);
-  k_predict_v<<<blocks((long long)nV), LT, 0, st>>>(sg.dev<double>(iu), sg.dev<double>(iv), sg.dev<double>(ivs),
-                                                    sg.dev<double>(ip), sg.dev<uint8_t>(im), nx, ny, dx, dy, dx * dx,
-                                                    dy * dy, dt, nu, rho, centered ? 1 : 0);
+  const Spacing h = spacing_of(dx, dy, rho);
+  const PredictArgs a{sg.dev<double>(iu), sg.dev<double>(iv), sg.dev<double>(ip), sg.dev<double>(ii), sg.dev<uint8_t>(im), nx, ny, h,
+                      dt, nu, slip_walls ? 1 : 0, centered ? 1 : 0};
+  k_predict<<<blocks((long long)(nU + nV)), LT, 0, st>>>(a, sg.dev<double>(ius), sg.dev<double>(ivs), -1, 0.0, 0.0, nullptr, nullptr,
+                                                       nullptr);
   k_poisson_rhs<<<blocks((long long)nP), LT, 0, st>>>(sg.dev<double>(ius), sg.dev<double>(ivs), sg.dev<uint8_t>(im),
-                                                      sg.dev<double>(ir), nx, ny, dx, dy, rho / dt);
-  gmk::kernel_launch_adjust(3);
+                                                      sg.dev<double>(ir), nx, ny, h, rho / dt);
+  gmk::kernel_launch_adjust(2);
   if (cudaError_t e = cudaGetLastError()) return cuda_fail(e);
   if (cudaError_t e = sg.finish()) return cuda_fail(e);
   return GM_OK;
@@ -679,7 +763,7 @@ int gm_mac_corrector(double* u, double* v, const double* u_star, const double* v
   k_correct<<<blocks((long long)(nU + nV)), LT, 0, sg.st>>>(sg.dev<double>(iu), sg.dev<double>(iv),
                                                               sg.dev<double>(ius), sg.dev<double>(ivs),
                                                               sg.dev<double>(iph), sg.dev<uint8_t>(im),
-                                                              sg.dev<double>(ii), nx, ny, dx, dy, dt / rho);
+                                                              sg.dev<double>(ii), nx, ny, spacing_of(dx, dy, rho), dt / rho, nullptr, 0, nullptr);
   gmk::kernel_launch_adjust(1);
   if (cudaError_t e = cudaGetLastError()) return cuda_fail(e);
   if (cudaError_t e = sg.finish()) return cuda_fail(e);
@@ -705,13 +789,13 @@ int gm_mac_ab2_rhs(const double* u, const double* v, double* u_star, double* v_s
   if (what & 1) {
     k_ab2<<<blocks((long long)(nU + nV)), LT, 0, st>>>(sg.dev<double>(iu), sg.dev<double>(iv), sg.dev<double>(ius),
                                                        sg.dev<double>(ivs), sg.dev<double>(idu), sg.dev<double>(idv),
-                                                       nx, ny, dt, dt * alpha, has_prev ? 1 : 0);
+                                                       nx, ny, dt, dt * alpha, has_prev ? 1 : 0, nullptr);
     gmk::kernel_launch_adjust(1);
   }
   if (what & 2) {
     k_legacy_rhs<<<blocks((long long)nP), LT, 0, st>>>(sg.dev<double>(ius), sg.dev<double>(ivs),
-                                                       sg.dev<uint8_t>(im), sg.dev<double>(ir), nx, ny, dx, dy,
-                                                       rho / dt);
+                                                       sg.dev<uint8_t>(im), sg.dev<double>(ir), nx, ny, spacing_of(dx, dy, rho),
+                                                       rho / dt, nullptr, nullptr, nullptr);
     gmk::kernel_launch_adjust(1);
   }
   if (cudaError_t e = cudaGetLastError()) return cuda_fail(e);
@@ -736,11 +820,11 @@ int gm_mac_ghost_apply(double* field, int64_t field_size, int64_t n_ghost, const
   if (cudaError_t e = sg.begin(ng * 8, &snap)) return cuda_fail(e);
   const unsigned nb = blocks((long long)n_ghost);
   const long long* tg = sg.dev<const long long>(it);
-  k_ghost_save<<<nb, LT, 0, sg.st>>>(sg.dev<double>(iff), field_size, tg, n_ghost, snap);
+  k_ghost_save<<<nb, LT, 0, sg.st>>>(sg.dev<double>(iff), field_size, tg, n_ghost, snap, nullptr);
   for (int l = 0; l < n_levels; ++l)
     k_ghost_level<<<nb, LT, 0, sg.st>>>(sg.dev<double>(iff), field_size, tg, sg.dev<const long long>(is),
                                         sg.dev<const int>(io), sg.dev<const double>(iw), sg.dev<const double>(ig),
-                                        sg.dev<const int>(il), n_ghost, l, snap, wall);
+                                        sg.dev<const int>(il), n_ghost, l, snap, wall, nullptr);
   gmk::kernel_launch_adjust(1 + n_levels);
   if (cudaError_t e = cudaGetLastError()) return cuda_fail(e);
   if (cudaError_t e = sg.finish()) return cuda_fail(e);
@@ -764,11 +848,11 @@ int gm_mac_ghost_correct(double* u, double* v, const double* u_star, const doubl
   const long long n = (long long)(nU + nV);
   if (boundary_faces)
     k_ghost_boundary<<<blocks(n), LT, 0, sg.st>>>(sg.dev<double>(iu), sg.dev<double>(iv), sg.dev<double>(ius),
-                                                  sg.dev<double>(ivs), sg.dev<uint8_t>(im), nx, ny);
+                                                  sg.dev<double>(ivs), sg.dev<uint8_t>(im), nx, ny, nullptr, nullptr, 0, nullptr);
   else
     k_ghost_correct<<<blocks(n), LT, 0, sg.st>>>(sg.dev<double>(iu), sg.dev<double>(iv), sg.dev<double>(ius),
                                                  sg.dev<double>(ivs), sg.dev<double>(iph), sg.dev<uint8_t>(im),
-                                                 sg.dev<double>(ii), nx, ny, dx, dy, dt / rho);
+                                                 sg.dev<double>(ii), nx, ny, dx, dy, dt / rho, nullptr);
   gmk::kernel_launch_adjust(1);
   if (cudaError_t e = cudaGetLastError()) return cuda_fail(e);
   if (cudaError_t e = sg.finish()) return cuda_fail(e);
@@ -791,7 +875,7 @@ int gm_mac_ghost_forces(const double* u, const double* v, const double* p, int32
   double* res = nullptr;
   if (cudaError_t e = sg.begin(8 * 8, &res)) return cuda_fail(e);
   k_ghost_forces<<<1, 256, 0, sg.st>>>(sg.dev<double>(iu), sg.dev<double>(iv), sg.dev<double>(ip), nx, ny, dx, dy,
-                                       xc, yc, radius, n_theta, mu, res);
+                                       xc, yc, radius, n_theta, mu, res, StepRecord{});
   gmk::kernel_launch_adjust(1);
   if (cudaError_t e = cudaGetLastError()) return cuda_fail(e);
   if (cudaError_t e = cudaMemcpyAsync(out, res, 4 * sizeof(double), cudaMemcpyDeviceToHost, sg.st))
@@ -815,7 +899,7 @@ int gm_mac_forces(const double* u, const double* v, const double* p, const uint8
   double* res = part + (size_t)nb * 4;
   k_forces_part<<<nb, LT, 0, sg.st>>>(sg.dev<double>(iu), sg.dev<double>(iv), sg.dev<double>(ip), sg.dev<uint8_t>(im),
                                       nx, ny, dx, dy, mu, part);
-  k_fold<<<1, LT, 0, sg.st>>>(part, (int)nb, 4, 0, res);
+  k_fold<<<1, LT, 0, sg.st>>>(part, (int)nb, 0, res, StepRecord{});
   gmk::kernel_launch_adjust(2);
   if (cudaError_t e = cudaGetLastError()) return cuda_fail(e);
   if (cudaError_t e = cudaMemcpyAsync(out, res, 4 * sizeof(double), cudaMemcpyDeviceToHost, sg.st))
@@ -837,7 +921,7 @@ int gm_mac_divergence(const double* u, const double* v, const uint8_t* mask, int
   if (cudaError_t e = sg.begin(((size_t)nb * 5 + 8) * 8, &part)) return cuda_fail(e);
   double* res = part + (size_t)nb * 5;
   k_div_part<<<nb, LT, 0, sg.st>>>(sg.dev<double>(iu), sg.dev<double>(iv), sg.dev<uint8_t>(im), nx, ny, dx, dy, part);
-  k_fold<<<1, LT, 0, sg.st>>>(part, (int)nb, 4, 1, res);
+  k_fold<<<1, LT, 0, sg.st>>>(part, (int)nb, 1, res, StepRecord{});
   gmk::kernel_launch_adjust(2);
   if (cudaError_t e = cudaGetLastError()) return cuda_fail(e);
   double r[5];

@@ -27,6 +27,7 @@
 #include <vector>
 
 #include "../../include/ghostmac.h"
+#include "exactdiv.cuh"
 #include "fftplan.hpp"
 #include "transforms.cuh"
 
@@ -163,13 +164,6 @@ __device__ __forceinline__ bool tg_short(unsigned long long* red, const TgHeld& 
     red[RED_ERR] = (unsigned long long)step_index;
   }
   return true;
-}
-// a / b for a divisor known in advance (rb = 1 / b, correctly rounded): one multiplication and two fused
-// multiply-adds give the correctly rounded quotient (Brisebarre, Muller and Raina, IEEE Trans. Computers
-// 53, 2004), a third of a divide's FP64 instructions and the same bits
-__device__ __forceinline__ double div_by(double a, double b, double rb) {
-  const double q = a * rb;
-  return fma(fma(-q, b, a), rb, q);
 }
 
 // ---- kernels ------------------------------------------------------------------------------

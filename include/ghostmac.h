@@ -408,9 +408,9 @@ typedef struct gm_legacy_step_diag {
  * (predictor_rhs_cpp), ghost velocities (ghost-cell branch), the loop's AB2 step, the
  * right-hand side, the pressure solve of `p` (built over the loop's staircase mask), the
  * corrector (corrector_cpp, or the ghost-cell branch's), the pressure update and the forces
- * (calculate_mac_forces_cpp, or extract_true_surface_forces on the circle).  One stream
- * synchronisation per step, at the pressure gate, before the corrector: a failed solve leaves
- * u, v and p as they were.  Ordered after the work on `stream` (a cudaStream_t or NULL) and
+ * (calculate_mac_forces_cpp, or extract_true_surface_forces on the circle).  The steps queue
+ * without a host check between them: a failed pressure gate stops the kernels behind it, so it
+ * leaves u, v and p as the last good step left them.  Ordered after the work on `stream` (a cudaStream_t or NULL) and
  * before later work there. */
 int gm_poisson_legacy_step(gm_poisson* p, gm_legacy_state* s, double dt, int32_t n_steps, gm_legacy_step_diag* diag,
                            void* stream);
