@@ -10,9 +10,11 @@
 
 namespace gmk {
 
-inline FftPlan make_plan(int M) {
+// fixed7: radix-7 stages by their own butterfly (FP64 handles; see FftPlan)
+inline FftPlan make_plan(int M, bool fixed7) {
   FftPlan p{};
   p.M = M;
+  p.fixed7 = fixed7 ? 1 : 0;
   int m = M, s = 0;
   while (m % 8 == 0) { p.radix[s++] = 8; m /= 8; }
   while (m % 4 == 0) { p.radix[s++] = 4; m /= 4; }
@@ -33,7 +35,7 @@ inline FftPlan make_plan(int M) {
   for (int k = 0; k < s; ++k) {
     p.ns_magic[k] = Ns == 1 ? 0u : (unsigned)(((1ull << 32) + (unsigned long long)Ns - 1) / (unsigned long long)Ns);
     const int R = p.radix[k];
-    if (R == 2 || R == 3 || R == 4 || R == 5 || R == 8) {
+    if (p.fixed_radix(R)) {
       p.tw_off[k] = off;
       off += (int)Ns * (R - 1);
     } else {
@@ -43,7 +45,7 @@ inline FftPlan make_plan(int M) {
   }
   for (int k = 0; k < s; ++k) {
     const int R = p.radix[k];
-    if (!(R == 2 || R == 3 || R == 4 || R == 5 || R == 8)) p.tw_off[k] = off;  // the full table follows
+    if (!p.fixed_radix(R)) p.tw_off[k] = off;  // the full table follows
   }
   p.tw_len = off + (generic ? M : 0);
   return p;
@@ -62,7 +64,7 @@ inline std::vector<double> plan_twiddles(const FftPlan& p) {
   bool generic = false;
   for (int s = 0; s < p.nstages; ++s) {
     const int R = p.radix[s];
-    if (R == 2 || R == 3 || R == 4 || R == 5 || R == 8) {
+    if (p.fixed_radix(R)) {
       const long long tws = p.M / (Ns * R);
       for (long long k = 0; k < Ns; ++k)
         for (int r = 1; r < R; ++r) put(p.tw_off[s] + (int)(k * (R - 1) + r - 1), r * k * tws);

@@ -554,7 +554,7 @@ void build_rect_tables(gm_handle* h, RectDev& rd, int kind, double dt) {
   TransformTables& tt = rd.tt;
   tt.tx_fwd = tx_f; tt.tx_inv = tx_i;
   int Mx = r2r_fft_length(tx_f, cols);
-  tt.plan_x = make_plan(Mx);
+  tt.plan_x = make_plan(Mx, h->precision == 0);
   cudaStream_t st = h->st;
   rd.Wx.upload(plan_twiddles(tt.plan_x), st);
   // type IV: pre exp(-i pi (4m+1)/(4n)), post exp(-i pi k/n); Makhoul: (cos, sin)(pi k/(2n))

@@ -883,7 +883,7 @@ int gm_tg_create(int32_t n, double nu, int32_t precision, gm_tg** out) {
   t->precision = precision;
   int rc = tg_guard(t.get(), [&] {
     TG_CK(cudaStreamCreateWithFlags(&t->st, cudaStreamNonBlocking));
-    t->plan = make_plan(n);
+    t->plan = make_plan(n, precision == 0);
     std::vector<double> tw = plan_twiddles(t->plan);
     t->tw64.alloc(tw.size());
     TG_CK(cudaMemcpy(t->tw64.p, tw.data(), tw.size() * sizeof(double), cudaMemcpyHostToDevice));

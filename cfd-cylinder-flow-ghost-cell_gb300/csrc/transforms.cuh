@@ -64,8 +64,13 @@ struct FftPlan {
   unsigned ns_magic[20];  // ceil(2^32 / Ns) of stage s (Ns = product of the earlier radices; 0 when Ns = 1)
   int tw_off[20];         // offset of stage s's twiddles in the plan's twiddle table
   int tw_len;             // length (complex entries) of the plan's twiddle table
+  int fixed7;             // whether radix 7 has its own butterfly here: in FP64 handles.  The FP32 mode keeps the
+                          // direct sum, whose rounding its results hold
+  __host__ __device__ bool fixed_radix(int R) const {
+    return R == 2 || R == 3 || R == 4 || R == 5 || R == 8 || (R == 7 && fixed7);
+  }
 };
-// The plan's twiddle table: for a radix-R stage (R in 2, 3, 4, 5, 8) the Ns x (R-1) entries
+// The plan's twiddle table: for a radix-R stage with its own butterfly the Ns x (R-1) entries
 // W_M^(r k M/(Ns R)), k < Ns, r = 1..R-1, stored k-major so that one butterfly reads R-1
 // consecutive entries; for any other radix the full table W_M^t, t < M.
 
@@ -118,6 +123,26 @@ __device__ __forceinline__ void dft_small(cplx<T>* v, int dir) {
     v[4] = csub(q1, r1);
     v[2] = cadd(q2, r2);
     v[3] = csub(q2, r2);
+  } else if constexpr (R == 7) {
+    // cos and sin of 2 pi k / 7
+    const T c1 = (T)0.62348980185873353052500488400424, c2 = (T)-0.22252093395631440428890256449679,
+            c3 = (T)-0.90096886790241912623610231950745;
+    const T s1 = (T)dir * (T)0.78183148246802980870844452667406, s2 = (T)dir * (T)0.97492791218182360701813168299393,
+            s3 = (T)dir * (T)0.43388373911755812047576833284836;
+    const cplx<T> a = v[0];
+    const cplx<T> p1 = cadd(v[1], v[6]), m1 = csub(v[1], v[6]);
+    const cplx<T> p2 = cadd(v[2], v[5]), m2 = csub(v[2], v[5]);
+    const cplx<T> p3 = cadd(v[3], v[4]), m3 = csub(v[3], v[4]);
+    v[0] = {a.x + p1.x + p2.x + p3.x, a.y + p1.y + p2.y + p3.y};
+    auto pair = [&](int i, T ca, T cb, T cc, T sa, T sb, T sc) {
+      const cplx<T> q = {a.x + ca * p1.x + cb * p2.x + cc * p3.x, a.y + ca * p1.y + cb * p2.y + cc * p3.y};
+      const cplx<T> r = {-(sa * m1.y + sb * m2.y + sc * m3.y), sa * m1.x + sb * m2.x + sc * m3.x};
+      v[i] = cadd(q, r);
+      v[7 - i] = csub(q, r);
+    };
+    pair(1, c1, c2, c3, s1, s2, s3);
+    pair(2, c2, c3, c1, s2, -s3, -s1);
+    pair(3, c3, c1, c2, s3, -s1, s2);
   } else if constexpr (R == 8) {
     const T h = (T)0.70710678118654752440084436210485;
     // radix-2 over stride 4
@@ -235,6 +260,13 @@ __device__ cplx<T>* fft_run_dir(cplx<T>* a, cplx<T>* b, const FftPlan& plan, int
       case 4: stage_fixed<T, 4, DIR>(a, b, plan.M, nfft, Ns, mg, ts, G); break;
       case 5: stage_fixed<T, 5, DIR>(a, b, plan.M, nfft, Ns, mg, ts, G); break;
       case 8: stage_fixed<T, 8, DIR>(a, b, plan.M, nfft, Ns, mg, ts, G); break;
+      case 7:
+        if constexpr (sizeof(T) == 8)
+          if (plan.fixed7) {  // 13 FP64 instructions a point against 42 and an integer remainder a term (a periodic step at 700^2 797 -> 569 us)
+            stage_fixed<T, 7, DIR>(a, b, plan.M, nfft, Ns, mg, ts, G);
+            break;
+          }
+        [[fallthrough]];
       default: stage_generic<T>(a, b, plan.M, nfft, Ns, mg, R, ts, DIR, G); break;
     }
     G.sync();

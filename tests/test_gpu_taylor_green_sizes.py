@@ -11,7 +11,7 @@ from conftest import load_package
 pytestmark = pytest.mark.gpu
 
 
-@pytest.mark.parametrize('n', [8, 9, 15, 21, 26, 63, 64, 100, 129, 250])
+@pytest.mark.parametrize('n', [8, 9, 14, 15, 21, 26, 49, 63, 64, 100, 129, 196, 250])
 def test_sizes_match_oracle(n):
     """Six steps; the oracle solves the CN system with GMRES to rtol 1e-12, so fields agree to
     1e-11 of their maxima (velocity) and 1e-10 (pressure), as on the reference's own runs."""
