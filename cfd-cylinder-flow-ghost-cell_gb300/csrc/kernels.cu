@@ -1255,9 +1255,10 @@ struct TileGrid {
 
 // The FP32 mode converts as it fills the tiles (integer pipe; the halo points twice): a kernel that
 // wrote FP32 copies of the state first took 12 us of the 800x820 step, and its own launch.
-template <typename T, typename S>
 __global__ void __launch_bounds__(MTI * MTJ) k_momentum_tiled(CaseDev c, MomentumArgs a, const double* __restrict__ Us,
                                                               const double* __restrict__ Ps, Gate gate) {
+  using T = float;
+  using S = float;
   constexpr int W = TileGrid::W, H = TileGrid::H, WP = TileGrid::WP;
   __shared__ S suv[2 * H * W];
   __shared__ S sp[(MTJ + 1) * WP];
@@ -1287,8 +1288,7 @@ __global__ void __launch_bounds__(MTI * MTJ) k_momentum_tiled(CaseDev c, Momentu
     sp[e] = (j >= 0 && j < ny && i >= 0 && i < nx) ? cvt_to<S>(Ps[g.p(j, i)]) : (S)0;
   }
   __syncthreads();
-  constexpr bool F32 = sizeof(T) == 4;
-  const T dx = F32 ? (T)c.fdx : (T)c.dx, dy = F32 ? (T)c.fdy : (T)c.dy;
+  const T dx = c.fdx, dy = c.fdy;
   const T hh = (T)0.5;
   auto U = [&](int j, int i) -> T { return (T)suv[tg.u(j, i)]; };
   auto V = [&](int j, int i) -> T { return (T)suv[tg.v(j, i)]; };
@@ -1330,10 +1330,10 @@ __global__ void __launch_bounds__(MTI * MTJ) k_momentum_tiled(CaseDev c, Momentu
   __syncthreads();
   const int r = threadIdx.y, q = threadIdx.x;
   const int j = j0 + r, i = i0 + q;
-  const T idx2 = F32 ? (T)c.fidx2 : (T)c.idx2, idy2 = F32 ? (T)c.fidy2 : (T)c.idy2;
-  const T iarea = F32 ? (T)c.fiarea : (T)c.iarea, nu = F32 ? (T)c.fnu : (T)c.nu;
-  const T dt = F32 ? (T)a.dt32 : (T)a.dt;
-  const T alpha = F32 ? (T)a.alpha32 : (T)a.alpha;
+  const T idx2 = c.fidx2, idy2 = c.fidy2;
+  const T iarea = c.fiarea, nu = c.fnu;
+  const T dt = a.dt32;
+  const T alpha = a.alpha32;
   auto FX = [&](int jj, int ii) -> T { return fx[(jj - j0) * (MTI + 1) + (ii - i0)]; };
   auto FY = [&](int jj, int ii) -> T { return fy[(jj - j0) * (MTI + 1) + (ii - i0)]; };
   auto XU = [&](int jj, int ii) -> T { return xu[(jj - j0) * (MTI + 1) + (ii - i0)]; };
@@ -1352,7 +1352,7 @@ __global__ void __launch_bounds__(MTI * MTJ) k_momentum_tiled(CaseDev c, Momentu
     T lq, gp, now, off = 0;
     if (comp == 0) {
       lq = nu * lap_u<T>(suv, tg, j, i, idx2, idy2, true);
-      gp = grad_u<T>(sp, tg, j, i, F32 ? (T)c.fgx : (T)c.gx);
+      gp = grad_u<T>(sp, tg, j, i, c.fgx);
       T adv;
       if (i < nx) {
         adv = (XU(j, i + 1) - XU(j, i)) + (FX(j + 1, i) - FX(j, i));
@@ -1365,26 +1365,148 @@ __global__ void __launch_bounds__(MTI * MTJ) k_momentum_tiled(CaseDev c, Momentu
       if (i == 1) off = nu * (idx2 * (T)c.inlet[j]);
     } else {
       lq = nu * lap_v<T>(suv, tg, j, i, idx2, idy2);
-      gp = grad_v<T>(sp, tg, j, i, F32 ? (T)c.fgy : (T)c.gy);
+      gp = grad_v<T>(sp, tg, j, i, c.fgy);
       now = ((FY(j, i + 1) - FY(j, i)) + (YV(j + 1, i) - YV(j, i))) * iarea;
     }
     const T expl = ((T)1 + alpha) * now - alpha * cvt_to<T>(a.prev[t]);
     a.now[t] = cvt_to<double>(now);
-    if constexpr (sizeof(T) == 8)
-      a.out[t] = (qv + (double)(dt * (expl + (T)0.5 * lq - gp))) + (double)(((T)0.5 * dt) * off);
-    else
-      a.out[t] = qv + cvt_to<double>(dt * (expl + (T)0.5 * lq - gp) + ((T)0.5 * dt) * off);
+    a.out[t] = qv + cvt_to<double>(dt * (expl + (T)0.5 * lq - gp) + ((T)0.5 * dt) * off);
   }
 }
 
-// whether the AB2 right-hand side runs from shared-memory tiles (GHOSTMAC_MOMENTUM_TILED=0: the
-// one-thread-per-face kernel; read at every launch, which graph replays do not repeat)
-static bool momentum_tiled() {
-  const char* e = std::getenv("GHOSTMAC_MOMENTUM_TILED");
-  return !(e && e[0] == '0');
+// The FP64 form.  The FP64 pipe is the bound (1/64 of the FP32 rate), so every constant is formed on the host
+// and multiplied last: the tiles hold the unscaled products 4 C, (u + u)^2 and (v + v)^2 (seven
+// instructions a point), and a face away from the channel's edges takes thirteen.  At 800x820 94 us with the
+// fluxes scaled where they are formed (about 86 instructions a point), 67 now; other faces go the long way
+// through the same functions as k_momentum.
+struct MomentumC {
+  double ax, ay;       // -dy / (4 dx dy), -dx / (4 dx dy): of the products' differences along x and y
+  double c1, c2;       // dt (1 + alpha), dt alpha
+  double lx, ly, lc;   // dt nu / (2 dx^2), dt nu / (2 dy^2), 1 - 2 (lx + ly)
+  double gx, gy;       // dt / (rho dx), dt / (rho dy)
+};
+__global__ void __launch_bounds__(MTI * MTJ, 4) k_momentum_tiled64(CaseDev c, MomentumArgs a, MomentumC m, Gate gate) {
+  constexpr int W = TileGrid::W, H = TileGrid::H, WP = TileGrid::WP, WC = MTI + 1;
+  __shared__ double suv[2 * H * W];
+  __shared__ double sp[(MTJ + 1) * WP];
+  __shared__ double cc[(MTJ + 1) * WC];  // 4 C at corner (j0 + r, i0 + q), zero on the walls
+  __shared__ double xu[MTJ * WC];        // (u(j, ii - 1) + u(j, ii))^2 at (j0 + r, i0 + q)
+  __shared__ double yv[(MTJ + 1) * MTI]; // (v(jj - 1, i) + v(jj, i))^2 at (j0 + r, i0 + q)
+  if (!gate_open(gate)) return;
+  // a raised screen stops every kernel behind this one, whose outputs are scratch until the step ends
+  if (a.state_max && blockIdx.x + blockIdx.y + threadIdx.x + threadIdx.y == 0)
+    check_cfl(gate.ctl, a.state_max, a.state_max + 1, a.dt, c.dx, c.dy, a.screen, a.counter);
+  const int nx = c.nx, ny = c.ny;
+  const int j0 = blockIdx.y * MTJ, i0 = blockIdx.x * MTI;
+  const int tid = threadIdx.y * MTI + threadIdx.x;
+  const Grid g{nx, ny, c.usize};
+  const TileGrid tg{nx, ny, j0, i0};
+  for (int e = tid; e < H * W; e += MTI * MTJ) {
+    const int r = e / W, q = e - r * W;
+    const int j = j0 - 1 + r, i = i0 - 1 + q;
+    suv[e] = (j >= 0 && j < ny && i >= 0 && i <= nx) ? a.U[g.u(j, i)] : 0.0;
+    suv[H * W + e] = (j >= 0 && j <= ny && i >= 0 && i < nx) ? a.U[g.v(j, i)] : 0.0;
+  }
+  for (int e = tid; e < (MTJ + 1) * WP; e += MTI * MTJ) {
+    const int r = e / WP, q = e - r * WP;
+    const int j = j0 - 1 + r, i = i0 - 1 + q;
+    sp[e] = (j >= 0 && j < ny && i >= 0 && i < nx) ? a.P[g.p(j, i)] : 0.0;
+  }
+  __syncthreads();
+  auto U = [&](int j, int i) { return suv[tg.u(j, i)]; };
+  auto V = [&](int j, int i) { return suv[tg.v(j, i)]; };
+  for (int e = tid; e < (MTJ + 1) * WC; e += MTI * MTJ) {
+    const int r = e / WC, q = e - r * WC, jj = j0 + r, ii = i0 + q;
+    double x = 0.0;
+    if (jj >= 1 && jj <= ny - 1 && ii >= 1 && ii <= nx)
+      x = (V(jj, ii - 1) + V(jj, ii == nx ? nx - 1 : ii)) * (U(jj - 1, ii) + U(jj, ii));
+    cc[e] = x;
+  }
+  for (int e = tid; e < MTJ * WC; e += MTI * MTJ) {
+    const int r = e / WC, q = e - r * WC, j = j0 + r, ii = i0 + q;
+    double x = 0.0;
+    if (j < ny && ii >= 1 && ii <= nx) { x = U(j, ii - 1) + U(j, ii); x *= x; }
+    xu[e] = x;
+  }
+  for (int e = tid; e < (MTJ + 1) * MTI; e += MTI * MTJ) {
+    const int r = e / MTI, q = e - r * MTI, jj = j0 + r, i = i0 + q;
+    double y = 0.0;
+    if (jj >= 1 && jj <= ny && i < nx) { y = V(jj - 1, i) + V(jj, i); y *= y; }
+    yv[e] = y;
+  }
+  __syncthreads();
+  const int r = threadIdx.y, q = threadIdx.x;
+  const int j = j0 + r, i = i0 + q;
+  auto C = [&](int jj, int ii) { return cc[(jj - j0) * WC + (ii - i0)]; };
+  auto XU = [&](int jj, int ii) { return xu[(jj - j0) * WC + (ii - i0)]; };
+  auto YV = [&](int jj, int ii) { return yv[(jj - j0) * MTI + (ii - i0)]; };
+  const bool inner = j >= 1 && j < ny - 1 && i >= 2 && i < nx - 1;
+  for (int comp = 0; comp < 2; ++comp) {
+    if (comp == 0 ? (j >= ny || i > nx) : (j > ny || i >= nx)) continue;
+    const int64_t t = comp == 0 ? g.u(j, i) : g.v(j, i);
+    const uint8_t cls = comp == 0 ? c.cls_u[t] : c.cls_v[t - c.usize];
+    if (!(cls & CLS_ACTIVE)) {
+      a.now[t] = 0.0;
+      a.out[t] = 0.0;
+      continue;
+    }
+    if (inner) {
+      double now, ew, ns, x, dp;
+      if (comp == 0) {
+        now = fma(m.ax, XU(j, i + 1) - XU(j, i), m.ay * (C(j + 1, i) - C(j, i)));
+        x = U(j, i);
+        ew = U(j, i - 1) + U(j, i + 1);
+        ns = U(j - 1, i) + U(j + 1, i);
+        dp = (sp[tg.p(j, i)] - sp[tg.p(j, i - 1)]) * m.gx;
+      } else {
+        now = fma(m.ax, C(j, i + 1) - C(j, i), m.ay * (YV(j + 1, i) - YV(j, i)));
+        x = V(j, i);
+        ew = V(j, i - 1) + V(j, i + 1);
+        ns = V(j - 1, i) + V(j + 1, i);
+        dp = (sp[tg.p(j, i)] - sp[tg.p(j - 1, i)]) * m.gy;
+      }
+      a.now[t] = now;
+      a.out[t] = fma(m.lc, x, fma(m.lx, ew, fma(m.ly, ns, fma(m.c1, now, fma(-m.c2, a.prev[t], -dp)))));
+      continue;
+    }
+    const double qv = a.U[t];
+    double lq, gp, now, off = 0.0;
+    if (comp == 0) {
+      lq = c.nu * lap_u<double>(suv, tg, j, i, c.idx2, c.idy2, true);
+      gp = grad_u<double>(sp, tg, j, i, c.gx);
+      if (i < nx) {
+        now = m.ax * (XU(j, i + 1) - XU(j, i)) + m.ay * (C(j + 1, i) - C(j, i));
+      } else {  // half a volume with the outlet's flux u^2
+        const double uC = U(j, i);
+        now = 2.0 * (m.ax * (4.0 * (uC * uC) - XU(j, nx)) + (0.5 * m.ay) * (C(j + 1, nx) - C(j, nx)));
+      }
+      if (i == 1) off = c.nu * (c.idx2 * c.inlet[j]);
+    } else {
+      lq = c.nu * lap_v<double>(suv, tg, j, i, c.idx2, c.idy2);
+      gp = grad_v<double>(sp, tg, j, i, c.gy);
+      // the corner at the outlet is 2 v (u + u): uf v whole there
+      now = m.ax * (C(j, i + 1) - C(j, i)) + m.ay * (YV(j + 1, i) - YV(j, i));
+    }
+    const double expl = (1.0 + a.alpha) * now - a.alpha * a.prev[t];
+    a.now[t] = now;
+    a.out[t] = (qv + a.dt * (expl + 0.5 * lq - gp)) + (0.5 * a.dt) * off;
+  }
 }
+
 static dim3 momentum_tiles(const CaseDev& c) {
   return dim3((unsigned)((c.nx + 1 + MTI - 1) / MTI), (unsigned)((c.ny + 1 + MTJ - 1) / MTJ));
+}
+
+// Whether the AB2 right-hand side runs from shared-memory tiles (GHOSTMAC_MOMENTUM_TILED=0: the
+// one-thread-per-face kernel, 1: the tiles; read at every launch, which graph replays do not repeat).
+// FP64 grids of fewer tiles than SMs go by face: two barriers and three passes over the tile cost more than
+// the instructions they save where most SMs idle (forty steps at 96x48, 28 tiles: 7.65 ms with tiles, 7.53
+// by face; twenty at 400x200, 338 tiles: 5.55 and 5.62).
+static bool momentum_tiled(const CaseDev& c, bool f32) {
+  const char* e = std::getenv("GHOSTMAC_MOMENTUM_TILED");
+  if (e && e[0]) return e[0] != '0';
+  const dim3 t = momentum_tiles(c);
+  return f32 || t.x * t.y >= 152;
 }
 
 __global__ void k_shadow(const double* __restrict__ U, float* __restrict__ U32, int64_t nf,
@@ -1406,8 +1528,11 @@ void launch_shadow(const double* U, float* U32, int64_t n_f, const double* P, fl
 void launch_momentum(const CaseDev& c, const MomentumArgs& a, const Gate& gate, cudaStream_t st) {
   note_launch();
   kt_mark(3, st);
-  if (a.mode == 0 && momentum_tiled())
-    launch_pdl(k_momentum_tiled<double, double>, dim3(momentum_tiles(c)), dim3(dim3(MTI, MTJ)), 0, st, c, a, a.U, a.P, gate);
+  if (a.mode == 0 && momentum_tiled(c, false))
+    launch_pdl(k_momentum_tiled64, dim3(momentum_tiles(c)), dim3(dim3(MTI, MTJ)), 0, st, c, a,
+               MomentumC{-0.25 * c.dy * c.iarea, -0.25 * c.dx * c.iarea, a.dt * (1 + a.alpha), a.dt * a.alpha,
+                         0.5 * a.dt * c.nu * c.idx2, 0.5 * a.dt * c.nu * c.idy2, 1 - a.dt * c.nu * (c.idx2 + c.idy2),
+                         a.dt * c.gx, a.dt * c.gy}, gate);
   else
     launch_pdl(k_momentum<double, double>, dim3(blocks_for(c.usize + c.vsize)), dim3(TPB), 0, st, c, a, a.U, a.P, gate);
   // algorithmic bytes: U, prev, class map read; now, out written; P read
@@ -1417,12 +1542,12 @@ void launch_momentum_f32(const CaseDev& c, const MomentumArgs& a_in, const Gate&
   MomentumArgs a = a_in;
   a.dt32 = (float)a.dt;
   a.alpha32 = (float)a.alpha;
-  const bool tiled = momentum_tiled(), shadow = a.mode == 0 && !tiled;
+  const bool tiled = momentum_tiled(c, true), shadow = a.mode == 0 && !tiled;
   if (shadow) launch_shadow(a.U, a.U32, c.usize + c.vsize, a.P, a.P32, c.psize, gate, st);
   note_launch();
   kt_mark(3, st);
   if (a.mode == 0 && tiled)
-    launch_pdl(k_momentum_tiled<float, float>, dim3(momentum_tiles(c)), dim3(dim3(MTI, MTJ)), 0, st, c, a, a.U, a.P, gate);
+    launch_pdl(k_momentum_tiled, dim3(momentum_tiles(c)), dim3(dim3(MTI, MTJ)), 0, st, c, a, a.U, a.P, gate);
   else if (shadow)
     launch_pdl(k_momentum<float, float>, dim3(blocks_for(c.usize + c.vsize)), dim3(TPB), 0, st, c, a, a.U32, a.P32, gate);
   else
