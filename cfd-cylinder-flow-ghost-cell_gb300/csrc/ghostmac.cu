@@ -417,7 +417,6 @@ void autotune_shapes(gm_handle* h, RectDev& rd, int kind, bool fp32) {
   TransformTables& tt = fp32 ? rd.tt32 : rd.tt;
   const RectView& v = rd.view;
   cudaStream_t st = h->st;
-  const size_t per = std::max(xpass_smem_per_group(tt.tx_fwd, v.cols, fp32), xpass_smem_per_group(tt.tx_inv, v.cols, fp32));
   const size_t tabs = std::max(xpass_smem_tables(tt.tx_fwd, v.cols, tt.plan_x.tw_len, fp32),
                                xpass_smem_tables(tt.tx_inv, v.cols, tt.plan_x.tw_len, fp32));
   double* field = kind == 0 ? h->ptmp.p : h->ftmp.p;
@@ -448,9 +447,18 @@ void autotune_shapes(gm_handle* h, RectDev& rd, int kind, bool fp32) {
   };
   // x pass
   float best = 1e30f;
-  int bt = 32, bg = 1;
+  int bt = 32, bg = 1, b2 = 0;
+  // (FP64 type-IV passes of at least four lines an SM also with two lines a group, whose butterflies fill the
+  // warps of a stage better: 38 instead of 43 us at 800x820; fewer lines split worse over the SMs, and the
+  // timing itself costs set-up.  The values are the same.)
+  const int most = !fp32 && !r2r_paired(tt.tx_fwd) && v.rows >= 4 * 152 ? 1 : 0;
+  for (int two = 0; two <= most; ++two)
   for (int gt : {64, 128, 256, 512}) {
+    if (two && gt == 64) continue;
+    const size_t per = std::max(xpass_smem_per_group(tt.tx_fwd, v.cols, fp32, two), xpass_smem_per_group(tt.tx_inv, v.cols, fp32, two));
+    tt.xg_two = two;
     for (int gp : {1, 2, 4}) {
+      if (two && gp > 1) continue;
       if (gt * gp > 512 || tabs + per * gp > h->smem_optin) continue;
       tt.xg_threads = gt;
       tt.xg_pb = gp;
@@ -468,13 +476,14 @@ void autotune_shapes(gm_handle* h, RectDev& rd, int kind, bool fp32) {
                                                v.pitch, nullptr, nullptr, none64, open, st);
         }
       });
-      if (ms < best) { best = ms; bt = gt; bg = gp; }
+      if (ms < best) { best = ms; bt = gt; bg = gp; b2 = two; }
     }
   }
   if (best >= 1e30f) throw CudaError("row transforms do not fit the shared memory");
+  tt.xg_two = b2;
   tt.xg_threads = bt;
   tt.xg_pb = bg;
-  tt.smem_x = tabs + per * bg;
+  tt.smem_x = tabs + bg * std::max(xpass_smem_per_group(tt.tx_fwd, v.cols, fp32, b2), xpass_smem_per_group(tt.tx_inv, v.cols, fp32, b2));
   // column solve: L columns per block and the block's threads (at least L x P: one per chunk in
   // the solve phases; more threads only shorten the load and store phases)
   best = 1e30f;
@@ -507,9 +516,11 @@ void autotune_shapes(gm_handle* h, RectDev& rd, int kind, bool fp32) {
   // computes the same values)
   if (const char* e = std::getenv("GHOSTMAC_SHAPES")) {
     int gt = 0, gp = 0, L = 0;
+    const size_t per = std::max(xpass_smem_per_group(tt.tx_fwd, v.cols, fp32, 0), xpass_smem_per_group(tt.tx_inv, v.cols, fp32, 0));
     if (std::sscanf(e, "%d,%d,%d", &gt, &gp, &L) == 3 && gt >= 32 && gt % 32 == 0 && gp >= 1 && gt * gp <= 512 &&
         tabs + per * gp <= h->smem_optin && (L == 2 || L == 4 || L == 8 || L == 16) &&
         ((L * tt.ych.P + 31) / 32) * 32 <= 1024 && ysolve_smem(v.rows, L, fp32) <= h->smem_optin) {
+      tt.xg_two = 0;
       tt.xg_threads = gt;
       tt.xg_pb = gp;
       tt.smem_x = tabs + per * gp;
@@ -525,13 +536,14 @@ void autotune_shapes(gm_handle* h, RectDev& rd, int kind, bool fp32) {
 bool apply_shape(gm_handle* h, RectDev& rd, bool fp32, int gt, int gp, int L) {
   TransformTables& tt = fp32 ? rd.tt32 : rd.tt;
   const RectView& v = rd.view;
-  const size_t per = std::max(xpass_smem_per_group(tt.tx_fwd, v.cols, fp32), xpass_smem_per_group(tt.tx_inv, v.cols, fp32));
+  const size_t per = std::max(xpass_smem_per_group(tt.tx_fwd, v.cols, fp32, 0), xpass_smem_per_group(tt.tx_inv, v.cols, fp32, 0));
   const size_t tabs = std::max(xpass_smem_tables(tt.tx_fwd, v.cols, tt.plan_x.tw_len, fp32),
                                xpass_smem_tables(tt.tx_inv, v.cols, tt.plan_x.tw_len, fp32));
   const int thr = ((L * tt.ych.P + 31) / 32) * 32;
   if (!(gt >= 32 && gt % 32 == 0 && gp >= 1 && gt * gp <= 512 && tabs + per * gp <= h->smem_optin &&
         (L == 2 || L == 4 || L == 8 || L == 16) && thr <= 1024 && ysolve_smem(v.rows, L, fp32) <= h->smem_optin))
     return false;
+  tt.xg_two = 0;
   tt.xg_threads = gt;
   tt.xg_pb = gp;
   tt.smem_x = tabs + per * gp;
@@ -3257,6 +3269,7 @@ void batch_groups(gm_batch* b) {
     }
   b->groups = std::move(gs);
   auto copy_shape = [](TransformTables& d, const TransformTables& s) {
+    d.xg_two = s.xg_two;
     d.xg_threads = s.xg_threads;
     d.xg_pb = s.xg_pb;
     d.smem_x = s.smem_x;

@@ -218,14 +218,14 @@ void ktimer_read(int cls, double* total_ms, long long* count, double* bytes) {
 // ---------------------------------------------------------------------------
 // Row transforms.  A group of `gthreads` threads (one warp, or whole warps on a named
 // barrier) transforms one line group -- two paired lines for the Makhoul and DST-I
-// transforms, one line for the type-IV transforms -- and a block holds `gpb` groups.
+// transforms, one line or two (TransformTables::xg_two) for the type-IV transforms -- and a block holds
+// `gpb` groups.
 // Rows r0 .. r0+nr-1 are transformed.  Masked load with the optional spectral correction
 // of the boundary term (YCorr); masked store with the optional epilogue out = add + v.
 // shared memory of one line group: the two FFT buffers (the real results go to the buffer the
 // FFT does not end in)
 template <typename T>
-__host__ __device__ inline size_t xpass_group_smem(int type, int n) {
-  const int lpw = r2r_paired(type) ? 2 : 1;
+__host__ __device__ inline size_t xpass_group_smem(int type, int n, int lpw) {
   return 2 * (size_t)r2r_buffer_elems(type, n, lpw) * sizeof(cplx<T>);
 }
 // lengths (complex entries) of the plan's twiddles, the pre- and the post-twiddles of a transform
@@ -240,8 +240,10 @@ __host__ __device__ inline size_t xpass_tw_bytes(int type, int n, int plan_tw) {
   return ((size_t)(xpass_tw_len(type, n, 0, plan_tw) + xpass_tw_len(type, n, 1, plan_tw) +
                    xpass_tw_len(type, n, 2, plan_tw)) * sizeof(cplx<T>) + 15) / 16 * 16;
 }
-size_t xpass_smem_per_group(int type, int n, bool fp32) {
-  return fp32 ? xpass_group_smem<float>(type, n) : xpass_group_smem<double>(type, n);
+int xpass_lines(int type, int two) { return r2r_paired(type) || two ? 2 : 1; }
+size_t xpass_smem_per_group(int type, int n, bool fp32, int two) {
+  const int lpw = xpass_lines(type, two);
+  return fp32 ? xpass_group_smem<float>(type, n, lpw) : xpass_group_smem<double>(type, n, lpw);
 }
 size_t xpass_smem_tables(int type, int n, int plan_tw, bool fp32) {
   return fp32 ? xpass_tw_bytes<float>(type, n, plan_tw) : xpass_tw_bytes<double>(type, n, plan_tw);
@@ -281,19 +283,19 @@ __device__ __forceinline__ R2RTables<T> xpass_stage_tables(int type, int n, cons
 // The line groups of (virtual) block bi: group grp of the block transforms lines
 // (bi * gpb + grp) * lpw ... of rows r0 .. r0+nr-1.  Groups past the end return at once; every
 // group synchronises on its own named barrier only, so a block may run this for several bi in turn.
-template <typename T, typename TI, typename TO>
+template <typename T, typename TI, typename TO, bool TWO>
 __device__ __forceinline__ void xpass_block(int bi, int n, int r0, int nr, int type, const FftPlan& plan,
                                             const R2RTables<T>& ts, const TI* __restrict__ in, int64_t ibase,
                                             int64_t ipitch, const uint8_t* __restrict__ icls, TO* __restrict__ out,
                                             int64_t obase, int64_t opitch, const uint8_t* __restrict__ ocls,
                                             const double* __restrict__ add, const YCorr<T>& corr, int gthreads,
                                             int gpb, unsigned char* smem_raw) {
+  const int lpw = r2r_paired(type) || TWO ? 2 : 1;
   const int grp = threadIdx.x / gthreads, tid = threadIdx.x - grp * gthreads;
-  const int lpw = r2r_paired(type) ? 2 : 1;
   const int l0 = (bi * gpb + grp) * lpw;
   if (grp >= gpb || l0 >= nr) return;
   const int nl = min(lpw, nr - l0);
-  unsigned char* mine = smem_raw + xpass_tw_bytes<T>(type, n, plan.tw_len) + (size_t)grp * xpass_group_smem<T>(type, n);
+  unsigned char* mine = smem_raw + xpass_tw_bytes<T>(type, n, plan.tw_len) + (size_t)grp * xpass_group_smem<T>(type, n, lpw);
   cplx<T>* a = reinterpret_cast<cplx<T>*>(mine);
   cplx<T>* b = a + r2r_buffer_elems(type, n, lpw);
   const Grp G{tid, gthreads, grp + 1};
@@ -331,7 +333,7 @@ __device__ __forceinline__ void xpass_block(int bi, int n, int r0, int nr, int t
     const T cv = cb ? (cf ? cf[e] * cb[e] : cb[e]) : (T)0;
     return ((mk & CLS_ACTIVE) ? cvt_to<T>(v) : (T)0) - cv;
   };
-  const T* stage = r2r_lines<T>(type, n, nl, a, b, plan, ts, G, x);
+  const T* stage = r2r_lines<T, TWO>(type, n, nl, a, b, plan, ts, G, x);
   for (int l = 0; l < nl; ++l) {
     const int64_t row = obase + (int64_t)(r0 + l0 + l) * opitch;
     for (int e0 = tid; e0 < n; e0 += XB * gthreads) {
@@ -361,7 +363,7 @@ __device__ __forceinline__ void xpass_block(int bi, int n, int r0, int nr, int t
   }
 }
 
-template <typename T, typename TI, typename TO>
+template <typename T, typename TI, typename TO, bool TWO>
 __global__ void k_xpass(int n, int r0, int nr, int type, FftPlan plan, R2RTables<T> tb, const TI* __restrict__ in,
                         int64_t ibase, int64_t ipitch, const uint8_t* __restrict__ icls, TO* __restrict__ out,
                         int64_t obase, int64_t opitch, const uint8_t* __restrict__ ocls, const double* __restrict__ add,
@@ -369,7 +371,7 @@ __global__ void k_xpass(int n, int r0, int nr, int type, FftPlan plan, R2RTables
   extern __shared__ __align__(16) unsigned char smem_raw[];
   const R2RTables<T> ts = xpass_stage_tables<T>(type, n, plan, tb, smem_raw);
   if (!gate_open(gate)) return;
-  xpass_block<T, TI, TO>(blockIdx.x, n, r0, nr, type, plan, ts, in, ibase, ipitch, icls, out, obase, opitch, ocls,
+  xpass_block<T, TI, TO, TWO>(blockIdx.x, n, r0, nr, type, plan, ts, in, ibase, ipitch, icls, out, obase, opitch, ocls,
                          add, corr, gthreads, gpb, smem_raw);
 }
 
@@ -382,14 +384,16 @@ void launch_xpass(const TransformTables& tt, bool inverse, int r0, int nr, const
   const int type = inverse ? tt.tx_inv : tt.tx_fwd;
   R2RTables<T> tb{(const C*)tt.Wx, (const C*)(inverse ? tt.prex_inv : tt.prex),
                   (const C*)(inverse ? tt.postx_inv : tt.postx)};
-  const int lpw = r2r_paired(type) ? 2 : 1;
+  const int lpw = xpass_lines(type, tt.xg_two);
   const int per_block = tt.xg_pb * lpw;
   const unsigned grid = (unsigned)((nr + per_block - 1) / per_block);
   note_launch();
   kt_mark(1, st);
-  launch_pdl(k_xpass<T, TI, TO>, dim3(grid), dim3(tt.xg_threads * tt.xg_pb), tt.smem_x, st, tt.n, r0, nr, type,
-             tt.plan_x, tb, in, ibase, ipitch, icls, out, obase, opitch, ocls, add, corr, tt.xg_threads, tt.xg_pb,
-             gate);
+  auto* kernel = k_xpass<T, TI, TO, false>;
+  if constexpr (sizeof(T) == 8)
+    if (lpw == 2 && !r2r_paired(type)) kernel = k_xpass<T, TI, TO, true>;
+  launch_pdl(kernel, dim3(grid), dim3(tt.xg_threads * tt.xg_pb), tt.smem_x, st, tt.n, r0, nr, type, tt.plan_x, tb, in, ibase,
+             ipitch, icls, out, obase, opitch, ocls, add, corr, tt.xg_threads, tt.xg_pb, gate);
   // algorithmic bytes: one read and one write per point, class maps, the added field and the
   // correction band (tables of the decay factors once per point)
   kt_mark(1, st, (double)nr * tt.n * (sizeof(TI) + sizeof(TO) + (icls ? 1 : 0) + (ocls ? 1 : 0) + (add ? 8 : 0) +
@@ -638,10 +642,11 @@ static int allow_dynamic_smem(K kernel, int optin) {
 }
 int configure_kernels(int smem_optin) {
   int d = smem_optin;
-  d = std::min(d, allow_dynamic_smem(k_xpass<double, double, double>, smem_optin));
-  d = std::min(d, allow_dynamic_smem(k_xpass<float, double, float>, smem_optin));
-  d = std::min(d, allow_dynamic_smem(k_xpass<float, float, float>, smem_optin));
-  d = std::min(d, allow_dynamic_smem(k_xpass<float, float, double>, smem_optin));
+  d = std::min(d, allow_dynamic_smem(k_xpass<double, double, double, false>, smem_optin));
+  d = std::min(d, allow_dynamic_smem(k_xpass<double, double, double, true>, smem_optin));
+  d = std::min(d, allow_dynamic_smem(k_xpass<float, double, float, false>, smem_optin));
+  d = std::min(d, allow_dynamic_smem(k_xpass<float, float, float, false>, smem_optin));
+  d = std::min(d, allow_dynamic_smem(k_xpass<float, float, double, false>, smem_optin));
   d = std::min(d, allow_dynamic_smem(k_ysolve<double, 2>, smem_optin));
   d = std::min(d, allow_dynamic_smem(k_ysolve<double, 4>, smem_optin));
   d = std::min(d, allow_dynamic_smem(k_ysolve<double, 8>, smem_optin));
@@ -3319,7 +3324,7 @@ __global__ void k_xpass_multi(const __grid_constant__ ArgPack<XpassArgs<T, TI, T
   extern __shared__ __align__(16) unsigned char smem_raw[];
   const R2RTables<T> ts = xpass_stage_tables<T>(a.type, a.n, a.plan, a.tb, smem_raw);
   if (!gate_open(a.gate)) return;
-  xpass_block<T, TI, TO>(blockIdx.x, a.n, a.r0, a.nr, a.type, a.plan, ts, a.in, a.ibase, a.ipitch, a.icls, a.out,
+  xpass_block<T, TI, TO, false>(blockIdx.x, a.n, a.r0, a.nr, a.type, a.plan, ts, a.in, a.ibase, a.ipitch, a.icls, a.out,
                          a.obase, a.opitch, a.ocls, a.add, a.corr, a.gthreads, a.gpb, smem_raw);
 }
 template <typename T, int L>
@@ -3413,7 +3418,7 @@ XpassArgs<T, TI, TO> xpass_args(const TransformTables& tt, bool inverse, int r0,
   a.gthreads = tt.xg_threads;
   a.gpb = tt.xg_pb;
   a.gate = gate;
-  const int per_block = tt.xg_pb * (r2r_paired(a.type) ? 2 : 1);
+  const int per_block = tt.xg_pb * xpass_lines(a.type, 0);
   a.nblk = (nr + per_block - 1) / per_block;
   return a;
 }

@@ -263,6 +263,7 @@ struct TransformTables {      // device tables of one rectangle kind (T = double
   const void* phi;            // bj0 x cols decay factors below the band
   const void* psi;            // (rows-1-bj1) x cols decay factors above the band
   // launch shapes (picked by timing candidates at set-up)
+  int xg_two = 0;             // x pass: a type-IV line group holds two lines (their butterflies in one loop)
   int xg_threads, xg_pb;      // x pass: threads per line group, groups per block
   size_t smem_x;
   int lpb_y, threads_y;       // y solve: columns per block, threads
@@ -397,7 +398,7 @@ void ktimer_enable(int on);
 void ktimer_collect();
 bool ktimer_active();
 void ktimer_read(int cls, double* total_ms, long long* count, double* bytes);
-size_t xpass_smem_per_group(int type, int n, bool fp32);
+size_t xpass_smem_per_group(int type, int n, bool fp32, int two);
 size_t xpass_smem_tables(int type, int n, int plan_tw, bool fp32);  // twiddle tables staged once per block
 size_t ysolve_smem(int rows, int lpb, bool fp32);
 // Row transforms of rows r0..r0+nr-1: forward (tx_fwd) or inverse (tx_inv).  Element (r, e)

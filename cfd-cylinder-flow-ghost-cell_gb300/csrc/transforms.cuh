@@ -14,6 +14,8 @@
 #include <cuda_runtime.h>
 #include <stdint.h>
 
+#include <type_traits>
+
 namespace gmk {
 
 enum R2R : int { DCT2 = 0, DCT3 = 1, DCT4 = 2, DST1 = 3, DST2 = 4, DST3 = 5, DST4 = 6 };
@@ -217,6 +219,39 @@ __device__ __forceinline__ void stage_fixed(const cplx<T>* __restrict__ in, cplx
   }
 }
 
+// The same stage over two transforms at once (FP64): their butterflies share one loop and fill the warps
+// better, as an FP64 warp instruction takes its 16 cycles whatever lanes it has.  (Compiled into kernels of its own: one loop for
+// both cases, or both loops in a kernel, cost single transforms 1 % of a 96x48 step.)
+template <typename T, int R, int DIR>
+__device__ __forceinline__ void stage_two(const cplx<T>* __restrict__ in, cplx<T>* __restrict__ out, int M, int nfft, int Ns,
+                                          unsigned magic, const cplx<T>* __restrict__ tw, const Grp& G) {
+  const int MR = M / R;
+  for (int t = G.tid; t < nfft * MR; t += G.n) {
+    const int f = t >= MR ? 1 : 0, j = t - f * MR;
+    const cplx<T>* src = in + f * M;
+    cplx<T>* dst = out + f * M;
+    const int jq = div_ns(j, Ns, magic);
+    const int k = j - jq * Ns;
+    const cplx<T>* w = tw + k * (R - 1);
+    cplx<T> v[R];
+    v[0] = src[j];
+#pragma unroll
+    for (int r = 1; r < R; ++r) v[r] = src[j + r * MR];
+    if (Ns > 1) {
+#pragma unroll
+      for (int r = 1; r < R; ++r) {
+        cplx<T> ww = w[r - 1];
+        if (DIR > 0) ww.y = -ww.y;
+        v[r] = cmul(v[r], ww);
+      }
+    }
+    dft_small<T, R>(v, DIR);
+    const int base = jq * Ns * R + k;
+#pragma unroll
+    for (int q = 0; q < R; ++q) dst[base + q * Ns] = v[q];
+  }
+}
+
 // Generic odd radix (any R up to 64): direct R-point DFT per output; W is the full table.
 template <typename T>
 __device__ void stage_generic(const cplx<T>* __restrict__ in, cplx<T>* __restrict__ out, int M, int nfft, int Ns,
@@ -246,7 +281,7 @@ __device__ void stage_generic(const cplx<T>* __restrict__ in, cplx<T>* __restric
   }
 }
 
-template <typename T, int DIR>
+template <typename T, int DIR, bool TWO>
 __device__ cplx<T>* fft_run_dir(cplx<T>* a, cplx<T>* b, const FftPlan& plan, int nfft, const cplx<T>* tw,
                                const Grp& G) {
   int Ns = 1;
@@ -254,16 +289,21 @@ __device__ cplx<T>* fft_run_dir(cplx<T>* a, cplx<T>* b, const FftPlan& plan, int
     const int R = plan.radix[s];
     const unsigned mg = plan.ns_magic[s];
     const cplx<T>* ts = tw + plan.tw_off[s];
+    auto fixed = [&](auto r) {
+      constexpr int RR = decltype(r)::value;
+      if constexpr (TWO) stage_two<T, RR, DIR>(a, b, plan.M, nfft, Ns, mg, ts, G);
+      else stage_fixed<T, RR, DIR>(a, b, plan.M, nfft, Ns, mg, ts, G);
+    };
     switch (R) {
-      case 2: stage_fixed<T, 2, DIR>(a, b, plan.M, nfft, Ns, mg, ts, G); break;
-      case 3: stage_fixed<T, 3, DIR>(a, b, plan.M, nfft, Ns, mg, ts, G); break;
-      case 4: stage_fixed<T, 4, DIR>(a, b, plan.M, nfft, Ns, mg, ts, G); break;
-      case 5: stage_fixed<T, 5, DIR>(a, b, plan.M, nfft, Ns, mg, ts, G); break;
-      case 8: stage_fixed<T, 8, DIR>(a, b, plan.M, nfft, Ns, mg, ts, G); break;
+      case 2: fixed(std::integral_constant<int, 2>{}); break;
+      case 3: fixed(std::integral_constant<int, 3>{}); break;
+      case 4: fixed(std::integral_constant<int, 4>{}); break;
+      case 5: fixed(std::integral_constant<int, 5>{}); break;
+      case 8: fixed(std::integral_constant<int, 8>{}); break;
       case 7:
         if constexpr (sizeof(T) == 8)
           if (plan.fixed7) {  // 13 FP64 instructions a point against 42 and an integer remainder a term (a periodic step at 700^2 797 -> 569 us)
-            stage_fixed<T, 7, DIR>(a, b, plan.M, nfft, Ns, mg, ts, G);
+            fixed(std::integral_constant<int, 7>{});
             break;
           }
         [[fallthrough]];
@@ -280,10 +320,11 @@ __device__ cplx<T>* fft_run_dir(cplx<T>* a, cplx<T>* b, const FftPlan& plan, int
 
 // Runs the FFT on nfft transforms held in a (length M each); the result is in
 // the returned buffer (a or b).  dir = -1 forward, +1 inverse (unnormalised).
-template <typename T>
+// TWO: at most two transforms, in one loop.
+template <typename T, bool TWO = false>
 __device__ cplx<T>* fft_run(cplx<T>* a, cplx<T>* b, const FftPlan& plan, int nfft, const cplx<T>* tw, int dir,
                            const Grp& G) {
-  return dir > 0 ? fft_run_dir<T, 1>(a, b, plan, nfft, tw, G) : fft_run_dir<T, -1>(a, b, plan, nfft, tw, G);
+  return dir > 0 ? fft_run_dir<T, 1, TWO>(a, b, plan, nfft, tw, G) : fft_run_dir<T, -1, TWO>(a, b, plan, nfft, tw, G);
 }
 
 // Twiddle tables of one r2r transform of length n (T precision), device pointers.
@@ -447,13 +488,13 @@ __host__ __device__ inline int r2r_nfft(int type, int nl) { return r2r_paired(ty
 // Full r2r transform of nl lines read through x(l, i) (see r2r_pre), through the FFT buffers
 // a/b; the real results are left line-major (l * n + i) in the buffer the FFT does not end in,
 // which is returned.
-template <typename T, typename X>
+template <typename T, bool TWO, typename X>
 __device__ __forceinline__ T* r2r_lines(int type, int n, int nl, cplx<T>* a, cplx<T>* b, const FftPlan& plan,
                                         const R2RTables<T>& tb, const Grp& G, X&& x) {
   const int fam = r2r_family(type);
   r2r_pre<T>(type, n, nl, a, tb, G, x);
   G.sync();
-  cplx<T>* res = fft_run<T>(a, b, plan, r2r_nfft(type, nl), tb.W, fam == 1 ? +1 : -1, G);
+  cplx<T>* res = fft_run<T, TWO>(a, b, plan, r2r_nfft(type, nl), tb.W, fam == 1 ? +1 : -1, G);
   T* out = reinterpret_cast<T*>(res == a ? b : a);
   r2r_post<T>(type, res, n, nl, out, tb, G);
   G.sync();
