@@ -14,8 +14,9 @@
 // A Fourier solve is three kernels: rows forward, columns (forward, symbol, inverse, in place),
 // rows inverse.  In FP64 the real fields share complex transforms: the two velocity components as
 // u + i v (the CN operator is real and the same for both), two rows of the divergence for the
-// pressure, whose spectrum then has n / 2 + 1 columns.  An FP64 step decides nothing on the
-// host: its launches are queued for all steps and the failed-gate word is read once.
+// pressure, whose spectrum then has n / 2 + 1 columns.  A step decides nothing on the host: the
+// launches of up to 64 steps are queued, the FP32 mode's with a held number of refinement sweeps
+// gated on the device, and the failed-gate word is read once.
 #include <cuda_runtime.h>
 
 #include <algorithm>
