@@ -435,8 +435,9 @@ __device__ __forceinline__ void ysolve_body(int n /*rows*/, int cols, const YChu
   const int ns = n | 1;                                  // odd stride between the columns
   T* col = reinterpret_cast<T*>(smem_raw);              // L x ns values
   T* piv = col + (size_t)L * ns;                         // L x ns reciprocal pivots
-  T* sl = piv + (size_t)L * ns;                          // L x ns left spikes (t1)
-  T* sr = sl + (size_t)L * ns;                           // L x ns right spikes (t2)
+  T* s1 = piv + (size_t)L * ns;                          // spikes at the interface rows: L x YCHUNK_MAX left (t1),
+  T* s2 = s1 + L * YCHUNK_MAX;                           // right (t2)
+  uint8_t* chunk_of = reinterpret_cast<uint8_t*>(s2 + L * YCHUNK_MAX);  // of each row; 255 at an interface row
   const int c0 = bid * L;
   const int P = ch.P;
   const int l = threadIdx.x & (L - 1);                   // column of this thread
@@ -444,35 +445,39 @@ __device__ __forceinline__ void ysolve_body(int n /*rows*/, int cols, const YChu
   const int rstep = blockDim.x / L;
   const bool colok = c0 + l < cols;
   const int64_t cc = c0 + l;
-  // load the column values and all three tables in one phase: 4 x 4 loads in flight per thread,
-  // so the solve phases below wait on shared memory only
-  for (int e0 = rsub; e0 < n; e0 += 4 * rstep) {
-    T sv[4], pvv[4], v1[4], v2[4];
+  // load the column values and pivots in one phase, 2 x 8 loads in flight per thread, so that the
+  // recurrences wait on shared memory only.  The spikes of the inner rows are read where they are used,
+  // once, in the store phase: staged here as well they doubled a block's shared memory, and at 800x820
+  // eight FP64 columns were one block an SM whose loads, recurrences and stores did not overlap
+  // (35 us a solve, now 31; the 400x200 step 277 -> 271 us)
+  for (int e0 = rsub; e0 < n; e0 += 8 * rstep) {
+    T sv[8], pvv[8];
 #pragma unroll
-    for (int u = 0; u < 4; ++u) {
+    for (int u = 0; u < 8; ++u) {
       const int e = e0 + u * rstep;
       if (colok && e < n) {
         const int64_t o = (int64_t)e * cols + cc;
         sv[u] = S[o];
         pvv[u] = t0[o];
-        if (P > 1) {
-          v1[u] = t1[o];
-          v2[u] = t2[o];
-        }
       }
     }
 #pragma unroll
-    for (int u = 0; u < 4; ++u) {
+    for (int u = 0; u < 8; ++u) {
       const int e = e0 + u * rstep;
       if (colok && e < n) {
         col[l * ns + e] = sv[u] * scale;
         piv[l * ns + e] = pvv[u];
-        if (P > 1) {
-          sl[l * ns + e] = v1[u];
-          sr[l * ns + e] = v2[u];
-        }
       }
     }
+  }
+  if (colok && rsub < P - 1) {
+    const int64_t o = (int64_t)(ch.end[rsub] + 1) * cols + cc;
+    s1[l * YCHUNK_MAX + rsub] = t1[o];
+    s2[l * YCHUNK_MAX + rsub] = t2[o];
+  }
+  if (l == 0 && rsub < P) {
+    for (int j = ch.start[rsub]; j <= ch.end[rsub]; ++j) chunk_of[j] = (uint8_t)rsub;
+    if (rsub < P - 1) chunk_of[ch.end[rsub] + 1] = 255;
   }
   __syncthreads();
   const int p = rsub;
@@ -481,8 +486,6 @@ __device__ __forceinline__ void ysolve_body(int n /*rows*/, int cols, const YChu
   if (work) { a = ch.start[p]; b = ch.end[p]; }
   T* x = col + l * ns;
   const T* pv = piv + l * ns;
-  const T* s1 = sl + l * ns;
-  const T* s2 = sr + l * ns;
   // phase 1: chunk-local Thomas
   if (work) {
     T prev = 0;
@@ -504,27 +507,44 @@ __device__ __forceinline__ void ysolve_body(int n /*rows*/, int cols, const YChu
     for (int q = 0; q < P - 1; ++q) {
       const int e = ch.end[q] + 1;
       const T rhs = x[e] - gamma * x[e - 1] - gamma * x[e + 1];
-      z = (rhs - s1[e] * z) * pv[e];
+      z = (rhs - s1[l * YCHUNK_MAX + q] * z) * pv[e];
       x[e] = z;
     }
     T y = 0;
     for (int q = P - 2; q >= 0; --q) {
       const int e = ch.end[q] + 1;
-      y = x[e] - s2[e] * y;
+      y = x[e] - s2[l * YCHUNK_MAX + q] * y;
       x[e] = y;
     }
   }
   __syncthreads();
-  // phase 3: spike corrections of the inner rows
-  if (work && P > 1) {
-    const T yl = p > 0 ? x[ch.end[p - 1] + 1] : (T)0;
-    const T yr = p < P - 1 ? x[b + 1] : (T)0;
-    for (int j = a; j <= b; ++j) x[j] = x[j] - yl * s1[j] - yr * s2[j];
+  // phase 3: spike corrections of the inner rows, on the way out
+  if (!colok) return;
+  for (int e0 = rsub; e0 < n; e0 += 4 * rstep) {
+    T v1[4], v2[4];
+#pragma unroll
+    for (int u = 0; u < 4; ++u) {
+      const int e = e0 + u * rstep;
+      if (P > 1 && e < n) {
+        const int64_t o = (int64_t)e * cols + cc;
+        v1[u] = t1[o];
+        v2[u] = t2[o];
+      }
+    }
+#pragma unroll
+    for (int u = 0; u < 4; ++u) {
+      const int e = e0 + u * rstep;
+      if (e >= n) continue;
+      T v = x[e];
+      const int q = P > 1 ? chunk_of[e] : 255;
+      if (q != 255) {
+        const T yl = q > 0 ? x[ch.end[q - 1] + 1] : (T)0;
+        const T yr = q < P - 1 ? x[ch.end[q] + 1] : (T)0;
+        v = v - yl * v1[u] - yr * v2[u];
+      }
+      S[(int64_t)e * cols + cc] = v;
+    }
   }
-  __syncthreads();
-  T* s_out = S + cc;
-  if (colok)
-    for (int e = rsub; e < n; e += rstep) s_out[(int64_t)e * cols] = col[l * ns + e];
 }
 template <typename T, int L>
 __global__ void k_ysolve(int n /*rows*/, int cols, YChunks ch, T gamma, T scale, const T* __restrict__ t0,
@@ -534,7 +554,8 @@ __global__ void k_ysolve(int n /*rows*/, int cols, YChunks ch, T gamma, T scale,
 }
 size_t ysolve_smem(int rows, int lpb, bool fp32) {
   const size_t esz = fp32 ? 4 : 8;
-  return (size_t)lpb * (rows | 1) * 4 * esz;  // values, pivots, left and right spikes
+  // values and pivots, the interface rows' spikes, the rows' chunks
+  return (size_t)lpb * ((rows | 1) * 2 + 2 * YCHUNK_MAX) * esz + (size_t)(rows + 15) / 16 * 16;
 }
 
 template <typename T>
