@@ -247,6 +247,7 @@ struct gm_handle {
   // the step.  FP64 starts with none, the FP32 mode with the one that it always needs.
   bool looped = false;  // the solves of this capture are the loops of a batch group
   int sweeps[5] = {0, 0, 0, 0, 0};
+  long long repeats = 0;  // steps repeated for a sweep more
   // launch-by-launch steps decide every refinement sweep on the host (one synchronisation
   // per sweep) instead of launching all sweeps gated: then every launched kernel does work,
   // which per-kernel timing and profiling need (environment GHOSTMAC_HOST_REFINE=1)
@@ -269,6 +270,7 @@ struct gm_handle {
     cudaGraphExec_t exec = nullptr;
     const double* key[6] = {};
     double dt = 0;
+    int sweeps[5] = {};   // held when it was captured
     long long nodes = 0;  // kernel nodes
   } graphs[2];
   bool has_history = false;
@@ -2065,14 +2067,16 @@ void swap_state(gm_handle* h) {
   std::swap(h->hist.p, h->now.p);
 }
 
-// Graph of one steady step for the current buffer assignment and dt (captured on demand,
+// Graph of one steady step for the current buffer assignment, dt and held sweeps (captured on demand,
 // two alternate between the ping-pong buffer assignments).
 cudaGraphExec_t step_graph(gm_handle* h, double dt) {
   const double* key[6] = {h->U.p, h->Unext.p, h->phalf.p, h->phalf_next.p, h->hist.p, h->now.p};
+  auto current = [&](const gm_handle::StepGraph& gr) {
+    return gr.exec && gr.dt == dt && std::equal(h->sweeps, h->sweeps + 5, gr.sweeps);
+  };
   for (auto& gr : h->graphs)
-    if (gr.exec && gr.dt == dt && std::equal(key, key + 6, gr.key)) return gr.exec;
-  gm_handle::StepGraph* slot = !h->graphs[0].exec || h->graphs[0].dt != dt ? &h->graphs[0]
-                               : (!h->graphs[1].exec || h->graphs[1].dt != dt ? &h->graphs[1] : &h->graphs[0]);
+    if (current(gr) && std::equal(key, key + 6, gr.key)) return gr.exec;
+  gm_handle::StepGraph* slot = current(h->graphs[0]) && !current(h->graphs[1]) ? &h->graphs[1] : &h->graphs[0];
   if (slot->exec) { cudaGraphExecDestroy(slot->exec); slot->exec = nullptr; }
   const long long c0 = kernel_launch_count();
   h->capturing = true;
@@ -2098,6 +2102,7 @@ cudaGraphExec_t step_graph(gm_handle* h, double dt) {
   slot->exec = ex;
   slot->dt = dt;
   std::copy(key, key + 6, slot->key);
+  std::copy(h->sweeps, h->sweeps + 5, slot->sweeps);
   return ex;
 }
 
@@ -2357,13 +2362,12 @@ void step_loop(gm_handle* h, double dt, int32_t n_steps, int64_t first_step_inde
       if (!direct) kernel_launch_adjust(batch * (h->graphs[0].exec ? h->graphs[0] : h->graphs[1]).nodes);
       if (good < batch && h->host_ring[good].err == ERR_SWEEPS) {
         // a solve of step s + good needs one sweep more than the graph holds: back to the state before
-        // that step, and on from there with graphs that have it
+        // that step, and on from there with graphs that have it (step_graph)
         for (int k = 0; k < good; ++k)
           if (diag) fill_diag(h, h->host_ring[k], start_time + (s + k + 1) * dt, dt, false, &diag[s + k]);
         if ((batch - good) % 2) swap_state(h);
         ++h->sweeps[h->host_ring[good].gate];
-        for (auto& gr : h->graphs)
-          if (gr.exec) { cudaGraphExecDestroy(gr.exec); gr.exec = nullptr; }
+        ++h->repeats;
         s += good;
         counter = first_step_index + s;
         CK(cudaMemsetAsync(h->ctl.p, 0, sizeof(StepCtl), st));
@@ -2968,6 +2972,13 @@ int gm_divergence_stats(gm_handle* h, const double* u, const double* v, double o
 }  // extern "C"
 
 extern "C" {
+
+int gm_held_sweeps(const gm_handle* h, int32_t held[5], int64_t* repeats) {
+  if (!h) return GM_EVALUE;
+  if (held) std::copy(h->sweeps, h->sweeps + 5, held);
+  if (repeats) *repeats = h->repeats;
+  return GM_OK;
+}
 
 int64_t gm_kernel_launches(void) { return (int64_t)kernel_launch_count(); }
 
@@ -3643,6 +3654,7 @@ int gm_batch_step(gm_batch* b, double dt, int32_t n_steps, int64_t first_step_in
             if (diag) fill_diag(h, h->host_ring[k], t0 + (s + k + 1) * dt, dt, false, &diag[(size_t)c * n_steps + s + k]);
           if ((batch - good) % 2) swap_state(h);
           ++h->sweeps[h->host_ring[good].gate];
+          ++h->repeats;
           std::vector<gm_step_diag> rest(batch - good);
           int done = 0;
           try {

@@ -443,6 +443,10 @@ int gm_host_free(void* p);
 
 /* --- instrumentation (no reference counterpart) -------------------------------- */
 
+/* Refinement sweeps that the graphs of a handle's steady steps hold for each solve (Helmholtz u and v,
+ * the start-up's pressure, the step's first and second pressure), and how many times a step was repeated
+ * because one of its solves needed more.  Either pointer may be NULL. */
+int gm_held_sweeps(const gm_handle* h, int32_t held[5], int64_t* repeats);
 /* Number of CUDA kernels this library has launched in this process. */
 int64_t gm_kernel_launches(void);
 /* Event times (ms) of the last step run by gm_step when the environment variable
