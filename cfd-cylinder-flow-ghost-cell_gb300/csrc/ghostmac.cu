@@ -19,6 +19,7 @@
 #include "geometry.hpp"
 #include "fftplan.hpp"
 #include "kernels.cuh"
+#include "heldcount.hpp"
 #include "internal.hpp"
 
 using namespace gmk;
@@ -244,9 +245,12 @@ struct gm_handle {
   // conditional node costs 8 us even when its body does not run and 4 more per pass (a kernel node 1.2),
   // 25 us of a 220 us step in FP64, which needs no sweep, and about 50 in the FP32 mode.  A solve that
   // needs more than its slot's stops the steps behind it (ERR_SWEEPS); the host adds one and repeats
-  // the step.  FP64 starts with none, the FP32 mode with the one that it always needs.
+  // the step.  The handle's first step, which runs launch by launch with every sweep, sets the counts, and
+  // a count falls again when the steps no longer use it (HeldCount): the FP32 mode's pressure solves
+  // need two sweeps for some twenty steps from rest and one from there on.
   bool looped = false;  // the solves of this capture are the loops of a batch group
-  int sweeps[5] = {0, 0, 0, 0, 0};
+  HeldCount sweeps[5];
+  bool sweeps_known = false;  // a first step has set them
   long long repeats = 0;  // steps repeated for a sweep more
   // launch-by-launch steps decide every refinement sweep on the host (one synchronisation
   // per sweep) instead of launching all sweeps gated: then every launched kernel does work,
@@ -270,7 +274,7 @@ struct gm_handle {
     cudaGraphExec_t exec = nullptr;
     const double* key[6] = {};
     double dt = 0;
-    int sweeps[5] = {};   // held when it was captured
+    std::array<int, 5> sweeps{};  // held when it was captured
     long long nodes = 0;  // kernel nodes
   } graphs[2];
   bool has_history = false;
@@ -1563,7 +1567,7 @@ void gmres_monitored(gm_handle* h, const double* b, double* x, double* res, int 
 // reference's residual target (solver/pressure_schur.py:16-72, direct branch).
 // refinement sweeps launched for a slot
 int sweeps_of(const gm_handle* h, int slot) {
-  return h->capturing && !h->looped ? std::min(h->sweeps[slot], h->nchk - 1) : h->nchk - 1;
+  return h->capturing && !h->looped ? std::min(h->sweeps[slot].n, h->nchk - 1) : h->nchk - 1;
 }
 void schur_solve(gm_handle* h, int lane, RectDev& rd, int kind, double hc, const double* b, double* x, double* res,
                  double* first, double* w2, int slot) {
@@ -2067,13 +2071,36 @@ void swap_state(gm_handle* h) {
   std::swap(h->hist.p, h->now.p);
 }
 
+std::array<int, 5> held_sweeps(const gm_handle* h) {
+  std::array<int, 5> n;
+  for (int s = 0; s < 5; ++s) n[s] = h->sweeps[s].n;
+  return n;
+}
+// refinement sweeps that a recorded solve ran (the host's form of last_check)
+int sweeps_run(const SolveCtl& sc, int nchk) {
+  const double tg = std::max(1e-10, 32 * 2.220446049250313e-16 * std::max(1.0, bits2d(sc.bmax)));
+  int k = 0;
+  while (k + 1 < nchk && bits2d(sc.rmax[k]) > tg) ++k;
+  return k;
+}
+// the held sweeps after `n` good steps recorded in host_ring: the handle's first step sets them, steps of a
+// graph lower them
+void note_sweeps(gm_handle* h, int n, bool first, bool graph) {
+  for (int k = 0; k < n; ++k)
+    for (int s : {S_HELM_U, S_HELM_V, S_P1, S_P2}) {
+      const int used = sweeps_run(h->host_ring[k].solve[s], h->nchk);
+      if (first && !h->sweeps_known) h->sweeps[s].raise(used);
+      else if (graph) h->sweeps[s].steps(used, 1);
+    }
+  if (first && n > 0) h->sweeps_known = true;
+}
+
 // Graph of one steady step for the current buffer assignment, dt and held sweeps (captured on demand,
 // two alternate between the ping-pong buffer assignments).
 cudaGraphExec_t step_graph(gm_handle* h, double dt) {
   const double* key[6] = {h->U.p, h->Unext.p, h->phalf.p, h->phalf_next.p, h->hist.p, h->now.p};
-  auto current = [&](const gm_handle::StepGraph& gr) {
-    return gr.exec && gr.dt == dt && std::equal(h->sweeps, h->sweeps + 5, gr.sweeps);
-  };
+  const std::array<int, 5> sweeps = held_sweeps(h);
+  auto current = [&](const gm_handle::StepGraph& gr) { return gr.exec && gr.dt == dt && gr.sweeps == sweeps; };
   for (auto& gr : h->graphs)
     if (current(gr) && std::equal(key, key + 6, gr.key)) return gr.exec;
   gm_handle::StepGraph* slot = current(h->graphs[0]) && !current(h->graphs[1]) ? &h->graphs[1] : &h->graphs[0];
@@ -2102,7 +2129,7 @@ cudaGraphExec_t step_graph(gm_handle* h, double dt) {
   slot->exec = ex;
   slot->dt = dt;
   std::copy(key, key + 6, slot->key);
-  std::copy(h->sweeps, h->sweeps + 5, slot->sweeps);
+  slot->sweeps = sweeps;
   return ex;
 }
 
@@ -2124,9 +2151,7 @@ void fill_diag(gm_handle* h, const StepCtl& c, double t, double dt, bool first, 
   int mref = 0;
   for (int s = 0; s < 2; ++s) {
     const SolveCtl& sc = c.solve[s];
-    double b = bits2d(sc.bmax), tg = std::max(1e-10, 32 * 2.220446049250313e-16 * std::max(1.0, b));
-    int k = 0;
-    while (k + 1 < h->nchk && bits2d(sc.rmax[k]) > tg) ++k;
+    const int k = sweeps_run(sc, h->nchk);
     mres = std::max(mres, bits2d(sc.rmax[k]));
     mref += k;
   }
@@ -2138,9 +2163,7 @@ void fill_diag(gm_handle* h, const StepCtl& c, double t, double dt, bool first, 
   int its = 0;
   for (int s = first ? 2 : 3; s < 5; ++s) {
     const SolveCtl& sc = c.solve[s];
-    double b = bits2d(sc.bmax), tg = std::max(1e-10, 32 * 2.220446049250313e-16 * std::max(1.0, b));
-    int k = 0;
-    while (k + 1 < h->nchk && bits2d(sc.rmax[k]) > tg) ++k;
+    int k = sweeps_run(sc, h->nchk);
     if (sc.gk1) k = sc.gk1 - 1;
     its += sc.gits;
     ++count;
@@ -2274,7 +2297,7 @@ void create_device(gm_handle* H) {
   H->spectral.alloc(std::max<int64_t>(H->Pn, (int64_t)g.ny * g.nx));
   H->spectral_b.alloc(H->spectral.n);
   if (H->precision == 1) {
-    std::fill(H->sweeps, H->sweeps + 5, 1);
+    for (HeldCount& c : H->sweeps) c.n = 1;
     H->spectral32.alloc(H->spectral.n);
     H->spectral32_b.alloc(H->spectral.n);
     H->pres32.alloc(H->Pn);
@@ -2366,7 +2389,9 @@ void step_loop(gm_handle* h, double dt, int32_t n_steps, int64_t first_step_inde
         for (int k = 0; k < good; ++k)
           if (diag) fill_diag(h, h->host_ring[k], start_time + (s + k + 1) * dt, dt, false, &diag[s + k]);
         if ((batch - good) % 2) swap_state(h);
-        ++h->sweeps[h->host_ring[good].gate];
+        note_sweeps(h, good, false, true);
+        HeldCount& held = h->sweeps[h->host_ring[good].gate];
+        held.raise(held.n + 1);
         ++h->repeats;
         s += good;
         counter = first_step_index + s;
@@ -2376,6 +2401,7 @@ void step_loop(gm_handle* h, double dt, int32_t n_steps, int64_t first_step_inde
       }
       for (int k = 0; k < std::min(batch, good + 1); ++k)
         if (diag) fill_diag(h, h->host_ring[k], start_time + (s + k + 1) * dt, dt, first && k == 0, &diag[s + k]);
+      note_sweeps(h, good, first, !direct);
       if (good < batch) {
         // back to the state after the last good step
         if ((batch - good) % 2) swap_state(h);
@@ -2975,7 +3001,8 @@ extern "C" {
 
 int gm_held_sweeps(const gm_handle* h, int32_t held[5], int64_t* repeats) {
   if (!h) return GM_EVALUE;
-  if (held) std::copy(h->sweeps, h->sweeps + 5, held);
+  if (held)
+    for (int s = 0; s < 5; ++s) held[s] = h->sweeps[s].n;
   if (repeats) *repeats = h->repeats;
   return GM_OK;
 }
@@ -3481,7 +3508,7 @@ gm_batch::Graph& batch_graph(gm_batch* b, double dt) {
   std::vector<long long> gens;  // what else a captured step depends on: Helmholtz tables, sweeps
   for (gm_handle* h : b->cases) {
     gens.push_back(h->helm_gen);
-    gens.insert(gens.end(), h->sweeps, h->sweeps + 5);
+    for (int n : held_sweeps(h)) gens.push_back(n);
   }
   for (auto& gr : b->graphs)
     if (gr.exec && gr.dt == dt && gr.key == key && gr.gens == gens) return gr;
@@ -3653,7 +3680,9 @@ int gm_batch_step(gm_batch* b, double dt, int32_t n_steps, int64_t first_step_in
           for (int k = 0; k < good; ++k)
             if (diag) fill_diag(h, h->host_ring[k], t0 + (s + k + 1) * dt, dt, false, &diag[(size_t)c * n_steps + s + k]);
           if ((batch - good) % 2) swap_state(h);
-          ++h->sweeps[h->host_ring[good].gate];
+          note_sweeps(h, good, false, true);
+          HeldCount& held = h->sweeps[h->host_ring[good].gate];
+          held.raise(held.n + 1);
           ++h->repeats;
           std::vector<gm_step_diag> rest(batch - good);
           int done = 0;
@@ -3680,6 +3709,7 @@ int gm_batch_step(gm_batch* b, double dt, int32_t n_steps, int64_t first_step_in
         for (int k = 0; k < std::min(batch, good + 1); ++k)
           if (diag) fill_diag(h, h->host_ring[k], t0 + (s + k + 1) * dt, dt, first && k == 0,
                               &diag[(size_t)c * n_steps + s + k]);
+        note_sweeps(h, good, first, steady);
         if (steps_done) steps_done[c] = s + good;
         if (good > 0) { h->has_history = true; h->prev_dt = dt; }
         if (good < batch) {
@@ -3768,7 +3798,7 @@ int check(gm_handle* h, const char* where, std::string& err) {
 }
 
 int failed_gate(const gm_handle* h) { return h->host_ctl->gate; }
-void add_sweep(gm_handle* h, int slot) { ++h->sweeps[slot]; }
+void add_sweep(gm_handle* h, int slot) { h->sweeps[slot].raise(h->sweeps[slot].n + 1); }
 
 int64_t schur_rank(const gm_handle* h) { return h->rp.rank; }
 

@@ -53,3 +53,37 @@ def test_batch_replays_no_graph_of_fewer_sweeps():
     assert out[0][:2] == out[1][:2]
     for a, b in zip(out[0][2:], out[1][2:]):
         assert np.array_equal(a, b)
+
+
+def test_first_step_sets_and_later_steps_lower(monkeypatch):
+    """From rest the FP32 mode's pressure solves need two sweeps for some twenty steps and one from there
+    on: the first step sets the counts, so no step is repeated, and 64 steps that use one lower them."""
+    pkg = load_package()
+    a = make(pkg, precision='fp32')
+    a.solve(n_steps=5, **QUIET)
+    assert held(pkg, a) == ([1, 1, 1, 2, 2], 0)
+    a.solve(n_steps=160, **QUIET)
+    assert held(pkg, a) == ([1, 1, 1, 1, 1], 0)
+    monkeypatch.setenv('GHOSTMAC_NO_GRAPHS', '1')
+    b = make(pkg, precision='fp32')
+    b.solve(n_steps=165, **QUIET)
+    for name in ('u', 'v', 'p'):
+        assert np.array_equal(getattr(a, name), getattr(b, name))
+
+
+@pytest.mark.parametrize('batch', [False, True])
+def test_one_hard_step_is_not_kept(batch):
+    """A perturbed FP64 state needs a sweep that later steps do not: the count goes up and down again."""
+    pkg = load_package()
+    cases = [make(pkg), make(pkg, 96, 48)]
+    b = pkg.CylinderBatch(cases)
+    step = (lambda n: b.solve(n, dt=0.002)) if batch else (lambda n: [s.solve(n_steps=n, **QUIET) for s in cases])
+    step(4)
+    assert [held(pkg, s) for s in cases] == [([0] * 5, 0)] * 2
+    for k, s in enumerate(cases):
+        shake(s, 0.3, k)
+    step(3)
+    assert [held(pkg, s) for s in cases] == [([0, 0, 0, 1, 1], 2)] * 2
+    step(130)
+    assert [held(pkg, s) for s in cases] == [([0] * 5, 2)] * 2
+    b.close()
