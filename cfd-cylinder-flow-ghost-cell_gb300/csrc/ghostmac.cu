@@ -11,6 +11,7 @@
 #include <cstring>
 #include <functional>
 #include <memory>
+#include <numeric>
 #include <string>
 #include <array>
 #include <vector>
@@ -248,8 +249,9 @@ struct gm_handle {
   // the step.  The handle's first step, which runs launch by launch with every sweep, sets the counts, and
   // a count falls again when the steps no longer use it (HeldCount): the FP32 mode's pressure solves
   // need two sweeps for some twenty steps from rest and one from there on.
-  bool looped = false;  // the solves of this capture are the loops of a batch group
+  bool looped = false;  // the solves of this capture are loops (WHILE nodes): a batch's (batch_loops)
   HeldCount sweeps[5];
+  long long loop_nodes[5] = {};  // looped: kernels of a pass of each slot's loop
   bool sweeps_known = false;  // a first step has set them
   long long repeats = 0;  // steps repeated for a sweep more
   // launch-by-launch steps decide every refinement sweep on the host (one synchronisation
@@ -1579,6 +1581,30 @@ void schur_solve(gm_handle* h, int lane, RectDev& rd, int kind, double hc, const
   SolveCtl* sc = &h->ctl.p->solve[slot];
   const bool f32 = h->precision == 1;
   void* resb = f32 ? (void*)(kind == 0 ? h->pres32.p : h->fres32.p) : (void*)res;
+  if (h->capturing && h->looped) {
+    // the sweeps as the body of a WHILE node, which runs while the residual check asks for it
+    cudaStream_t body_st = lane == 0 ? h->st_body : h->st2_body;
+    const Gate g0 = gate_of(h, slot, 0);
+    apply_inverse(h, lane, rd, kind, b, false, x, false, first, w2, g0, st);
+    launch_residual(h->cd, h->rcoef[kind], kind, b, x, resb, f32, sc, 0, true, g0, st);
+    ArgPack<StepCtl*> ctls{};
+    ctls.a[0] = h->ctl.p;
+    cudaStreamCaptureStatus cs;
+    cudaGraph_t graph, body;
+    CK(cudaStreamGetCaptureInfo(st, &cs, nullptr, &graph, nullptr, nullptr, nullptr));
+    cudaGraphConditionalHandle cond;
+    CK(cudaGraphConditionalHandleCreate(&cond, graph, 0, 0));
+    launch_refine_decide_multi(ctls, 1, slot, h->nchk, cond, st);
+    add_conditional(st, cond, cudaGraphCondTypeWhile, &body);
+    CK(cudaStreamBeginCaptureToGraph(body_st, body, nullptr, nullptr, 0, cudaStreamCaptureModeRelaxed));
+    const long long c0 = kernel_launch_count();
+    apply_inverse(h, lane, rd, kind, resb, f32, x, true, first, w2, g0, body_st);
+    launch_residual(h->cd, h->rcoef[kind], kind, b, x, resb, f32, sc, -1, false, g0, body_st);
+    launch_refine_decide_multi(ctls, 1, slot, h->nchk, cond, body_st);
+    h->loop_nodes[slot] = kernel_launch_count() - c0;
+    CK(cudaStreamEndCapture(body_st, &body));
+    return;
+  }
   const int last = sweeps_of(h, slot);
   for (int sweep = 0; sweep <= last; ++sweep) {
     Gate gt = gate_of(h, slot, sweep);
@@ -3097,7 +3123,8 @@ struct gm_batch {
     std::vector<const double*> key;
     std::vector<long long> gens;
     double dt = 0;
-    std::vector<long long> outer;  // kernel nodes of a case's own branch
+    std::vector<long long> outer;  // kernel nodes of a case's own branch, outside its loops
+    std::vector<std::array<long long, 5>> loop;  // and of a pass of its loops, per solve slot
     long long group_outer = 0;                          // case-indexed solves: nodes outside the loops
     std::vector<std::array<long long, 5>> group_body;   // and per group, one sweep per solve slot
   } graphs[2];
@@ -3503,12 +3530,35 @@ std::vector<const double*> batch_key(gm_batch* b) {
   return k;
 }
 
+// Whether the FP32 cases' refinement sweeps are loops (WHILE nodes) in the batch's graph instead of held
+// and gated ones (FP64 cases hold none).  A loop costs its branch some 20 us of latency a solve; a sweep
+// that is held and not needed costs its blocks, which a full GPU no longer hides.  Held against
+// loops, ms a step from rest and later: 64 cases of 96x48 1.50 and 1.44 against 2.27 and 2.25, of 256x128
+// 2.60 and 2.40 against 3.09 and 2.90; of 400x200 12 cases 0.94 and 0.87 against 0.95 and 0.84, 64 cases 4.69
+// and 4.30 against 4.64 and 4.13; of 800x410 4 cases 0.95 and 0.85 against 1.03 and 0.87, 24 cases 4.76 and 4.35
+// against 4.76 and 4.23, 48 cases 9.69 and 8.87 against 9.35 and 8.34; the sweep over three grids (143,000
+// cells a case) 24 cases 2.56 and 2.42 against 2.67 and 2.49, 40 cases 4.05 and 3.84 against 4.07 and 3.79, 64
+// cases 6.58 and 6.17 against 6.16 and 5.70.  GHOSTMAC_BATCH_LOOPS=0 or 1 decides instead.
+bool batch_loops(const gm_batch* b) {
+  if (const char* e = std::getenv("GHOSTMAC_BATCH_LOOPS"))
+    if (e[0]) return e[0] != '0';
+  int64_t cells = 0, cases = 0;
+  for (const gm_handle* h : b->cases)
+    if (h->precision == 1) {
+      cells += h->Pn;
+      ++cases;
+    }
+  return cells >= 5000000 && cells >= 60000 * cases;
+}
+
 gm_batch::Graph& batch_graph(gm_batch* b, double dt) {
   std::vector<const double*> key = batch_key(b);
-  std::vector<long long> gens;  // what else a captured step depends on: Helmholtz tables, sweeps
+  const bool loops = batch_loops(b);
+  std::vector<long long> gens{loops};  // what else a captured step depends on: Helmholtz tables, sweeps
   for (gm_handle* h : b->cases) {
     gens.push_back(h->helm_gen);
-    for (int n : held_sweeps(h)) gens.push_back(n);
+    if (!(loops && h->precision == 1))
+      for (int n : held_sweeps(h)) gens.push_back(n);
   }
   for (auto& gr : b->graphs)
     if (gr.exec && gr.dt == dt && gr.key == key && gr.gens == gens) return gr;
@@ -3519,6 +3569,7 @@ gm_batch::Graph& batch_graph(gm_batch* b, double dt) {
     slot->exec = nullptr;
   }
   slot->outer.assign(b->cases.size(), 0);
+  slot->loop.assign(b->cases.size(), {});
   slot->group_outer = 0;
   slot->group_body.clear();
   batch_shapes(b);
@@ -3547,11 +3598,15 @@ gm_batch::Graph& batch_graph(gm_batch* b, double dt) {
       gm_handle* h = b->cases[c];
       CK(cudaStreamWaitEvent(h->st, b->fork, 0));
       const long long c0 = kernel_launch_count();
+      std::fill(h->loop_nodes, h->loop_nodes + 5, 0LL);
       h->capturing = true;
+      h->looped = loops && h->precision == 1;
       step_once(h, dt, -1);
-      h->capturing = false;
-      slot->outer[c] = kernel_launch_count() - c0;
-      kernel_launch_adjust(-slot->outer[c]);
+      h->capturing = h->looped = false;
+      const long long captured = kernel_launch_count() - c0;
+      kernel_launch_adjust(-captured);
+      std::copy(h->loop_nodes, h->loop_nodes + 5, slot->loop[c].begin());
+      slot->outer[c] = captured - std::accumulate(h->loop_nodes, h->loop_nodes + 5, 0LL);
       CK(cudaEventRecord(b->join[c], h->st));
       CK(cudaStreamWaitEvent(b->root, b->join[c], 0));
     }
@@ -3672,7 +3727,12 @@ int gm_batch_step(gm_batch* b, double dt, int32_t n_steps, int64_t first_step_in
         int good = 0;
         while (good < batch && h->host_ring[good].err == 0) ++good;
         const double t0 = start_times ? start_times[c] : 0.0;
-        if (steady) nodes += batch * (b->graphs[0].exec ? b->graphs[0] : b->graphs[1]).outer[c];
+        if (steady) {
+          const gm_batch::Graph& gr = b->graphs[0].exec ? b->graphs[0] : b->graphs[1];
+          nodes += batch * gr.outer[c];
+          for (int k = 0; k < batch; ++k)
+            for (int sl = 0; sl < 5; ++sl) nodes += gr.loop[c][sl] * h->host_ring[k].solve[sl].k;
+        }
         if (good < batch && h->host_ring[good].err == ERR_SWEEPS) {
           // a solve needs a sweep more than the graph holds: this case goes back to the state before
           // that step and takes the rest of the graph batch alone (the same kernels, so the same
