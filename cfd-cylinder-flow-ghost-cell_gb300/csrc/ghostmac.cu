@@ -3128,6 +3128,7 @@ struct gm_batch {
     long long group_outer = 0;                          // case-indexed solves: nodes outside the loops
     std::vector<std::array<long long, 5>> group_body;   // and per group, one sweep per solve slot
   } graphs[2];
+  const Graph* last = nullptr;  // the one used last
   std::string err;
 };
 
@@ -3561,10 +3562,14 @@ gm_batch::Graph& batch_graph(gm_batch* b, double dt) {
       for (int n : held_sweeps(h)) gens.push_back(n);
   }
   for (auto& gr : b->graphs)
-    if (gr.exec && gr.dt == dt && gr.key == key && gr.gens == gens) return gr;
-  gm_batch::Graph* slot = !b->graphs[0].exec ? &b->graphs[0] : (!b->graphs[1].exec ? &b->graphs[1] : nullptr);
-  if (!slot) {
-    slot = (b->graphs[0].key == key || b->graphs[0].dt != dt) ? &b->graphs[0] : &b->graphs[1];
+    if (gr.exec && gr.dt == dt && gr.key == key && gr.gens == gens) {
+      b->last = &gr;
+      return gr;
+    }
+  // in the place of the other graph than the last one used: the buffers of two steps alternate, so the
+  // two that a batch needs stay, whatever pairs of buffers its cases bring (a case stepped alone in between)
+  gm_batch::Graph* slot = b->last == &b->graphs[0] ? &b->graphs[1] : &b->graphs[0];
+  if (slot->exec) {
     cudaGraphExecDestroy(slot->exec);
     slot->exec = nullptr;
   }
@@ -3626,6 +3631,7 @@ gm_batch::Graph& batch_graph(gm_batch* b, double dt) {
   slot->dt = dt;
   slot->key = key;
   slot->gens = gens;
+  b->last = slot;
   return *slot;
 }
 

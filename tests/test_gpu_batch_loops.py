@@ -1,5 +1,7 @@
 """A batch whose FP32 cases refine in loops (WHILE nodes; large batches of large grids) against held, gated
 sweeps and against the cases stepped alone: the same kernels, so the same bits."""
+import time
+
 import numpy as np
 import pytest
 
@@ -51,3 +53,28 @@ def test_loops_never_repeat_a_step(monkeypatch):
         b.solve(3, dt=0.002)
     assert np.isfinite(cases[1].u).all() and not np.array_equal(cases[1].u, good)
     b.close()
+
+
+def test_case_stepped_alone_in_between():
+    """After one step of one case alone the batch pairs its cases' buffers anew and captures its two graphs
+    again, once: its steps then replay them (a step that captures eight cases takes many times as long)."""
+    pkg = load_package()
+    cases = [make(pkg, 96, 48) for _ in range(8)]
+    b = pkg.CylinderBatch(cases)
+
+    def fastest():
+        times = []
+        for _ in range(6):
+            t0 = time.perf_counter()
+            rc, _, _ = b.step_raw(0.002, 1)
+            times.append(time.perf_counter() - t0)
+            b._check(rc)
+        return min(times)
+
+    fastest()
+    before = fastest()
+    rc, _ = cases[3].step_raw(0.002, 1)
+    pkg._lib.check(rc, cases[3]._h)
+    after = fastest()
+    b.close()
+    assert after < 3 * before
