@@ -37,6 +37,7 @@
 
 #include "../../include/ghostmac.h"
 #include "geometry.hpp"
+#include "heldcount.hpp"
 #include "internal.hpp"
 #include "kernels.cuh"
 
@@ -1277,17 +1278,21 @@ struct gm_cc {
   Buf<double> nval;
   CnOp cn{};
   bool offset_stale = true;  // the inlet changed since offset was formed
-  int cn_steps = 6;          // Arnoldi steps that a step graph holds; above CN_M: restart cycles in a WHILE node
+  HeldCount arnoldi{6, 1};   // Arnoldi steps that a step graph holds; above CN_M: restart cycles in a WHILE node
+  bool counts_known = false; // a first step, which holds plenty, has set them and the pressure solves' sweeps
+  long long repeats = 0;     // steps repeated for a refinement sweep or Arnoldi steps more
   Buf<double> V, gpart, gpart2;
   Buf<CnDev> gdev;
   // per-step diagnostics
   Buf<CcDiagDev> diag;
   CcDiagDev* host_diag = nullptr;
-  // step graphs keyed by (dt, history, previous dt)
+  // step graphs keyed by (dt, history, previous dt) and what they hold
   struct Graph {
     cudaGraphExec_t exec = nullptr;
     double dt = 0, prev_dt = 0;
     bool hist = false;
+    std::array<int, 5> sweeps{};
+    int arnoldi = 0;
     long long outer = 0, per_cycle = 0;
   };
   Graph graphs[3];
@@ -1413,8 +1418,8 @@ void gmres(gm_cc* c, const double* b, double* x, double dt, gm_cc::Graph& gr, cu
     counted();
     k_cn_combine<<<std::min<unsigned>(nblk(c->F), 1216), CC_TPB, 0, s>>>(c->V.p, c->F, c->gdev.p, x);
   };
-  if (c->cn_steps <= CN_M) {
-    cycle(1, c->cn_steps, gmi::control(c->P), st);
+  if (c->arnoldi.n <= CN_M) {
+    cycle(1, c->arnoldi.n, gmi::control(c->P), st);
     return;
   }
   CCK(cudaMemsetAsync(&c->gdev.p->jend, 0, sizeof(CnDev) - offsetof(CnDev, jend), st));
@@ -1504,8 +1509,11 @@ void step_body(gm_cc* c, double dt, gm_cc::Graph& gr, cudaStream_t st) {
 }
 
 gm_cc::Graph& step_graph(gm_cc* c, double dt) {
+  const std::array<int, 5> sweeps = gmi::held_sweeps(c->P);
   for (auto& g : c->graphs)
-    if (g.exec && g.dt == dt && g.hist == c->has_history && (!g.hist || g.prev_dt == c->prev_dt)) return g;
+    if (g.exec && g.dt == dt && g.hist == c->has_history && (!g.hist || g.prev_dt == c->prev_dt) && g.sweeps == sweeps &&
+        g.arnoldi == c->arnoldi.n)
+      return g;
   gm_cc::Graph& gr = c->graphs[c->next_graph];
   c->next_graph = (c->next_graph + 1) % 3;
   if (gr.exec) { cudaGraphExecDestroy(gr.exec); gr.exec = nullptr; }
@@ -1537,6 +1545,8 @@ gm_cc::Graph& step_graph(gm_cc* c, double dt) {
   gr.dt = dt;
   gr.hist = c->has_history;
   gr.prev_dt = c->prev_dt;
+  gr.sweeps = sweeps;
+  gr.arnoldi = c->arnoldi.n;
   return gr;
 }
 
@@ -2182,6 +2192,10 @@ int gm_cc_step(gm_cc* c, double dt, int32_t n_steps, double start_time, gm_cc_st
     cudaStream_t st = c->st;
     for (int32_t k = 0; k < n_steps; ++k) {
       refresh_offset(c);
+      if (!c->counts_known) {
+        for (int s : {S_P0, S_P1, S_P2}) gmi::set_sweeps(c->P, s, gmi::checks(c->P) - 1);
+        c->arnoldi.raise(12);
+      }
       gm_cc::Graph& gr = step_graph(c, dt);
       CCK(cudaMemsetAsync(gmi::control(c->P), 0, sizeof(StepCtl), st));
       CCK(cudaGraphLaunch(gr.exec, st));
@@ -2194,14 +2208,23 @@ int gm_cc_step(gm_cc* c, double dt, int32_t n_steps, double start_time, gm_cc_st
       kernel_launch_adjust(gr.outer + (long long)cycles * gr.per_cycle);
       if (prc == ERR_SWEEPS) {
         // a solve needs more than the graph holds; the state is as before the step: once more with more
-        const int what = gmi::failed_gate(c->P);
-        if (what == CN_SHORT) c->cn_steps = c->cn_steps < CN_M ? std::min(c->cn_steps + 4, CN_M) : CN_M + 1;
+        const int what = gmi::failed_gate(c->P), n = c->arnoldi.n;
+        if (what == CN_SHORT) c->arnoldi.raise(n < CN_M ? std::min(n + 2, CN_M) : CN_M + 1);
         else gmi::add_sweep(c->P, what);
-        for (auto& g : c->graphs)
-          if (g.exec) { cudaGraphExecDestroy(g.exec); g.exec = nullptr; }
+        ++c->repeats;
         --k;
         continue;
       }
+      // the first step sets the counts, and those that later steps do not use fall (HeldCount)
+      const int used = cycles > 0 ? CN_M + 1 : its;
+      if (!c->counts_known) c->arnoldi.n = std::max(used, c->arnoldi.least);
+      c->arnoldi.steps(used, 1);
+      for (int s : {S_P0, S_P1, S_P2}) {
+        const int run = gmi::sweeps_run(c->P, s);
+        if (!c->counts_known) gmi::set_sweeps(c->P, s, run);
+        if (s != S_P0) gmi::note_sweeps(c->P, s, run, 1);
+      }
+      c->counts_known = true;
       if (c->phase_on)
         for (int q = 0; q < gm_cc::NPHASE; ++q) {
           float ms = 0.f;
@@ -2340,6 +2363,17 @@ int gm_cc_get_legacy_history(gm_cc* c, int32_t* has_history, double* prev_accel,
       CCK(cudaStreamSynchronize(c->st));
     }
   });
+}
+
+int gm_cc_held_sweeps(const gm_cc* c, int32_t held[6], int64_t* repeats) {
+  if (!c) return GM_EVALUE;
+  if (held) {
+    const std::array<int, 5> n = gmi::held_sweeps(c->P);
+    std::copy(n.begin(), n.end(), held);
+    held[5] = c->arnoldi.n;
+  }
+  if (repeats) *repeats = c->repeats;
+  return GM_OK;
 }
 
 int gm_cc_phase_timing(const gm_cc* c, double out[8]) {
@@ -2495,6 +2529,8 @@ struct gm_poisson {
   Buf<int32_t> cell_type;
   // the legacy loop's device scratch and per-step records (see gml::forces)
   Buf<double> lscratch, lrec;
+  bool counts_known = false;  // a first step of the loop has set the sweeps its solves hold
+  long long repeats = 0;      // solves that went on with a refinement sweep more
   cudaEvent_t ev_in = nullptr, ev_out = nullptr;
 };
 
@@ -2589,9 +2625,11 @@ int gm_poisson_legacy_step(gm_poisson* p, gm_legacy_state* s, double dt, int32_t
     // All steps queue behind each other: a failed pressure gate stops the kernels behind it, and a solve
     // that needs more refinement sweeps than are held (FP64 starts with none) goes on from there with one
     // more.  With a read-back a step and two idle sweeps a solve a step took 229 us at 350x213, now 154.
+    // The loop's first step holds every sweep and sets the count (HeldCount).
     bool predicted = false;
     for (int32_t k = 0; k < n_steps;) {
-      for (; k < n_steps; ++k) {
+      if (!p->counts_known) gmi::set_sweeps(p->P, S_P1, gmi::checks(p->P) - 1);
+      for (const int32_t end = p->counts_known ? n_steps : 1; k < end; ++k) {
         if (!predicted) {
           gml::predict(*s, dt, p->lscratch.p, p->cell_type.p, p->ikappa.p, &ctl->err, st);
           if (s->centered) {  // the loop keeps the AB2 history before its pressure solve (solver/main.py:320)
@@ -2611,15 +2649,21 @@ int gm_poisson_legacy_step(gm_poisson* p, gm_legacy_state* s, double dt, int32_t
       CCK(cudaGetLastError());
       std::string m;
       const int rc = gmi::check(p->P, "pressure solve", m);  // synchronises the stream
-      if (rc == GM_OK) break;
+      if (rc == GM_OK) {
+        if (!p->counts_known) gmi::set_sweeps(p->P, S_P1, (int)rec[5] - 1);
+        p->counts_known = true;
+        continue;
+      }
       if (rc != ERR_SWEEPS) throw CcFail(rc, m);
       gmi::add_sweep(p->P, gmi::failed_gate(p->P));
+      ++p->repeats;
       for (k = 0; k < n_steps && rec[(size_t)k * NR + 5] != 0.0; ++k) {}
       CCK(cudaMemsetAsync(ctl, 0, sizeof(StepCtl), st));
       predicted = true;
     }
     CCK(cudaEventRecord(p->ev_out, st));
     CCK(cudaStreamWaitEvent(cs, p->ev_out, 0));
+    for (int32_t k = 0; k < n_steps; ++k) gmi::note_sweeps(p->P, S_P1, (int)rec[(size_t)k * NR + 5] - 1, 1);
     if (diag)
       for (int32_t k = 0; k < n_steps; ++k) {
         for (int q = 0; q < 4; ++q) diag[k].forces[q] = rec[(size_t)k * NR + q];
@@ -2632,6 +2676,13 @@ int gm_poisson_legacy_step(gm_poisson* p, gm_legacy_state* s, double dt, int32_t
     p->err = e.what();
     return GM_ECUDA;
   }
+  return GM_OK;
+}
+
+int gm_poisson_held_sweeps(const gm_poisson* p, int32_t* held, int64_t* repeats) {
+  if (!p) return GM_EVALUE;
+  if (held) *held = gmi::held_sweeps(p->P)[S_P1];
+  if (repeats) *repeats = p->repeats;
   return GM_OK;
 }
 

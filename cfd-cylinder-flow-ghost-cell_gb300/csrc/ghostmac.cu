@@ -3865,6 +3865,10 @@ int check(gm_handle* h, const char* where, std::string& err) {
 
 int failed_gate(const gm_handle* h) { return h->host_ctl->gate; }
 void add_sweep(gm_handle* h, int slot) { h->sweeps[slot].raise(h->sweeps[slot].n + 1); }
+std::array<int, 5> held_sweeps(const gm_handle* h) { return ::held_sweeps(h); }
+int sweeps_run(const gm_handle* h, int slot) { return ::sweeps_run(h->host_ctl->solve[slot], h->nchk); }
+void set_sweeps(gm_handle* h, int slot, int n) { h->sweeps[slot].n = n; }
+void note_sweeps(gm_handle* h, int slot, int used, int count) { h->sweeps[slot].steps(used, count); }
 
 int64_t schur_rank(const gm_handle* h) { return h->rp.rank; }
 

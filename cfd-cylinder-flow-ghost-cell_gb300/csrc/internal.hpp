@@ -5,6 +5,7 @@
 #pragma once
 #include <cuda_runtime.h>
 
+#include <array>
 #include <cstdint>
 #include <functional>
 #include <string>
@@ -41,7 +42,14 @@ gmk::StepCtl* control(gm_handle* h);
 // GM_OK or the class of a failed gate / CUDA error recorded in the control block (message in err)
 int check(gm_handle* h, const char* where, std::string& err);
 int failed_gate(const gm_handle* h);       // the gate word that check read
-void add_sweep(gm_handle* h, int slot);    // one more sweep in graphs captured from here on
+// The held sweeps (HeldCount): one more for a slot; a slot's, set; those of every slot; the sweeps that a slot's
+// solve ran, of the control block that check read; and `count` solves of a slot that ran at most `used` each.
+// What is captured or queued from here on holds the new counts.
+void add_sweep(gm_handle* h, int slot);
+void set_sweeps(gm_handle* h, int slot, int n);
+std::array<int, 5> held_sweeps(const gm_handle* h);
+int sweeps_run(const gm_handle* h, int slot);
+void note_sweeps(gm_handle* h, int slot, int used, int count);
 int64_t schur_rank(const gm_handle* h);
 // surface point-pressure reconstruction (rows = quadrature points, columns = pressure cells)
 struct SurfaceCsr {
@@ -70,7 +78,7 @@ void predict(const gm_legacy_state& s, double dt, double* scratch, const int32_t
 // p = phi (centred) or p += phi
 void correct(const gm_legacy_state& s, double dt, double* scratch, const int* err, cudaStream_t st);
 // the step's record: forces (fx_p, fy_p, fx_v, fy_v), the bits of max |residual| of the solve in `slot`, and
-// 1, into out[0..5] (device)
+// one more than its refinement sweeps, into out[0..5] (device)
 void forces(const gm_legacy_state& s, double* scratch, double* out, const gmk::StepCtl* ctl, int slot, int nchk,
             cudaStream_t st);
 }  // namespace gml

@@ -310,7 +310,7 @@ __global__ void k_ghost_boundary(double* __restrict__ u, double* __restrict__ v,
 }
 
 // A step's record behind its four forces: max |residual| of the pressure solve's last check (out[4], its bits)
-// and a mark that the step is complete (out[5]).
+// and, as a mark that the step is complete, one more than the refinement sweeps that the solve ran (out[5]).
 struct StepRecord {
   const gmk::StepCtl* ctl;  // null: no record
   int slot, nchk;
@@ -318,8 +318,9 @@ struct StepRecord {
   __device__ void close(double* out) const {
     if (!ctl) return;
     const gmk::SolveCtl* sc = &ctl->solve[slot];
-    out[4] = gmk::bits2d(sc->rmax[gmk::last_check(sc, nchk)]);
-    out[5] = 1.0;
+    const int k = gmk::last_check(sc, nchk);
+    out[4] = gmk::bits2d(sc->rmax[k]);
+    out[5] = 1.0 + k;
   }
 };
 

@@ -414,6 +414,8 @@ typedef struct gm_legacy_step_diag {
  * before later work there. */
 int gm_poisson_legacy_step(gm_poisson* p, gm_legacy_state* s, double dt, int32_t n_steps, gm_legacy_step_diag* diag,
                            void* stream);
+/* Refinement sweeps that the loop's solves hold, and how many solves went on with one more. */
+int gm_poisson_held_sweeps(const gm_poisson* p, int32_t* held, int64_t* repeats);
 
 /* --- snapshot POD (postprocessing/modal_analysis.py:17-98) ------------------------ */
 /* Method of snapshots for M snapshots of N points (row-major M x N, host or device memory):
@@ -596,6 +598,8 @@ int gm_cc_get_legacy_history(gm_cc* c, int32_t* has_history, double* prev_accel,
  * its residual check, projection 1, CN action and defect, projection 2, outputs (pressure,
  * history, step maxima, forces).  No counterpart in the reference. */
 int gm_cc_phase_timing(const gm_cc* c, double out[8]);
+/* gm_held_sweeps of a cut-cell case; held[5]: Arnoldi steps of the CN system's GMRES (31: restart cycles). */
+int gm_cc_held_sweeps(const gm_cc* c, int32_t held[6], int64_t* repeats);
 
 #define GM_CC_OP_MOMENTUM_ADVECTION 1 /* (u|v grids) -> a (u|v), y2: rhs; compute_momentum_rhs(u, v, 0, rho) :790-957 */
 #define GM_CC_OP_MOMENTUM_DIFFUSION 2 /* same with nu = param and include_advection=False */
