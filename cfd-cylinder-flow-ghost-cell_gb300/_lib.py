@@ -23,7 +23,7 @@ SYMBOLS = ('gm_create', 'gm_create_host', 'gm_prepare_dt', 'gm_destroy', 'gm_las
            'gm_get_surface_points', 'gm_set_state', 'gm_get_state', 'gm_set_inlet', 'gm_set_history',
            'gm_get_history', 'gm_step', 'gm_solve_io', 'gm_apply', 'gm_project', 'gm_pressure_solve', 'gm_rectangle_solve',
            'gm_surface_forces', 'gm_divergence_stats', 'gm_held_sweeps', 'gm_cc_held_sweeps',
-           'gm_poisson_held_sweeps', 'gm_kernel_launches', 'gm_kernel_timing',
+           'gm_poisson_held_sweeps', 'gm_tg_held_sweeps', 'gm_kernel_launches', 'gm_kernel_timing',
            'gm_divergence_stats_noalloc', 'gm_batch_create', 'gm_batch_destroy', 'gm_batch_last_error',
            'gm_batch_step', 'gm_phase_timing', 'gm_tg_create', 'gm_tg_destroy', 'gm_tg_last_error',
            'gm_tg_set_state', 'gm_tg_get_state', 'gm_tg_step', 'gm_unet_layers', 'gm_unet_create',
@@ -170,6 +170,7 @@ def _load():
         'gm_surface_forces': ([P, P, P, P, D, P], C.c_int),
         'gm_divergence_stats': ([P, P, P, P, P], C.c_int),
         'gm_held_sweeps': ([P, P, C.POINTER(I64)], C.c_int),
+        'gm_tg_held_sweeps': ([P, P, C.POINTER(I64)], C.c_int),
         'gm_cc_held_sweeps': ([P, P, C.POINTER(I64)], C.c_int),
         'gm_poisson_held_sweeps': ([P, P, C.POINTER(I64)], C.c_int),
         'gm_kernel_launches': ([], I64),

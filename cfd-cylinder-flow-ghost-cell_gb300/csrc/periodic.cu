@@ -30,6 +30,7 @@
 #include "../../include/ghostmac.h"
 #include "exactdiv.cuh"
 #include "fftplan.hpp"
+#include "heldcount.hpp"
 #include "transforms.cuh"
 
 namespace gmk {
@@ -122,9 +123,10 @@ __device__ __forceinline__ T lap_p(const S* f, int n, int j, int i, T h, T nu) {
 // ---- a step's control words -----------------------------------------------------------------
 // Reductions (bits of non-negative doubles), the step whose gate failed (RED_ERR, from 1) and, when it
 // failed because a solve needed more refinement sweeps than were queued, that solve's slot + 1
-// (RED_SHORT); then the residual of every check of every refined solve (FP32 mode).
-enum : int { RED_CN = 0, RED_RHS = 1, RED_DIV = 2, RED_COUPLED = 3, RED_SHORT = 4, RED_ERR = 5, RED_W = 8 };
-enum : int { SLOT_START = 0, SLOT_CN = 1, SLOT_P1 = 2, SLOT_P2 = 3, NSLOT = 4, SLOT_CHECKS = 9, RED_N = RED_W + NSLOT * SLOT_CHECKS };
+// (RED_SHORT); then, of every refined solve (FP32 mode), the most sweeps that it ran in a step since the words
+// were read (RED_USED) and this step's residual at every check.
+enum : int { RED_CN = 0, RED_RHS = 1, RED_DIV = 2, RED_COUPLED = 3, RED_SHORT = 4, RED_ERR = 5, RED_USED = 6, NSLOT = 4, RED_W = RED_USED + NSLOT };
+enum : int { SLOT_START = 0, SLOT_CN = 1, SLOT_P1 = 2, SLOT_P2 = 3, SLOT_CHECKS = 9, RED_N = RED_W + NSLOT * SLOT_CHECKS };
 // Whether an earlier gate of this call failed: the state writers of the steps queued behind it return.
 __device__ __forceinline__ bool tg_failed(const unsigned long long* red) {
   return *(const volatile unsigned long long*)(red + RED_ERR) != 0;
@@ -159,7 +161,10 @@ struct TgHeld {
   double step;
 };
 __device__ __forceinline__ bool tg_short(unsigned long long* red, const TgHeld& h, int step_index) {
-  if (h.slot < 0 || h.held >= h.most || !tg_above(red, h.slot, h.held, h.step)) return false;
+  if (h.slot < 0) return false;
+  if (blockIdx.x == 0 && (int)threadIdx.x < h.held && tg_above(red, h.slot, threadIdx.x, h.step))
+    atomicMax(red + RED_USED + h.slot, (unsigned long long)threadIdx.x + 1);  // a sweep ran behind this check
+  if (h.held >= h.most || !tg_above(red, h.slot, h.held, h.step)) return false;
   if (blockIdx.x == 0 && threadIdx.x == 0) {
     red[RED_SHORT] = (unsigned long long)h.slot + 1;
     red[RED_ERR] = (unsigned long long)step_index;
@@ -650,8 +655,11 @@ struct gm_tg {
   unsigned long long* host_red = nullptr;  // its page-locked copy
   // FP32 mode: refinement sweeps queued for each solve.  A read-back per check held the stream for some
   // 20 us, six to eight times a step; now the steps of a call queue behind each other, a step that needs
-  // one sweep more than is held leaves its state alone, and the host repeats it with the sweep.
-  int held[NSLOT] = {1, 1, 1, 1};
+  // one sweep more than is held leaves its state alone, and the host repeats it with the sweep.  The
+  // first step holds as many as the mode takes and sets the counts, which fall when unused (HeldCount).
+  HeldCount held[NSLOT];
+  bool held_known = false;
+  long long repeats = 0;  // steps repeated for a sweep more
   ~gm_tg() { if (host_red) cudaFreeHost(host_red); }
   bool has_history = false;
   double prev_dt = 0;
@@ -683,7 +691,7 @@ TgC stencil_consts(const gm_tg* t, double dt) {
 // refinement sweeps at most: CN 6 (then a last check), pressure 8 (none behind the last)
 int most_of(int slot) { return slot == SLOT_CN ? 6 : 8; }
 TgHeld held_of(const gm_tg* t, int slot, double step) {
-  return t->precision ? TgHeld{slot, t->held[slot], most_of(slot), step} : TgHeld{-1, 0, 0, 0.0};
+  return t->precision ? TgHeld{slot, t->held[slot].n, most_of(slot), step} : TgHeld{-1, 0, 0, 0.0};
 }
 
 // One application of a solve: kind 0 Poisson, 1 Helmholtz (coef = dt nu / 2), the forward rows as LINE:
@@ -713,7 +721,7 @@ void fourier_solve(gm_tg* t, int kind, double coef, const double* b, double* x, 
 }
 
 const unsigned long long* read_red(gm_tg* t) {
-  TG_CK(cudaMemcpyAsync(t->host_red, t->red.p, 8 * sizeof(unsigned long long), cudaMemcpyDeviceToHost, t->st));
+  TG_CK(cudaMemcpyAsync(t->host_red, t->red.p, RED_W * sizeof(unsigned long long), cudaMemcpyDeviceToHost, t->st));
   TG_CK(cudaStreamSynchronize(t->st));
   return t->host_red;
 }
@@ -727,7 +735,7 @@ double bitsd(unsigned long long b) {
 // k - 1, so a sweep is three kernels; a last check follows the last sweep.
 template <int FIRST, int RES>
 void refined_solve(gm_tg* t, int slot, double coef, const double* b, const double* rhs, double* x, double dt, double step) {
-  const int fields = slot == SLOT_CN ? 2 : 1, kind = slot == SLOT_CN ? 1 : 0, held = std::min(t->held[slot], most_of(slot));
+  const int fields = slot == SLOT_CN ? 2 : 1, kind = slot == SLOT_CN ? 1 : 0, held = std::min(t->held[slot].n, most_of(slot));
   unsigned long long* w = t->red.p + RED_W + slot * SLOT_CHECKS;
   unsigned long long* bmax = slot == SLOT_CN ? t->red.p + RED_RHS : nullptr;
   const TgC c = stencil_consts(t, dt);
@@ -833,21 +841,35 @@ void tg_steps(gm_tg* t, double dt, int n_steps, double* max_div) {
   const double prev = t->prev_dt;
   TG_CK(cudaMemsetAsync(t->red.p, 0, RED_N * sizeof(unsigned long long), t->st));
   const unsigned long long* r = t->host_red;
-  for (int done = 0; done < n_steps;) {
+  const bool f32 = t->precision != 0;
+  for (int done = 0, read = 0; done < n_steps;) {
+    if (f32 && !t->held_known)
+      for (int s = 0; s < NSLOT; ++s) t->held[s].n = most_of(s);
     tg_step(t, dt, done + 1);
     tg_swap(t);
     t->has_history = true;
     t->prev_dt = dt;
     ++done;
-    if (done != n_steps && done % 64 != 0) continue;
+    if (done != n_steps && done - read < 64 && (!f32 || t->held_known)) continue;
     const int err = (int)read_red(t)[RED_ERR];
-    if (!err) continue;
+    if (!err) {
+      for (int s = 0; f32 && s < NSLOT; ++s) {
+        const int used = (int)r[RED_USED + s];
+        if (!t->held_known) t->held[s].n = used;
+        else if (s != SLOT_START) t->held[s].steps(used, done - read);
+      }
+      t->held_known = f32;
+      if (f32) TG_CK(cudaMemsetAsync(t->red.p + RED_USED, 0, NSLOT * sizeof(unsigned long long), t->st));
+      read = done;
+      continue;
+    }
     if ((done - (err - 1)) % 2) tg_swap(t);  // step err failed: the state is that after err - 1 steps
     if (err == 1) { t->has_history = had; t->prev_dt = prev; }
     const int slot = (int)r[RED_SHORT] - 1;
     if (slot < 0) throw TgError(GM_ERUNTIME, "CN momentum solve failed: residual=" + std::to_string(bitsd(r[RED_CN])));
-    ++t->held[slot];
-    done = err - 1;
+    t->held[slot].raise(t->held[slot].n + 1);
+    ++t->repeats;
+    done = read = err - 1;
     TG_CK(cudaMemsetAsync(t->red.p + RED_SHORT, 0, 2 * sizeof(unsigned long long), t->st));
   }
   *max_div = std::max(*max_div, bitsd(r[RED_DIV]));
@@ -954,7 +976,7 @@ int gm_tg_create(int32_t n, double nu, int32_t precision, gm_tg** out) {
       TG_CK(cudaGetLastError());
     }
     t->red.alloc(RED_N);
-    TG_CK(cudaMallocHost(&t->host_red, 8 * sizeof(unsigned long long)));
+    TG_CK(cudaMallocHost(&t->host_red, RED_W * sizeof(unsigned long long)));
     TG_CK(cudaMemset(t->red.p, 0, RED_N * sizeof(unsigned long long)));
   });
   if (rc != GM_OK) { g_tg_create_error = t->err; return rc; }
@@ -996,6 +1018,13 @@ int gm_tg_get_state(gm_tg* t, double* q, double* p_half, double* p_out) {
     if (p_out) TG_CK(cudaMemcpyAsync(p_out, t->pout.p, nn * sizeof(double), cudaMemcpyDefault, t->st));
     TG_CK(cudaStreamSynchronize(t->st));
   });
+}
+
+int gm_tg_held_sweeps(const gm_tg* t, int32_t held[4], int64_t* repeats) {
+  if (!t) return GM_EVALUE;
+  for (int s = 0; held && s < NSLOT; ++s) held[s] = t->held[s].n;
+  if (repeats) *repeats = t->repeats;
+  return GM_OK;
 }
 
 int gm_tg_step(gm_tg* t, double dt, int32_t n_steps, double* max_divergence) {

@@ -237,6 +237,9 @@ int gm_tg_get_state(gm_tg* t, double* q, double* p_half, double* p_out);
 /* n_steps AB2/CN steps of size dt; *max_divergence (in/out) is raised to the largest
  * max |div q| after any step */
 int gm_tg_step(gm_tg* t, double dt, int32_t n_steps, double* max_divergence);
+/* Refinement sweeps that the FP32 mode's steps hold for each solve (the start-up's pressure, the CN system,
+ * the step's first and second pressure) and how many times a step was repeated for one more. */
+int gm_tg_held_sweeps(const gm_tg* t, int32_t held[4], int64_t* repeats);
 
 /* --- learned pressure preconditioner (no reference counterpart) ----------------- */
 
