@@ -8,6 +8,7 @@
 #include <utility>
 
 #include "kernels.cuh"
+#include "momentum.cuh"
 
 namespace gmk {
 
@@ -1402,15 +1403,9 @@ __global__ void __launch_bounds__(MTI * MTJ) k_momentum_tiled(CaseDev c, Momentu
 
 // The FP64 form.  The FP64 pipe is the bound (1/64 of the FP32 rate), so every constant is formed on the host
 // and multiplied last: the tiles hold the unscaled products 4 C, (u + u)^2 and (v + v)^2 (seven
-// instructions a point), and a face away from the channel's edges takes thirteen.  At 800x820 94 us with the
+// instructions a point), and a face away from the channel's edges takes fifteen.  At 800x820 94 us with the
 // fluxes scaled where they are formed (about 86 instructions a point), 67 now; other faces go the long way
 // through the same functions as k_momentum.
-struct MomentumC {
-  double ax, ay;       // -dy / (4 dx dy), -dx / (4 dx dy): of the products' differences along x and y
-  double c1, c2;       // dt (1 + alpha), dt alpha
-  double lx, ly, lc;   // dt nu / (2 dx^2), dt nu / (2 dy^2), 1 - 2 (lx + ly)
-  double gx, gy;       // dt / (rho dx), dt / (rho dy)
-};
 __global__ void __launch_bounds__(MTI * MTJ, 4) k_momentum_tiled64(CaseDev c, MomentumArgs a, MomentumC m, Gate gate) {
   constexpr int W = TileGrid::W, H = TileGrid::H, WP = TileGrid::WP, WC = MTI + 1;
   __shared__ double suv[2 * H * W];
@@ -1492,7 +1487,7 @@ __global__ void __launch_bounds__(MTI * MTJ, 4) k_momentum_tiled64(CaseDev c, Mo
         dp = (sp[tg.p(j, i)] - sp[tg.p(j - 1, i)]) * m.gy;
       }
       a.now[t] = now;
-      a.out[t] = fma(m.lc, x, fma(m.lx, ew, fma(m.ly, ns, fma(m.c1, now, fma(-m.c2, a.prev[t], -dp)))));
+      a.out[t] = momentum_rhs(m, x, ew, ns, now, a.prev[t], dp);
       continue;
     }
     const double qv = a.U[t];
@@ -1557,8 +1552,7 @@ void launch_momentum(const CaseDev& c, const MomentumArgs& a, const Gate& gate, 
   if (a.mode == 0 && momentum_tiled(c, false))
     launch_pdl(k_momentum_tiled64, dim3(momentum_tiles(c)), dim3(dim3(MTI, MTJ)), 0, st, c, a,
                MomentumC{-0.25 * c.dy * c.iarea, -0.25 * c.dx * c.iarea, a.dt * (1 + a.alpha), a.dt * a.alpha,
-                         0.5 * a.dt * c.nu * c.idx2, 0.5 * a.dt * c.nu * c.idy2, 1 - a.dt * c.nu * (c.idx2 + c.idy2),
-                         a.dt * c.gx, a.dt * c.gy}, gate);
+                         0.5 * a.dt * c.nu * c.idx2, 0.5 * a.dt * c.nu * c.idy2, a.dt * c.gx, a.dt * c.gy}, gate);
   else
     launch_pdl(k_momentum<double, double>, dim3(blocks_for(c.usize + c.vsize)), dim3(TPB), 0, st, c, a, a.U, a.P, gate);
   // algorithmic bytes: U, prev, class map read; now, out written; P read
