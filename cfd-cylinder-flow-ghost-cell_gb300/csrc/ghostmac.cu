@@ -520,15 +520,17 @@ void autotune_shapes(gm_handle* h, RectDev& rd, int kind, bool fp32) {
   CK(cudaEventDestroy(e0));
   CK(cudaEventDestroy(e1));
   CK(cudaGetLastError());
-  // GHOSTMAC_SHAPES="gthreads,gpb,L" replaces the timed choice (shape studies; every shape
+  // GHOSTMAC_SHAPES="gthreads,gpb,L[,two]" replaces the timed choice (shape studies; every shape
   // computes the same values)
   if (const char* e = std::getenv("GHOSTMAC_SHAPES")) {
-    int gt = 0, gp = 0, L = 0;
-    const size_t per = std::max(xpass_smem_per_group(tt.tx_fwd, v.cols, fp32, 0), xpass_smem_per_group(tt.tx_inv, v.cols, fp32, 0));
-    if (std::sscanf(e, "%d,%d,%d", &gt, &gp, &L) == 3 && gt >= 32 && gt % 32 == 0 && gp >= 1 && gt * gp <= 512 &&
+    int gt = 0, gp = 0, L = 0, two = 0;
+    const int n = std::sscanf(e, "%d,%d,%d,%d", &gt, &gp, &L, &two);
+    two = two == 1 && !fp32 && !r2r_paired(tt.tx_fwd) ? 1 : 0;
+    const size_t per = std::max(xpass_smem_per_group(tt.tx_fwd, v.cols, fp32, two), xpass_smem_per_group(tt.tx_inv, v.cols, fp32, two));
+    if (n >= 3 && gt >= 32 && gt % 32 == 0 && gp >= 1 && gt * gp <= 512 &&
         tabs + per * gp <= h->smem_optin && (L == 2 || L == 4 || L == 8 || L == 16) &&
         ((L * tt.ych.P + 31) / 32) * 32 <= 1024 && ysolve_smem(v.rows, L, fp32) <= h->smem_optin) {
-      tt.xg_two = 0;
+      tt.xg_two = two;
       tt.xg_threads = gt;
       tt.xg_pb = gp;
       tt.smem_x = tabs + per * gp;
