@@ -1326,7 +1326,7 @@ void copy_in(double* dst, const double* src, size_t n, cudaStream_t st) {
   CCK(cudaMemcpyAsync(dst, src, n * sizeof(double), cudaMemcpyDefault, st));
 }
 
-// ---- momentum evaluation (five launches) ----------------------------------------------------
+// ---- momentum evaluation (three launches) ---------------------------------------------------
 void momentum(gm_cc* c, bool adv, const double* X, const double* inl, double nu, int mode, double hdt, double* Y,
               double* Rout, cudaStream_t st, bool upwind = false) {
   const double rnu = c->rho * nu;

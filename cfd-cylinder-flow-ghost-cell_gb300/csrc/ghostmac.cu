@@ -253,6 +253,7 @@ struct gm_handle {
   HeldCount sweeps[5];
   long long loop_nodes[5] = {};  // looped: kernels of a pass of each slot's loop
   bool sweeps_known = false;  // a first step has set them
+  int settled = 0;            // graph steps since, up to the counts' first window, which one batch of steps ends with
   long long repeats = 0;  // steps repeated for a sweep more
   // launch-by-launch steps decide every refinement sweep on the host (one synchronisation
   // per sweep) instead of launching all sweeps gated: then every launched kernel does work,
@@ -2121,6 +2122,12 @@ void note_sweeps(gm_handle* h, int n, bool first, bool graph) {
       else if (graph) h->sweeps[s].steps(used, 1);
     }
   if (first && n > 0) h->sweeps_known = true;
+  if (graph) h->settled = std::min(h->settled + n, HeldCount::FIRST);
+}
+
+// steps that are queued before the host reads their records, so that the first window's counts take effect at its end
+int queue_steps(const gm_handle* h) {
+  return h->settled < HeldCount::FIRST ? HeldCount::FIRST - h->settled : (int)gm_handle::RING_CAP;
 }
 
 // Graph of one steady step for the current buffer assignment, dt and held sweeps (captured on demand,
@@ -2382,7 +2389,7 @@ void step_loop(gm_handle* h, double dt, int32_t n_steps, int64_t first_step_inde
       // a changed dt, or per-kernel event timing
       const bool direct = !h->has_history || h->prev_dt != dt || !h->use_graphs || ktimer_active() || h->rec_rhs;
       const bool first = !h->has_history;
-      const int batch = direct ? 1 : std::min(n_steps - s, (int)gm_handle::RING_CAP);
+      const int batch = direct ? 1 : std::min(n_steps - s, queue_steps(h));
       CK(cudaMemsetAsync(h->ridx.p, 0, sizeof(int), st));
       if (direct) {
         step_once(h, dt, ((first_step_index + s) % 100) == 0 ? 1 : 0);
@@ -3705,7 +3712,8 @@ int gm_batch_step(gm_batch* b, double dt, int32_t n_steps, int64_t first_step_in
     while (s < n_steps && first_error == GM_OK) {
       bool steady = !ktimer_active();
       for (gm_handle* h : b->cases) steady = steady && h->has_history && h->prev_dt == dt && h->use_graphs;
-      const int batch = steady ? std::min(n_steps - s, (int)gm_handle::RING_CAP) : 1;
+      int batch = steady ? n_steps - s : 1;
+      for (gm_handle* h : b->cases) batch = std::min(batch, queue_steps(h));
       for (gm_handle* h : b->cases) CK(cudaMemsetAsync(h->ridx.p, 0, sizeof(int), h->st));
       long long nodes = 0;
       if (!steady) {

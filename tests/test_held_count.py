@@ -20,16 +20,16 @@ int main() {
   expect(c.n == 2, "raise");
   c.raise(1);
   expect(c.n == 2, "raise to less");
-  for (int k = 0; k < 63; ++k) expect(!c.steps(1, 1), "before the window's end");
+  for (int k = 0; k < 15; ++k) expect(!c.steps(1, 1), "before the first window's end");
   expect(c.steps(0, 1) && c.n == 1, "to the window's largest need");
   c.raise(2);
-  expect(c.window == 128, "a need that came back");
-  for (int k = 0; k < 127; ++k) expect(!c.steps(k == 5 ? 2 : 1, 1), "window of 128");
+  expect(c.window == 64, "a need that came back");
+  for (int k = 0; k < 63; ++k) expect(!c.steps(k == 5 ? 2 : 1, 1), "window of 64");
   expect(!c.steps(1, 1) && c.n == 2, "used once in the window");
-  expect(c.steps(1, 128) && c.n == 1, "counted steps");
+  expect(c.steps(1, 64) && c.n == 1, "counted steps");
   c.raise(3);
   c.raise(4);
-  expect(c.window == 256, "one doubling for a rise in two parts");
+  expect(c.window == 128, "one doubling for a rise in two parts");
   for (int r = 0; r < 12; ++r) { c.steps(0, 1 << 20); c.raise(4); }
   expect(c.window == 4096, "the largest window");
   HeldCount m;
@@ -37,6 +37,9 @@ int main() {
   m.least = 1;
   expect(m.steps(0, 64) && m.n == 1, "not below the least");
   expect(!m.steps(0, 64) && m.n == 1, "stays");
+  HeldCount q;
+  q.raise(1);
+  expect(!q.steps(1, 16) && q.window == 32 && !q.steps(0, 31) && q.steps(0, 1) && q.n == 0, "the windows behind the first");
   return bad;
 }
 """
