@@ -96,7 +96,7 @@ DEFAULT_WORKLOAD = 'wide_800x820_re100'
 # FP64 instructions (dadd + dmul + dfma, thread level) per cell update of the plain FP64 step on
 # the 800x820 case, and the measured FP64 instruction rate of a GB300 (independent FMA chains on
 # every SM, profiles/gb300_rates.md); the count comes from the ncu capture in FP64_OPS_SOURCE.
-FP64_OPS_PER_CELL_UPDATE = 424.4
+FP64_OPS_PER_CELL_UPDATE = 356.5
 FP64_OPS_SOURCE = 'profiles/fp64_instructions_wide_800x820.md'
 FP64_INST_RATE = 499e9
 # DRAM bytes (read + write) per launch of the dominant kernel class, averaged over the launches
@@ -689,7 +689,8 @@ def run_ours_gmres(args, w, rank, world):
                                ms_per_step_plain=ms_plain, ms_per_step_learned=ms_net, ms_per_step_direct=ms_dir,
                                ms_per_step_plain_host_control=ms_host,
                                iterations_per_solve_plain_host_control=per(its_host, n_host),
-                               control='device (graph: restart cycles as a WHILE node, Arnoldi steps as IF nodes)',
+                               control='device (graph: restart cycles as a WHILE node, Arnoldi steps ' +
+                                       ('in one cluster kernel)' if args.precision == 'fp64' else 'as IF nodes)'),
                                cd_rel_diff_plain_vs_direct=abs(cd_plain - cd_dir) / abs(cd_dir),
                                cd_rel_diff_learned_vs_direct=abs(cd_net - cd_dir) / abs(cd_dir),
                                cl_abs_diff_learned_vs_plain=abs(cl_net - cl_plain),
@@ -973,10 +974,9 @@ def profile_step(args, w):
 
 
 def profile_cutcell_ops(args, w):
-    """Profiling driver of the cut-cell path: its step graph holds conditional nodes, whose kernel
-    nodes ncu does not profile, so the operator calls that launch the same kernels one by one run
-    inside the NVTX range "one_step": one viscous and one advective momentum evaluation and one
-    projection of the seeded state."""
+    """Profiling driver of the cut-cell path's flux operators, launched one by one inside the NVTX
+    range "one_step": one viscous and one advective momentum evaluation and one projection of the
+    seeded state."""
     import torch
     pkg = load_package()
     kw = {k: w[k] for k in ('nx', 'ny', 'Lx', 'Ly', 'D', 'xc', 'yc', 'nu')}
@@ -1014,8 +1014,8 @@ def run_ours_cutcell(args, w, rank, world):
 
 def run_ours_legacy(args, w, rank, world):
     """A legacy loop alone (1 GPU): K steps of MAC_CylinderFlow(time_scheme='legacy') after W
-    warm-up steps, one solve() call, wall clock between two device synchronisations (each step
-    is a few library calls from the host and reads the forces back)."""
+    warm-up steps, one solve() call, wall clock between two device synchronisations (one library
+    call for all steps; the cut-cell loop reads each step's diagnostics back)."""
     import torch
     pkg = load_package()
     torch.zeros(1, device='cuda')

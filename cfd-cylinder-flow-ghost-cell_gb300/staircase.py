@@ -7,12 +7,12 @@ Poisson right-hand side, a pressure solve of the staircase Poisson matrix (build
 solver/mac_solver.py:5-87, which the reference factors with a sparse LU or solves by
 ILU-GMRES), the native corrector (or the ghost-cell branch's) and the force sums (staircase
 sums, or the integral on the true circle).  One library call (gm_poisson_legacy_step) runs a
-chunk of steps on the device with one synchronisation per step; the state stays on the device
-between calls (torch tensors serve as device buffers), and the host arrays u, v, p are written
-back after each solve() call.  The staircase Poisson matrix is the aperture-weighted cut-cell matrix with
-open fractions 0 or 1 taken from the cell mask, solved to rounding by the boundary-corrected
-separable inverse; both pressure_solver choices of the reference solve that system (the LU
-exactly, ILU-GMRES to rtol 1e-8).
+chunk of steps on the device, queued behind each other without a host check in between; the
+state stays on the device between calls (torch tensors serve as device buffers), and the host
+arrays u, v, p are written back after each solve() call.  The staircase Poisson matrix is the
+aperture-weighted cut-cell matrix with open fractions 0 or 1 taken from the cell mask, solved to
+rounding by the boundary-corrected separable inverse; both pressure_solver choices of the
+reference solve that system (the LU exactly, ILU-GMRES to rtol 1e-8).
 """
 from __future__ import annotations
 
