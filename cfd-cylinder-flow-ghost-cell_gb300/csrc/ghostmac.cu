@@ -246,14 +246,16 @@ struct gm_handle {
   // conditional node costs 8 us even when its body does not run and 4 more per pass (a kernel node 1.2),
   // 25 us of a 220 us step in FP64, which needs no sweep, and about 50 in the FP32 mode.  A solve that
   // needs more than its slot's stops the steps behind it (ERR_SWEEPS); the host adds one and repeats
-  // the step.  The handle's first step, which runs launch by launch with every sweep, sets the counts, and
-  // a count falls again when the steps no longer use it (HeldCount): the FP32 mode's pressure solves
-  // need two sweeps for some twenty steps from rest and one from there on.
+  // the step.  FP64 starts with none.  In the FP32 mode the handle's first step, which runs launch by launch
+  // with every sweep, sets the counts: its pressure solves need two sweeps for some twenty steps from rest
+  // and one from there on.  (FP64 solves that need a sweep in the first step seldom do in the second; the
+  // sweep held for it cost the first twenty steps at 400x200 5 %.)  A count falls again when the steps
+  // no longer use it (HeldCount).
   bool looped = false;  // the solves of this capture are loops (WHILE nodes): a batch's (batch_loops)
   HeldCount sweeps[5];
   long long loop_nodes[5] = {};  // looped: kernels of a pass of each slot's loop
-  bool sweeps_known = false;  // a first step has set them
-  int settled = 0;            // graph steps since, up to the counts' first window, which one batch of steps ends with
+  bool sweeps_known = false;  // a first step has set them (FP32 mode)
+  int settled = HeldCount::FIRST;  // graph steps since, up to the counts' first window, which one batch of steps ends with
   long long repeats = 0;  // steps repeated for a sweep more
   // launch-by-launch steps decide every refinement sweep on the host (one synchronisation
   // per sweep) instead of launching all sweeps gated: then every launched kernel does work,
@@ -2112,17 +2114,22 @@ int sweeps_run(const SolveCtl& sc, int nchk) {
   while (k + 1 < nchk && bits2d(sc.rmax[k]) > tg) ++k;
   return k;
 }
-// the held sweeps after `n` good steps recorded in host_ring: the handle's first step sets them, steps of a
-// graph lower them
+// the held sweeps after `n` good steps recorded in host_ring: the handle's first step sets them (FP32 mode),
+// steps of a graph lower them
 void note_sweeps(gm_handle* h, int n, bool first, bool graph) {
+  const bool set = first && n > 0 && h->precision == 1 && !h->sweeps_known;
   for (int k = 0; k < n; ++k)
     for (int s : {S_HELM_U, S_HELM_V, S_P1, S_P2}) {
       const int used = sweeps_run(h->host_ring[k].solve[s], h->nchk);
-      if (first && !h->sweeps_known) h->sweeps[s].raise(used);
+      if (set) h->sweeps[s].raise(used);
       else if (graph) h->sweeps[s].steps(used, 1);
     }
-  if (first && n > 0) h->sweeps_known = true;
-  if (graph) h->settled = std::min(h->settled + n, HeldCount::FIRST);
+  if (set) {
+    h->sweeps_known = true;
+    h->settled = 0;
+  } else if (graph) {
+    h->settled = std::min(h->settled + n, HeldCount::FIRST);
+  }
 }
 
 // steps that are queued before the host reads their records, so that the first window's counts take effect at its end
