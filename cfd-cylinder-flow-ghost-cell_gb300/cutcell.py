@@ -485,8 +485,9 @@ class CutCellFlow:
     # -- checkpoints (schema 1, solver/main.py:503-567)
     def _source_hashes(self):
         files = ['cutcell.py', 'cutcell_geometry.py', '_lib.py', 'csrc/cutcell.cu', 'csrc/ghostmac.cu',
-                 'csrc/kernels.cu', 'csrc/kernels.cuh', 'csrc/transforms.cuh', 'csrc/geometry.cpp',
-                 'csrc/geometry.hpp', 'csrc/internal.hpp']
+                 'csrc/kernels.cu', 'csrc/kernels.cuh', 'csrc/momentum.cuh', 'csrc/transforms.cuh',
+                 'csrc/fftplan.hpp', 'csrc/geometry.cpp', 'csrc/geometry.hpp', 'csrc/heldcount.hpp',
+                 'csrc/internal.hpp']
         return {name: hashlib.sha256((_PKG / name).read_bytes()).hexdigest() for name in files}
 
     def metadata(self, dt, n_steps, perturb_transient=True, perturb_duration=None, perturb_amp=.15):

@@ -502,7 +502,8 @@ class MAC_CylinderFlow:
     # -- checkpoints (solver/main.py:503-585), schema 1
     def _source_hashes(self):
         files = ['ghost.py', '_lib.py', 'csrc/ghostmac.cu', 'csrc/kernels.cu', 'csrc/kernels.cuh',
-                 'csrc/transforms.cuh', 'csrc/geometry.cpp', 'csrc/geometry.hpp']
+                 'csrc/momentum.cuh', 'csrc/transforms.cuh', 'csrc/fftplan.hpp', 'csrc/geometry.cpp',
+                 'csrc/geometry.hpp', 'csrc/heldcount.hpp', 'csrc/internal.hpp']
         return {name: hashlib.sha256((_PKG / name).read_bytes()).hexdigest() for name in files}
 
     def metadata(self, dt, n_steps, perturb_transient=True, perturb_duration=None, perturb_amp=.15):

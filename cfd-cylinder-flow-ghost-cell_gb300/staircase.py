@@ -184,8 +184,10 @@ class StaircaseFlow:
 
     def _source_hashes(self):
         root = Path(__file__).resolve().parent
-        files = ['staircase.py', '_lib.py', '_args.py', 'csrc/legacy.cu', 'csrc/cutcell.cu', 'csrc/ghostmac.cu',
-                 'csrc/kernels.cu', 'csrc/geometry.cpp', 'csrc/internal.hpp']
+        files = ['staircase.py', '_lib.py', '_args.py', 'csrc/legacy.cu', 'csrc/exactdiv.cuh', 'csrc/cutcell.cu',
+                 'csrc/ghostmac.cu', 'csrc/kernels.cu', 'csrc/kernels.cuh', 'csrc/momentum.cuh',
+                 'csrc/transforms.cuh', 'csrc/fftplan.hpp', 'csrc/geometry.cpp', 'csrc/geometry.hpp',
+                 'csrc/heldcount.hpp', 'csrc/internal.hpp']
         return {name: hashlib.sha256((root / name).read_bytes()).hexdigest() for name in files}
 
     def metadata(self, dt, n_steps, perturb_transient=True, perturb_duration=None, perturb_amp=.15):
